@@ -287,7 +287,8 @@ def f16_to_f32(h):
 
 
 def reference_available():
-    return os.path.isdir(REFERENCE_SOURCES)
+    # An empty directory is no source tree.
+    return os.path.isdir(os.path.join(REFERENCE_SOURCES, "renderer"))
 
 
 def _make_env():
