@@ -2154,20 +2154,35 @@ __device__ __forceinline__ uint32_t f2h(float f)
     return (uint32_t)__half_as_ushort(__float2half_rn(f));
 }
 __device__ __forceinline__ float clamp01(float x) { return fminf(fmaxf(x, 0.f), 1.f); }
-__device__ __forceinline__ uint32_t unorm8(float x)
+// The nearest integer (ties to even) of 255 x, x clamped to [0, 1], in the low
+// byte of the result: adding 3 * 2^22 leaves it in the mantissa's low bits, on
+// the full-rate fp32 pipe (a float-to-int conversion runs at 1/8 of it).
+__device__ __forceinline__ uint32_t unorm8_bits(float x)
 {
-    return (uint32_t)__float2int_rn(clamp01(x) * 255.f);
+    return __float_as_uint(__fadd_rn(clamp01(x) * 255.f, 12582912.f));
+}
+__device__ __forceinline__ uint32_t unorm8(float x) { return unorm8_bits(x) & 0xffu; }
+// b / 255, correctly rounded, for an integer b in [0, 255]: 1/255 as a sum of
+// two floats (kHi + kLo), b * kLo rounded, then one fused step. Equal to the
+// IEEE division for all 256 values (tests/test_gpu_raster_cover.py) at 2 instructions
+// instead of a division's ten; a resolve unpacks up to 24 bytes.
+constexpr float kUnormHi = 0x1.010102p-8f, kUnormLo = -0x1.fdfdfep-33f;
+__device__ __forceinline__ float unorm_float(uint32_t b)
+{
+    const float f = __fsub_rn(__uint_as_float(0x4b000000u | b), 8388608.f); // exact
+    return __fmaf_rn(f, kUnormHi, __fmul_rn(f, kUnormLo));
 }
 __device__ __forceinline__ void unpack_rgba8(uint32_t c, float out[4])
 {
-    out[0] = (float)(c & 0xffu) / 255.f;
-    out[1] = (float)((c >> 8) & 0xffu) / 255.f;
-    out[2] = (float)((c >> 16) & 0xffu) / 255.f;
-    out[3] = (float)(c >> 24) / 255.f;
+    out[0] = unorm_float(c & 0xffu);
+    out[1] = unorm_float((c >> 8) & 0xffu);
+    out[2] = unorm_float((c >> 16) & 0xffu);
+    out[3] = unorm_float(c >> 24);
 }
 __device__ __forceinline__ uint32_t pack_rgba8(const float c[4])
 {
-    return unorm8(c[0]) | (unorm8(c[1]) << 8) | (unorm8(c[2]) << 16) | (unorm8(c[3]) << 24);
+    return __byte_perm(__byte_perm(unorm8_bits(c[0]), unorm8_bits(c[1]), 0x0040),
+                       __byte_perm(unorm8_bits(c[2]), unorm8_bits(c[3]), 0x0040), 0x5410);
 }
 
 __device__ __forceinline__ float min3f(float a, float b, float c) { return fminf(fminf(a, b), c); }
@@ -2311,26 +2326,36 @@ __device__ __noinline__ void sample_grad(const FlushParams& P, float u, float v,
             int yj = min(max(y0 + j, 0), H - 1);
             float wgt = __fmul_rn(i ? ax : __fsub_rn(1.f, ax), j ? ay : __fsub_rn(1.f, ay));
             uchar4 t = P.grad[(size_t)yj * kGradTextureWidth + xi];
-            out[0] = __fadd_rn(out[0], __fmul_rn(wgt, __fdiv_rn((float)t.x, 255.f)));
-            out[1] = __fadd_rn(out[1], __fmul_rn(wgt, __fdiv_rn((float)t.y, 255.f)));
-            out[2] = __fadd_rn(out[2], __fmul_rn(wgt, __fdiv_rn((float)t.z, 255.f)));
-            out[3] = __fadd_rn(out[3], __fmul_rn(wgt, __fdiv_rn((float)t.w, 255.f)));
+            out[0] = __fadd_rn(out[0], __fmul_rn(wgt, unorm_float(t.x)));
+            out[1] = __fadd_rn(out[1], __fmul_rn(wgt, unorm_float(t.y)));
+            out[2] = __fadd_rn(out[2], __fmul_rn(wgt, unorm_float(t.z)));
+            out[3] = __fadd_rn(out[3], __fmul_rn(wgt, unorm_float(t.w)));
         }
 }
 
-// Pixel-local storage of one pixel (draw_raster_order_path.frag:7-12), plus
-// the path whose fragments are still being accumulated.
-struct Pixel
+// The pixel-local-storage planes a resolve reads and writes
+// (draw_raster_order_path.frag:7-12). Passed and returned by value: a
+// reference to an out-of-line function would keep every plane of the pixel in
+// local memory for the whole tile.
+struct Planes
 {
-    uint32_t color;    // RGBA8, the colour before the pending path
-    uint32_t clip;     // packHalf2x16(coverage, clipID)
-    uint32_t scratch;  // RGBA8 scratch plane
-    uint32_t key;      // coverage plane's path key (fp16 bits of the pathID)
-    float count;       // coverage plane's count (always an fp16 value)
-    uint32_t pendMeta; // pathAndFeatures of the pending path (0: none)
-    uint32_t pendPaintX, pendPaintY;
-    uint32_t pendFrags; // fragments of the pending path so far (saturating)
+    uint32_t color;   // RGBA8, the colour before the pending path
+    uint32_t clip;    // packHalf2x16(coverage, clipID)
+    uint32_t scratch; // RGBA8 scratch plane
 };
+
+// common.glsl:269-274 interleaved gradient noise (depends on the pixel only).
+// Rounded step by step as the C restatement rounds it: the noise wraps at
+// fract(), where a fused multiply-add's last bit moves a pixel's dither by a
+// whole step, and chains of advanced blends amplify it.
+__device__ __forceinline__ float pixel_dither(const FlushParams& P, float fx, float fy)
+{
+    float v1 = __fadd_rn(__fmul_rn(0.06711056f, fx), __fmul_rn(0.00583715f, fy));
+    v1 = __fsub_rn(v1, floorf(v1));
+    float v2 = __fmul_rn(52.9829189f, v1);
+    v2 = __fsub_rn(v2, floorf(v2));
+    return __fadd_rn(__fmul_rn(v2, P.ditherScale), P.ditherBias);
+}
 
 // min_component of find_clip_rect_coverage_distances (common.glsl:376-400)
 // at the pixel centre, for the clip-rect inverse matrix cm (2x2) and its
@@ -2459,10 +2484,10 @@ __device__ void sample_image_level(const ImageTex& t, int level, float u, float 
         const int x = wrap_texel((int)floorf(__fmul_rn(u, (float)w)), w, wrapX);
         const int y = wrap_texel((int)floorf(__fmul_rn(v, (float)h)), h, wrapY);
         const uchar4 c = tex[(size_t)y * w + x];
-        out[0] = __fdiv_rn((float)c.x, 255.f);
-        out[1] = __fdiv_rn((float)c.y, 255.f);
-        out[2] = __fdiv_rn((float)c.z, 255.f);
-        out[3] = __fdiv_rn((float)c.w, 255.f);
+        out[0] = unorm_float(c.x);
+        out[1] = unorm_float(c.y);
+        out[2] = unorm_float(c.z);
+        out[3] = unorm_float(c.w);
         return;
     }
     const float fx = __fsub_rn(__fmul_rn(u, (float)w), .5f);
@@ -2479,10 +2504,10 @@ __device__ void sample_image_level(const ImageTex& t, int level, float u, float 
             const int xi = wrap_texel(x0 + i, w, wrapX), yj = wrap_texel(y0 + j, h, wrapY);
             const float wgt = __fmul_rn(i ? ax : __fsub_rn(1.f, ax), j ? ay : __fsub_rn(1.f, ay));
             const uchar4 c = tex[(size_t)yj * w + xi];
-            out[0] = __fadd_rn(out[0], __fmul_rn(wgt, __fdiv_rn((float)c.x, 255.f)));
-            out[1] = __fadd_rn(out[1], __fmul_rn(wgt, __fdiv_rn((float)c.y, 255.f)));
-            out[2] = __fadd_rn(out[2], __fmul_rn(wgt, __fdiv_rn((float)c.z, 255.f)));
-            out[3] = __fadd_rn(out[3], __fmul_rn(wgt, __fdiv_rn((float)c.w, 255.f)));
+            out[0] = __fadd_rn(out[0], __fmul_rn(wgt, unorm_float(c.x)));
+            out[1] = __fadd_rn(out[1], __fmul_rn(wgt, unorm_float(c.y)));
+            out[2] = __fadd_rn(out[2], __fmul_rn(wgt, unorm_float(c.z)));
+            out[3] = __fadd_rn(out[3], __fmul_rn(wgt, unorm_float(c.w)));
         }
 }
 
@@ -2501,10 +2526,10 @@ __device__ void sample_image(const ImageTex& t, float u, float v, float lod, flo
 // cut by the clip rect and the clip, then times the draw's opacity; advanced
 // blending unmultiplies the texel first; dither, then src-over onto the
 // colour. The coverage plane keeps what it held (a mesh is no path).
-__device__ __noinline__ void resolve_mesh(const FlushParams& P, Pixel& s, uint32_t meta,
-                                          uint32_t imageDraw, uint32_t imageWord,
-                                          const float4* __restrict__ planes, float fx, float fy,
-                                          float dither)
+__device__ __noinline__ uint32_t resolve_mesh(const FlushParams& P, uint32_t dstColor,
+                                              uint32_t clip, uint32_t meta, uint32_t imageDraw,
+                                              uint32_t imageWord,
+                                              const float4* __restrict__ planes, float fx, float fy)
 {
     const uint32_t features = meta >> 16;
     const float4 f0 = planes[0], f1 = planes[1];
@@ -2529,13 +2554,13 @@ __device__ __noinline__ void resolve_mesh(const FlushParams& P, Pixel& s, uint32
         const uint32_t clipBits = id_bits_to_f16(__float_as_uint(packed.y), P.pathIDGranularity);
         if (clipBits != 0)
         {
-            const float clipCoverage = (s.clip >> 16) == clipBits ? h2f(s.clip & 0xffffu) : 0.f;
+            const float clipCoverage = (clip >> 16) == clipBits ? h2f(clip & 0xffffu) : 0.f;
             coverage = fminf(coverage, fmaxf(clipCoverage, 0.f));
         }
     }
     coverage = __fmul_rn(coverage, packed.x); // opacity, after clipping
     float dst[4];
-    unpack_rgba8(s.color, dst);
+    unpack_rgba8(dstColor, dst);
     if (features & SF_ADVANCED_BLEND)
     {
         // unmultiply_rgb (common.glsl:210-216): images are premultiplied.
@@ -2558,6 +2583,7 @@ __device__ __noinline__ void resolve_mesh(const FlushParams& P, Pixel& s, uint32
     }
     if ((features & SF_DITHER) && color[3] != 0.f)
     {
+        const float dither = pixel_dither(P, fx, fy);
         color[0] += dither;
         color[1] += dither;
         color[2] += dither;
@@ -2565,7 +2591,7 @@ __device__ __noinline__ void resolve_mesh(const FlushParams& P, Pixel& s, uint32
     const float a = color[3];
     for (int k = 0; k < 4; ++k)
         color[k] = dst[k] * (1.f - a) + color[k];
-    s.color = pack_rgba8(color);
+    return pack_rgba8(color);
 }
 
 // ENABLE_MODULATED_IMAGE (draw_path.vert:343-361, 478-493): the paint's
@@ -2611,12 +2637,11 @@ __device__ __noinline__ void image_modulate(const FlushParams& P, uint32_t pathI
 // which batches with images or feathers use); the plain variant's resolve
 // stays without it.
 template <bool kImages>
-__device__ __noinline__ void resolve_path(const FlushParams& P, Pixel& s, float fx, float fy,
-                                          float dither)
+__device__ __noinline__ Planes resolve_path(const FlushParams& P, Planes s, float count,
+                                            uint32_t meta, uint32_t paintX, uint32_t paintY,
+                                            bool oneFragment, float fx, float fy)
 {
-    const uint32_t meta = s.pendMeta;
     const uint32_t pathID = meta & 0xffffu, features = meta >> 16;
-    const uint32_t paintX = s.pendPaintX, paintY = s.pendPaintY;
     const uint32_t paintType = paintX & 0xfu;
     const bool evenOdd = (paintX & PAINT_FLAG_EVEN_ODD_FILL) != 0;
     // draw_raster_order_path.frag:63-82: clockwise fills keep positive
@@ -2624,11 +2649,11 @@ __device__ __noinline__ void resolve_path(const FlushParams& P, Pixel& s, float 
     float coverage;
     if (features & FEATURE_CLOCKWISE_FILL)
     {
-        coverage = fminf(fmaxf(s.count, 0.f), 1.f);
+        coverage = fminf(fmaxf(count, 0.f), 1.f);
     }
     else
     {
-        coverage = fabsf(s.count);
+        coverage = fabsf(count);
         if ((features & SF_EVEN_ODD) && evenOdd)
             coverage = 1.f - fabsf((coverage * .5f - floorf(coverage * .5f)) * 2.f + -1.f);
         coverage = fminf(coverage, 1.f);
@@ -2652,18 +2677,18 @@ __device__ __noinline__ void resolve_path(const FlushParams& P, Pixel& s, float 
                         outer = contentID == outerBits ? h2f(s.clip & 0xffffu) : 0.f;
                         const uint32_t stash = unorm8(outer);
                         s.scratch = stash;
-                        if (s.pendFrags > 1)
-                            outer = (float)stash / 255.f;
+                        if (!oneFragment)
+                            outer = unorm_float(stash);
                     }
                     else
                     {
-                        outer = (float)(s.scratch & 0xffu) / 255.f;
+                        outer = unorm_float(s.scratch & 0xffu);
                     }
                     coverage = fminf(coverage, outer);
                 }
             }
             s.clip = (clipBits << 16) | f2h(coverage);
-            return;
+            return s;
         }
         if (clipBits != 0)
             coverage = (s.clip >> 16) == clipBits ? fminf(h2f(s.clip & 0xffffu), coverage) : 0.f;
@@ -2693,11 +2718,13 @@ __device__ __noinline__ void resolve_path(const FlushParams& P, Pixel& s, float 
         color[k] += dst[k] * (1.f - paintAlpha);
     if ((features & SF_DITHER) && paintAlpha != 0.f)
     {
+        const float dither = pixel_dither(P, fx, fy);
         color[0] += dither;
         color[1] += dither;
         color[2] += dither;
     }
     s.color = pack_rgba8(color);
+    return s;
 }
 
 // The feather atlas at atlas pixel coordinates (x, y): the atlas sampler's
@@ -2732,9 +2759,10 @@ __device__ __noinline__ float atlas_coverage(const FlushParams& P, float x, floa
 // the atlas sample, cut by the clip rect and the clip; the paint blends
 // straight into the colour (dither before the blend, as that shader does);
 // the coverage plane keeps what it held.
-__device__ __noinline__ void resolve_blit(const FlushParams& P, Pixel& s, uint32_t meta,
-                                          uint32_t paintX, uint32_t paintY, float ax, float ay,
-                                          float fx, float fy, float dither)
+__device__ __noinline__ uint32_t resolve_blit(const FlushParams& P, uint32_t dstColor,
+                                              uint32_t clip, uint32_t meta, uint32_t paintX,
+                                              uint32_t paintY, float ax, float ay, float fx,
+                                              float fy)
 {
     const uint32_t pathID = meta & 0xffffu, features = meta >> 16;
     const uint32_t paintType = paintX & 0xfu;
@@ -2747,7 +2775,7 @@ __device__ __noinline__ void resolve_blit(const FlushParams& P, Pixel& s, uint32
             (paintType == CLIP_UPDATE_PAINT_TYPE ? paintY : paintX) >> 16, P.pathIDGranularity);
         if (clipBits != 0)
         {
-            float clipCoverage = (s.clip >> 16) == clipBits ? h2f(s.clip & 0xffffu) : 0.f;
+            float clipCoverage = (clip >> 16) == clipBits ? h2f(clip & 0xffffu) : 0.f;
             coverage = fminf(coverage, fmaxf(clipCoverage, 0.f));
         }
     }
@@ -2755,7 +2783,7 @@ __device__ __noinline__ void resolve_blit(const FlushParams& P, Pixel& s, uint32
     float color[4];
     paint_color(P, paintX, paintY, pathID, fx, fy, 1.f, unmultiplied, color, features);
     float dst[4];
-    unpack_rgba8(s.color, dst);
+    unpack_rgba8(dstColor, dst);
     if (unmultiplied)
     {
         uint32_t mode = (paintX >> 4) & 0xfu;
@@ -2773,6 +2801,7 @@ __device__ __noinline__ void resolve_blit(const FlushParams& P, Pixel& s, uint32
     }
     if ((features & SF_DITHER) && color[3] != 0.f)
     {
+        const float dither = pixel_dither(P, fx, fy);
         color[0] += dither;
         color[1] += dither;
         color[2] += dither;
@@ -2780,15 +2809,17 @@ __device__ __noinline__ void resolve_blit(const FlushParams& P, Pixel& s, uint32
     const float a = color[3];
     for (int k = 0; k < 4; ++k)
         color[k] = dst[k] * (1.f - a) + color[k];
-    s.color = pack_rgba8(color);
+    return pack_rgba8(color);
 }
 } // namespace
 
 // One CTA per 16x16 tile, one thread per pixel; warp w owns the 8x4 block at
 // (8 (w & 1), 4 (w >> 1)). The tile's bin entries (triangle slots in
 // primitive order) are staged 256 at a time into shared memory in tile-local
-// form, each with a mask of the warp blocks it may cover; warps then walk
-// their own triangles in order and keep every pixel's planes in registers.
+// form, each with the warp blocks it may cover. Each warp then takes the
+// triangles of its own block 32 at a time, works out which pixels each covers
+// with one lane per triangle, and hands every pixel (lane) the triangles that
+// cover it, in primitive order; a pixel's planes stay in registers.
 struct __align__(16) TileTri
 {
     float4 v0; // coverage key (bits), C0, A0, B0
@@ -2882,91 +2913,165 @@ __device__ __noinline__ float feathered_fragment(const float4* __restrict__ plan
 #ifndef RIVE_RASTER_MIN_BLOCKS
 #define RIVE_RASTER_MIN_BLOCKS 5
 #endif
-// Prefetch of the next chunk's records into L2 while a chunk is walked (off:
-// measured slower, the staging's loads are not what the barrier waits for).
-#ifndef RIVE_RASTER_PREFETCH
-#define RIVE_RASTER_PREFETCH 0
-#endif
-// Bin entries each thread stages per chunk (8x8 and 16x16 tiles): a chunk of
-// kStage x threads entries between two CTA barriers.
-#ifndef RIVE_RASTER_STAGE
-#define RIVE_RASTER_STAGE 1
-#endif
 
 // Tile geometry: a CTA of T x T threads, one per pixel; warp w owns the 8x4
-// block at (8 (w % (T/8)), 4 (w / (T/8))).
+// block at (8 (w % (T/8)), 4 (w / (T/8))). A chunk of bin entries, one per
+// thread, is staged between two CTA barriers.
 template <int TL> struct RasterTile
 {
     static constexpr int T = 1 << TL;
     static constexpr int kThreads = T * T;
     static constexpr int kWarpCols = T / 8;
-    static constexpr int kBlocks = kThreads / 32;
-    using Mask = typename std::conditional<(kBlocks <= 8), uint8_t, uint32_t>::type;
+    static constexpr int kBlocks = kThreads / 32; // warps, one 8x4 block each
+    static constexpr int kChunk = kThreads;
+    using Index = typename std::conditional<(kChunk <= 256), uint8_t, uint16_t>::type;
 };
 
-template <int TL, bool kFeather, int kStage>
+// A tile's shared state: its flush's parameters, the staged triangles, per
+// block the staged triangles that may cover it (bit i % 32 of word i / 32),
+// and each warp's list of them.
+template <int TL> struct RasterShared
+{
+    using G = RasterTile<TL>;
+    TileTri tris[G::kChunk];
+    uint32_t bits[G::kBlocks][G::kChunk / 32];
+    typename G::Index list[G::kBlocks][G::kChunk];
+    FlushParams params;
+};
+
+// ones << (n & 31).
+__device__ __forceinline__ uint32_t ones_from(uint32_t n)
+{
+    return __funnelshift_l(0u, 0xffffffffu, n);
+}
+
+// The pixels of the 8x4 block at tile offset (qx, qy) inside a staged
+// triangle, bit 8 r + c for pixel (qx + c, qy + r): exactly those for which
+// local_inside holds on all three of E = fma(A, lx, fma(B, ly, C)).
+//
+// Along a pixel row, E's sign is that of the exact A lx + t (t = fma(B, ly, C);
+// one rounding, and no underflow: every term is a multiple of 2^-16), so an
+// edge's pixels are all those from some column on (A > 0: E >= 0 is inside, by
+// the tie rule) or all those before one (A < 0: E > 0). With A, B and C negated
+// in the second case both look for the first column s with |A| s + t >= 0,
+// which is inside, or outside. The column nearest to -t / |A|, from an
+// approximate reciprocal, is s or s - 1, and the sign of E there says which.
+// A horizontal edge (A = 0) takes all of a row or nothing of it: its
+// "reciprocal" is a huge number, so t < 0 gives column 8 and t >= 0 column 0.
+// About 28 instructions a row for all eight pixels, against 8 x 9 for testing
+// each, with one lane per triangle, where the test by pixels leaves idle the
+// three quarters of the lanes that a triangle does not cover.
+__device__ __forceinline__ uint32_t block_coverage(const TileTri& T, float qx, float qy)
+{
+    const float4 v0 = T.v0, v1 = T.v1, v2 = T.v2;
+    float a[3] = {v0.z, v1.y, v2.x}, b[3] = {v0.w, v1.z, v2.y}, c[3] = {v0.y, v1.x, v1.w};
+    float k[3];
+    uint32_t flip[3];
+#pragma unroll
+    for (int e = 0; e < 3; ++e)
+    {
+        const bool pos = a[e] > 0.f || (a[e] == 0.f && b[e] > 0.f);
+        flip[e] = pos ? 0u : 0xffffffffu;
+        k[e] = a[e] == 0.f ? -1e30f : __fdividef(-.125f, fabsf(a[e]));
+        if (!pos)
+        {
+            b[e] = -b[e];
+            c[e] = -c[e];
+        }
+        a[e] = fabsf(a[e]);
+    }
+    const float kMagic = 12582912.f; // 3 * 2^22: the column ends up in the low bits
+    const float off = -.125f * qx, back = kMagic - qx;
+    uint32_t out = 0;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+    {
+        uint32_t m[3];
+#pragma unroll
+        for (int e = 0; e < 3; ++e)
+        {
+            const float t = __fmaf_rn(b[e], qy + (float)r, c[e]);
+            const float u = __saturatef(__fmaf_rn(t, k[e], off)); // column / 8 in the block
+            const float n = __fmaf_rn(u, 8.f, kMagic);
+            const float E = __fmaf_rn(a[e], n - back, t);
+            m[e] = ones_from(__float_as_uint(n));
+            m[e] = (E < 0.f ? m[e] << 1 : m[e]) ^ flip[e];
+        }
+        out |= (m[0] & m[1] & m[2] & 0xffu) << (8 * r);
+    }
+    return out;
+}
+
+// Transposes a 32x32 bit matrix held one row per lane: bit i of lane p's
+// result is bit p of lane i's word.
+__device__ __forceinline__ uint32_t transpose_bits(uint32_t x, int lane)
+{
+#pragma unroll
+    for (int j = 16; j >= 1; j >>= 1)
+    {
+        constexpr uint32_t kMasks[5] = {0x55555555u, 0x33333333u, 0x0f0f0f0fu, 0x00ff00ffu,
+                                        0x0000ffffu};
+        const uint32_t lo = kMasks[j == 1 ? 0 : j == 2 ? 1 : j == 4 ? 2 : j == 8 ? 3 : 4];
+        const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
+        // A lane with bit j clear keeps its low halves and takes the other's
+        // low halves as its high ones; the other lane does the opposite.
+        const bool up = (lane & j) != 0;
+        const uint32_t keep = up ? ~lo : lo;
+        const uint32_t turned = __funnelshift_l(y, y, up ? 32 - j : j);
+        x = (x & keep) | (turned & ~keep);
+    }
+    return x;
+}
+
+template <int TL, bool kFeather>
 __device__ __forceinline__ void raster_tile(const BatchTables& B,
                                             const TriRecord* __restrict__ tris,
                                             const uint32_t* __restrict__ sortedSlots,
                                             const uint2* __restrict__ ranges,
-                                            TileTri* __restrict__ sTris,
-                                            typename RasterTile<TL>::Mask* __restrict__ sMask,
+                                            RasterShared<TL>& sh,
                                             uint32_t gtile)
 {
     using G = RasterTile<TL>;
+    constexpr uint32_t kChunk = G::kChunk;
     static_assert(sizeof(FlushParams) / 4 <= G::kThreads, "one word of FlushParams per thread");
-    __shared__ FlushParams sP;
     const uint2 range = ranges[gtile];
     // The tile's scene: its parameters are staged once for the whole CTA.
     const uint32_t scene = find_range(B.tileBase, B.sceneCount, gtile);
     if (threadIdx.x < sizeof(FlushParams) / 4)
-        reinterpret_cast<uint32_t*>(&sP)[threadIdx.x] =
+        reinterpret_cast<uint32_t*>(&sh.params)[threadIdx.x] =
             reinterpret_cast<const uint32_t*>(B.scenes + scene)[threadIdx.x];
     __syncthreads();
-    const FlushParams& P = sP;
+    const FlushParams& P = sh.params;
     uint32_t* __restrict__ fb = P.fb;
     const uint32_t tilesX = P.tilesX;
     const uint32_t tile = gtile - B.tileBase[scene];
     const int tx = (int)(tile % tilesX), ty = (int)(tile / tilesX);
     const int ox = tx * G::T, oy = ty * G::T;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int lxi = (warp % G::kWarpCols) * 8 + (lane & 7), lyi = (warp / G::kWarpCols) * 4 + (lane >> 3);
+    const int qx = (warp % G::kWarpCols) * 8, qy = (warp / G::kWarpCols) * 4;
+    const int lxi = qx + (lane & 7), lyi = qy + (lane >> 3);
     const int px = ox + lxi, py = oy + lyi;
     const float lx = (float)lxi, ly = (float)lyi;
     const bool inBounds = px < (int)P.width && py < (int)P.height;
     if (range.y <= range.x && !P.loadClear)
         return;
-    Pixel s;
+    const float fx = (float)px + .5f, fy = (float)py + .5f;
+    Planes s;
     s.color = P.loadClear ? P.clearColorPremulRGBA : (inBounds ? fb[(size_t)py * P.width + px] : 0u);
     s.clip = 0;
     s.scratch = 0;
-    s.key = 0;
-    s.count = 0.f;
-    s.pendMeta = 0;
-    s.pendPaintX = s.pendPaintY = 0;
-    s.pendFrags = 0;
-    const float fx = (float)px + .5f, fy = (float)py + .5f;
-    // common.glsl:269-274 interleaved gradient noise (depends on the pixel
-    // only). Rounded step by step as the C restatement rounds it: the noise
-    // wraps at fract(), where a fused multiply-add's last bit moves a pixel's
-    // dither by a whole step, and chains of advanced blends amplify it.
-    float v1 = __fadd_rn(__fmul_rn(0.06711056f, fx), __fmul_rn(0.00583715f, fy));
-    v1 = __fsub_rn(v1, floorf(v1));
-    float v2 = __fmul_rn(52.9829189f, v1);
-    v2 = __fsub_rn(v2, floorf(v2));
-    const float dither = __fadd_rn(__fmul_rn(v2, P.ditherScale), P.ditherBias);
+    uint32_t key = 0;      // coverage plane's path key (fp16 bits of the pathID)
+    float count = 0.f;     // coverage plane's count (always an fp16 value)
+    uint32_t pendMeta = 0; // pathAndFeatures of the pending path (0: none)
+    uint32_t pendPaintX = 0, pendPaintY = 0;
+    bool oneFragment = false; // the pending path has had one fragment here
     uint32_t streamPath = 0xffffffffu; // coverage key of the warp's current path
 
-    constexpr uint32_t kChunk = (uint32_t)G::kThreads * kStage;
     for (uint32_t base = range.x; base < range.y; base += kChunk)
     {
-        // Each thread stages kStage triangles in tile-local form and marks
-        // which of the warp blocks may hold a pixel each covers.
-#pragma unroll
-        for (int j = 0; j < kStage; ++j)
-        {
-        const uint32_t si = (uint32_t)j * G::kThreads + threadIdx.x;
-        const uint32_t k = base + si;
+        // Each thread stages one triangle in tile-local form and marks which
+        // of the warp blocks may hold a pixel it covers.
+        const uint32_t k = base + threadIdx.x;
         uint32_t m = 0;
         const uint32_t entry = k < range.y ? sortedSlots[k] : 0u;
         if (k < range.y && (entry & BIN_WINDING_ENTRY))
@@ -2988,8 +3093,8 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
             L.v2 = make_float4(0.f, 0.f, W, 0.f);
             L.v3 = make_float4(0.f, -1.f, 0.f, 0.f);
             L.v4 = make_uint4(__float_as_uint(cv.z), __float_as_uint(cv.w), meta.x, 0u);
-            sTris[si] = L;
-            m = G::kBlocks >= 32 ? 0xffffffffu : ((1u << (G::kBlocks & 31)) - 1u);
+            sh.tris[threadIdx.x] = L;
+            m = 0xffffffffu >> (32 - G::kBlocks);
         }
         else if (k < range.y)
         {
@@ -3008,146 +3113,154 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
                                T.cov1.y);
             L.v4 = make_uint4(__float_as_uint(T.cov1.z), __float_as_uint(T.cov1.w), T.meta.x,
                               entry);
-            sTris[si] = L;
+            sh.tris[threadIdx.x] = L;
             const int4 bb = unpack_bbox(T.meta);
             const int bx0 = bb.x - ox, bx1 = bb.z - ox, by0 = bb.y - oy, by1 = bb.w - oy;
 #pragma unroll
             for (int b = 0; b < G::kBlocks; ++b)
             {
-                const int qx = (b % G::kWarpCols) * 8, qy = (b / G::kWarpCols) * 4;
-                const int x0 = max(bx0, qx), x1 = min(bx1, qx + 8);
-                const int y0 = max(by0, qy), y1 = min(by1, qy + 4);
+                const int bx = (b % G::kWarpCols) * 8, by = (b / G::kWarpCols) * 4;
+                const int x0 = max(bx0, bx), x1 = min(bx1, bx + 8);
+                const int y0 = max(by0, by), y1 = min(by1, by + 4);
                 if (x0 < x1 && y0 < y1 && local_rect_overlaps(c, e, x0, x1, y0, y1))
                     m |= 1u << b;
             }
         }
-        sMask[si] = (typename G::Mask)m;
+        // Per block, the staged triangles that may cover it.
+#pragma unroll
+        for (int b = 0; b < G::kBlocks; ++b)
+        {
+            const uint32_t bits = __ballot_sync(0xffffffffu, (m >> b) & 1u);
+            if (lane == b)
+                sh.bits[b][warp] = bits;
         }
         __syncthreads();
-#if RIVE_RASTER_PREFETCH
-        // The next chunk's records are pulled into L2 while this one is
-        // walked, so the staging after the next barrier does not wait on DRAM.
-        if (kStage == 1)
+        // This warp's triangles of the chunk, in primitive order.
+        uint32_t n = 0;
+        const uint32_t words = (min(kChunk, range.y - base) + 31) / 32;
+        for (uint32_t w = 0; w < words; ++w)
         {
-            const uint32_t kn = base + kChunk + threadIdx.x;
-            if (kn < range.y)
-            {
-                const uint32_t en = __ldg(sortedSlots + kn) & ~BIN_WINDING_ENTRY;
-                const char* a = reinterpret_cast<const char*>(tris + en);
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(a));
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(a + sizeof(TriRecord) - 1));
-            }
+            const uint32_t bits = sh.bits[warp][w];
+            if ((bits >> lane) & 1u)
+                sh.list[warp][n + __popc(bits & ((1u << lane) - 1u))] =
+                    (typename G::Index)(w * 32 + lane);
+            n += __popc(bits);
         }
-#endif
-        const uint32_t n = min(kChunk, range.y - base);
+        __syncwarp();
         for (uint32_t g = 0; g < n; g += 32)
         {
-            // Triangles of this group touching this warp's block, in order.
-            uint32_t bits = __ballot_sync(0xffffffffu, (sMask[g + lane] >> warp) & 1u);
-            while (bits)
+            // One lane per triangle: the pixels of the block it covers, and
+            // where the stream moves to another path.
+            const typename G::Index* const list = sh.list[warp] + g;
+            const uint32_t cnt = min(32u, n - g);
+            uint32_t cover = 0, path = 0;
+            if (lane < cnt)
             {
-                const uint32_t i = g + (uint32_t)(__ffs(bits) - 1);
-                bits &= bits - 1;
-                const TileTri& T = sTris[i];
-                const float4 v0 = T.v0;
-                const uint32_t vPathID = __float_as_uint(v0.x);
-                // A path's triangles are contiguous in primitive order, so when
-                // the warp's stream moves to another path every pixel still
-                // holding the previous path's coverage has seen all of it:
-                // resolve them together (one convergent call per path).
-                if (vPathID != streamPath)
+                const TileTri& T = sh.tris[list[lane]];
+                path = __float_as_uint(T.v0.x);
+                cover = block_coverage(T, (float)qx, (float)qy);
+            }
+            uint32_t before = __shfl_up_sync(0xffffffffu, path, 1);
+            if (lane == 0)
+                before = streamPath;
+            uint32_t moves = __ballot_sync(0xffffffffu, lane < cnt && path != before);
+            streamPath = __shfl_sync(0xffffffffu, path, cnt - 1);
+            // One lane per pixel: the triangles that cover it.
+            uint32_t hits = transpose_bits(cover, lane);
+            if (!inBounds)
+                hits = 0;
+            uint32_t from = 0;
+            while (from < cnt)
+            {
+                // The run [from, to) of one path. A path's triangles are
+                // contiguous in primitive order, so when the stream moves to
+                // another path every pixel still holding the previous path's
+                // coverage has seen all of it: resolve them together.
+                if ((moves >> from) & 1u)
                 {
-                    if (s.pendMeta)
+                    if (pendMeta)
                     {
-                        resolve_path<kFeather>(P, s, fx, fy, dither);
-                        s.pendMeta = 0;
+                        s = resolve_path<kFeather>(P, s, count, pendMeta, pendPaintX, pendPaintY,
+                                                   oneFragment, fx, fy);
+                        pendMeta = 0;
                     }
-                    streamPath = vPathID;
+                    moves &= moves - 1; // the lowest set bit is `from`
                 }
-                const float4 v1 = T.v1, v2 = T.v2;
-                const float E0 = local_edge(v0.y, v0.z, v0.w, lx, ly);
-                const float E1 = local_edge(v1.x, v1.y, v1.z, lx, ly);
-                const float E2 = local_edge(v1.w, v2.x, v2.y, lx, ly);
-                const float emin = fminf(fminf(E0, E1), E2);
-                if (!(emin > 0.f) &&
-                    !(emin == 0.f && local_inside(v0.z, v0.w, E0) && local_inside(v1.y, v1.z, E1) &&
-                      local_inside(v2.x, v2.y, E2)))
-                    continue;
-                if (!inBounds)
-                    continue;
-                const float4 v3 = T.v3;
-                const float covx = __fmaf_rn(v2.w, lx, __fmaf_rn(v3.x, ly, v2.z));
-                const float covy = __fmaf_rn(v3.z, lx, __fmaf_rn(v3.w, ly, v3.y));
-                if (kFeather && ((T.v4.z >> 16) & FEATURE_IMAGE_MESH))
+                const uint32_t to = moves ? (uint32_t)__ffs(moves) - 1u : cnt;
+                uint32_t h = hits & (to < 32 ? (1u << to) - 1u : 0xffffffffu);
+                hits &= ~h;
+                from = to;
+                while (h)
                 {
-                    // An image-mesh triangle blends at once, like a blit.
-                    if (s.pendMeta)
+                    const TileTri& T = sh.tris[list[__ffs(h) - 1]];
+                    h &= h - 1;
+                    const float4 v2 = T.v2, v3 = T.v3;
+                    const float covx = __fmaf_rn(v2.w, lx, __fmaf_rn(v3.x, ly, v2.z));
+                    const float covy = __fmaf_rn(v3.z, lx, __fmaf_rn(v3.w, ly, v3.y));
+                    const uint32_t vPathID = __float_as_uint(T.v0.x);
+                    if (kFeather && ((T.v4.z >> 16) & (FEATURE_IMAGE_MESH | FEATURE_ATLAS_BLIT)))
                     {
-                        resolve_path<kFeather>(P, s, fx, fy, dither);
-                        s.pendMeta = 0;
-                    }
-                    const uint4 v4 = T.v4;
-                    resolve_mesh(P, s, v4.z, v4.x, v4.y, B.featherPlanes + 2 * (size_t)v4.w, fx, fy,
-                                 dither);
-                    continue;
-                }
-                if (kFeather && ((T.v4.z >> 16) & FEATURE_ATLAS_BLIT))
-                {
-                    // A blit: the pending path is complete here; the blit
-                    // writes its colour at once and leaves the coverage plane
-                    // (key and count) to whichever path owns it.
-                    if (s.pendMeta)
-                    {
-                        resolve_path<kFeather>(P, s, fx, fy, dither);
-                        s.pendMeta = 0;
-                    }
-                    const uint4 v4 = T.v4;
-                    resolve_blit(P, s, v4.z, v4.x, v4.y, covx, covy, fx, fy, dither);
-                    continue;
-                }
-                float count;
-                if (s.key != vPathID)
-                {
-                    if (s.pendMeta)
-                        resolve_path<kFeather>(P, s, fx, fy, dither);
-                    const uint4 v4 = T.v4;
-                    s.pendMeta = v4.z;
-                    s.pendPaintX = v4.x;
-                    s.pendPaintY = v4.y;
-                    s.pendFrags = 1;
-                    s.key = vPathID;
-                    count = 0.f;
-                }
-                else
-                {
-                    count = s.count;
-                    s.pendFrags = 2;
-                    if (!s.pendMeta) // the key's path came back after a resolve
-                    {
+                        // An image-mesh triangle or a feather-atlas blit: the
+                        // pending path is complete here; it writes its colour
+                        // at once and leaves the coverage plane (key and
+                        // count) to whichever path owns it.
+                        if (pendMeta)
+                        {
+                            s = resolve_path<kFeather>(P, s, count, pendMeta, pendPaintX,
+                                                       pendPaintY, oneFragment, fx, fy);
+                            pendMeta = 0;
+                        }
                         const uint4 v4 = T.v4;
-                        s.pendMeta = v4.z;
-                        s.pendPaintX = v4.x;
-                        s.pendPaintY = v4.y;
+                        s.color = ((v4.z >> 16) & FEATURE_IMAGE_MESH)
+                                      ? resolve_mesh(P, s.color, s.clip, v4.z, v4.x, v4.y,
+                                                     B.featherPlanes + 2 * (size_t)v4.w, fx, fy)
+                                      : resolve_blit(P, s.color, s.clip, v4.z, v4.x, v4.y, covx,
+                                                     covy, fx, fy);
+                        continue;
                     }
+                    if (key != vPathID)
+                    {
+                        // The path's first fragment here. (Nothing is pending:
+                        // the pending path is the stream's, whose key is this.)
+                        const uint4 v4 = T.v4;
+                        pendMeta = v4.z;
+                        pendPaintX = v4.x;
+                        pendPaintY = v4.y;
+                        oneFragment = true;
+                        key = vPathID;
+                        count = 0.f;
+                    }
+                    else
+                    {
+                        oneFragment = false;
+                        if (!pendMeta) // the key's path came back after a resolve
+                        {
+                            const uint4 v4 = T.v4;
+                            pendMeta = v4.z;
+                            pendPaintX = v4.x;
+                            pendPaintY = v4.y;
+                        }
+                    }
+                    // Strokes (covy >= 0) keep the maximum coverage, fills add
+                    // (find_stroke_coverage / find_fill_coverage,
+                    // draw_path.vert:501-519); feathered ones are marked by a
+                    // coverage below the feather threshold.
+                    const bool stroke = covy >= 0.f;
+                    float frag = stroke ? fminf(covx, covy) : covx;
+                    // (pendMeta is this triangle's pathAndFeatures here.)
+                    if (kFeather && (stroke ? covx : covy) < kFeatherCoverageThreshold &&
+                        ((pendMeta >> 16) & SF_FEATHER))
+                        frag = feathered_fragment(B.featherPlanes, T.v4.w, fx, fy, covx, covy);
+                    count = h2f(f2h(stroke ? fmaxf(frag, count) : count + frag)); // fp16 plane
                 }
-                // Strokes (covy >= 0) keep the maximum coverage, fills add
-                // (find_stroke_coverage / find_fill_coverage,
-                // draw_path.vert:501-519); feathered ones are marked by a
-                // coverage below the feather threshold.
-                const bool stroke = covy >= 0.f;
-                float frag = stroke ? fminf(covx, covy) : covx;
-                // (s.pendMeta is this triangle's pathAndFeatures here.)
-                if (kFeather && (stroke ? covx : covy) < kFeatherCoverageThreshold &&
-                    ((s.pendMeta >> 16) & SF_FEATHER))
-                    frag = feathered_fragment(B.featherPlanes, T.v4.w, fx, fy, covx, covy);
-                count = stroke ? fmaxf(frag, count) : count + frag;
-                s.count = h2f(f2h(count)); // the plane stores fp16
+                __syncwarp();
             }
         }
         __syncthreads();
     }
-    if (s.pendMeta)
-        resolve_path<kFeather>(P, s, fx, fy, dither);
+    if (pendMeta)
+        s = resolve_path<kFeather>(P, s, count, pendMeta, pendPaintX, pendPaintY, oneFragment, fx,
+                                   fy);
     if (inBounds)
         fb[(size_t)py * P.width + px] = s.color;
 }
@@ -3159,10 +3272,8 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
         BatchTables B, const TriRecord* __restrict__ tris,                                        \
         const uint32_t* __restrict__ sortedSlots, const uint2* __restrict__ ranges)               \
     {                                                                                             \
-        __shared__ TileTri sTris[256 * RIVE_RASTER_STAGE];                                        \
-        __shared__ uint8_t sMask[256 * RIVE_RASTER_STAGE];                                        \
-        raster_tile<4, FEATHER, RIVE_RASTER_STAGE>(B, tris, sortedSlots, ranges, sTris, sMask,   \
-                                                    blockIdx.x);                                  \
+        __shared__ RasterShared<4> sh;                                                            \
+        raster_tile<4, FEATHER>(B, tris, sortedSlots, ranges, sh, blockIdx.x);                    \
     }
 RIVE_RASTER_KERNELS(raster_tile_kernel, false)
 RIVE_RASTER_KERNELS(raster_tile_feather_kernel, true)
@@ -3179,8 +3290,7 @@ RIVE_RASTER_KERNELS(raster_tile_feather_kernel, true)
         const uint32_t* __restrict__ sortedSlots, const uint2* __restrict__ ranges,               \
         const uint32_t* __restrict__ order, uint32_t* __restrict__ cursor, uint32_t tiles)        \
     {                                                                                             \
-        __shared__ TileTri sTris[256];                                                            \
-        __shared__ uint8_t sMask[256];                                                            \
+        __shared__ RasterShared<4> sh;                                                            \
         __shared__ uint32_t sNext;                                                                \
         for (;;)                                                                                  \
         {                                                                                         \
@@ -3191,7 +3301,7 @@ RIVE_RASTER_KERNELS(raster_tile_feather_kernel, true)
             const uint32_t t = sNext;                                                             \
             if (t >= tiles)                                                                       \
                 break;                                                                            \
-            raster_tile<4, FEATHER, 1>(B, tris, sortedSlots, ranges, sTris, sMask, order[t]);     \
+            raster_tile<4, FEATHER>(B, tris, sortedSlots, ranges, sh, order[t]);                  \
         }                                                                                         \
     }
 RIVE_RASTER_QUEUE_KERNELS(raster_queue_kernel, false)
@@ -3301,16 +3411,14 @@ __global__ void __launch_bounds__(256) tile_order_keys_kernel(uint32_t tiles,
                                                const uint32_t* __restrict__ sortedSlots,         \
                                                const uint2* __restrict__ ranges)                 \
     {                                                                                             \
-        __shared__ TileTri sTris[64 * RIVE_RASTER_STAGE];                                         \
-        __shared__ uint8_t sMask[64 * RIVE_RASTER_STAGE];                                         \
-        raster_tile<3, FEATHER, RIVE_RASTER_STAGE>(B, tris, sortedSlots, ranges, sTris, sMask,   \
-                                                    blockIdx.x);                                  \
+        __shared__ RasterShared<3> sh;                                                            \
+        raster_tile<3, FEATHER>(B, tris, sortedSlots, ranges, sh, blockIdx.x);                    \
     }
 RIVE_RASTER8_KERNELS(raster_tile8_kernel, false)
 RIVE_RASTER8_KERNELS(raster_tile8_feather_kernel, true)
 #undef RIVE_RASTER8_KERNELS
 
-// 32x32 tiles: 1,024 threads, the staged records in dynamic shared memory
+// 32x32 tiles: 1,024 threads, the tile's shared state in dynamic shared memory
 // (kRaster32SmemBytes).
 #define RIVE_RASTER32_KERNELS(NAME, FEATHER)                                                      \
     __global__ void __launch_bounds__(1024, 1) NAME(                                              \
@@ -3318,10 +3426,10 @@ RIVE_RASTER8_KERNELS(raster_tile8_feather_kernel, true)
         const uint32_t* __restrict__ sortedSlots, const uint2* __restrict__ ranges)               \
     {                                                                                             \
         extern __shared__ uint4 dyn[];                                                            \
-        TileTri* sTris = reinterpret_cast<TileTri*>(dyn);                                         \
-        uint32_t* sMask = reinterpret_cast<uint32_t*>(sTris + 1024);                              \
-        raster_tile<5, FEATHER, 1>(B, tris, sortedSlots, ranges, sTris, sMask, blockIdx.x);       \
+        RasterShared<5>& sh = *reinterpret_cast<RasterShared<5>*>(dyn);                           \
+        raster_tile<5, FEATHER>(B, tris, sortedSlots, ranges, sh, blockIdx.x);                    \
     }
+static_assert(sizeof(RasterShared<5>) <= kRaster32SmemBytes, "kRaster32SmemBytes");
 RIVE_RASTER32_KERNELS(raster_tile32_kernel, false)
 RIVE_RASTER32_KERNELS(raster_tile32_feather_kernel, true)
 #undef RIVE_RASTER32_KERNELS

@@ -157,7 +157,8 @@ constexpr float kWindingMaxEdgeShare = .75f;
 // choices (rive_cuda_set_raster_config).
 constexpr int kTileSize = 16;
 constexpr int kTileLog2 = 4;
-constexpr int kRaster32SmemBytes = 1024 * 80 + 1024 * 4; // staged records + block masks
+// 32x32 tiles: staged records, block bits and per-warp triangle lists.
+constexpr int kRaster32SmemBytes = 1024 * 80 + 32 * 32 * 4 + 32 * 1024 * 2 + 512;
 
 // Device error word bits (read by rive_cuda_sync).
 constexpr uint32_t ERR_BAD_TESS_INDEX = 1u << 0;

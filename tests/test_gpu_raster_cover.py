@@ -1,0 +1,127 @@
+"""Which pixels the raster gives a triangle, against the edge rule evaluated
+pixel by pixel in numpy: every (triangle, pixel) decision must agree exactly.
+
+The triangles are interior triangles (opaque, undithered, one path each), so a
+pixel's colour names the last triangle that covers it. An edge's value is
+E = fma(A, x, fma(B, y, C)) with C = fma(A, dx, B dy) at the tile's first pixel
+centre; with coordinates on the 1/256-pixel grid all exact values here are
+multiples of 2^-16 below 2^33, so float64 holds them exactly and one rounding
+to float32 restates each fused step."""
+import numpy as np
+import pytest
+
+from conftest import device_buffers, load_golden, load_package
+
+load_package()
+W, H = 331, 203  # ragged at every tile size
+
+
+def triangles(kind, n, rng):
+    """n clockwise (y down) triangles, (n, 3, 2) on the 1/256-pixel grid."""
+    if kind == "ties":  # corners on and half-way between pixel centres, axis-aligned edges
+        p = (rng.integers(-4, 2 * max(W, H) + 4, (n, 1, 2)) + rng.integers(-50, 50, (n, 3, 2))) / 2.0
+        p[::3, 1, 1] = p[::3, 0, 1]
+        p[1::3, 2, 0] = p[1::3, 1, 0]
+    elif kind == "slivers":  # long and thin, far outside the canvas, rounded edge values
+        a = rng.integers(-2000 * 256, 2400 * 256, (n, 1, 2)) / 256.0
+        b = rng.integers(-2000 * 256, 2400 * 256, (n, 1, 2)) / 256.0
+        p = np.concatenate([a, b, b + rng.integers(-300, 300, (n, 1, 2)) / 256.0], 1)
+    else:  # "small": a few pixels
+        p = rng.integers(0, max(W, H) * 256, (n, 1, 2)) + rng.integers(-1400, 1400, (n, 3, 2))
+        p = p / 256.0
+    u, v = p[:, 1] - p[:, 0], p[:, 2] - p[:, 0]
+    area = u[:, 0] * v[:, 1] - v[:, 0] * u[:, 1]
+    p[area < 0] = p[area < 0][:, [0, 2, 1]]
+    return p
+
+
+def f32(x):
+    return np.asarray(x, np.float64).astype(np.float32).astype(np.float64)
+
+
+def expected(tris, tile):
+    """Per pixel the last covering triangle's number + 1, or 0."""
+    out = np.zeros((H, W), np.int64)
+    for i, p in enumerate(tris):
+        u, v = p[1] - p[0], p[2] - p[0]
+        if u[0] * v[1] - v[0] * u[1] <= 0:
+            continue
+        lo = np.maximum(np.ceil(p.min(0) - .5), 0)
+        hi = np.minimum(np.floor(p.max(0) - .5) + 1, (W, H))
+        if (lo >= hi).any():
+            continue
+        ly0, lx0 = (lo[::-1] // 8 * 8).astype(int)  # whole 8x4 blocks about the pixel box
+        ly1, lx1 = (-(-hi[::-1] // 8) * 8).astype(int)
+        ys, xs = np.mgrid[ly0:min(ly1, H), lx0:min(lx1, W)]
+        ox, oy = xs // tile * tile, ys // tile * tile
+        lx, ly = xs - ox, ys - oy
+        bx, by = lx // 8 * 8, ly // 4 * 4  # the pixel's 8x4 block in its tile
+        # The part of the block inside the pixel box, tile-local, empty or not.
+        x0, x1 = np.maximum(lo[0] - ox, bx), np.minimum(hi[0] - ox, bx + 8)
+        y0, y1 = np.maximum(lo[1] - oy, by), np.minimum(hi[1] - oy, by + 4)
+        inside = (x0 < x1) & (y0 < y1)
+        for k in range(3):
+            a, b = p[k], p[(k + 1) % 3]
+            first, last = (a, b) if (a[1], a[0]) < (b[1], b[0]) else (b, a)
+            A, B = -(b[1] - a[1]), b[0] - a[0]
+            assert first is not last
+            C = f32(A * (ox + .5 - first[0]) + f32(B * (oy + .5 - first[1])))
+            E = A * lx + f32(B * ly + C)
+            edge_in = A > 0 or (A == 0 and B > 0)
+            # The block's corner that maximises E must not be outside.
+            corner = A * (x1 - 1 if A > 0 else x0) + f32(B * (y1 - 1 if B > 0 else y0) + C)
+            inside &= ((E >= 0) if edge_in else (E > 0)) & (corner >= 0)
+        out[ys[inside], xs[inside]] = i + 1
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("queue", [False, True])
+@pytest.mark.parametrize("tile", [8, 16, 32])
+@pytest.mark.parametrize("kind,n", [("ties", 700), ("slivers", 700), ("small", 3000)])
+def test_covered_pixels_are_exact(kind, n, tile, queue):
+    import torch
+    from rive_runtime_gb300 import rive_cuda
+    if queue and tile != 16:
+        pytest.skip("the work queue takes 16-pixel tiles")
+    tris = triangles(kind, n, np.random.default_rng(7))
+    cap = load_golden("tri_fills_s21")[0]  # for a FlushUniforms record and a descriptor
+    f = cap.flushes[0]
+    paths = np.zeros((n + 1, 16), np.float32)
+    paths[1:, 0] = paths[1:, 3] = 1.0
+    ids = np.arange(n + 1, dtype=np.uint32)
+    paints = np.zeros((n + 1, 2), np.uint32)
+    paints[:, 0] = 1  # solid
+    paints[:, 1] = ids | 0xFF000000
+    verts = np.zeros((n, 3, 3), np.uint32)
+    verts[..., :2] = tris.astype(np.float32).view(np.uint32)
+    verts[..., 2] = ids[1:, None] | 0x10000  # weight 1
+    cap.buffers = {"flush_uniforms": cap.buffers["flush_uniforms"], "paths": paths.tobytes(),
+                   "paints": paints.tobytes(), "paint_aux": bytes(128 * (n + 1)),
+                   "triangles": verts.tobytes()}
+    f.desc.update(render_target_width=W, render_target_height=H, ub2=W, ub3=H, path_count=n + 1,
+                  contour_count=0, tess_span_count=0, tess_data_height=0, dither_mode=0,
+                  color_clear_value=0xFF000000, combined_shader_features=0)
+    f.batches = np.array([[3, 3 * n, 0, 0, 16, 0, 3, 0]], np.uint32)
+    bufs, keep = device_buffers(cap)
+    ctx = rive_cuda.Context(0)
+    ctx.set_raster_config(tile)
+    ctx.set_raster_queue(queue)
+    target = torch.zeros((H, W, 4), dtype=torch.uint8, device="cuda")
+    ctx.flush_device(f, bufs, target.data_ptr())
+    ctx.sync()
+    img = target.cpu().numpy().astype(np.int64)
+    ctx.close()
+    got = img[..., 0] | (img[..., 1] << 8) | (img[..., 2] << 16)
+    want = expected(tris, tile)
+    assert (want > 0).mean() > .02
+    assert np.array_equal(got, want), np.argwhere(got != want)[:5]
+
+
+def test_unorm_float_is_the_correctly_rounded_quotient():
+    """kUnormHi / kUnormLo of kernels_raster.cu: b / 255 for every byte by one
+    rounded product and one fused step (float64 holds both exactly)."""
+    hi, lo = np.float64(float.fromhex("0x1.010102p-8")), np.float64(float.fromhex("-0x1.fdfdfep-33"))
+    b = np.arange(256, dtype=np.float64)
+    got = (b * hi + f32(b * lo)).astype(np.float32)
+    assert np.array_equal(got, np.arange(256, dtype=np.float32) / np.float32(255))
