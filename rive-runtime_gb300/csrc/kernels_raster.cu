@@ -2185,6 +2185,86 @@ __device__ __forceinline__ uint32_t pack_rgba8(const float c[4])
                        __byte_perm(unorm8_bits(c[2]), unorm8_bits(c[3]), 0x0040), 0x5410);
 }
 
+// Two fp32 lanes of a 64-bit register pair and the packed operations on them
+// (one issue slot for both; each lane rounds as the scalar operation does).
+struct Pair
+{
+    unsigned long long v;
+};
+__device__ __forceinline__ Pair pair(float x, float y)
+{
+    Pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float2 split(Pair p)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p.v));
+    return r;
+}
+__device__ __forceinline__ Pair mul2(Pair a, Pair b)
+{
+    Pair r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+// The product where an add2 follows: the assembler fuses a packed multiply and
+// a packed add into one rounding (measured: 10% of random sums differ in the
+// last bit, bytes of the image change), which it does not do to scalar ones.
+__device__ __forceinline__ Pair mul2_rounded(Pair a, Pair b)
+{
+    const float2 x = split(a), y = split(b);
+    return pair(__fmul_rn(x.x, y.x), __fmul_rn(x.y, y.y));
+}
+__device__ __forceinline__ Pair add2(Pair a, Pair b)
+{
+    Pair r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c)
+{
+    Pair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+
+// An RGBA colour as two pairs.
+struct Color
+{
+    Pair rg, ba;
+};
+__device__ __forceinline__ Pair unorm_pair(uint32_t c, uint32_t selX, uint32_t selY)
+{
+    // Bytes into the mantissas of 2^23 + byte, then as in unorm_float.
+    const Pair f = add2(pair(__uint_as_float(__byte_perm(c, 0x4b000000u, selX)),
+                             __uint_as_float(__byte_perm(c, 0x4b000000u, selY))),
+                        pair(-8388608.f, -8388608.f));
+    return fma2(f, pair(kUnormHi, kUnormHi), mul2(f, pair(kUnormLo, kUnormLo)));
+}
+__device__ __forceinline__ Color unpack_color(uint32_t c)
+{
+    return {unorm_pair(c, 0x7650, 0x7651), unorm_pair(c, 0x7652, 0x7653)};
+}
+// pack_rgba8 of the colour with `dither` added to r, g and b: the clamp is the
+// saturation of that addition.
+__device__ __forceinline__ uint32_t pack_color(Color c, float dither)
+{
+    const float2 rg = split(c.rg), ba = split(c.ba);
+    const Pair k255 = pair(255.f, 255.f), magic = pair(12582912.f, 12582912.f);
+    const float2 x = split(add2(mul2_rounded(pair(__saturatef(__fadd_rn(rg.x, dither)),
+                                          __saturatef(__fadd_rn(rg.y, dither))),
+                                     k255),
+                                magic));
+    const float2 y = split(add2(mul2_rounded(pair(__saturatef(__fadd_rn(ba.x, dither)),
+                                          __saturatef(ba.y)),
+                                     k255),
+                                magic));
+    return __byte_perm(__byte_perm(__float_as_uint(x.x), __float_as_uint(x.y), 0x0040),
+                       __byte_perm(__float_as_uint(y.x), __float_as_uint(y.y), 0x0040), 0x5410);
+}
+
 __device__ __forceinline__ float min3f(float a, float b, float c) { return fminf(fminf(a, b), c); }
 __device__ __forceinline__ float max3f(float a, float b, float c) { return fmaxf(fmaxf(a, b), c); }
 
@@ -2307,7 +2387,7 @@ __device__ __noinline__ void advanced_blend(float src[3], const float dp[4], uin
 // fused multiply-adds), in the oracle's order: a gradient coordinate is a
 // difference of large terms, and a contracted evaluation lands on the other
 // side of a hard colour step at a few pixels.
-__device__ __noinline__ void sample_grad(const FlushParams& P, float u, float v, float out[4])
+__device__ __noinline__ Color sample_grad(const FlushParams& P, float u, float v)
 {
     float fx = __fsub_rn(__fmul_rn(u, (float)kGradTextureWidth), .5f);
     // The gradient texture always has at least one row allocated.
@@ -2316,21 +2396,25 @@ __device__ __noinline__ void sample_grad(const FlushParams& P, float u, float v,
     float x0f = floorf(fx), y0f = floorf(fy);
     float ax = __fsub_rn(fx, x0f), ay = __fsub_rn(fy, y0f);
     int x0 = (int)x0f, y0 = (int)y0f;
-    out[0] = out[1] = out[2] = out[3] = 0.f;
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-        {
-            int xi = min(max(x0 + i, 0), kGradTextureWidth - 1);
-            int yj = min(max(y0 + j, 0), H - 1);
-            float wgt = __fmul_rn(i ? ax : __fsub_rn(1.f, ax), j ? ay : __fsub_rn(1.f, ay));
-            uchar4 t = P.grad[(size_t)yj * kGradTextureWidth + xi];
-            out[0] = __fadd_rn(out[0], __fmul_rn(wgt, unorm_float(t.x)));
-            out[1] = __fadd_rn(out[1], __fmul_rn(wgt, unorm_float(t.y)));
-            out[2] = __fadd_rn(out[2], __fmul_rn(wgt, unorm_float(t.z)));
-            out[3] = __fadd_rn(out[3], __fmul_rn(wgt, unorm_float(t.w)));
-        }
+    const int xa = min(max(x0, 0), kGradTextureWidth - 1);
+    const int xb = min(max(x0 + 1, 0), kGradTextureWidth - 1);
+    const uint32_t* __restrict__ grad = reinterpret_cast<const uint32_t*>(P.grad);
+    Color out = {pair(0.f, 0.f), pair(0.f, 0.f)};
+    // A row's centre (where the front end puts a gradient's coordinate, to
+    // rounding) gives the second row the weight 0: it would add zeros.
+    const int rows = ay == 0.f ? 1 : 2;
+    for (int j = 0; j < rows; ++j)
+    {
+        const uint32_t* row = grad + (size_t)min(max(y0 + j, 0), H - 1) * kGradTextureWidth;
+        const float wy = j ? ay : __fsub_rn(1.f, ay);
+        const float wa = __fmul_rn(__fsub_rn(1.f, ax), wy), wb = __fmul_rn(ax, wy);
+        const Color ca = unpack_color(row[xa]), cb = unpack_color(row[xb]);
+        out.rg = add2(add2(out.rg, mul2_rounded(pair(wa, wa), ca.rg)),
+                      mul2_rounded(pair(wb, wb), cb.rg));
+        out.ba = add2(add2(out.ba, mul2_rounded(pair(wa, wa), ca.ba)),
+                      mul2_rounded(pair(wb, wb), cb.ba));
+    }
+    return out;
 }
 
 // The pixel-local-storage planes a resolve reads and writes
@@ -2396,25 +2480,27 @@ __device__ __forceinline__ float clip_rect_distance(const FlushParams& P, uint32
 __device__ __noinline__ void image_modulate(const FlushParams& P, uint32_t pathID, float fx,
                                             float fy, bool unmultiplied, float color[4]);
 
-__device__ __forceinline__ void paint_color(const FlushParams& P, uint32_t paintX, uint32_t paintY,
-                                            uint32_t pathID, float fx, float fy, float coverage,
-                                            bool unmultiplied, float color[4],
-                                            uint32_t features = 0)
+__device__ __forceinline__ Color paint_color(const FlushParams& P, uint32_t paintX,
+                                             uint32_t paintY, uint32_t pathID, float fx, float fy,
+                                             float coverage, bool unmultiplied,
+                                             uint32_t features = 0)
 {
     const uint32_t paintType = paintX & 0xfu;
+    Color c;
     if (paintType == SOLID_COLOR_PAINT_TYPE)
     {
-        unpack_rgba8(paintY, color);
+        c = unpack_color(paintY);
         if (!unmultiplied)
         {
-            color[0] *= color[3];
-            color[1] *= color[3];
-            color[2] *= color[3];
-            for (int k = 0; k < 4; ++k)
-                color[k] *= coverage;
+            const float a = split(c.ba).y;
+            const Pair cov = pair(coverage, coverage);
+            c.rg = mul2_rounded(mul2(c.rg, pair(a, a)), cov);
+            c.ba = mul2_rounded(mul2(c.ba, pair(a, 1.f)), cov);
         }
         else
-            color[3] *= coverage;
+        {
+            c.ba = mul2_rounded(c.ba, pair(1.f, coverage));
+        }
     }
     else if (paintType == LINEAR_GRADIENT_PAINT_TYPE || paintType == RADIAL_GRADIENT_PAINT_TYPE)
     {
@@ -2430,21 +2516,27 @@ __device__ __forceinline__ void paint_color(const FlushParams& P, uint32_t paint
         float x = spanB > 1.f ? __fadd_rn(__fmul_rn(1.f - 1.f / kGradTextureWidth, t),
                                           .5f / kGradTextureWidth)
                               : __fadd_rn(__fmul_rn(1.f / kGradTextureWidth, t), spanB);
-        sample_grad(P, x, __uint_as_float(paintY), color);
-        color[3] *= coverage;
+        c = sample_grad(P, x, __uint_as_float(paintY));
+        c.ba = mul2_rounded(c.ba, pair(1.f, coverage));
         if (!unmultiplied)
         {
-            color[0] *= color[3];
-            color[1] *= color[3];
-            color[2] *= color[3];
+            const float a = split(c.ba).y;
+            c.rg = mul2_rounded(c.rg, pair(a, a));
+            c.ba = mul2_rounded(c.ba, pair(a, 1.f));
         }
     }
     else
     {
-        color[0] = color[1] = color[2] = color[3] = 0.f;
+        c.rg = c.ba = pair(0.f, 0.f);
     }
     if ((features & SF_MODULATED_IMAGE) && (paintX & PAINT_FLAG_HAS_IMAGE) && P.pathImage)
+    {
+        const float2 rg = split(c.rg), ba = split(c.ba);
+        float color[4] = {rg.x, rg.y, ba.x, ba.y};
         image_modulate(P, pathID, fx, fy, unmultiplied, color);
+        c = {pair(color[0], color[1]), pair(color[2], color[3])};
+    }
+    return c;
 }
 
 // An image texel address under a wrap mode (the Vulkan sampler address modes
@@ -2529,7 +2621,8 @@ __device__ void sample_image(const ImageTex& t, float u, float v, float lod, flo
 __device__ __noinline__ uint32_t resolve_mesh(const FlushParams& P, uint32_t dstColor,
                                               uint32_t clip, uint32_t meta, uint32_t imageDraw,
                                               uint32_t imageWord,
-                                              const float4* __restrict__ planes, float fx, float fy)
+                                              const float4* __restrict__ planes, float fx, float fy,
+                                              float dither)
 {
     const uint32_t features = meta >> 16;
     const float4 f0 = planes[0], f1 = planes[1];
@@ -2583,7 +2676,6 @@ __device__ __noinline__ uint32_t resolve_mesh(const FlushParams& P, uint32_t dst
     }
     if ((features & SF_DITHER) && color[3] != 0.f)
     {
-        const float dither = pixel_dither(P, fx, fy);
         color[0] += dither;
         color[1] += dither;
         color[2] += dither;
@@ -2637,9 +2729,10 @@ __device__ __noinline__ void image_modulate(const FlushParams& P, uint32_t pathI
 // which batches with images or feathers use); the plain variant's resolve
 // stays without it.
 template <bool kImages>
-__device__ __noinline__ Planes resolve_path(const FlushParams& P, Planes s, float count,
+__device__ __forceinline__ Planes resolve_path(const FlushParams& P, Planes s, float count,
                                             uint32_t meta, uint32_t paintX, uint32_t paintY,
-                                            bool oneFragment, float fx, float fy)
+                                            bool oneFragment, float fx, float fy,
+                                            float dither)
 {
     const uint32_t pathID = meta & 0xffffu, features = meta >> 16;
     const uint32_t paintType = paintX & 0xfu;
@@ -2697,34 +2790,46 @@ __device__ __noinline__ Planes resolve_path(const FlushParams& P, Planes s, floa
         coverage = fminf(fmaxf(clip_rect_distance(P, pathID, fx, fy), 0.f), coverage);
 
     const bool unmultiplied = (features & SF_ADVANCED_BLEND) != 0;
-    float color[4];
-    paint_color(P, paintX, paintY, pathID, fx, fy, coverage, unmultiplied, color,
-                kImages ? features : 0u);
-
-    float dst[4];
-    unpack_rgba8(s.color, dst);
-    s.scratch = s.color;
+    uint32_t mode = unmultiplied ? (paintX >> 4) & 0xfu : 0u;
+    if (mode >= 12 && !(features & SF_HSL_BLEND_MODES))
+        mode = 0;
+    const uint32_t dstColor = s.color;
+    s.scratch = dstColor;
+    // No coverage (the fan's triangles cancel, or the clip is empty here): the
+    // blend below would give back the destination.
+    if (coverage == 0.f && mode == 0)
+        return s;
+    Color c = paint_color(P, paintX, paintY, pathID, fx, fy, coverage, unmultiplied,
+                          kImages ? features : 0u);
+    const Color dst = unpack_color(dstColor);
+    if (mode != 0)
+    {
+        const float2 rg = split(c.rg), ba = split(c.ba);
+        const float2 drg = split(dst.rg), dba = split(dst.ba);
+        float color[4] = {rg.x, rg.y, ba.x, ba.y};
+        const float d[4] = {drg.x, drg.y, dba.x, dba.y};
+        advanced_blend(color, d, mode);
+        c = {pair(color[0], color[1]), pair(color[2], color[3])};
+    }
+    const float paintAlpha = split(c.ba).y;
     if (unmultiplied)
     {
-        uint32_t mode = (paintX >> 4) & 0xfu;
-        if (mode != 0 && (mode < 12 || (features & SF_HSL_BLEND_MODES)))
-            advanced_blend(color, dst, mode);
-        color[0] *= color[3];
-        color[1] *= color[3];
-        color[2] *= color[3];
+        c.rg = mul2_rounded(c.rg, pair(paintAlpha, paintAlpha));
+        c.ba = mul2_rounded(c.ba, pair(paintAlpha, 1.f));
     }
-    const float paintAlpha = color[3];
-    for (int k = 0; k < 4; ++k)
-        color[k] += dst[k] * (1.f - paintAlpha);
-    if ((features & SF_DITHER) && paintAlpha != 0.f)
-    {
-        const float dither = pixel_dither(P, fx, fy);
-        color[0] += dither;
-        color[1] += dither;
-        color[2] += dither;
-    }
-    s.color = pack_rgba8(color);
+    const Pair keep = pair(1.f - paintAlpha, 1.f - paintAlpha);
+    c.rg = add2(c.rg, mul2_rounded(dst.rg, keep));
+    c.ba = add2(c.ba, mul2_rounded(dst.ba, keep));
+    s.color = pack_color(c, (features & SF_DITHER) && paintAlpha != 0.f ? dither : 0.f);
     return s;
+}
+
+// The same out of line, for the raster's rarely taken second call site.
+__device__ __noinline__ Planes resolve_path_call(const FlushParams& P, Planes s, float count,
+                                                 uint32_t meta, uint32_t paintX, uint32_t paintY,
+                                                 bool oneFragment, float fx, float fy, float dither)
+{
+    return resolve_path<true>(P, s, count, meta, paintX, paintY, oneFragment, fx, fy, dither);
 }
 
 // The feather atlas at atlas pixel coordinates (x, y): the atlas sampler's
@@ -2762,7 +2867,7 @@ __device__ __noinline__ float atlas_coverage(const FlushParams& P, float x, floa
 __device__ __noinline__ uint32_t resolve_blit(const FlushParams& P, uint32_t dstColor,
                                               uint32_t clip, uint32_t meta, uint32_t paintX,
                                               uint32_t paintY, float ax, float ay, float fx,
-                                              float fy)
+                                              float fy, float dither)
 {
     const uint32_t pathID = meta & 0xffffu, features = meta >> 16;
     const uint32_t paintType = paintX & 0xfu;
@@ -2780,8 +2885,9 @@ __device__ __noinline__ uint32_t resolve_blit(const FlushParams& P, uint32_t dst
         }
     }
     const bool unmultiplied = (features & SF_ADVANCED_BLEND) != 0;
-    float color[4];
-    paint_color(P, paintX, paintY, pathID, fx, fy, 1.f, unmultiplied, color, features);
+    const Color paint = paint_color(P, paintX, paintY, pathID, fx, fy, 1.f, unmultiplied, features);
+    const float2 prg = split(paint.rg), pba = split(paint.ba);
+    float color[4] = {prg.x, prg.y, pba.x, pba.y};
     float dst[4];
     unpack_rgba8(dstColor, dst);
     if (unmultiplied)
@@ -2801,7 +2907,6 @@ __device__ __noinline__ uint32_t resolve_blit(const FlushParams& P, uint32_t dst
     }
     if ((features & SF_DITHER) && color[3] != 0.f)
     {
-        const float dither = pixel_dither(P, fx, fy);
         color[0] += dither;
         color[1] += dither;
         color[2] += dither;
@@ -2822,10 +2927,10 @@ __device__ __noinline__ uint32_t resolve_blit(const FlushParams& P, uint32_t dst
 // cover it, in primitive order; a pixel's planes stay in registers.
 struct __align__(16) TileTri
 {
-    float4 v0; // coverage key (bits), C0, A0, B0
-    float4 v1; // C1, A1, B1, C2
-    float4 v2; // A2, B2, covx at the tile origin, d covx/dx
-    float4 v3; // d covx/dy, covy at the tile origin, d covy/dx, d covy/dy
+    float4 v0; // C0, A0, B0, C1
+    float4 v1; // A1, B1, C2, A2
+    float4 v2; // B2, covy at the tile origin, d covy/dx, d covy/dy
+    float4 v3; // covx at the tile origin, d covx/dx, d covx/dy, coverage key (bits)
     uint4 v4;  // paint.x, paint.y, pathAndFeatures, triangle slot
 };
 static_assert(sizeof(TileTri) == 80, "TileTri layout");
@@ -2909,10 +3014,10 @@ __device__ __noinline__ float feathered_fragment(const float4* __restrict__ plan
     return eval_feathered_fill(covx, covy, covz, covw);
 }
 
-// Resident CTAs per SM the register allocation is bounded for (16x16 tiles).
-#ifndef RIVE_RASTER_MIN_BLOCKS
-#define RIVE_RASTER_MIN_BLOCKS 5
-#endif
+// Resident CTAs per SM the register allocation is bounded for (16x16 tiles): 5
+// (48 registers; 64 UI screens 1.94 ms against 2.15 ms with 4), with the feather
+// paths 4 (64 registers; 16 recorded frames 2.69 ms against 2.76 ms with 5).
+#define RIVE_RASTER_MIN_BLOCKS(FEATHER) ((FEATHER) ? 4 : 5)
 
 // Tile geometry: a CTA of T x T threads, one per pixel; warp w owns the 8x4
 // block at (8 (w % (T/8)), 4 (w / (T/8))). A chunk of bin entries, one per
@@ -2939,6 +3044,60 @@ template <int TL> struct RasterShared
     FlushParams params;
 };
 
+// The warp blocks whose part inside the pixel box bb may hold a pixel inside
+// all three edges (tile constants c[k], slopes e[k].z, e[k].w): the test of
+// local_rect_overlaps on every block, with each edge's values at the block
+// rows' and columns' decisive corners shared between blocks and no branches.
+template <int TL>
+__device__ __forceinline__ uint32_t blocks_overlapped(const float* c, const float4* e, int4 bb,
+                                                      int ox, int oy)
+{
+    using G = RasterTile<TL>;
+    constexpr int kCols = G::kWarpCols, kRows = G::kBlocks / kCols;
+    const float x0 = (float)(bb.x - ox), x1 = (float)(bb.z - 1 - ox);
+    const float y0 = (float)(bb.y - oy), y1 = (float)(bb.w - 1 - oy);
+    float emin[kRows][kCols];
+    uint32_t valid = 0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+    {
+        float xs[kCols];
+#pragma unroll
+        for (int i = 0; i < kCols; ++i)
+            xs[i] = e[k].z > 0.f ? fminf(x1, 8.f * i + 7.f) : fmaxf(x0, 8.f * i);
+#pragma unroll
+        for (int j = 0; j < kRows; ++j)
+        {
+            const float y = e[k].w > 0.f ? fminf(y1, 4.f * j + 3.f) : fmaxf(y0, 4.f * j);
+            const float t = __fmaf_rn(e[k].w, y, c[k]);
+#pragma unroll
+            for (int i = 0; i < kCols; ++i)
+            {
+                const float E = __fmaf_rn(e[k].z, xs[i], t);
+                emin[j][i] = k == 0 ? E : fminf(emin[j][i], E);
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < kRows; ++j)
+#pragma unroll
+        for (int i = 0; i < kCols; ++i)
+            valid |= (emin[j][i] < 0.f ? 0u : 1u) << (j * kCols + i);
+    // Blocks that the pixel box does not reach: whole columns and rows.
+#pragma unroll
+    for (int i = 0; i < kCols; ++i)
+    {
+        constexpr uint32_t kColumn = kCols == 1 ? 0xffffffffu : kCols == 2 ? 0x55555555u : 0x11111111u;
+        if (x0 > 8.f * i + 7.f || x1 < 8.f * i)
+            valid &= ~(kColumn << i);
+    }
+#pragma unroll
+    for (int j = 0; j < kRows; ++j)
+        if (y0 > 4.f * j + 3.f || y1 < 4.f * j)
+            valid &= ~(((1u << kCols) - 1u) << (j * kCols));
+    return valid;
+}
+
 // ones << (n & 31).
 __device__ __forceinline__ uint32_t ones_from(uint32_t n)
 {
@@ -2961,10 +3120,10 @@ __device__ __forceinline__ uint32_t ones_from(uint32_t n)
 // About 28 instructions a row for all eight pixels, against 8 x 9 for testing
 // each, with one lane per triangle, where the test by pixels leaves idle the
 // three quarters of the lanes that a triangle does not cover.
-__device__ __forceinline__ uint32_t block_coverage(const TileTri& T, float qx, float qy)
+__device__ __forceinline__ uint32_t block_coverage(float4 v0, float4 v1, float b2, float qx,
+                                                   float qy)
 {
-    const float4 v0 = T.v0, v1 = T.v1, v2 = T.v2;
-    float a[3] = {v0.z, v1.y, v2.x}, b[3] = {v0.w, v1.z, v2.y}, c[3] = {v0.y, v1.x, v1.w};
+    float a[3] = {v0.y, v1.x, v1.w}, b[3] = {v0.z, v1.y, b2}, c[3] = {v0.x, v0.w, v1.z};
     float k[3];
     uint32_t flip[3];
 #pragma unroll
@@ -3002,22 +3161,39 @@ __device__ __forceinline__ uint32_t block_coverage(const TileTri& T, float qx, f
     return out;
 }
 
+// Up to this many triangles of a batch are tested pixel by pixel, one after
+// another (about 20 instructions each); more take block_coverage and the
+// transpose (about 200 for up to 32).
+#ifndef RIVE_RASTER_FEW
+#define RIVE_RASTER_FEW 6
+#endif
+constexpr uint32_t kFewTriangles = RIVE_RASTER_FEW;
+__device__ __forceinline__ bool pixel_inside(const TileTri& T, float lx, float ly)
+{
+    const float4 v0 = T.v0, v1 = T.v1;
+    const float b2 = T.v2.x;
+    const float E0 = local_edge(v0.x, v0.y, v0.z, lx, ly);
+    const float E1 = local_edge(v0.w, v1.x, v1.y, lx, ly);
+    const float E2 = local_edge(v1.z, v1.w, b2, lx, ly);
+    const float emin = fminf(fminf(E0, E1), E2);
+    return emin > 0.f || (emin == 0.f && local_inside(v0.y, v0.z, E0) &&
+                          local_inside(v1.x, v1.y, E1) && local_inside(v1.w, b2, E2));
+}
+
 // Transposes a 32x32 bit matrix held one row per lane: bit i of lane p's
-// result is bit p of lane i's word.
+// result is bit p of lane i's word. Each step swaps the off-diagonal halves of
+// 2j x 2j blocks between lanes j apart; whole bytes move by one permutation.
 __device__ __forceinline__ uint32_t transpose_bits(uint32_t x, int lane)
 {
+    x = __byte_perm(x, __shfl_xor_sync(0xffffffffu, x, 16), (lane & 16) ? 0x3276 : 0x5410);
+    x = __byte_perm(x, __shfl_xor_sync(0xffffffffu, x, 8), (lane & 8) ? 0x3715 : 0x6240);
 #pragma unroll
-    for (int j = 16; j >= 1; j >>= 1)
+    for (int j = 4; j >= 1; j >>= 1)
     {
-        constexpr uint32_t kMasks[5] = {0x55555555u, 0x33333333u, 0x0f0f0f0fu, 0x00ff00ffu,
-                                        0x0000ffffu};
-        const uint32_t lo = kMasks[j == 1 ? 0 : j == 2 ? 1 : j == 4 ? 2 : j == 8 ? 3 : 4];
+        const uint32_t low = j == 4 ? 0x0f0f0f0fu : j == 2 ? 0x33333333u : 0x55555555u;
         const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
-        // A lane with bit j clear keeps its low halves and takes the other's
-        // low halves as its high ones; the other lane does the opposite.
-        const bool up = (lane & j) != 0;
-        const uint32_t keep = up ? ~lo : lo;
-        const uint32_t turned = __funnelshift_l(y, y, up ? 32 - j : j);
+        const uint32_t keep = (lane & j) ? ~low : low;
+        const uint32_t turned = __funnelshift_l(y, y, (lane & j) ? 32 - j : j);
         x = (x & keep) | (turned & ~keep);
     }
     return x;
@@ -3056,6 +3232,7 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
     if (range.y <= range.x && !P.loadClear)
         return;
     const float fx = (float)px + .5f, fy = (float)py + .5f;
+    const float dither = pixel_dither(P, fx, fy);
     Planes s;
     s.color = P.loadClear ? P.clearColorPremulRGBA : (inBounds ? fb[(size_t)py * P.width + px] : 0u);
     s.clip = 0;
@@ -3088,10 +3265,10 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
             const uint4 meta = R.meta;
             const float4 cv = R.cov1;
             TileTri L;
-            L.v0 = make_float4(__uint_as_float(meta.w & 0xffffu), 1.f, 0.f, 0.f);
-            L.v1 = make_float4(1.f, 0.f, 0.f, 1.f);
-            L.v2 = make_float4(0.f, 0.f, W, 0.f);
-            L.v3 = make_float4(0.f, -1.f, 0.f, 0.f);
+            L.v0 = make_float4(1.f, 0.f, 0.f, 1.f);
+            L.v1 = make_float4(0.f, 0.f, 1.f, 0.f);
+            L.v2 = make_float4(0.f, -1.f, 0.f, 0.f);
+            L.v3 = make_float4(W, 0.f, 0.f, __uint_as_float(meta.w & 0xffffu));
             L.v4 = make_uint4(__float_as_uint(cv.z), __float_as_uint(cv.w), meta.x, 0u);
             sh.tris[threadIdx.x] = L;
             m = 0xffffffffu >> (32 - G::kBlocks);
@@ -3105,26 +3282,16 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
                                 tile_edge_origin(e[2], tx, ty, TL)};
             const float dx0 = (float)ox + .5f - T.e0.x, dy0 = (float)oy + .5f - T.e0.y;
             TileTri L;
-            L.v0 = make_float4(__uint_as_float(T.meta.w & 0xffffu), c[0], e[0].z, e[0].w);
-            L.v1 = make_float4(c[1], e[1].z, e[1].w, c[2]);
-            L.v2 = make_float4(e[2].z, e[2].w, T.cov0.x + T.cov0.y * dx0 + T.cov0.z * dy0,
-                               T.cov0.y);
-            L.v3 = make_float4(T.cov0.z, T.cov0.w + T.cov1.x * dx0 + T.cov1.y * dy0, T.cov1.x,
+            L.v0 = make_float4(c[0], e[0].z, e[0].w, c[1]);
+            L.v1 = make_float4(e[1].z, e[1].w, c[2], e[2].z);
+            L.v2 = make_float4(e[2].w, T.cov0.w + T.cov1.x * dx0 + T.cov1.y * dy0, T.cov1.x,
                                T.cov1.y);
+            L.v3 = make_float4(T.cov0.x + T.cov0.y * dx0 + T.cov0.z * dy0, T.cov0.y, T.cov0.z,
+                               __uint_as_float(T.meta.w & 0xffffu));
             L.v4 = make_uint4(__float_as_uint(T.cov1.z), __float_as_uint(T.cov1.w), T.meta.x,
                               entry);
             sh.tris[threadIdx.x] = L;
-            const int4 bb = unpack_bbox(T.meta);
-            const int bx0 = bb.x - ox, bx1 = bb.z - ox, by0 = bb.y - oy, by1 = bb.w - oy;
-#pragma unroll
-            for (int b = 0; b < G::kBlocks; ++b)
-            {
-                const int bx = (b % G::kWarpCols) * 8, by = (b / G::kWarpCols) * 4;
-                const int x0 = max(bx0, bx), x1 = min(bx1, bx + 8);
-                const int y0 = max(by0, by), y1 = min(by1, by + 4);
-                if (x0 < x1 && y0 < y1 && local_rect_overlaps(c, e, x0, x1, y0, y1))
-                    m |= 1u << b;
-            }
+            m = blocks_overlapped<TL>(c, e, unpack_bbox(T.meta), ox, oy);
         }
         // Per block, the staged triangles that may cover it.
 #pragma unroll
@@ -3154,19 +3321,35 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
             const typename G::Index* const list = sh.list[warp] + g;
             const uint32_t cnt = min(32u, n - g);
             uint32_t cover = 0, path = 0;
+            bool fill = true, special = false;
             if (lane < cnt)
             {
                 const TileTri& T = sh.tris[list[lane]];
-                path = __float_as_uint(T.v0.x);
-                cover = block_coverage(T, (float)qx, (float)qy);
+                const float4 v2 = T.v2;
+                path = __float_as_uint(T.v3.w);
+                if (cnt > kFewTriangles)
+                    cover = block_coverage(T.v0, T.v1, v2.x, (float)qx, (float)qy);
+                fill = v2.y < 0.f && v2.z == 0.f && v2.w == 0.f;
+                if (kFeather)
+                    special = ((T.v4.z >> 16) &
+                               (FEATURE_IMAGE_MESH | FEATURE_ATLAS_BLIT | SF_FEATHER)) != 0;
             }
+            // Triangles that are not plain fills (a constant negative covy),
+            // and those that take the general fragment below.
+            const uint32_t strokes = __ballot_sync(0xffffffffu, !fill);
+            const uint32_t specials = kFeather ? __ballot_sync(0xffffffffu, special) : 0u;
             uint32_t before = __shfl_up_sync(0xffffffffu, path, 1);
             if (lane == 0)
                 before = streamPath;
             uint32_t moves = __ballot_sync(0xffffffffu, lane < cnt && path != before);
             streamPath = __shfl_sync(0xffffffffu, path, cnt - 1);
             // One lane per pixel: the triangles that cover it.
-            uint32_t hits = transpose_bits(cover, lane);
+            uint32_t hits = 0;
+            if (cnt > kFewTriangles)
+                hits = transpose_bits(cover, lane);
+            else
+                for (uint32_t i = 0; i < cnt; ++i)
+                    hits |= (pixel_inside(sh.tris[list[i]], lx, ly) ? 1u : 0u) << i;
             if (!inBounds)
                 hits = 0;
             uint32_t from = 0;
@@ -3175,83 +3358,116 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
                 // The run [from, to) of one path. A path's triangles are
                 // contiguous in primitive order, so when the stream moves to
                 // another path every pixel still holding the previous path's
-                // coverage has seen all of it: resolve them together.
+                // coverage has seen all of it: resolve them together. (Inlined
+                // here and at the tile's end: out of line it cost 8% of the 20
+                // plain canvases' frame time, and one shared site 1%.)
                 if ((moves >> from) & 1u)
                 {
                     if (pendMeta)
                     {
                         s = resolve_path<kFeather>(P, s, count, pendMeta, pendPaintX, pendPaintY,
-                                                   oneFragment, fx, fy);
+                                                   oneFragment, fx, fy, dither);
                         pendMeta = 0;
                     }
                     moves &= moves - 1; // the lowest set bit is `from`
                 }
                 const uint32_t to = moves ? (uint32_t)__ffs(moves) - 1u : cnt;
-                uint32_t h = hits & (to < 32 ? (1u << to) - 1u : 0xffffffffu);
-                hits &= ~h;
+                const uint32_t run = (to < 32 ? (1u << to) - 1u : 0xffffffffu) & ~((1u << from) - 1u);
+                uint32_t h = hits & run;
+                const uint32_t runPath = __shfl_sync(0xffffffffu, path, from);
                 from = to;
-                while (h)
+                if (kFeather && (specials & run))
                 {
-                    const TileTri& T = sh.tris[list[__ffs(h) - 1]];
-                    h &= h - 1;
-                    const float4 v2 = T.v2, v3 = T.v3;
-                    const float covx = __fmaf_rn(v2.w, lx, __fmaf_rn(v3.x, ly, v2.z));
-                    const float covy = __fmaf_rn(v3.z, lx, __fmaf_rn(v3.w, ly, v3.y));
-                    const uint32_t vPathID = __float_as_uint(T.v0.x);
-                    if (kFeather && ((T.v4.z >> 16) & (FEATURE_IMAGE_MESH | FEATURE_ATLAS_BLIT)))
+                    while (h)
                     {
-                        // An image-mesh triangle or a feather-atlas blit: the
-                        // pending path is complete here; it writes its colour
-                        // at once and leaves the coverage plane (key and
-                        // count) to whichever path owns it.
-                        if (pendMeta)
+                        const TileTri& T = sh.tris[list[__ffs(h) - 1]];
+                        h &= h - 1;
+                        const float4 v2 = T.v2, v3 = T.v3;
+                        const uint4 v4 = T.v4;
+                        const float covx = __fmaf_rn(v3.y, lx, __fmaf_rn(v3.z, ly, v3.x));
+                        const float covy = __fmaf_rn(v2.z, lx, __fmaf_rn(v2.w, ly, v2.y));
+                        const uint32_t features = v4.z >> 16;
+                        if (features & (FEATURE_IMAGE_MESH | FEATURE_ATLAS_BLIT))
                         {
-                            s = resolve_path<kFeather>(P, s, count, pendMeta, pendPaintX,
-                                                       pendPaintY, oneFragment, fx, fy);
-                            pendMeta = 0;
+                            // An image-mesh triangle or a feather-atlas blit:
+                            // the pending path is complete here; it writes its
+                            // colour at once and leaves the coverage plane
+                            // (key and count) to whichever path owns it.
+                            if (pendMeta)
+                            {
+                                s = resolve_path_call(P, s, count, pendMeta, pendPaintX, pendPaintY,
+                                                      oneFragment, fx, fy, dither);
+                                pendMeta = 0;
+                            }
+                            s.color = (features & FEATURE_IMAGE_MESH)
+                                          ? resolve_mesh(P, s.color, s.clip, v4.z, v4.x, v4.y,
+                                                         B.featherPlanes + 2 * (size_t)v4.w, fx, fy,
+                                                         dither)
+                                          : resolve_blit(P, s.color, s.clip, v4.z, v4.x, v4.y, covx,
+                                                         covy, fx, fy, dither);
+                            continue;
                         }
-                        const uint4 v4 = T.v4;
-                        s.color = ((v4.z >> 16) & FEATURE_IMAGE_MESH)
-                                      ? resolve_mesh(P, s.color, s.clip, v4.z, v4.x, v4.y,
-                                                     B.featherPlanes + 2 * (size_t)v4.w, fx, fy)
-                                      : resolve_blit(P, s.color, s.clip, v4.z, v4.x, v4.y, covx,
-                                                     covy, fx, fy);
-                        continue;
-                    }
-                    if (key != vPathID)
-                    {
-                        // The path's first fragment here. (Nothing is pending:
-                        // the pending path is the stream's, whose key is this.)
-                        const uint4 v4 = T.v4;
-                        pendMeta = v4.z;
-                        pendPaintX = v4.x;
-                        pendPaintY = v4.y;
-                        oneFragment = true;
-                        key = vPathID;
-                        count = 0.f;
-                    }
-                    else
-                    {
-                        oneFragment = false;
-                        if (!pendMeta) // the key's path came back after a resolve
+                        oneFragment = key != runPath;
+                        if (key != runPath)
+                            count = 0.f;
+                        key = runPath;
+                        if (!pendMeta)
                         {
-                            const uint4 v4 = T.v4;
                             pendMeta = v4.z;
                             pendPaintX = v4.x;
                             pendPaintY = v4.y;
                         }
+                        // A feathered fragment is marked by a coverage below
+                        // the feather threshold.
+                        const bool stroke = covy >= 0.f;
+                        float frag = stroke ? fminf(covx, covy) : covx;
+                        if ((stroke ? covx : covy) < kFeatherCoverageThreshold &&
+                            ((pendMeta >> 16) & SF_FEATHER))
+                            frag = feathered_fragment(B.featherPlanes, v4.w, fx, fy, covx, covy);
+                        count = h2f(f2h(stroke ? fmaxf(frag, count) : count + frag));
                     }
-                    // Strokes (covy >= 0) keep the maximum coverage, fills add
-                    // (find_stroke_coverage / find_fill_coverage,
-                    // draw_path.vert:501-519); feathered ones are marked by a
-                    // coverage below the feather threshold.
-                    const bool stroke = covy >= 0.f;
-                    float frag = stroke ? fminf(covx, covy) : covx;
-                    // (pendMeta is this triangle's pathAndFeatures here.)
-                    if (kFeather && (stroke ? covx : covy) < kFeatherCoverageThreshold &&
-                        ((pendMeta >> 16) & SF_FEATHER))
-                        frag = feathered_fragment(B.featherPlanes, T.v4.w, fx, fy, covx, covy);
-                    count = h2f(f2h(stroke ? fmaxf(frag, count) : count + frag)); // fp16 plane
+                }
+                else if (h)
+                {
+                    // The path's first fragment here starts its coverage; its
+                    // paint is the path's, from any of its triangles. (Nothing
+                    // else is pending: the pending path is the stream's.)
+                    oneFragment = key != runPath && (h & (h - 1)) == 0;
+                    if (key != runPath)
+                        count = 0.f;
+                    key = runPath;
+                    if (!pendMeta)
+                    {
+                        const uint4 v4 = sh.tris[list[__ffs(h) - 1]].v4;
+                        pendMeta = v4.z;
+                        pendPaintX = v4.x;
+                        pendPaintY = v4.y;
+                    }
+                    // Fills add their coverage, strokes (covy >= 0) keep the
+                    // maximum (find_fill_coverage / find_stroke_coverage,
+                    // draw_path.vert:501-519); the plane stores fp16.
+                    if (!(strokes & run))
+                    {
+                        do
+                        {
+                            const float4 v3 = sh.tris[list[__ffs(h) - 1]].v3;
+                            h &= h - 1;
+                            count = h2f(f2h(count + __fmaf_rn(v3.y, lx, __fmaf_rn(v3.z, ly, v3.x))));
+                        } while (h);
+                    }
+                    else
+                    {
+                        do
+                        {
+                            const TileTri& T = sh.tris[list[__ffs(h) - 1]];
+                            h &= h - 1;
+                            const float4 v2 = T.v2, v3 = T.v3;
+                            const float covx = __fmaf_rn(v3.y, lx, __fmaf_rn(v3.z, ly, v3.x));
+                            const float covy = __fmaf_rn(v2.z, lx, __fmaf_rn(v2.w, ly, v2.y));
+                            count = h2f(f2h(covy >= 0.f ? fmaxf(fminf(covx, covy), count)
+                                                        : count + covx));
+                        } while (h);
+                    }
                 }
                 __syncwarp();
             }
@@ -3260,7 +3476,7 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
     }
     if (pendMeta)
         s = resolve_path<kFeather>(P, s, count, pendMeta, pendPaintX, pendPaintY, oneFragment, fx,
-                                   fy);
+                                   fy, dither);
     if (inBounds)
         fb[(size_t)py * P.width + px] = s.color;
 }
@@ -3268,7 +3484,7 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
 // The raster kernels, each without and with the feather paths (the host
 // launches the feather variant only for batches with ENABLE_FEATHER draws).
 #define RIVE_RASTER_KERNELS(NAME, FEATHER)                                                        \
-    __global__ void __launch_bounds__(256, RIVE_RASTER_MIN_BLOCKS) NAME(                           \
+    __global__ void __launch_bounds__(256, RIVE_RASTER_MIN_BLOCKS(FEATHER)) NAME(                           \
         BatchTables B, const TriRecord* __restrict__ tris,                                        \
         const uint32_t* __restrict__ sortedSlots, const uint2* __restrict__ ranges)               \
     {                                                                                             \
@@ -3285,7 +3501,7 @@ RIVE_RASTER_KERNELS(raster_tile_feather_kernel, true)
 // first, so the longest tiles start first and the last wave has no straggler
 // behind it. The cursor starts at zero on every launch.
 #define RIVE_RASTER_QUEUE_KERNELS(NAME, FEATHER)                                                  \
-    __global__ void __launch_bounds__(256, RIVE_RASTER_MIN_BLOCKS) NAME(                           \
+    __global__ void __launch_bounds__(256, RIVE_RASTER_MIN_BLOCKS(FEATHER)) NAME(                           \
         BatchTables B, const TriRecord* __restrict__ tris,                                        \
         const uint32_t* __restrict__ sortedSlots, const uint2* __restrict__ ranges,               \
         const uint32_t* __restrict__ order, uint32_t* __restrict__ cursor, uint32_t tiles)        \
