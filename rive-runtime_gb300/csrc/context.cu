@@ -56,7 +56,8 @@ __global__ void center_setup_kernel(BatchTables B,
                                     TriRecord* tris,
                                     uint32_t* tileCounts,
                                     uint8_t* tileMasks);
-__global__ void scene_uniforms_kernel(FlushParams* scenes, uint32_t sceneCount);
+__global__ void scene_uniforms_kernel(FlushParams* scenes, uint32_t sceneCount, uint32_t* wide);
+__global__ void wide_count_kernel(BatchTables B, const TriRecord* tris, uint32_t* tileCounts);
 __global__ void bin_fill_kernel(const uint32_t* pairTotal,
                                 uint32_t capacity,
                                 uint32_t sentinel,
@@ -71,7 +72,8 @@ __global__ void bin_scatter_kernel(uint32_t slotCount,
                                    uint32_t capacity,
                                    uint32_t* error,
                                    uint32_t* keys,
-                                   uint32_t* vals);
+                                   uint32_t* vals,
+                                   WideScatter wide);
 __global__ void tile_ranges_kernel(uint32_t pairCount,
                                    uint32_t tileCount,
                                    const uint32_t* keys,
@@ -91,7 +93,8 @@ __global__ void bin_scatter16_kernel(uint32_t slotCount,
                                      uint32_t capacity,
                                      uint32_t* error,
                                      uint16_t* keys,
-                                     uint32_t* vals);
+                                     uint32_t* vals,
+                                     WideScatter wide);
 __global__ void tile_ranges16_kernel(uint32_t pairCount,
                                      uint32_t tileCount,
                                      const uint16_t* keys,
@@ -298,7 +301,7 @@ struct rive_cuda_context
     RecordRing rings[RIVE_CUDA_BUFFER_KIND_COUNT];
     DeviceBuffer tess, grad;
     uint32_t tessWidth = 0, tessHeight = 0, gradWidth = 0, gradHeight = 0;
-    DeviceBuffer tris, tileCounts, tileMasks, offsets, featherPlanes;
+    DeviceBuffer tris, tileCounts, tileMasks, offsets, featherPlanes, wide;
     DeviceBuffer keys, vals, keysAlt, valsAlt, sortTemp, scanTemp, ranges;
     DeviceBuffer dTables;  // batch tables (device)
     // Pinned staging of the tables, a ring of three, so the host writes the
@@ -362,7 +365,7 @@ struct rive_cuda_graph
     DeviceBuffer tables, tess, grad, tris, counts, masks, offsets, keys, vals, keysAlt, valsAlt,
         scanTemp, sortTemp, ranges, error, featherPlanes, pathGrids, gridWinding, gridEdge,
         gridCounters, queueKeys, queueVals, queueKeysAlt, queueValsAlt, queueTemp, queueCursor,
-        atlas, pathImage;
+        atlas, pathImage, wide;
     cudaStream_t stream = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -687,6 +690,10 @@ struct BatchLayout
     // then take fanStride slots (their 24 triangles and a winding slot).
     bool winding = false;
     uint32_t fanStride = kPatchTriangleCount;
+    // Some scene has enough tiles for a wide triangle (BatchTables::wide).
+    bool wide = false;
+    uint32_t wideCap() const { return wide ? std::min(slots, kWideCapacity) : 0u; }
+    size_t wideBytes() const { return wide ? 4 + (size_t)wideCap() * 4 * (1 + kWideStrips) : 0; }
     uint64_t tessRows = 0, gradRows = 0;
     std::vector<uint64_t> tessRow0, gradRow0;
     // Table blob offsets.
@@ -756,8 +763,10 @@ int plan_batch(rive_cuda_context* ctx, const FlushInput* in, uint32_t n, BatchLa
         L.gradRow0[i] = L.gradRows;
         L.tessRows += std::max(d->tess_data_height, 1u);
         L.gradRows += std::max(d->grad_data_height, 1u);
-        tiles += (uint64_t)((d->render_target_width + ts - 1) / ts) *
-                 ((d->render_target_height + ts - 1) / ts);
+        const uint64_t sceneTiles = (uint64_t)((d->render_target_width + ts - 1) / ts) *
+                                    ((d->render_target_height + ts - 1) / ts);
+        tiles += sceneTiles;
+        L.wide = L.wide || sceneTiles > kWideTiles;
         gradSpans += d->grad_span_count;
         tessSpans += d->tess_span_count;
         paths += d->path_count;
@@ -771,8 +780,10 @@ int plan_batch(rive_cuda_context* ctx, const FlushInput* in, uint32_t n, BatchLa
         L.atlasScene[i] = n + L.atlasScenes++;
         L.atlasTexel0[i] = L.atlasTexels;
         L.atlasTexels += (uint64_t)d->atlas_content_width * d->atlas_content_height;
-        tiles += (uint64_t)((d->atlas_content_width + ts - 1) / ts) *
-                 ((d->atlas_content_height + ts - 1) / ts);
+        const uint64_t sceneTiles = (uint64_t)((d->atlas_content_width + ts - 1) / ts) *
+                                    ((d->atlas_content_height + ts - 1) / ts);
+        tiles += sceneTiles;
+        L.wide = L.wide || sceneTiles > kWideTiles;
         L.feather = true;
         for (uint32_t b = 0; b < atlas_batch_count(d); ++b)
         {
@@ -794,6 +805,7 @@ int plan_batch(rive_cuda_context* ctx, const FlushInput* in, uint32_t n, BatchLa
     {
         L.fanStride = kPatchTriangleCount + 1;
         slots += items[0]; // one winding slot per midpoint-fan patch
+        L.wide = false;    // the winding binner walks its triangles in place
     }
     if (slots > 0xffffffffull || tiles >= 0x7fffffffull || gradSpans > 0x7fffffffull ||
         tessSpans * 32 > 0xffffffffull || paths > 0x7fffffffull)
@@ -863,6 +875,7 @@ struct Scratch
     // null; a scratch word for speculative passes, whose overflow is
     // handled by re-running the back half).
     uint32_t* binError = nullptr;
+    uint32_t* wide = nullptr;        // wide triangles (BatchLayout::wide)
     float4* featherPlanes = nullptr; // 2 per slot, only with center-AA patches
     uint16_t* atlas = nullptr;       // the batch's feather atlases, fp16 texels
     uint32_t* pathImage = nullptr;   // per path of the batch: its image slot
@@ -1091,6 +1104,9 @@ BatchTables write_tables(rive_cuda_context* ctx,
     B.featherPlanes = S.featherPlanes;
     B.meshes = L.meshes ? (const MeshDesc*)(dT + L.oMeshes) : nullptr;
     B.fanSlotStride = L.fanStride;
+    B.wide = L.wide ? S.wide : nullptr;
+    B.wideCap = L.wideCap();
+    B.wideStrips = L.wide ? S.wide + 1 + B.wideCap : nullptr;
     B.pathBase = (const uint32_t*)(dT + L.oPathBase);
     if (L.winding)
     {
@@ -1115,7 +1131,7 @@ int enqueue_front(rive_cuda_context* ctx,
                   cudaStream_t stream)
 {
     scene_uniforms_kernel<<<(L.scenes() + 127) / 128, 128, 0, stream>>>(
-        const_cast<FlushParams*>(B.scenes), L.scenes());
+        const_cast<FlushParams*>(B.scenes), L.scenes(), B.wide);
     // Texels no span covers are never sampled; zero them so the gradient
     // texture is deterministic.
     CK(cudaMemsetAsync(S.grad, 0, L.gradBytes(), stream));
@@ -1172,6 +1188,8 @@ int enqueue_front(rive_cuda_context* ctx,
                                                                                    S.counts, S.masks);
             path_winding_kernel<<<(L.paths + 7) / 8, 256, 0, stream>>>(B, S.counts);
         }
+        if (L.wide)
+            wide_count_kernel<<<kWideBlocks, 256, 0, stream>>>(B, S.tris, S.counts);
         stage_end(ctx, stream);
         stage_begin(ctx, RIVE_CUDA_STAGE_BIN, stream);
         size_t tempBytes = S.scanTempBytes;
@@ -1317,15 +1335,24 @@ int enqueue_back(rive_cuda_context* ctx,
     if (entries && L.slots)
     {
         stage_begin(ctx, RIVE_CUDA_STAGE_BIN, stream);
+        WideScatter wide;
+        if (L.wide)
+        {
+            wide.list = B.wide;
+            wide.strips = B.wideStrips;
+            wide.cap = B.wideCap;
+            wide.blocks = kWideBlocks;
+        }
+        const uint32_t binBlocks = wide.blocks + (L.slots + 255) / 256;
         if (S.keys16)
         {
             uint16_t* keys = (uint16_t*)S.keys;
             if (padded)
                 bin_fill16_kernel<<<(entries + 255) / 256, 256, 0, stream>>>(
                     S.offsets + L.slots, entries, L.tiles, keys);
-            bin_scatter16_kernel<<<(L.slots + 255) / 256, 256, 0, stream>>>(
+            bin_scatter16_kernel<<<binBlocks, 256, 0, stream>>>(
                 L.slots, L.tileLog2, B.sceneTiles, S.tris, S.counts, S.masks, S.offsets, entries,
-                binError, keys, S.vals);
+                binError, keys, S.vals, wide);
         }
         else
         {
@@ -1338,9 +1365,9 @@ int enqueue_back(rive_cuda_context* ctx,
                     B, S.tris, S.counts, S.masks, S.offsets, L.slots, entries, binError, keys,
                     S.vals);
             else
-                bin_scatter_kernel<<<(L.slots + 255) / 256, 256, 0, stream>>>(
+                bin_scatter_kernel<<<binBlocks, 256, 0, stream>>>(
                     L.slots, L.tileLog2, B.sceneTiles, S.tris, S.counts, S.masks, S.offsets, entries,
-                    binError, keys, S.vals);
+                    binError, keys, S.vals, wide);
         }
         stage_end(ctx, stream);
         cub::DoubleBuffer<uint32_t> v(S.vals, S.valsAlt);
@@ -1547,6 +1574,8 @@ int run_batch_body(rive_cuda_context* ctx,
     CK(ctx->tileCounts.reserve((size_t)std::max(L.slots, 1u) * 4));
     CK(ctx->tileMasks.reserve((size_t)std::max(L.slots, 1u)));
     CK(ctx->offsets.reserve((size_t)L.slots * 4 + 4));
+    if (L.wide)
+        CK(ctx->wide.reserve(L.wideBytes()));
     if (L.planes())
         CK(ctx->featherPlanes.reserve((size_t)L.slots * 2 * sizeof(float4)));
     if (L.atlasTexels)
@@ -1589,6 +1618,7 @@ int run_batch_body(rive_cuda_context* ctx,
     S.tess = (uint4*)ctx->tess.ptr;
     S.grad = (uchar4*)ctx->grad.ptr;
     S.tris = (TriRecord*)ctx->tris.ptr;
+    S.wide = L.wide ? (uint32_t*)ctx->wide.ptr : nullptr;
     S.featherPlanes = L.planes() ? (float4*)ctx->featherPlanes.ptr : nullptr;
     S.atlas = L.atlasTexels ? (uint16_t*)ctx->atlas.ptr : nullptr;
     S.pathImage = L.imageSlots ? (uint32_t*)ctx->pathImage.ptr : nullptr;
@@ -1665,6 +1695,7 @@ int run_batch_body(rive_cuda_context* ctx,
         ctx->stats.winding_entries = 0;
         ctx->stats.tiles = L.tiles;
         ctx->stats.kernel_launches = 1 + (L.gradSpans ? 1 : 0) + (L.tessSpans ? 1 : 0) + 1 + 5 +
+                                     (L.wide ? 1 : 0) +
                                      1 + (L.tiles > L.mainTiles ? 1 : 0);
         return RIVE_CUDA_OK;
     }
@@ -1702,7 +1733,7 @@ int run_batch_body(rive_cuda_context* ctx,
     ctx->stats.winding_entries = windingEntries;
     ctx->stats.tiles = L.tiles;
     ctx->stats.kernel_launches = 1 + (L.gradSpans ? 1 : 0) + (L.tessSpans ? 1 : 0) +
-                                 (L.slots ? 1 : 0) + (pairs ? 3 : 0) + 1 +
+                                 (L.slots ? 1 + (L.wide ? 1 : 0) : 0) + (pairs ? 3 : 0) + 1 +
                                  (L.tiles > L.mainTiles ? 1 : 0) +
                                  (L.winding ? 3 + (L.tessSpans ? 1 : 0) + 1 : 0);
     return RIVE_CUDA_OK;
@@ -1842,7 +1873,7 @@ void rive_cuda_context_destroy(rive_cuda_context* ctx)
         }
     }
     for (DeviceBuffer* b : {&ctx->tess, &ctx->grad, &ctx->tris, &ctx->tileCounts, &ctx->tileMasks,
-                            &ctx->offsets, &ctx->featherPlanes,
+                            &ctx->offsets, &ctx->featherPlanes, &ctx->wide,
                             &ctx->keys, &ctx->vals, &ctx->keysAlt, &ctx->valsAlt,
                             &ctx->sortTemp, &ctx->scanTemp, &ctx->ranges, &ctx->dTables,
                             &ctx->pathGrids, &ctx->gridWinding, &ctx->gridEdge,
@@ -2218,7 +2249,7 @@ void graph_free(rive_cuda_graph* g)
                             &g->sortTemp, &g->ranges, &g->error, &g->featherPlanes,
                             &g->pathGrids, &g->gridWinding, &g->gridEdge, &g->gridCounters,
                             &g->queueKeys, &g->queueVals, &g->queueKeysAlt, &g->queueValsAlt,
-                            &g->queueTemp, &g->queueCursor, &g->atlas, &g->pathImage})
+                            &g->queueTemp, &g->queueCursor, &g->atlas, &g->pathImage, &g->wide})
         b->release();
     if (g->hError)
         cudaFreeHost(g->hError);
@@ -2246,6 +2277,8 @@ int graph_build(rive_cuda_context* ctx,
     CK(g->counts.reserve((size_t)std::max(L.slots, 1u) * 4));
     CK(g->masks.reserve((size_t)std::max(L.slots, 1u)));
     CK(g->offsets.reserve((size_t)L.slots * 4 + 4));
+    if (L.wide)
+        CK(g->wide.reserve(L.wideBytes()));
     if (L.planes())
         CK(g->featherPlanes.reserve((size_t)L.slots * 2 * sizeof(float4)));
     if (L.atlasTexels)
@@ -2273,6 +2306,7 @@ int graph_build(rive_cuda_context* ctx,
     S.tess = (uint4*)g->tess.ptr;
     S.grad = (uchar4*)g->grad.ptr;
     S.tris = (TriRecord*)g->tris.ptr;
+    S.wide = L.wide ? (uint32_t*)g->wide.ptr : nullptr;
     S.featherPlanes = L.planes() ? (float4*)g->featherPlanes.ptr : nullptr;
     S.atlas = L.atlasTexels ? (uint16_t*)g->atlas.ptr : nullptr;
     S.pathImage = L.imageSlots ? (uint32_t*)g->pathImage.ptr : nullptr;
@@ -2391,7 +2425,7 @@ int graph_build(rive_cuda_context* ctx,
     g->stats.bin_entries = g->measured;
     g->stats.tiles = L.tiles;
     g->stats.kernel_launches = 1 + (L.gradSpans ? 1 : 0) + (L.tessSpans ? 1 : 0) +
-                               (L.slots ? 2 : 0) + (capacity ? 4 : 0) + 1;
+                               (L.slots ? 2 + (L.wide ? 1 : 0) : 0) + (capacity ? 4 : 0) + 1;
     return RIVE_CUDA_OK;
 }
 } // namespace

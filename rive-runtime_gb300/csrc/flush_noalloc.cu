@@ -35,7 +35,8 @@ __global__ void outer_setup_kernel(BatchTables B,
                                    TriRecord* tris,
                                    uint32_t* tileCounts,
                                    uint8_t* tileMasks);
-__global__ void scene_uniforms_kernel(FlushParams* scenes, uint32_t sceneCount);
+__global__ void scene_uniforms_kernel(FlushParams* scenes, uint32_t sceneCount, uint32_t* wide);
+__global__ void wide_count_kernel(BatchTables B, const TriRecord* tris, uint32_t* tileCounts);
 __global__ void bin_scatter_kernel(uint32_t slotCount,
                                    int tileLog2,
                                    const uint2* sceneTiles,
@@ -46,7 +47,8 @@ __global__ void bin_scatter_kernel(uint32_t slotCount,
                                    uint32_t capacity,
                                    uint32_t* error,
                                    uint32_t* keys,
-                                   uint32_t* vals);
+                                   uint32_t* vals,
+                                   WideScatter wide);
 __global__ void tile_ranges_kernel(uint32_t pairCount,
                                    uint32_t tileCount,
                                    const uint32_t* keys,
@@ -104,6 +106,9 @@ constexpr size_t kTablesOff = kSortTempOff + kSortTempBytes;
 constexpr size_t kPoolBytes = kTablesOff + kTablesBytes;
 static_assert(kPoolBytes == RIVE_CUDA_NOALLOC_POOL_BYTES,
               "RIVE_CUDA_NOALLOC_POOL_BYTES must match the pool layout");
+
+// Wide triangles kept (list and strips fit the alternate keys' region).
+constexpr uint32_t kWideCap = (uint32_t)(kPairBytes / 4 - 1) / (1 + kWideStrips);
 
 constexpr int kMaxDevices = 64;
 std::mutex gPoolMutex;
@@ -321,7 +326,11 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
     segBase[segCount] = instAcc;
     uint8_t* dTab = pool + kTablesOff;
     CKN(cudaMemcpyAsync(dTab, tab, sizeof(tab), cudaMemcpyHostToDevice, stream));
-    scene_uniforms_kernel<<<1, 32, 0, stream>>>((FlushParams*)(dTab + kTabScenes), 1u);
+    // Wide triangles: their list and strips sit in the alternate keys, which
+    // only the sort uses, after them.
+    uint32_t* const wideList = tiles > (uint32_t)kWideTiles ? (uint32_t*)(pool + kKeysAltOff) : nullptr;
+    scene_uniforms_kernel<<<1, 32, 0, stream>>>((FlushParams*)(dTab + kTabScenes), 1u,
+                                             wideList);
     BatchTables B = {};
     B.scenes = (const FlushParams*)(dTab + kTabScenes);
     B.gradSpanBase = (const uint32_t*)(dTab + kTabPrefix);
@@ -342,6 +351,12 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
     B.totalGradSpans = d->grad_span_count;
     B.totalTessSpans = d->tess_span_count;
     B.totalTiles = tiles;
+    if (wideList)
+    {
+        B.wide = wideList;
+        B.wideCap = kWideCap;
+        B.wideStrips = wideList + 1 + kWideCap;
+    }
 
     // What must start at zero on every call: the error word, the tile
     // ranges, the gradient rows in use and the scan's leading offset.
@@ -368,6 +383,8 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
         (feather ? patch_setup_feather_kernel : patch_setup_kernel)<<<(instAcc + 3) / 4, 128, 0,
                                                                      stream>>>(B, tris, counts,
                                                                                masks);
+        if (wideList)
+            wide_count_kernel<<<kWideBlocks, 256, 0, stream>>>(B, tris, counts);
         size_t tempBytes = 0;
         CKN(cub::DeviceScan::InclusiveSum(nullptr, tempBytes, counts, offs + 1, slots, stream));
         if (tempBytes > kScanTempBytes)
@@ -390,8 +407,17 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
     const uint32_t* sortedSlots = nullptr;
     if (pairs)
     {
-        bin_scatter_kernel<<<(slots + 255) / 256, 256, 0, stream>>>(
-            slots, kTileLog2, B.sceneTiles, tris, counts, masks, offs, pairs, dError, keys, vals);
+        WideScatter wide;
+        if (wideList)
+        {
+            wide.list = B.wide;
+            wide.strips = B.wideStrips;
+            wide.cap = B.wideCap;
+            wide.blocks = kWideBlocks;
+        }
+        bin_scatter_kernel<<<wide.blocks + (slots + 255) / 256, 256, 0, stream>>>(
+            slots, kTileLog2, B.sceneTiles, tris, counts, masks, offs, pairs, dError, keys, vals,
+            wide);
         int endBit = 1;
         while ((1u << endBit) <= tiles)
             ++endBit;

@@ -911,6 +911,20 @@ __device__ __forceinline__ void tile_span(int4 bb, int tileLog2, int& tx0, int& 
 }
 
 constexpr int kLaneTiles = 8;
+// tileMasks value of a triangle set aside in BatchTables::wide (its box holds
+// more than kLaneTiles tiles, so the byte carries no tile mask).
+constexpr uint8_t kWideMask = 1;
+
+// The strip of tiles [lo, hi) that a warp takes of a wide triangle's n tiles;
+// false when the triangle has no such strip.
+__device__ __forceinline__ bool wide_strip(int n, int strip, int& lo, int& hi)
+{
+    const int strips = min((n + kWideStripTiles - 1) / kWideStripTiles, kWideStrips);
+    const int len = (n + strips - 1) / strips;
+    lo = strip * len;
+    hi = min(lo + len, n);
+    return lo < hi;
+}
 
 // Counts the tiles of the warp's triangles: a lane counts its own triangle
 // when its box spans at most kLaneTiles tiles; the whole warp walks larger
@@ -921,6 +935,8 @@ __device__ __forceinline__ void count_tiles(bool has,
                                             int4 bb,
                                             uint32_t* __restrict__ countOut,
                                             uint8_t* __restrict__ maskOut,
+                                            const BatchTables& B,
+                                            uint32_t slot,
                                             const float4 (*warpEdges)[3],
                                             const int4* warpBoxes,
                                             uint32_t* const* warpOuts)
@@ -952,6 +968,20 @@ __device__ __forceinline__ void count_tiles(bool has,
             else
             {
                 big = true;
+                // (Past the capacity the counter is only read: no contention
+                // on batches with hundreds of thousands of such triangles.)
+                if (B.wide && ntx * nty > kWideTiles &&
+                    *(volatile const uint32_t*)B.wide < B.wideCap)
+                {
+                    const uint32_t i = atomicAdd(B.wide, 1u);
+                    if (i < B.wideCap)
+                    {
+                        B.wide[1 + i] = slot; // wide_count_kernel adds up its tiles
+                        *countOut = 0;
+                        big = false;
+                    }
+                }
+                *maskOut = big ? 0 : kWideMask;
             }
         }
         else
@@ -1327,8 +1357,8 @@ __device__ __forceinline__ void patch_setup(const BatchTables& B,
         }
         __syncwarp();
         count_tiles(has && !deferred, B.tileLog2, e, bb, tileCounts + slot0 + t,
-                    tileMasks + slot0 + t, sEdges[w] + pass * 32, sBox[w] + pass * 32,
-                    sOut[w] + pass * 32);
+                    tileMasks + slot0 + t, B, slot0 + t, sEdges[w] + pass * 32,
+                    sBox[w] + pass * 32, sOut[w] + pass * 32);
         if (deferred)
             tileCounts[slot0 + t] = kDeferredCount;
         __syncwarp();
@@ -1565,7 +1595,8 @@ __global__ void __launch_bounds__(256) interior_setup_kernel(BatchTables B,
         sOut[w][lane] = tileCounts + slot;
     }
     __syncwarp();
-    count_tiles(has, B.tileLog2, e, bb, tileCounts + slot, tileMasks + slot, sEdges[w], sBox[w], sOut[w]);
+    count_tiles(has, B.tileLog2, e, bb, tileCounts + slot, tileMasks + slot, B, slot, sEdges[w],
+                sBox[w], sOut[w]);
 }
 
 // ---- Winding grids: the per-path passes ------------------------------------
@@ -1848,14 +1879,50 @@ __global__ void __launch_bounds__(256) fan_filter_kernel(BatchTables B,
     }
 }
 
+// The tiles of the triangles set aside as wide: a warp per strip counts its
+// own, a triangle's total is their sum. (Latency bound: a strip is 4 to 32
+// rounds of one tile test per lane.)
+__global__ void __launch_bounds__(256) wide_count_kernel(BatchTables B,
+                                                         const TriRecord* __restrict__ tris,
+                                                         uint32_t* __restrict__ tileCounts)
+{
+    const uint32_t items = min(*B.wide, B.wideCap) * kWideStrips;
+    const int lane = threadIdx.x & 31;
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < items;
+         i += (gridDim.x * blockDim.x) >> 5)
+    {
+        const uint32_t slot = B.wide[1 + i / kWideStrips];
+        const TriRecord* T = tris + slot;
+        const int4 bb = unpack_bbox(T->meta);
+        int tx0, ty0, ntx, nty, lo, hi;
+        tile_span(bb, B.tileLog2, tx0, ty0, ntx, nty);
+        if (!wide_strip(ntx * nty, (int)(i % kWideStrips), lo, hi))
+            continue;
+        const float4 e[3] = {T->e0, T->e1, T->e2};
+        uint32_t count = 0;
+        for (int t = lo + lane; t < hi; t += 32)
+            count += tile_overlaps(e, bb, tx0 + t % ntx, ty0 + t / ntx, B.tileLog2) ? 1u : 0u;
+        count = __reduce_add_sync(0xffffffffu, count);
+        if (lane == 0)
+        {
+            B.wideStrips[i] = count;
+            atomicAdd(tileCounts + slot, count);
+        }
+    }
+}
+
 // FlushUniforms fields the passes use (gpu.hpp:1466-1537: pathIDGranularity
 // at byte 72, ditherScale at 88, ditherBias at 92), read on the device so no
 // pass waits for the host. One thread per flush of the batch.
-__global__ void scene_uniforms_kernel(FlushParams* __restrict__ scenes, uint32_t sceneCount)
+// The first of them also empties the list of wide triangles, if there is one.
+__global__ void scene_uniforms_kernel(FlushParams* __restrict__ scenes, uint32_t sceneCount,
+                                      uint32_t* __restrict__ wide)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= sceneCount)
         return;
+    if (i == 0 && wide)
+        *wide = 0;
     const uint8_t* u = scenes[i].uniforms;
     const uint32_t granularity = *reinterpret_cast<const uint32_t*>(u + 72);
     scenes[i].pathIDGranularity = granularity ? granularity : 1u;
@@ -1900,6 +1967,62 @@ __global__ void bin_fill16_kernel(const uint32_t* __restrict__ pairTotal,
 // winding records), a deferred fan triangle's large box keeps its path's
 // edge tiles only, and an anchor winding slot writes one entry per interior
 // tile of its path with a nonzero winding.
+// The wide triangles' part of the binner: the first `blocks` CTAs of its grid
+// (0: no list) write their pairs, a warp per strip, each after the entries of
+// the triangle's strips before it.
+template <typename K>
+__device__ __forceinline__ void bin_scatter_wide(int tileLog2,
+                                                 const uint2* __restrict__ sceneTiles,
+                                                 const TriRecord* __restrict__ tris,
+                                                 const uint32_t* __restrict__ offsets,
+                                                 uint32_t capacity,
+                                                 uint32_t* __restrict__ error,
+                                                 K* __restrict__ keys,
+                                                 uint32_t* __restrict__ vals,
+                                                 const WideScatter& wide)
+{
+    const uint32_t items = min(*wide.list, wide.cap) * kWideStrips;
+    const int lane = threadIdx.x & 31;
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < items;
+         i += (wide.blocks * blockDim.x) >> 5)
+    {
+        const uint32_t slot = wide.list[1 + i / kWideStrips], strip = i % kWideStrips;
+        const TriRecord* T = tris + slot;
+        const uint4 meta = T->meta;
+        const int4 bb = unpack_bbox(meta);
+        int tx0, ty0, ntx, nty, lo, hi;
+        tile_span(bb, tileLog2, tx0, ty0, ntx, nty);
+        if (!wide_strip(ntx * nty, (int)strip, lo, hi))
+            continue;
+        uint32_t before = 0;
+        for (uint32_t k = lane; k < strip; k += 32)
+            before += wide.strips[i - strip + k];
+        uint32_t o = offsets[slot] + __reduce_add_sync(0xffffffffu, before);
+        const uint2 st = sceneTiles[meta.w >> 16];
+        const float4 e[3] = {T->e0, T->e1, T->e2};
+        for (int base = lo; base < hi; base += 32)
+        {
+            const int t = base + lane, tx = tx0 + t % ntx, ty = ty0 + t / ntx;
+            const bool hit = t < hi && tile_overlaps(e, bb, tx, ty, tileLog2);
+            const uint32_t mask = __ballot_sync(0xffffffffu, hit);
+            if (hit)
+            {
+                const uint32_t pos = o + __popc(mask & ((1u << lane) - 1u));
+                if (pos < capacity)
+                {
+                    keys[pos] = (K)(st.x + (uint32_t)ty * st.y + (uint32_t)tx);
+                    vals[pos] = slot;
+                }
+                else
+                {
+                    atomicOr(error, ERR_BIN_OVERFLOW);
+                }
+            }
+            o += __popc(mask);
+        }
+    }
+}
+
 template <bool kWinding, typename K>
 __device__ __forceinline__ void bin_scatter(const BatchTables* __restrict__ Bw,
                                             uint32_t slotCount,
@@ -1912,11 +2035,16 @@ __device__ __forceinline__ void bin_scatter(const BatchTables* __restrict__ Bw,
                                             uint32_t capacity,
                                             uint32_t* __restrict__ error,
                                             K* __restrict__ keys,
-                                            uint32_t* __restrict__ vals)
+                                            uint32_t* __restrict__ vals,
+                                            const WideScatter& wide)
 {
-    constexpr int kLaneTiles = 8;
-    const uint32_t warpId = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
+    if (blockIdx.x < wide.blocks)
+    {
+        bin_scatter_wide(tileLog2, sceneTiles, tris, offsets, capacity, error, keys, vals, wide);
+        return;
+    }
+    const uint32_t warpId = ((blockIdx.x - wide.blocks) * blockDim.x + threadIdx.x) >> 5;
     const uint32_t first = warpId * 32;
     if (first >= slotCount)
         return;
@@ -1958,7 +2086,7 @@ __device__ __forceinline__ void bin_scatter(const BatchTables* __restrict__ Bw,
         }
         else
         {
-            isBig = true;
+            isBig = !(wide.blocks && tileMasks[mySlot] == kWideMask);
         }
     }
     uint32_t pending = __ballot_sync(0xffffffffu, isBig);
@@ -2057,10 +2185,11 @@ __global__ void __launch_bounds__(256, RIVE_BIN_MIN_BLOCKS) bin_scatter_kernel(u
                                                           uint32_t capacity,
                                                           uint32_t* __restrict__ error,
                                                           uint32_t* __restrict__ keys,
-                                                          uint32_t* __restrict__ vals)
+                                                          uint32_t* __restrict__ vals,
+                                                          WideScatter wide)
 {
     bin_scatter<false>(nullptr, slotCount, tileLog2, sceneTiles, tris, tileCounts, tileMasks,
-                       offsets, capacity, error, keys, vals);
+                       offsets, capacity, error, keys, vals, wide);
 }
 __global__ void __launch_bounds__(256, RIVE_BIN_MIN_BLOCKS) bin_scatter16_kernel(uint32_t slotCount,
                                                           int tileLog2,
@@ -2072,10 +2201,11 @@ __global__ void __launch_bounds__(256, RIVE_BIN_MIN_BLOCKS) bin_scatter16_kernel
                                                           uint32_t capacity,
                                                           uint32_t* __restrict__ error,
                                                           uint16_t* __restrict__ keys,
-                                                          uint32_t* __restrict__ vals)
+                                                          uint32_t* __restrict__ vals,
+                                                          WideScatter wide)
 {
     bin_scatter<false>(nullptr, slotCount, tileLog2, sceneTiles, tris, tileCounts, tileMasks,
-                       offsets, capacity, error, keys, vals);
+                       offsets, capacity, error, keys, vals, wide);
 }
 
 // The same, for batches that draw interior tiles as winding records.
@@ -2091,7 +2221,7 @@ __global__ void __launch_bounds__(256) bin_scatter_winding_kernel(BatchTables B,
                                                                   uint32_t* __restrict__ vals)
 {
     bin_scatter<true>(&B, slotCount, B.tileLog2, B.sceneTiles, tris, tileCounts, tileMasks,
-                      offsets, capacity, error, keys, vals);
+                      offsets, capacity, error, keys, vals, WideScatter());
 }
 
 // A speculative pass whose scanned bin-entry total exceeds the capacity its

@@ -284,6 +284,22 @@ struct PatchSegment
     uint32_t mesh;
 };
 
+// Triangles with large tile boxes. One warp tests a triangle's tiles 32 at a
+// time; a canvas-wide triangle of a backdrop has 8,000 to 65,000 of them, and a
+// patch of such triangles kept its warp busy for hundreds of microseconds while
+// the rest of the GPU was idle (a 1739x2831 recorded frame: set-up 589 us,
+// binner 550 us). Boxes above kWideTiles tiles are therefore set aside and cut
+// into up to kWideStrips strips of at least kWideStripTiles tiles, a warp each.
+// 1080x1920 UI screen with uploads and read-back: 556 -> 368 us; 16 recorded
+// frames alone: 3.71 -> 2.74 ms. The line lies where the two extra passes
+// stop costing batches whose many such triangles fill the GPU anyway (20 plain
+// canvases 10.57, 10.19 and 10.17 ms with it at 256, 512 and 1024 tiles,
+// 10.15 ms without).
+constexpr int kWideTiles = 1024;
+constexpr int kWideStrips = 64;
+constexpr int kWideStripTiles = 128;
+constexpr uint32_t kWideCapacity = 16384; // triangles kept; more are walked in place
+
 // Set-up work lists: midpoint-fan patches, outer-curve patches, interior
 // triangles, center-AA midpoint-fan patches (items: instances, instances,
 // triangles, instances).
@@ -318,6 +334,13 @@ struct BatchTables
     float4* featherPlanes;
     // Image meshes of the batch (PatchSegment::mesh indexes it).
     const MeshDesc* meshes;
+    // Triangles whose tile box holds more than kWideTiles tiles: wide[0] of
+    // them (at most wideCap are kept), slots from wide[1] on, and per kept
+    // triangle the entries of each of its kWideStrips strips. Null: no such
+    // triangle is set aside (no scene has that many tiles, or winding records).
+    uint32_t* wide;
+    uint32_t* wideStrips;
+    uint32_t wideCap;
     // Interior tiles as winding records (null grids: off). Midpoint-fan
     // patches then take fanSlotStride = 25 slots (24 triangles and the
     // winding slot), otherwise 24.
@@ -329,6 +352,19 @@ struct BatchTables
     uint32_t gridCapacity;     // cells in the pool
     uint32_t* gridCounters;    // [0] cells asked for, [1] winding entries
 };
+
+// The binner's view of BatchTables::wide and how many of its first CTAs write
+// those triangles' pairs (0: no list).
+struct WideScatter
+{
+    const uint32_t* list = nullptr;
+    const uint32_t* strips = nullptr;
+    uint32_t cap = 0;
+    uint32_t blocks = 0;
+};
+// CTAs (256 threads) of the two wide-triangle passes: two per SM's worth, a
+// strip for every warp of 38 triangles.
+constexpr uint32_t kWideBlocks = 304;
 
 // Index j with base[j] <= i < base[j + 1] (empty ranges skipped), n >= 1.
 __device__ __forceinline__ uint32_t find_range(const uint32_t* __restrict__ base, uint32_t n,

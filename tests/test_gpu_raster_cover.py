@@ -13,11 +13,14 @@ import pytest
 from conftest import device_buffers, load_golden, load_package
 
 load_package()
-W, H = 331, 203  # ragged at every tile size
+# Ragged at every tile size. "wide": more than kWideTiles tiles of 8 and of 16
+# pixels, so its largest triangles are binned strip by strip.
+SIZES = {"ties": (331, 203), "slivers": (331, 203), "small": (331, 203), "wide": (701, 475)}
 
 
 def triangles(kind, n, rng):
     """n clockwise (y down) triangles, (n, 3, 2) on the 1/256-pixel grid."""
+    W, H = SIZES[kind]
     if kind == "ties":  # corners on and half-way between pixel centres, axis-aligned edges
         p = (rng.integers(-4, 2 * max(W, H) + 4, (n, 1, 2)) + rng.integers(-50, 50, (n, 3, 2))) / 2.0
         p[::3, 1, 1] = p[::3, 0, 1]
@@ -26,6 +29,9 @@ def triangles(kind, n, rng):
         a = rng.integers(-2000 * 256, 2400 * 256, (n, 1, 2)) / 256.0
         b = rng.integers(-2000 * 256, 2400 * 256, (n, 1, 2)) / 256.0
         p = np.concatenate([a, b, b + rng.integers(-300, 300, (n, 1, 2)) / 256.0], 1)
+    elif kind == "wide":  # most of the canvas, and slivers across it
+        p = rng.integers(-200 * 256, 900 * 256, (n, 3, 2)) / 256.0
+        p[::4, 2] = p[::4, 1] + rng.integers(-900, 900, (len(p[::4]), 2)) / 256.0
     else:  # "small": a few pixels
         p = rng.integers(0, max(W, H) * 256, (n, 1, 2)) + rng.integers(-1400, 1400, (n, 3, 2))
         p = p / 256.0
@@ -39,7 +45,7 @@ def f32(x):
     return np.asarray(x, np.float64).astype(np.float32).astype(np.float64)
 
 
-def expected(tris, tile):
+def expected(tris, tile, W, H):
     """Per pixel the last covering triangle's number + 1, or 0."""
     out = np.zeros((H, W), np.int64)
     for i, p in enumerate(tris):
@@ -75,35 +81,33 @@ def expected(tris, tile):
     return out
 
 
-@pytest.mark.gpu
-@pytest.mark.parametrize("queue", [False, True])
-@pytest.mark.parametrize("tile", [8, 16, 32])
-@pytest.mark.parametrize("kind,n", [("ties", 700), ("slivers", 700), ("small", 3000)])
-def test_covered_pixels_are_exact(kind, n, tile, queue):
-    import torch
-    from rive_runtime_gb300 import rive_cuda
-    if queue and tile != 16:
-        pytest.skip("the work queue takes 16-pixel tiles")
-    tris = triangles(kind, n, np.random.default_rng(7))
+def flush_of(tris, path_ids, W, H):
+    """A capture of one batch of interior triangles, and its device buffers."""
+    n, paths_n = len(tris), int(path_ids.max())
     cap = load_golden("tri_fills_s21")[0]  # for a FlushUniforms record and a descriptor
     f = cap.flushes[0]
-    paths = np.zeros((n + 1, 16), np.float32)
+    paths = np.zeros((paths_n + 1, 16), np.float32)
     paths[1:, 0] = paths[1:, 3] = 1.0
-    ids = np.arange(n + 1, dtype=np.uint32)
-    paints = np.zeros((n + 1, 2), np.uint32)
+    paints = np.zeros((paths_n + 1, 2), np.uint32)
     paints[:, 0] = 1  # solid
-    paints[:, 1] = ids | 0xFF000000
+    paints[:, 1] = np.arange(paths_n + 1, dtype=np.uint32) | 0xFF000000
     verts = np.zeros((n, 3, 3), np.uint32)
     verts[..., :2] = tris.astype(np.float32).view(np.uint32)
-    verts[..., 2] = ids[1:, None] | 0x10000  # weight 1
+    verts[..., 2] = path_ids[:, None].astype(np.uint32) | 0x10000  # weight 1
     cap.buffers = {"flush_uniforms": cap.buffers["flush_uniforms"], "paths": paths.tobytes(),
-                   "paints": paints.tobytes(), "paint_aux": bytes(128 * (n + 1)),
+                   "paints": paints.tobytes(), "paint_aux": bytes(128 * (paths_n + 1)),
                    "triangles": verts.tobytes()}
-    f.desc.update(render_target_width=W, render_target_height=H, ub2=W, ub3=H, path_count=n + 1,
-                  contour_count=0, tess_span_count=0, tess_data_height=0, dither_mode=0,
-                  color_clear_value=0xFF000000, combined_shader_features=0)
+    f.desc.update(render_target_width=W, render_target_height=H, ub2=W, ub3=H,
+                  path_count=paths_n + 1, contour_count=0, tess_span_count=0, tess_data_height=0,
+                  dither_mode=0, color_clear_value=0xFF000000, combined_shader_features=0)
     f.batches = np.array([[3, 3 * n, 0, 0, 16, 0, 3, 0]], np.uint32)
-    bufs, keep = device_buffers(cap)
+    return f, device_buffers(cap)
+
+
+def render(f, bufs, W, H, tile=16, queue=False):
+    """The image as (H, W) path numbers, and the flush's statistics."""
+    import torch
+    from rive_runtime_gb300 import rive_cuda
     ctx = rive_cuda.Context(0)
     ctx.set_raster_config(tile)
     ctx.set_raster_queue(queue)
@@ -111,11 +115,38 @@ def test_covered_pixels_are_exact(kind, n, tile, queue):
     ctx.flush_device(f, bufs, target.data_ptr())
     ctx.sync()
     img = target.cpu().numpy().astype(np.int64)
+    stats = ctx.stats()
     ctx.close()
-    got = img[..., 0] | (img[..., 1] << 8) | (img[..., 2] << 16)
-    want = expected(tris, tile)
+    return img[..., 0] | (img[..., 1] << 8) | (img[..., 2] << 16), stats
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("queue", [False, True])
+@pytest.mark.parametrize("tile", [8, 16, 32])
+@pytest.mark.parametrize("kind,n", [("ties", 700), ("slivers", 700), ("small", 3000), ("wide", 80)])
+def test_covered_pixels_are_exact(kind, n, tile, queue):
+    if queue and tile != 16:
+        pytest.skip("the work queue takes 16-pixel tiles")
+    W, H = SIZES[kind]
+    tris = triangles(kind, n, np.random.default_rng(7))
+    f, (bufs, keep) = flush_of(tris, np.arange(1, n + 1), W, H)
+    got, _ = render(f, bufs, W, H, tile, queue)
+    want = expected(tris, tile, W, H)
     assert (want > 0).mean() > .02
     assert np.array_equal(got, want), np.argwhere(got != want)[:5]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 16383, 16384, 16400])
+def test_wide_triangles_around_the_capacity_of_their_list(n):
+    """Canvas-wide triangles, as many as the binner sets aside (kWideCapacity)
+    and some more, which it walks in place: every one has every tile."""
+    W, H = 16 * 33, 16 * 32
+    tris = np.tile(np.array([[[-10, -10], [3000, -10], [-10, 3000]]], np.float64), (n, 1, 1))
+    f, (bufs, keep) = flush_of(tris, np.full(n, 1), W, H)
+    got, stats = render(f, bufs, W, H)
+    assert stats["bin_entries"] == n * 33 * 32
+    assert (got == 1).all()
 
 
 def test_unorm_float_is_the_correctly_rounded_quotient():
