@@ -3171,6 +3171,9 @@ template <int TL> struct RasterShared
     TileTri tris[G::kChunk];
     uint32_t bits[G::kBlocks][G::kChunk / 32];
     typename G::Index list[G::kBlocks][G::kChunk];
+    // The coverage planes of each warp's current batch: covx and the coverage
+    // key (TileTri::v3), and v2 for triangles that are not plain fills.
+    float4 covx[G::kBlocks][32], covy[G::kBlocks][32];
     FlushParams params;
 };
 
@@ -3341,15 +3344,15 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
     constexpr uint32_t kChunk = G::kChunk;
     static_assert(sizeof(FlushParams) / 4 <= G::kThreads, "one word of FlushParams per thread");
     const uint2 range = ranges[gtile];
-    // The tile's scene: its parameters are staged once for the whole CTA.
+    // The tile's scene: its parameters are staged for the whole CTA (seen after
+    // the first chunk's barrier); what comes before reads them in place.
     const uint32_t scene = find_range(B.tileBase, B.sceneCount, gtile);
-    if (threadIdx.x < sizeof(FlushParams) / 4)
+    const FlushParams& G0 = B.scenes[scene];
+    if (range.y > range.x && threadIdx.x < sizeof(FlushParams) / 4)
         reinterpret_cast<uint32_t*>(&sh.params)[threadIdx.x] =
-            reinterpret_cast<const uint32_t*>(B.scenes + scene)[threadIdx.x];
-    __syncthreads();
+            reinterpret_cast<const uint32_t*>(&G0)[threadIdx.x];
     const FlushParams& P = sh.params;
-    uint32_t* __restrict__ fb = P.fb;
-    const uint32_t tilesX = P.tilesX;
+    const uint32_t tilesX = G0.tilesX;
     const uint32_t tile = gtile - B.tileBase[scene];
     const int tx = (int)(tile % tilesX), ty = (int)(tile / tilesX);
     const int ox = tx * G::T, oy = ty * G::T;
@@ -3358,13 +3361,15 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
     const int lxi = qx + (lane & 7), lyi = qy + (lane >> 3);
     const int px = ox + lxi, py = oy + lyi;
     const float lx = (float)lxi, ly = (float)lyi;
-    const bool inBounds = px < (int)P.width && py < (int)P.height;
-    if (range.y <= range.x && !P.loadClear)
+    const uint32_t width = G0.width, loadClear = G0.loadClear;
+    uint32_t* __restrict__ fb = G0.fb;
+    const bool inBounds = px < (int)width && py < (int)G0.height;
+    if (range.y <= range.x && !loadClear)
         return;
     const float fx = (float)px + .5f, fy = (float)py + .5f;
-    const float dither = pixel_dither(P, fx, fy);
+    const float dither = pixel_dither(G0, fx, fy);
     Planes s;
-    s.color = P.loadClear ? P.clearColorPremulRGBA : (inBounds ? fb[(size_t)py * P.width + px] : 0u);
+    s.color = loadClear ? G0.clearColorPremulRGBA : (inBounds ? fb[(size_t)py * width + px] : 0u);
     s.clip = 0;
     s.scratch = 0;
     uint32_t key = 0;      // coverage plane's path key (fp16 bits of the pathID)
@@ -3423,13 +3428,17 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
             sh.tris[threadIdx.x] = L;
             m = blocks_overlapped<TL>(c, e, unpack_bbox(T.meta), ox, oy);
         }
-        // Per block, the staged triangles that may cover it.
-#pragma unroll
-        for (int b = 0; b < G::kBlocks; ++b)
+        // Per block, the staged triangles that may cover it (nothing to say
+        // for a warp past the chunk's last entry).
+        if (base + warp * 32 < range.y)
         {
-            const uint32_t bits = __ballot_sync(0xffffffffu, (m >> b) & 1u);
-            if (lane == b)
-                sh.bits[b][warp] = bits;
+#pragma unroll
+            for (int b = 0; b < G::kBlocks; ++b)
+            {
+                const uint32_t bits = __ballot_sync(0xffffffffu, (m >> b) & 1u);
+                if (lane == b)
+                    sh.bits[b][warp] = bits;
+            }
         }
         __syncthreads();
         // This warp's triangles of the chunk, in primitive order.
@@ -3455,11 +3464,13 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
             if (lane < cnt)
             {
                 const TileTri& T = sh.tris[list[lane]];
-                const float4 v2 = T.v2;
-                path = __float_as_uint(T.v3.w);
+                const float4 v2 = T.v2, v3 = T.v3;
+                path = __float_as_uint(v3.w);
+                sh.covx[warp][lane] = v3;
                 if (cnt > kFewTriangles)
                     cover = block_coverage(T.v0, T.v1, v2.x, (float)qx, (float)qy);
                 fill = v2.y < 0.f && v2.z == 0.f && v2.w == 0.f;
+                sh.covy[warp][lane] = v2;
                 if (kFeather)
                     special = ((T.v4.z >> 16) &
                                (FEATURE_IMAGE_MESH | FEATURE_ATLAS_BLIT | SF_FEATHER)) != 0;
@@ -3482,16 +3493,17 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
                     hits |= (pixel_inside(sh.tris[list[i]], lx, ly) ? 1u : 0u) << i;
             if (!inBounds)
                 hits = 0;
-            uint32_t from = 0;
-            while (from < cnt)
+            __syncwarp();
+            uint32_t rest = 0xffffffffu >> (32 - cnt);
+            do
             {
-                // The run [from, to) of one path. A path's triangles are
-                // contiguous in primitive order, so when the stream moves to
-                // another path every pixel still holding the previous path's
-                // coverage has seen all of it: resolve them together. (Inlined
-                // here and at the tile's end: out of line it cost 8% of the 20
-                // plain canvases' frame time, and one shared site 1%.)
-                if ((moves >> from) & 1u)
+                // The next run of one path. A path's triangles are contiguous
+                // in primitive order, so when the stream moves to another path
+                // every pixel still holding the previous path's coverage has
+                // seen all of it: resolve them together. (Inlined here and at
+                // the tile's end: out of line it cost 8% of the 20 plain
+                // canvases' frame time, and one shared site 1%.)
+                if (moves & rest & (0u - rest))
                 {
                     if (pendMeta)
                     {
@@ -3499,13 +3511,11 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
                                                    oneFragment, fx, fy, dither);
                         pendMeta = 0;
                     }
-                    moves &= moves - 1; // the lowest set bit is `from`
+                    moves &= moves - 1; // the run's first triangle is the lowest
                 }
-                const uint32_t to = moves ? (uint32_t)__ffs(moves) - 1u : cnt;
-                const uint32_t run = (to < 32 ? (1u << to) - 1u : 0xffffffffu) & ~((1u << from) - 1u);
+                const uint32_t run = rest & ((moves & (0u - moves)) - 1u);
+                rest ^= run;
                 uint32_t h = hits & run;
-                const uint32_t runPath = __shfl_sync(0xffffffffu, path, from);
-                from = to;
                 if (kFeather && (specials & run))
                 {
                     while (h)
@@ -3537,10 +3547,11 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
                                                          covy, fx, fy, dither);
                             continue;
                         }
-                        oneFragment = key != runPath;
-                        if (key != runPath)
+                        const uint32_t path = __float_as_uint(v3.w);
+                        oneFragment = key != path;
+                        if (key != path)
                             count = 0.f;
-                        key = runPath;
+                        key = path;
                         if (!pendMeta)
                         {
                             pendMeta = v4.z;
@@ -3559,19 +3570,25 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
                 }
                 else if (h)
                 {
-                    // The path's first fragment here starts its coverage; its
-                    // paint is the path's, from any of its triangles. (Nothing
-                    // else is pending: the pending path is the stream's.)
-                    oneFragment = key != runPath && (h & (h - 1)) == 0;
-                    if (key != runPath)
-                        count = 0.f;
-                    key = runPath;
+                    // The path's first fragment here starts its coverage and
+                    // carries its paint. (Nothing else is pending: the pending
+                    // path is the stream's.)
+                    const int first = __ffs(h) - 1;
                     if (!pendMeta)
                     {
-                        const uint4 v4 = sh.tris[list[__ffs(h) - 1]].v4;
+                        const uint4 v4 = sh.tris[list[first]].v4;
+                        const uint32_t path = __float_as_uint(sh.covx[warp][first].w);
                         pendMeta = v4.z;
                         pendPaintX = v4.x;
                         pendPaintY = v4.y;
+                        oneFragment = key != path && (h & (h - 1)) == 0;
+                        if (key != path)
+                            count = 0.f;
+                        key = path;
+                    }
+                    else
+                    {
+                        oneFragment = false;
                     }
                     // Fills add their coverage, strokes (covy >= 0) keep the
                     // maximum (find_fill_coverage / find_stroke_coverage,
@@ -3580,7 +3597,7 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
                     {
                         do
                         {
-                            const float4 v3 = sh.tris[list[__ffs(h) - 1]].v3;
+                            const float4 v3 = sh.covx[warp][__ffs(h) - 1];
                             h &= h - 1;
                             count = h2f(f2h(count + __fmaf_rn(v3.y, lx, __fmaf_rn(v3.z, ly, v3.x))));
                         } while (h);
@@ -3589,9 +3606,9 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
                     {
                         do
                         {
-                            const TileTri& T = sh.tris[list[__ffs(h) - 1]];
+                            const int i = __ffs(h) - 1;
                             h &= h - 1;
-                            const float4 v2 = T.v2, v3 = T.v3;
+                            const float4 v3 = sh.covx[warp][i], v2 = sh.covy[warp][i];
                             const float covx = __fmaf_rn(v3.y, lx, __fmaf_rn(v3.z, ly, v3.x));
                             const float covy = __fmaf_rn(v2.z, lx, __fmaf_rn(v2.w, ly, v2.y));
                             count = h2f(f2h(covy >= 0.f ? fmaxf(fminf(covx, covy), count)
@@ -3600,15 +3617,18 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
                     }
                 }
                 __syncwarp();
-            }
+            } while (rest);
         }
-        __syncthreads();
+        // The next chunk overwrites this one. (After the last one warps go on
+        // by themselves.)
+        if (range.y - base > kChunk)
+            __syncthreads();
     }
     if (pendMeta)
         s = resolve_path<kFeather>(P, s, count, pendMeta, pendPaintX, pendPaintY, oneFragment, fx,
                                    fy, dither);
     if (inBounds)
-        fb[(size_t)py * P.width + px] = s.color;
+        fb[(size_t)py * width + px] = s.color;
 }
 
 // The raster kernels, each without and with the feather paths (the host

@@ -157,8 +157,9 @@ constexpr float kWindingMaxEdgeShare = .75f;
 // choices (rive_cuda_set_raster_config).
 constexpr int kTileSize = 16;
 constexpr int kTileLog2 = 4;
-// 32x32 tiles: staged records, block bits and per-warp triangle lists.
-constexpr int kRaster32SmemBytes = 1024 * 80 + 32 * 32 * 4 + 32 * 1024 * 2 + 512;
+// 32x32 tiles: staged records, block bits, per-warp triangle lists and coverage
+// planes.
+constexpr int kRaster32SmemBytes = 1024 * 80 + 32 * 32 * 4 + 32 * 1024 * 2 + 32 * 32 * 32 + 512;
 
 // Device error word bits (read by rive_cuda_sync).
 constexpr uint32_t ERR_BAD_TESS_INDEX = 1u << 0;
