@@ -330,6 +330,16 @@ struct VertexOut
     bool discard;
 };
 
+// What a patch vertex's shading knows beside its output: its path's transform,
+// its contour's midpoint, the flags of the tessellation vertex it starts from.
+struct VertexSource
+{
+    float4 M;
+    float2 translate, midpoint;
+    uint32_t flags;
+    bool stroke;
+};
+
 // GLSL mod(x, y) = x - y * floor(x / y)
 __device__ __forceinline__ float glsl_mod(float x, float y)
 {
@@ -380,7 +390,8 @@ __device__ bool shade_patch_vertex(const FlushParams& P,
                                    int span,
                                    uint32_t instanceID,
                                    VertexOut& o,
-                                   float2& cov2) // feathered fills: the corner's cotTheta, y0
+                                   float2& cov2, // feathered fills: the corner's cotTheta, y0
+                                   VertexSource* source = nullptr)
 {
     int localVertexID = (int)pv.localVertexID;
     float outset = pv.outset;
@@ -413,6 +424,8 @@ __device__ bool shade_patch_vertex(const FlushParams& P,
     float2 translate = make_float2(__uint_as_float(r1.x), __uint_as_float(r1.y));
     float strokeRadius = __uint_as_float(r1.z);
     float featherRadius = kFeather ? __uint_as_float(r1.w) : 0.f;
+    if (source)
+        *source = VertexSource{M, translate, midpoint, flags, strokeRadius != 0.f};
     uint32_t mirrored = flags & MIRRORED_CONTOUR_CONTOUR_FLAG;
     if (mirrored)
     {
@@ -756,32 +769,92 @@ __device__ __forceinline__ bool local_inside(float a, float b, float E)
     return E > 0.f || (E == 0.f && (a > 0.f || (a == 0.f && b > 0.f)));
 }
 
-// Can any pixel of the tile-local rectangle [x0, x1) x [y0, y1) lie inside
-// all three edges (tile constants c[k], slopes e[k].z, e[k].w)?
-__device__ __forceinline__ bool local_rect_overlaps(const float* c, const float4* e, int x0, int x1,
-                                                    int y0, int y1)
+// A triangle's pixel box for the tile tests: first and last pixels, as floats
+// (exact).
+struct PixelBox
 {
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-    {
-        const float lx = (float)(e[k].z > 0.f ? x1 - 1 : x0);
-        const float ly = (float)(e[k].w > 0.f ? y1 - 1 : y0);
-        if (local_edge(c[k], e[k].z, e[k].w, lx, ly) < 0.f)
-            return false;
-    }
-    return true;
+    float x0, x1, y0, y1;
+};
+__device__ __forceinline__ PixelBox pixel_box(int4 bb)
+{
+    return PixelBox{(float)bb.x, (float)(bb.z - 1), (float)bb.y, (float)(bb.w - 1)};
 }
 
-__device__ __forceinline__ bool tile_overlaps(const float4* e, int4 bb, int tx, int ty,
+// Can any pixel of the triangle's box within the tile at (tx, ty) lie inside
+// all three edges? Each edge is evaluated at the corner of that rectangle that
+// maximises it.
+__device__ __forceinline__ bool tile_overlaps(const float4* e, const PixelBox& bb, int tx, int ty,
                                               int tileLog2)
 {
-    const int ts = 1 << tileLog2;
-    const int ox = tx << tileLog2, oy = ty << tileLog2;
-    const float c[3] = {tile_edge_origin(e[0], tx, ty, tileLog2),
-                        tile_edge_origin(e[1], tx, ty, tileLog2),
-                        tile_edge_origin(e[2], tx, ty, tileLog2)};
-    return local_rect_overlaps(c, e, max(ox, bb.x) - ox, min(ox + ts, bb.z) - ox,
-                               max(oy, bb.y) - oy, min(oy + ts, bb.w) - oy);
+    const float last = (float)((1 << tileLog2) - 1);
+    const float ox = (float)(tx << tileLog2), oy = (float)(ty << tileLog2);
+    const float px = ox + .5f, py = oy + .5f;
+    const float x0 = fmaxf(bb.x0 - ox, 0.f), x1 = fminf(bb.x1 - ox, last);
+    const float y0 = fmaxf(bb.y0 - oy, 0.f), y1 = fminf(bb.y1 - oy, last);
+    float E[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        E[k] = local_edge(edge_eval(e[k], px, py), e[k].z, e[k].w, e[k].z > 0.f ? x1 : x0,
+                          e[k].w > 0.f ? y1 : y0);
+    return !(fminf(fminf(E[0], E[1]), E[2]) < 0.f);
+}
+
+// Tiles i, i + 32, ... of a box nx tiles wide, in row-major order: one division
+// to start with, additions from then on.
+struct TileWalk
+{
+    int x, y, dx, dy, nx;
+    __device__ __forceinline__ TileWalk(int i, int nx_) : nx(nx_)
+    {
+        y = i / nx;
+        x = i - y * nx;
+        dy = 32 / nx;
+        dx = 32 - dy * nx;
+    }
+    __device__ __forceinline__ void next()
+    {
+        x += dx;
+        y += dy;
+        if (x >= nx)
+        {
+            x -= nx;
+            ++y;
+        }
+    }
+};
+
+// The tiles of a small box (at most 8) that the triangle overlaps, as bits in
+// row-major order: tile_overlaps on each, with the row's terms shared.
+__device__ __forceinline__ uint32_t overlapped_tiles(const float4* e, const PixelBox& bb, int tx0,
+                                                     int ty0, int ntx, int nty, int tileLog2)
+{
+    const float size = (float)(1 << tileLog2), last = size - 1.f;
+    uint32_t mask = 0, bit = 1;
+    float oy = (float)(ty0 << tileLog2);
+    for (int j = 0; j < nty; ++j, oy += size)
+    {
+        const float y0 = fmaxf(bb.y0 - oy, 0.f), y1 = fminf(bb.y1 - oy, last);
+        float ly[3], by[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+        {
+            ly[k] = e[k].w > 0.f ? y1 : y0;
+            by[k] = __fmul_rn(e[k].w, __fsub_rn(oy + .5f, e[k].y));
+        }
+        float ox = (float)(tx0 << tileLog2);
+        for (int i = 0; i < ntx; ++i, ox += size, bit <<= 1)
+        {
+            const float x0 = fmaxf(bb.x0 - ox, 0.f), x1 = fminf(bb.x1 - ox, last);
+            float E[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                E[k] = local_edge(__fmaf_rn(e[k].z, __fsub_rn(ox + .5f, e[k].x), by[k]), e[k].z,
+                                  e[k].w, e[k].z > 0.f ? x1 : x0, ly[k]);
+            if (!(fminf(fminf(E[0], E[1]), E[2]) < 0.f))
+                mask |= bit;
+        }
+    }
+    return mask;
 }
 
 __device__ __forceinline__ int4 unpack_bbox(uint4 meta)
@@ -791,69 +864,54 @@ __device__ __forceinline__ int4 unpack_bbox(uint4 meta)
 }
 } // namespace
 
-// Sets up one triangle for the tile raster: snaps the vertices to the
-// 1/256-pixel grid, culls counterclockwise and degenerate triangles (exact
-// integer area), clips the pixel box to the target, and builds the edge
-// functions and coverage planes. Returns false for a triangle that draws
-// nothing (bb stays empty).
+// Sets up one triangle for the tile raster from vertices snapped to the
+// 1/256-pixel grid (V as 1/256 px and v in pixels): culls counterclockwise and
+// degenerate triangles (exact integer area), clips the pixel box to the target,
+// and builds the edge functions and coverage planes. Returns false for a
+// triangle that draws nothing (bb stays empty).
 // `clip` bounds the pixels (an atlas batch's scissor; the canvas always).
 // `twoSided` keeps counterclockwise triangles (the atlas fill pipeline culls
 // nothing, gpu.hpp:2076-2077): they are turned clockwise and marked
 // FEATURE_ATLAS_NEGATE, since a back-facing atlas fill subtracts coverage.
-__device__ bool setup_triangle(const FlushParams& P,
-                               const VertexOut& A,
-                               const VertexOut& Bv,
-                               const VertexOut& Cv,
-                               uint32_t features,
-                               uint32_t scene,
-                               TriRecord& T,
-                               int4& bb,
-                               float4* featherPlanes = nullptr,
-                               float2 zwA = {}, float2 zwB = {}, float2 zwC = {},
-                               int4 clip = make_int4(0, 0, 0x7fffffff, 0x7fffffff),
-                               bool twoSided = false)
+__device__ __forceinline__ bool setup_snapped(const FlushParams& P,
+                                              int2 V0, int2 V1, int2 V2,
+                                              float2 p0, float2 p1, float2 p2,
+                                              float2 covA, float2 covB, float2 covC,
+                                              uint32_t pathID,
+                                              uint32_t features,
+                                              uint32_t scene,
+                                              TriRecord& T,
+                                              int4& bb,
+                                              float4* featherPlanes,
+                                              float2 zwA, float2 zwB, float2 zwC,
+                                              int4 clip,
+                                              bool twoSided)
 {
-    bb = make_int4(0, 0, 0, 0);
-    if (A.discard || Bv.discard || Cv.discard)
-        return false;
-    float m = fmaxf(fmaxf(fmaxf(fabsf(A.pos.x), fabsf(A.pos.y)), fmaxf(fabsf(Bv.pos.x), fabsf(Bv.pos.y))),
-                    fmaxf(fabsf(Cv.pos.x), fabsf(Cv.pos.y)));
-    if (!(m < 32768.f)) // NaN or outside the exact snapping range
-    {
-        if (!isnan(m))
-            atomicOr(P.error, ERR_COORD_RANGE);
-        return false;
-    }
-    const VertexOut* pB = &Bv;
-    const VertexOut* pC = &Cv;
-    int X1 = __float2int_rn(Bv.pos.x * 256.f), Y1 = __float2int_rn(Bv.pos.y * 256.f);
-    int X2 = __float2int_rn(Cv.pos.x * 256.f), Y2 = __float2int_rn(Cv.pos.y * 256.f);
-    const int X0 = __float2int_rn(A.pos.x * 256.f), Y0 = __float2int_rn(A.pos.y * 256.f);
     // Exact twice-area in 1/65536 px^2: counterclockwise culled (or turned,
     // when two-sided), degenerate dropped.
-    long long area2 = (long long)(X1 - X0) * (Y2 - Y0) - (long long)(X2 - X0) * (Y1 - Y0);
+    long long area2 = (long long)(V1.x - V0.x) * (V2.y - V0.y) -
+                      (long long)(V2.x - V0.x) * (V1.y - V0.y);
     if (area2 < 0 && twoSided)
     {
-        int t = X1;
-        X1 = X2;
-        X2 = t;
-        t = Y1;
-        Y1 = Y2;
-        Y2 = t;
-        pB = &Cv;
-        pC = &Bv;
-        const float2 z = zwB;
+        const int2 v = V1;
+        V1 = V2;
+        V2 = v;
+        float2 f = p1;
+        p1 = p2;
+        p2 = f;
+        f = covB;
+        covB = covC;
+        covC = f;
+        f = zwB;
         zwB = zwC;
-        zwC = z;
+        zwC = f;
         area2 = -area2;
         features |= FEATURE_ATLAS_NEGATE;
     }
     if (area2 <= 0)
         return false;
-    const VertexOut& B = *pB;
-    const VertexOut& C = *pC;
-    const int mnx = min(min(X0, X1), X2), mxx = max(max(X0, X1), X2);
-    const int mny = min(min(Y0, Y1), Y2), mxy = max(max(Y0, Y1), Y2);
+    const int mnx = min(min(V0.x, V1.x), V2.x), mxx = max(max(V0.x, V1.x), V2.x);
+    const int mny = min(min(V0.y, V1.y), V2.y), mxy = max(max(V0.y, V1.y), V2.y);
     // Pixels k whose centres (256 k + 128) lie in [min, max].
     const int bx0 = max(max(-((-(mnx - 128)) >> 8), 0), clip.x);
     const int bx1 = min(min(((mxx - 128) >> 8) + 1, (int)P.width), clip.z);
@@ -862,8 +920,6 @@ __device__ bool setup_triangle(const FlushParams& P,
     if (bx0 >= bx1 || by0 >= by1)
         return false;
     const float s = 1.f / 256.f;
-    const float2 p0 = make_float2(X0 * s, Y0 * s), p1 = make_float2(X1 * s, Y1 * s);
-    const float2 p2 = make_float2(X2 * s, Y2 * s);
     T.e0 = make_edge(p0, p1);
     T.e1 = make_edge(p1, p2);
     T.e2 = make_edge(p2, p0);
@@ -871,12 +927,12 @@ __device__ bool setup_triangle(const FlushParams& P,
     const float d2x = p2.x - p0.x, d2y = p2.y - p0.y;
     const float inv = 1.f / ((float)area2 * (s * s));
     const float ax = T.e0.x - p0.x, ay = T.e0.y - p0.y;
-    const float cxgx = ((B.cov.x - A.cov.x) * d2y - (C.cov.x - A.cov.x) * d1y) * inv;
-    const float cxgy = ((C.cov.x - A.cov.x) * d1x - (B.cov.x - A.cov.x) * d2x) * inv;
-    const float cygx = ((B.cov.y - A.cov.y) * d2y - (C.cov.y - A.cov.y) * d1y) * inv;
-    const float cygy = ((C.cov.y - A.cov.y) * d1x - (B.cov.y - A.cov.y) * d2x) * inv;
-    const uint2 paint = P.paints[P.firstPaint + A.pathID];
-    T.cov0 = make_float4(A.cov.x + cxgx * ax + cxgy * ay, cxgx, cxgy, A.cov.y + cygx * ax + cygy * ay);
+    const float cxgx = ((covB.x - covA.x) * d2y - (covC.x - covA.x) * d1y) * inv;
+    const float cxgy = ((covC.x - covA.x) * d1x - (covB.x - covA.x) * d2x) * inv;
+    const float cygx = ((covB.y - covA.y) * d2y - (covC.y - covA.y) * d1y) * inv;
+    const float cygy = ((covC.y - covA.y) * d1x - (covB.y - covA.y) * d2x) * inv;
+    const uint2 paint = P.paints[P.firstPaint + pathID];
+    T.cov0 = make_float4(covA.x + cxgx * ax + cxgy * ay, cxgx, cxgy, covA.y + cygx * ax + cygy * ay);
     T.cov1 = make_float4(cygx, cygy, __uint_as_float(paint.x), __uint_as_float(paint.y));
     if (featherPlanes)
     {
@@ -891,13 +947,60 @@ __device__ bool setup_triangle(const FlushParams& P,
     }
     // The fp16 coverage key of the path (draw_raster_order_path.frag: pathID
     // bits, sign bit flipped for even-odd fills).
-    uint32_t key = A.pathID == 0 ? 0u : ((A.pathID + MAX_DENORM_F16) * P.pathIDGranularity) & 0xffffu;
+    uint32_t key = pathID == 0 ? 0u : ((pathID + MAX_DENORM_F16) * P.pathIDGranularity) & 0xffffu;
     if (paint.x & PAINT_FLAG_EVEN_ODD_FILL)
         key ^= 0x8000u;
     bb = make_int4(bx0, by0, bx1, by1);
-    T.meta = make_uint4((A.pathID & 0xffffu) | (features << 16), (uint32_t)bx0 | ((uint32_t)bx1 << 16),
+    T.meta = make_uint4((pathID & 0xffffu) | (features << 16), (uint32_t)bx0 | ((uint32_t)bx1 << 16),
                         (uint32_t)by0 | ((uint32_t)by1 << 16), key | (scene << 16));
     return true;
+}
+
+// Vertex positions outside the exact snapping range draw nothing (m: the
+// largest coordinate of a triangle; NaN only when all are).
+__device__ __forceinline__ bool snapping_range(const FlushParams& P, float m)
+{
+    if (m < 32768.f)
+        return true;
+    if (!isnan(m))
+        atomicOr(P.error, ERR_COORD_RANGE);
+    return false;
+}
+__device__ __forceinline__ int2 snap(float2 p)
+{
+    return make_int2(__float2int_rn(p.x * 256.f), __float2int_rn(p.y * 256.f));
+}
+__device__ __forceinline__ float2 snapped_pixels(int2 V)
+{
+    const float s = 1.f / 256.f;
+    return make_float2(V.x * s, V.y * s);
+}
+
+// setup_snapped from shaded vertices.
+__device__ bool setup_triangle(const FlushParams& P,
+                               const VertexOut& A,
+                               const VertexOut& B,
+                               const VertexOut& C,
+                               uint32_t features,
+                               uint32_t scene,
+                               TriRecord& T,
+                               int4& bb,
+                               float4* featherPlanes = nullptr,
+                               float2 zwA = {}, float2 zwB = {}, float2 zwC = {},
+                               int4 clip = make_int4(0, 0, 0x7fffffff, 0x7fffffff),
+                               bool twoSided = false)
+{
+    bb = make_int4(0, 0, 0, 0);
+    if (A.discard || B.discard || C.discard)
+        return false;
+    if (!snapping_range(P, fmaxf(fmaxf(fmaxf(fabsf(A.pos.x), fabsf(A.pos.y)),
+                                       fmaxf(fabsf(B.pos.x), fabsf(B.pos.y))),
+                                 fmaxf(fabsf(C.pos.x), fabsf(C.pos.y)))))
+        return false;
+    const int2 V0 = snap(A.pos), V1 = snap(B.pos), V2 = snap(C.pos);
+    return setup_snapped(P, V0, V1, V2, snapped_pixels(V0), snapped_pixels(V1), snapped_pixels(V2),
+                         A.cov, B.cov, C.cov, A.pathID, features, scene, T, bb, featherPlanes, zwA,
+                         zwB, zwC, clip, twoSided);
 }
 
 // Tiles a set-up triangle touches (the same tile test as the binner's).
@@ -928,42 +1031,33 @@ __device__ __forceinline__ bool wide_strip(int n, int strip, int& lo, int& hi)
 
 // Counts the tiles of the warp's triangles: a lane counts its own triangle
 // when its box spans at most kLaneTiles tiles; the whole warp walks larger
-// ones in turn. `has` marks lanes holding a triangle; e/bb its edges and box.
+// ones in turn. `has` marks lanes holding a triangle of slot `slot`; e/bb its
+// edges and box.
 __device__ __forceinline__ void count_tiles(bool has,
-                                            int tileLog2,
+                                            const BatchTables& B,
                                             const float4* e,
                                             int4 bb,
-                                            uint32_t* __restrict__ countOut,
-                                            uint8_t* __restrict__ maskOut,
-                                            const BatchTables& B,
                                             uint32_t slot,
-                                            const float4 (*warpEdges)[3],
-                                            const int4* warpBoxes,
-                                            uint32_t* const* warpOuts)
+                                            uint32_t* __restrict__ tileCounts,
+                                            uint8_t* __restrict__ tileMasks)
 {
     const int lane = threadIdx.x & 31;
+    const int tileLog2 = B.tileLog2;
     bool big = false;
     if (has)
     {
         if (bb.z > bb.x)
         {
+            const PixelBox box = pixel_box(bb);
             int tx0, ty0, ntx, nty;
             tile_span(bb, tileLog2, tx0, ty0, ntx, nty);
             if (ntx * nty <= kLaneTiles)
             {
                 // The tiles it overlaps, as bits in row-major order over its
                 // tile box, so the binner need not test them again.
-                uint32_t count = 0, mask = 0;
-                int i = 0;
-                for (int ty = ty0; ty < ty0 + nty; ++ty)
-                    for (int tx = tx0; tx < tx0 + ntx; ++tx, ++i)
-                        if (tile_overlaps(e, bb, tx, ty, tileLog2))
-                        {
-                            ++count;
-                            mask |= 1u << i;
-                        }
-                *countOut = count;
-                *maskOut = (uint8_t)mask;
+                const uint32_t mask = overlapped_tiles(e, box, tx0, ty0, ntx, nty, tileLog2);
+                tileCounts[slot] = __popc(mask);
+                tileMasks[slot] = (uint8_t)mask;
             }
             else
             {
@@ -977,16 +1071,16 @@ __device__ __forceinline__ void count_tiles(bool has,
                     if (i < B.wideCap)
                     {
                         B.wide[1 + i] = slot; // wide_count_kernel adds up its tiles
-                        *countOut = 0;
+                        tileCounts[slot] = 0;
                         big = false;
                     }
                 }
-                *maskOut = big ? 0 : kWideMask;
+                tileMasks[slot] = big ? 0 : kWideMask;
             }
         }
         else
         {
-            *countOut = 0;
+            tileCounts[slot] = 0;
         }
     }
     uint32_t bigs = __ballot_sync(0xffffffffu, big);
@@ -994,19 +1088,24 @@ __device__ __forceinline__ void count_tiles(bool has,
     {
         const int t = __ffs(bigs) - 1;
         bigs &= bigs - 1;
-        const int4 tb = warpBoxes[t];
-        const float4 te[3] = {warpEdges[t][0], warpEdges[t][1], warpEdges[t][2]};
+        float4 te[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            te[k] = make_float4(__shfl_sync(0xffffffffu, e[k].x, t), __shfl_sync(0xffffffffu, e[k].y, t),
+                                __shfl_sync(0xffffffffu, e[k].z, t), __shfl_sync(0xffffffffu, e[k].w, t));
+        const int4 tb = make_int4(__shfl_sync(0xffffffffu, bb.x, t), __shfl_sync(0xffffffffu, bb.y, t),
+                                  __shfl_sync(0xffffffffu, bb.z, t), __shfl_sync(0xffffffffu, bb.w, t));
         int tx0, ty0, ntx, nty;
         tile_span(tb, tileLog2, tx0, ty0, ntx, nty);
         const int n = ntx * nty;
+        const PixelBox box = pixel_box(tb);
         uint32_t count = 0;
-        for (int i = lane; i < n; i += 32)
-            count += tile_overlaps(te, tb, tx0 + i % ntx, ty0 + i / ntx, tileLog2) ? 1u : 0u;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            count += __shfl_xor_sync(0xffffffffu, count, o);
-        if (lane == 0)
-            *warpOuts[t] = count;
+        TileWalk at(lane, ntx);
+        for (int i = lane; i < n; i += 32, at.next())
+            count += tile_overlaps(te, box, tx0 + at.x, ty0 + at.y, tileLog2) ? 1u : 0u;
+        count = __reduce_add_sync(0xffffffffu, count);
+        if (lane == t)
+            tileCounts[slot] = count;
     }
 }
 
@@ -1198,9 +1297,6 @@ __device__ __forceinline__ void patch_setup(const BatchTables& B,
     __shared__ VertexOut sv[4][kVerts];
     // The feathered-fill coverage components, kept only for feathered draws.
     __shared__ float2 sZW[4][kFeather ? kVerts : 1];
-    __shared__ float4 sEdges[4][kTriPasses * 32][3];
-    __shared__ int4 sBox[4][kTriPasses * 32];
-    __shared__ uint32_t* sOut[4][kTriPasses * 32];
     __shared__ bool sok[4];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t gi = blockIdx.x * 4 + w;
@@ -1347,26 +1443,133 @@ __device__ __forceinline__ void patch_setup(const BatchTables& B,
                 e[0] = T.e0;
                 e[1] = T.e1;
                 e[2] = T.e2;
-                sEdges[w][t][0] = T.e0;
-                sEdges[w][t][1] = T.e1;
-                sEdges[w][t][2] = T.e2;
                 deferred = fan;
             }
-            sBox[w][t] = bb;
-            sOut[w][t] = tileCounts + slot0 + t;
         }
         __syncwarp();
-        count_tiles(has && !deferred, B.tileLog2, e, bb, tileCounts + slot0 + t,
-                    tileMasks + slot0 + t, B, slot0 + t, sEdges[w] + pass * 32,
-                    sBox[w] + pass * 32, sOut[w] + pass * 32);
+        count_tiles(has && !deferred, B, e, bb, slot0 + t, tileCounts, tileMasks);
         if (deferred)
             tileCounts[slot0 + t] = kDeferredCount;
         __syncwarp();
     }
 }
 
+// patch_setup of a midpoint fan without feathers. Its 42 vertices are 32 of the
+// AA ramps, 9 of the fan and the contour's midpoint; a warp shades the 32 in one
+// pass and makes the others from them:
+//  * fan vertex i starts from the same tessellation vertex, with the same
+//    offset, as ramp vertex 4 i (4 i + 1 when that vertex is mirrored; for
+//    i = 8, ramp vertex 30, or 28), so position and coverage are the same bits;
+//    only the discard rules differ (a stroke has no fan, a retrofitted triangle
+//    strip no ramps);
+//  * the midpoint has no offset: a zero outset times a normal has the sign 0.
+// Shading the ten in a second pass cost as much as the 32. Vertices are snapped
+// once each, not once per triangle corner, and tile tests share their row's
+// terms: full-feature 1021x767 (356 k patches) 490 -> 372 us, 20 plain canvases
+// (653 k patches of large triangles) 1112 -> 896 us. Bound by issue slots.
+__device__ __forceinline__ void fan_setup(const BatchTables& B,
+                                          TriRecord* __restrict__ tris,
+                                          uint32_t* __restrict__ tileCounts,
+                                          uint8_t* __restrict__ tileMasks)
+{
+    // Snapped positions (1/256 px, and px), coverage, and the largest
+    // coordinate and path of every vertex (bit 31: discarded).
+    __shared__ int2 sV[4][kPatchVertexCount];
+    __shared__ float2 sP[4][kPatchVertexCount], sCov[4][kPatchVertexCount];
+    __shared__ uint2 sMeta[4][kPatchVertexCount];
+    constexpr uint32_t kDiscard = 1u << 31;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t gi = blockIdx.x * 4 + w;
+    if (gi >= B.totalItems[0])
+        return; // whole warp exits together
+    const uint32_t seg = find_range(B.segBase[0], B.segCount[0], gi);
+    const PatchSegment S = B.segments[0][seg];
+    const FlushParams& P = B.scenes[S.scene];
+    const uint32_t local = gi - B.segBase[0][seg];
+    VertexOut o;
+    VertexSource src;
+    float2 zw;
+    const bool shaded = shade_patch_vertex<false>(P, patch_vertex_desc(lane), kPatchSegmentSpan,
+                                                  S.baseElement + local, o, zw, &src);
+    const bool ok = __all_sync(0xffffffffu, shaded);
+    uint32_t strokes = 0, mirrored = 0;
+    if (ok)
+    {
+        const int2 V = snap(o.pos);
+        sV[w][lane] = V;
+        sP[w][lane] = snapped_pixels(V);
+        sCov[w][lane] = o.cov;
+        sMeta[w][lane] = make_uint2(__float_as_uint(fmaxf(fabsf(o.pos.x), fabsf(o.pos.y))),
+                                    o.pathID | (o.discard ? kDiscard : 0u));
+        strokes = __ballot_sync(0xffffffffu, src.stroke);
+        mirrored = __ballot_sync(0xffffffffu, (src.flags & MIRRORED_CONTOUR_CONTOUR_FLAG) != 0);
+        __syncwarp();
+        if (lane < 9)
+        {
+            const int first = lane < 8 ? 4 * lane : 28; // starts from the same tessellation vertex
+            const int v = ((mirrored >> first) & 1u) ? (lane < 8 ? first + 1 : 28)
+                                                     : (lane < 8 ? first : 30);
+            sV[w][32 + lane] = sV[w][v];
+            sP[w][32 + lane] = sP[w][v];
+            sCov[w][32 + lane] = sCov[w][v];
+            const uint2 m = sMeta[w][v];
+            sMeta[w][32 + lane] =
+                make_uint2(m.x, (m.y & ~kDiscard) | (((strokes >> v) & 1u) ? kDiscard : 0u));
+        }
+        if (lane == 0)
+        {
+            const float2 mo = mat_mul(src.M, src.midpoint);
+            const float2 pos = make_float2(__fadd_rn(mo.x, src.translate.x),
+                                           __fadd_rn(mo.y, src.translate.y));
+            const bool negate = ((src.flags & MIRRORED_CONTOUR_CONTOUR_FLAG) != 0) !=
+                                ((src.flags & NEGATE_PATH_FILL_COVERAGE_FLAG) != 0);
+            const int2 M = snap(pos);
+            sV[w][41] = M;
+            sP[w][41] = snapped_pixels(M);
+            sCov[w][41] = make_float2(negate && !P.wireframe ? -1.f : 1.f, -1.f);
+            sMeta[w][41] = make_uint2(
+                __float_as_uint(fmaxf(fabsf(pos.x), fabsf(pos.y))),
+                o.pathID |
+                    (src.stroke || (src.flags & RETROFIT_TRI_STRIP_CONTOUR_FLAG) ? kDiscard : 0u));
+            // The path's image slot, for the raster's image paint (every patch
+            // of the path writes the same value).
+            if (S.image != kNoImage && P.pathImage && o.pathID < P.pathCount)
+                P.pathImage[o.pathID] = S.image;
+        }
+        __syncwarp();
+    }
+    const uint32_t slot = S.slotBase + local * kPatchTriangleCount + lane;
+    const bool has = lane < kPatchTriangleCount;
+    int4 bb = make_int4(0, 0, 0, 0);
+    float4 e[3];
+    if (has && ok)
+    {
+        int ia, ib, ic;
+        patch_triangle(lane, ia, ib, ic);
+        const uint2 mA = sMeta[w][ia], mB = sMeta[w][ib], mC = sMeta[w][ic];
+        TriRecord T;
+        if (!((mA.y | mB.y | mC.y) & kDiscard) &&
+            snapping_range(P, fmaxf(fmaxf(__uint_as_float(mA.x), __uint_as_float(mB.x)),
+                                    __uint_as_float(mC.x))) &&
+            setup_snapped(P, sV[w][ia], sV[w][ib], sV[w][ic], sP[w][ia], sP[w][ib], sP[w][ic],
+                          sCov[w][ia], sCov[w][ib], sCov[w][ic], mA.y, S.features, S.scene, T, bb,
+                          nullptr, float2{}, float2{}, float2{},
+                          make_int4((int)(S.scissorLT & 0xffffu), (int)(S.scissorLT >> 16),
+                                    (int)(S.scissorRB & 0xffffu), (int)(S.scissorRB >> 16)),
+                          false))
+        {
+            tris[slot] = T;
+            e[0] = T.e0;
+            e[1] = T.e1;
+            e[2] = T.e2;
+        }
+    }
+    __syncwarp();
+    count_tiles(has, B, e, bb, slot, tileCounts, tileMasks);
+}
+
 // Resident 128-thread CTAs per SM the midpoint-fan set-up's registers are
-// bounded for.
+// bounded for (20 plain canvases 896, 915 and 944 us at 9, 10 and 11).
 #ifndef RIVE_SETUP_MIN_BLOCKS
 #define RIVE_SETUP_MIN_BLOCKS 9
 #endif
@@ -1375,7 +1578,7 @@ __global__ void __launch_bounds__(128, RIVE_SETUP_MIN_BLOCKS) patch_setup_kernel
                                                           uint32_t* __restrict__ tileCounts,
                                                           uint8_t* __restrict__ tileMasks)
 {
-    patch_setup<0, false>(B, tris, tileCounts, tileMasks);
+    fan_setup(B, tris, tileCounts, tileMasks);
 }
 
 // Midpoint-fan set-up for batches that draw interior tiles as winding records
@@ -1498,10 +1701,6 @@ __global__ void __launch_bounds__(256) interior_setup_kernel(BatchTables B,
                                                              uint32_t* __restrict__ tileCounts,
                                                              uint8_t* __restrict__ tileMasks)
 {
-    __shared__ float4 sEdges[8][32][3];
-    __shared__ int4 sBox[8][32];
-    __shared__ uint32_t* sOut[8][32];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t first = (blockIdx.x * blockDim.x) & ~31u;
     if (first >= B.totalItems[2])
         return; // whole warp exits together
@@ -1528,9 +1727,6 @@ __global__ void __launch_bounds__(256) interior_setup_kernel(BatchTables B,
                 e[0] = T.e0;
                 e[1] = T.e1;
                 e[2] = T.e2;
-                sEdges[w][lane][0] = T.e0;
-                sEdges[w][lane][1] = T.e1;
-                sEdges[w][lane][2] = T.e2;
             }
             ok = false; // set up already
         }
@@ -1587,16 +1783,10 @@ __global__ void __launch_bounds__(256) interior_setup_kernel(BatchTables B,
             e[0] = T.e0;
             e[1] = T.e1;
             e[2] = T.e2;
-            sEdges[w][lane][0] = T.e0;
-            sEdges[w][lane][1] = T.e1;
-            sEdges[w][lane][2] = T.e2;
         }
-        sBox[w][lane] = bb;
-        sOut[w][lane] = tileCounts + slot;
     }
     __syncwarp();
-    count_tiles(has, B.tileLog2, e, bb, tileCounts + slot, tileMasks + slot, B, slot, sEdges[w],
-                sBox[w], sOut[w]);
+    count_tiles(has, B, e, bb, slot, tileCounts, tileMasks);
 }
 
 // ---- Winding grids: the per-path passes ------------------------------------
@@ -1830,7 +2020,7 @@ __global__ void __launch_bounds__(256) fan_filter_kernel(BatchTables B,
                 int k = 0;
                 for (int ty = ty0; ty < ty0 + nty; ++ty)
                     for (int tx = tx0; tx < tx0 + ntx; ++tx, ++k)
-                        if (tile_overlaps(e, bb, tx, ty, tileLog2) &&
+                        if (tile_overlaps(e, pixel_box(bb), tx, ty, tileLog2) &&
                             keep_fan_tile(g, B.gridEdge, tx, ty))
                         {
                             ++count;
@@ -1867,7 +2057,7 @@ __global__ void __launch_bounds__(256) fan_filter_kernel(BatchTables B,
         for (int i = lane; i < n; i += 32)
         {
             const int tx = tx0 + i % ntx, ty = ty0 + i / ntx;
-            count += (tile_overlaps(te, tb, tx, ty, tileLog2) && keep_fan_tile(tg, B.gridEdge, tx, ty))
+            count += (tile_overlaps(te, pixel_box(tb), tx, ty, tileLog2) && keep_fan_tile(tg, B.gridEdge, tx, ty))
                          ? 1u
                          : 0u;
         }
@@ -1899,9 +2089,11 @@ __global__ void __launch_bounds__(256) wide_count_kernel(BatchTables B,
         if (!wide_strip(ntx * nty, (int)(i % kWideStrips), lo, hi))
             continue;
         const float4 e[3] = {T->e0, T->e1, T->e2};
+        const PixelBox box = pixel_box(bb);
         uint32_t count = 0;
-        for (int t = lo + lane; t < hi; t += 32)
-            count += tile_overlaps(e, bb, tx0 + t % ntx, ty0 + t / ntx, B.tileLog2) ? 1u : 0u;
+        TileWalk at(lo + lane, ntx);
+        for (int t = lo + lane; t < hi; t += 32, at.next())
+            count += tile_overlaps(e, box, tx0 + at.x, ty0 + at.y, B.tileLog2) ? 1u : 0u;
         count = __reduce_add_sync(0xffffffffu, count);
         if (lane == 0)
         {
@@ -2000,10 +2192,12 @@ __device__ __forceinline__ void bin_scatter_wide(int tileLog2,
         uint32_t o = offsets[slot] + __reduce_add_sync(0xffffffffu, before);
         const uint2 st = sceneTiles[meta.w >> 16];
         const float4 e[3] = {T->e0, T->e1, T->e2};
-        for (int base = lo; base < hi; base += 32)
+        const PixelBox box = pixel_box(bb);
+        TileWalk at(lo + lane, ntx);
+        for (int base = lo; base < hi; base += 32, at.next())
         {
-            const int t = base + lane, tx = tx0 + t % ntx, ty = ty0 + t / ntx;
-            const bool hit = t < hi && tile_overlaps(e, bb, tx, ty, tileLog2);
+            const int tx = tx0 + at.x, ty = ty0 + at.y;
+            const bool hit = base + lane < hi && tile_overlaps(e, box, tx, ty, tileLog2);
             const uint32_t mask = __ballot_sync(0xffffffffu, hit);
             if (hit)
             {
@@ -2135,19 +2329,18 @@ __device__ __forceinline__ void bin_scatter(const BatchTables* __restrict__ Bw,
         const PathGrid* g = (kWinding && (meta.x & (FEATURE_FAN_DEFERRED << 16)))
                                 ? winding_grid(*Bw, meta.w >> 16, meta.x & 0xffffu)
                                 : nullptr;
+        const PixelBox box = pixel_box(bb);
         int tx0, ty0, ntx, nty;
         tile_span(bb, tileLog2, tx0, ty0, ntx, nty);
         const int n = ntx * nty;
-        for (int base = 0; base < n; base += 32)
+        TileWalk at(lane, ntx);
+        for (int base = 0; base < n; base += 32, at.next())
         {
-            const int i = base + lane;
             bool hit = false;
-            int tx = 0, ty = 0;
-            if (i < n)
+            const int tx = tx0 + at.x, ty = ty0 + at.y;
+            if (base + lane < n)
             {
-                tx = tx0 + i % ntx;
-                ty = ty0 + i / ntx;
-                hit = tile_overlaps(e, bb, tx, ty, tileLog2) &&
+                hit = tile_overlaps(e, box, tx, ty, tileLog2) &&
                       (!kWinding || keep_fan_tile(g, kWinding ? Bw->gridEdge : nullptr, tx, ty));
             }
             const uint32_t mask = __ballot_sync(0xffffffffu, hit);
@@ -2169,11 +2362,12 @@ __device__ __forceinline__ void bin_scatter(const BatchTables* __restrict__ Bw,
     }
 }
 
-// Resident 256-thread CTAs per SM the binner's registers are bounded for: 6
-// (no spills) bins the full-feature frame in 0.98 ms against 1.10 ms at the
-// compiler's 45 registers (5 CTAs).
+// Resident 256-thread CTAs per SM the binner's registers are bounded for. It
+// waits for its scattered loads, so more warps win over a few spilled
+// registers: scan and binner of the full-feature 2048x2048 frame 1.06, 0.96 and
+// 0.85 ms at 5, 6 and 8 CTAs.
 #ifndef RIVE_BIN_MIN_BLOCKS
-#define RIVE_BIN_MIN_BLOCKS 6
+#define RIVE_BIN_MIN_BLOCKS 8
 #endif
 __global__ void __launch_bounds__(256, RIVE_BIN_MIN_BLOCKS) bin_scatter_kernel(uint32_t slotCount,
                                                           int tileLog2,
@@ -3179,7 +3373,7 @@ template <int TL> struct RasterShared
 
 // The warp blocks whose part inside the pixel box bb may hold a pixel inside
 // all three edges (tile constants c[k], slopes e[k].z, e[k].w): the test of
-// local_rect_overlaps on every block, with each edge's values at the block
+// tile_overlaps on every block, with each edge's values at the block
 // rows' and columns' decisive corners shared between blocks and no branches.
 template <int TL>
 __device__ __forceinline__ uint32_t blocks_overlapped(const float* c, const float4* e, int4 bb,
