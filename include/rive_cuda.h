@@ -551,10 +551,10 @@ int rive_cuda_get_raster_config(const rive_cuda_context* ctx, int* tile_size, in
 
 /*
  * Raster schedule (no counterpart in the reference; off by default, an
- * autotuner knob; 16-pixel tiles): with it on, the raster runs as a
- * persistent grid of resident CTAs that take tiles from an atomic cursor over
- * the batch's tiles sorted by bin entries, heaviest first, instead of one CTA
- * launched per tile. The image is the same either way.
+ * autotuner knob; 16-pixel tiles): with it on, the tiles of every batch are
+ * rendered heaviest first (by bin entries), so no long tile starts last; with
+ * it off, only those of batches where that is known to pay. The image is the
+ * same either way.
  */
 int rive_cuda_set_raster_queue(rive_cuda_context* ctx, int enabled);
 int rive_cuda_get_raster_queue(const rive_cuda_context* ctx, int* enabled);

@@ -12,7 +12,7 @@ fastest set on the context.
 
 The search space is tile size {8, 16, 32} x resident raster CTAs per SM
 {1, 2, 4, as many as fit} x winding records {off, on}, and for 16-pixel
-tiles the raster schedule {one CTA per tile, persistent work queue}; 32-pixel
+tiles the tile order {as they come, heaviest first}; 32-pixel
 tiles run one 1,024-thread CTA per SM at most, so only their "as many as fit"
 entry differs.
 """
@@ -38,7 +38,7 @@ def _candidates():
 
 
 # (tile size in pixels, resident raster CTAs per SM or 0, winding records,
-# work-queue raster)
+# tiles heaviest first)
 CANDIDATES = _candidates()
 
 

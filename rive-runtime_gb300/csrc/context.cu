@@ -103,21 +103,6 @@ __global__ void ranges_guard_kernel(const uint32_t* pairTotal,
                                     uint32_t capacity,
                                     uint2* ranges,
                                     uint32_t tiles);
-// The work-queue raster (kernels_raster.cu).
-__global__ void raster_queue_kernel(BatchTables B,
-                                    const TriRecord* tris,
-                                    const uint32_t* sortedSlots,
-                                    const uint2* ranges,
-                                    const uint32_t* order,
-                                    uint32_t* cursor,
-                                    uint32_t tiles);
-__global__ void raster_queue_feather_kernel(BatchTables B,
-                                            const TriRecord* tris,
-                                            const uint32_t* sortedSlots,
-                                            const uint2* ranges,
-                                            const uint32_t* order,
-                                            uint32_t* cursor,
-                                            uint32_t tiles);
 // One mip level of an image from the level above (kernels_raster.cu).
 __global__ void mip_level_kernel(const uchar4* src, uint32_t sw, uint32_t sh, uchar4* dst,
                                  uint32_t dw, uint32_t dh);
@@ -158,8 +143,13 @@ __global__ void bin_scatter_winding_kernel(BatchTables B,
 #define RIVE_DECLARE_RASTER(NAME)                                                                  \
     __global__ void NAME(BatchTables B, const TriRecord* tris, const uint32_t* sortedSlots,        \
                          const uint2* ranges);
-RIVE_DECLARE_RASTER(raster_tile_kernel)
-RIVE_DECLARE_RASTER(raster_tile_feather_kernel)
+// (16-pixel tiles: in the order of `order`, or as they come when it is null.)
+__global__ void raster_tile_kernel(BatchTables B, const TriRecord* tris, const uint32_t* sortedSlots,
+                                   const uint2* ranges, const uint32_t* order);
+__global__ void raster_tile_feather_kernel(BatchTables B, const TriRecord* tris,
+                                           const uint32_t* sortedSlots, const uint2* ranges,
+                                           const uint32_t* order);
+__global__ void tile_order_kernel(uint32_t tiles, const uint2* ranges, uint32_t* order);
 RIVE_DECLARE_RASTER(raster_tile8_kernel)
 RIVE_DECLARE_RASTER(raster_tile8_feather_kernel)
 RIVE_DECLARE_RASTER(raster_tile32_kernel)
@@ -301,7 +291,7 @@ struct rive_cuda_context
     RecordRing rings[RIVE_CUDA_BUFFER_KIND_COUNT];
     DeviceBuffer tess, grad;
     uint32_t tessWidth = 0, tessHeight = 0, gradWidth = 0, gradHeight = 0;
-    DeviceBuffer tris, tileCounts, tileMasks, offsets, featherPlanes, wide;
+    DeviceBuffer tris, tileCounts, tileMasks, offsets, featherPlanes, wide, order;
     DeviceBuffer keys, vals, keysAlt, valsAlt, sortTemp, scanTemp, ranges;
     DeviceBuffer dTables;  // batch tables (device)
     // Pinned staging of the tables, a ring of three, so the host writes the
@@ -327,12 +317,10 @@ struct rive_cuda_context
     // Interior tiles as winding records (rive_cuda_set_winding_tiles): per-path
     // grids and the cell pool, grown when a flush asked for more cells.
     bool windingTiles = false;
-    // Raster as a persistent work queue over heaviest-first tiles
-    // (rive_cuda_set_raster_queue; 16-pixel tiles).
+    // Every batch's tiles heaviest first (rive_cuda_set_raster_queue; 16-pixel
+    // tiles), not only those the grid orders by itself (orders_tiles).
     bool rasterQueue = false;
-    int queueCtas[2] = {0, 0}; // resident queue CTAs per SM [feather variant]
-    int smCount = 0;
-    DeviceBuffer queueKeys, queueVals, queueKeysAlt, queueValsAlt, queueTemp, queueCursor;
+    DeviceBuffer queueKeys, queueVals, queueKeysAlt, queueValsAlt, queueTemp;
     DeviceBuffer pathGrids, gridWinding, gridEdge, gridCounters;
     DeviceBuffer atlas; // the batch's feather atlases (fp16 texels)
     DeviceBuffer pathImage; // per path of the batch: the slot of its image
@@ -345,8 +333,6 @@ struct rive_cuda_context
     bool raster32Ready = false;
     size_t rasterPad[2][2] = {};      // [feather variant][8 or 16 pixel kernel]: padding
     int rasterPadFor[2] = {-1, -1};   // the CTAs-per-SM limit it was found for
-    size_t queuePad[2] = {};          // [feather variant]: the work-queue kernel's padding
-    int queuePadFor = -1;             // the CTAs-per-SM limit it was found for
     // Stage timing (rive_cuda_set_profiling).
     bool profiling = false;
     std::vector<cudaEvent_t> eventPool;
@@ -364,8 +350,8 @@ struct rive_cuda_graph
     rive_cuda_context* ctx = nullptr;
     DeviceBuffer tables, tess, grad, tris, counts, masks, offsets, keys, vals, keysAlt, valsAlt,
         scanTemp, sortTemp, ranges, error, featherPlanes, pathGrids, gridWinding, gridEdge,
-        gridCounters, queueKeys, queueVals, queueKeysAlt, queueValsAlt, queueTemp, queueCursor,
-        atlas, pathImage, wide;
+        gridCounters, queueKeys, queueVals, queueKeysAlt, queueValsAlt, queueTemp,
+        atlas, pathImage, wide, order;
     cudaStream_t stream = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -886,10 +872,11 @@ struct Scratch
     uint8_t* gridEdge = nullptr;
     uint32_t* gridCounters = nullptr;
     uint32_t gridCapacity = 0;
-    // Work-queue raster: the tile order (sorted keys/values and their
-    // alternates), the sort's temporaries and the cursor.
+    // Heaviest-first batches of more than kOrderTiles tiles: the tile order
+    // (sorted keys/values and their alternates) and the sort's temporaries.
     uint32_t *qKeys = nullptr, *qVals = nullptr, *qKeysAlt = nullptr, *qValsAlt = nullptr;
-    uint32_t* qCursor = nullptr;
+    uint32_t* order = nullptr; // the grid's tile order (kOrderTiles entries)
+    bool heaviestFirst = false; // whatever orders_tiles says
     void* qTemp = nullptr;
     size_t qTempBytes = 0;
 };
@@ -1232,14 +1219,6 @@ int prepare_raster(rive_cuda_context* ctx)
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, kRaster32SmemBytes));
         ctx->raster32Ready = true;
     }
-    if (ctx->rasterQueue && ctx->smCount == 0)
-    {
-        CK(cudaDeviceGetAttribute(&ctx->smCount, cudaDevAttrMultiProcessorCount, ctx->device));
-        const void* q[2] = {(const void*)raster_queue_kernel,
-                            (const void*)raster_queue_feather_kernel};
-        for (int f = 0; f < 2; ++f)
-            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->queueCtas[f], q[f], 256, 0));
-    }
     const int slot = ctx->tileLog2 == 3 ? 0 : ctx->tileLog2 == 4 ? 1 : -1;
     if (slot >= 0 && ctx->rasterCtasPerSm > 0 && ctx->rasterPadFor[slot] != ctx->rasterCtasPerSm)
     {
@@ -1252,18 +1231,19 @@ int prepare_raster(rive_cuda_context* ctx)
         cudaGetLastError(); // a failed query only leaves the launch unpadded
         ctx->rasterPadFor[slot] = ctx->rasterCtasPerSm;
     }
-    if (ctx->rasterQueue && ctx->rasterCtasPerSm > 0 && ctx->queuePadFor != ctx->rasterCtasPerSm)
-    {
-        // The queue kernels have their own static shared memory, so their own
-        // padding (and their own dynamic shared memory limit, set there).
-        const void* q[2] = {(const void*)raster_queue_kernel,
-                            (const void*)raster_queue_feather_kernel};
-        for (int f = 0; f < 2; ++f)
-            ctx->queuePad[f] = occupancy_pad(q[f], 256, ctx->rasterCtasPerSm);
-        cudaGetLastError();
-        ctx->queuePadFor = ctx->rasterCtasPerSm;
-    }
     return RIVE_CUDA_OK;
+}
+
+// Whether the 16-pixel grid takes its tiles heaviest first without being asked:
+// from about one wave of CTAs (760) to what one CTA can order, and where a tile
+// is long enough for the last ones to leave the GPU half empty. 3072 tiles of
+// 2366 entries: raster 737 -> 634 us; 16384 tiles of 450: 3.76 -> 3.57 ms; 1024
+// tiles of 610: no difference; UI screens (9 to 13 entries a tile) would pay the
+// order's 5 us for nothing.
+bool orders_tiles(const BatchLayout& L, uint32_t entries)
+{
+    return L.tileLog2 == 4 && L.mainTiles >= kOrderMinTiles && L.mainTiles <= kOrderTiles &&
+           entries / 64 >= L.mainTiles;
 }
 
 // Launches the raster for the batch's tile size (prepare_raster has run). A
@@ -1276,26 +1256,9 @@ int launch_raster(rive_cuda_context* ctx,
                   const TriRecord* tris,
                   const uint32_t* sortedSlots,
                   const uint2* ranges,
+                  uint32_t entries,
                   cudaStream_t stream)
 {
-    if (L.tileLog2 == 4 && S.qCursor)
-    {
-        // The work queue: tiles sorted by bin entries, heaviest first, taken
-        // in turn by a persistent grid of resident CTAs.
-        tile_order_keys_kernel<<<(L.mainTiles + 255) / 256, 256, 0, stream>>>(L.mainTiles, ranges,
-                                                                            S.qKeys, S.qVals);
-        cub::DoubleBuffer<uint32_t> k(S.qKeys, S.qKeysAlt), v(S.qVals, S.qValsAlt);
-        size_t tb = S.qTempBytes;
-        CK(cub::DeviceRadixSort::SortPairs(S.qTemp, tb, k, v, (int)L.mainTiles, 0, 32, stream));
-        CK(cudaMemsetAsync(S.qCursor, 0, 4, stream));
-        const size_t dyn = ctx->rasterCtasPerSm > 0 ? ctx->queuePad[L.feather] : 0;
-        const int per = ctx->rasterCtasPerSm > 0 ? ctx->rasterCtasPerSm : ctx->queueCtas[L.feather];
-        const uint32_t grid =
-            std::min<uint32_t>(L.mainTiles, (uint32_t)std::max(per * ctx->smCount, 1));
-        (L.feather ? raster_queue_feather_kernel : raster_queue_kernel)<<<grid, 256, dyn, stream>>>(
-            B, tris, sortedSlots, ranges, v.Current(), S.qCursor, L.mainTiles);
-        return RIVE_CUDA_OK;
-    }
     if (L.tileLog2 == 3)
     {
         const size_t dyn = ctx->rasterCtasPerSm > 0 ? ctx->rasterPad[L.feather][0] : 0;
@@ -1311,9 +1274,24 @@ int launch_raster(rive_cuda_context* ctx,
     else
     {
         const size_t dyn = ctx->rasterCtasPerSm > 0 ? ctx->rasterPad[L.feather][1] : 0;
+        const uint32_t* order = nullptr;
+        if (S.qKeys)
+        {
+            tile_order_keys_kernel<<<(L.mainTiles + 255) / 256, 256, 0, stream>>>(
+                L.mainTiles, ranges, S.qKeys, S.qVals);
+            cub::DoubleBuffer<uint32_t> k(S.qKeys, S.qKeysAlt), v(S.qVals, S.qValsAlt);
+            size_t tb = S.qTempBytes;
+            CK(cub::DeviceRadixSort::SortPairs(S.qTemp, tb, k, v, (int)L.mainTiles, 0, 32, stream));
+            order = v.Current();
+        }
+        else if (S.order && (S.heaviestFirst || orders_tiles(L, entries)))
+        {
+            tile_order_kernel<<<1, 1024, 0, stream>>>(L.mainTiles, ranges, S.order);
+            order = S.order;
+        }
         (L.feather ? raster_tile_feather_kernel : raster_tile_kernel)<<<L.mainTiles, 256, dyn,
                                                                          stream>>>(
-            B, tris, sortedSlots, ranges);
+            B, tris, sortedSlots, ranges, order);
     }
     return RIVE_CUDA_OK;
 }
@@ -1416,7 +1394,7 @@ int enqueue_back(rive_cuda_context* ctx,
     }
     if (ctx->rasterWait)
         CK(cudaStreamWaitEvent(stream, ctx->rasterWait, 0));
-    int rc = launch_raster(ctx, L, B, S, S.tris, sortedSlots, S.ranges, stream);
+    int rc = launch_raster(ctx, L, B, S, S.tris, sortedSlots, S.ranges, entries, stream);
     stage_end(ctx, stream);
     if (rc)
         return rc;
@@ -1432,7 +1410,7 @@ size_t scan_temp_bytes(uint32_t slots)
     return b;
 }
 
-// Temporary bytes of the work queue's sort of `tiles` tile indices.
+// Temporary bytes of the tile order's sort of `tiles` tile indices.
 size_t queue_temp_bytes(uint32_t tiles)
 {
     size_t b = 0;
@@ -1576,6 +1554,8 @@ int run_batch_body(rive_cuda_context* ctx,
     CK(ctx->offsets.reserve((size_t)L.slots * 4 + 4));
     if (L.wide)
         CK(ctx->wide.reserve(L.wideBytes()));
+    if (L.mainTiles <= kOrderTiles)
+        CK(ctx->order.reserve(kOrderTiles * 4));
     if (L.planes())
         CK(ctx->featherPlanes.reserve((size_t)L.slots * 2 * sizeof(float4)));
     if (L.atlasTexels)
@@ -1594,7 +1574,7 @@ int run_batch_body(rive_cuda_context* ctx,
         CK(ctx->gridEdge.reserve(ctx->gridCapacity));
         CK(ctx->gridCounters.reserve(8));
     }
-    const bool queue = ctx->rasterQueue && L.tileLog2 == 4;
+    const bool queue = ctx->rasterQueue && L.tileLog2 == 4 && L.mainTiles > kOrderTiles;
     size_t queueBytes = 0;
     if (queue)
     {
@@ -1603,7 +1583,6 @@ int run_batch_body(rive_cuda_context* ctx,
                                 &ctx->queueValsAlt})
             CK(b->reserve((size_t)L.tiles * 4));
         CK(ctx->queueTemp.reserve(queueBytes));
-        CK(ctx->queueCursor.reserve(4));
     }
     const size_t scanBytes = scan_temp_bytes(L.slots);
     CK(ctx->scanTemp.reserve(scanBytes));
@@ -1619,6 +1598,8 @@ int run_batch_body(rive_cuda_context* ctx,
     S.grad = (uchar4*)ctx->grad.ptr;
     S.tris = (TriRecord*)ctx->tris.ptr;
     S.wide = L.wide ? (uint32_t*)ctx->wide.ptr : nullptr;
+    S.order = L.mainTiles <= kOrderTiles ? (uint32_t*)ctx->order.ptr : nullptr;
+    S.heaviestFirst = ctx->rasterQueue;
     S.featherPlanes = L.planes() ? (float4*)ctx->featherPlanes.ptr : nullptr;
     S.atlas = L.atlasTexels ? (uint16_t*)ctx->atlas.ptr : nullptr;
     S.pathImage = L.imageSlots ? (uint32_t*)ctx->pathImage.ptr : nullptr;
@@ -1645,7 +1626,6 @@ int run_batch_body(rive_cuda_context* ctx,
         S.qValsAlt = (uint32_t*)ctx->queueValsAlt.ptr;
         S.qTemp = ctx->queueTemp.ptr;
         S.qTempBytes = queueBytes;
-        S.qCursor = (uint32_t*)ctx->queueCursor.ptr;
     }
     BatchTables B = write_tables(ctx, in, L, S, (uint8_t*)ctx->hTables[tslot].ptr);
     CK(cudaMemcpyAsync(S.tables, ctx->hTables[tslot].ptr, L.tableBytes, cudaMemcpyHostToDevice,
@@ -1873,13 +1853,13 @@ void rive_cuda_context_destroy(rive_cuda_context* ctx)
         }
     }
     for (DeviceBuffer* b : {&ctx->tess, &ctx->grad, &ctx->tris, &ctx->tileCounts, &ctx->tileMasks,
-                            &ctx->offsets, &ctx->featherPlanes, &ctx->wide,
+                            &ctx->offsets, &ctx->featherPlanes, &ctx->wide, &ctx->order,
                             &ctx->keys, &ctx->vals, &ctx->keysAlt, &ctx->valsAlt,
                             &ctx->sortTemp, &ctx->scanTemp, &ctx->ranges, &ctx->dTables,
                             &ctx->pathGrids, &ctx->gridWinding, &ctx->gridEdge,
                             &ctx->gridCounters, &ctx->queueKeys, &ctx->queueVals,
                             &ctx->queueKeysAlt, &ctx->queueValsAlt, &ctx->queueTemp,
-                            &ctx->queueCursor, &ctx->atlas, &ctx->pathImage})
+                            &ctx->atlas, &ctx->pathImage})
         b->release();
     for (int i = 0; i < rive_cuda_context::kTableRing; ++i)
     {
@@ -2249,7 +2229,8 @@ void graph_free(rive_cuda_graph* g)
                             &g->sortTemp, &g->ranges, &g->error, &g->featherPlanes,
                             &g->pathGrids, &g->gridWinding, &g->gridEdge, &g->gridCounters,
                             &g->queueKeys, &g->queueVals, &g->queueKeysAlt, &g->queueValsAlt,
-                            &g->queueTemp, &g->queueCursor, &g->atlas, &g->pathImage, &g->wide})
+                            &g->queueTemp, &g->atlas, &g->pathImage, &g->wide,
+                            &g->order})
         b->release();
     if (g->hError)
         cudaFreeHost(g->hError);
@@ -2279,6 +2260,8 @@ int graph_build(rive_cuda_context* ctx,
     CK(g->offsets.reserve((size_t)L.slots * 4 + 4));
     if (L.wide)
         CK(g->wide.reserve(L.wideBytes()));
+    if (L.mainTiles <= kOrderTiles)
+        CK(g->order.reserve(kOrderTiles * 4));
     if (L.planes())
         CK(g->featherPlanes.reserve((size_t)L.slots * 2 * sizeof(float4)));
     if (L.atlasTexels)
@@ -2287,7 +2270,7 @@ int graph_build(rive_cuda_context* ctx,
         CK(g->pathImage.reserve((size_t)std::max(L.paths, 1u) * 4));
     CK(g->ranges.reserve((size_t)L.tiles * sizeof(uint2)));
     CK(g->error.reserve(4));
-    const bool queue = ctx->rasterQueue && L.tileLog2 == 4;
+    const bool queue = ctx->rasterQueue && L.tileLog2 == 4 && L.mainTiles > kOrderTiles;
     size_t queueBytes = 0;
     if (queue)
     {
@@ -2295,7 +2278,6 @@ int graph_build(rive_cuda_context* ctx,
         for (DeviceBuffer* b : {&g->queueKeys, &g->queueVals, &g->queueKeysAlt, &g->queueValsAlt})
             CK(b->reserve((size_t)L.tiles * 4));
         CK(g->queueTemp.reserve(queueBytes));
-        CK(g->queueCursor.reserve(4));
     }
     const size_t scanBytes = scan_temp_bytes(L.slots);
     CK(g->scanTemp.reserve(scanBytes));
@@ -2307,6 +2289,8 @@ int graph_build(rive_cuda_context* ctx,
     S.grad = (uchar4*)g->grad.ptr;
     S.tris = (TriRecord*)g->tris.ptr;
     S.wide = L.wide ? (uint32_t*)g->wide.ptr : nullptr;
+    S.order = L.mainTiles <= kOrderTiles ? (uint32_t*)g->order.ptr : nullptr;
+    S.heaviestFirst = ctx->rasterQueue;
     S.featherPlanes = L.planes() ? (float4*)g->featherPlanes.ptr : nullptr;
     S.atlas = L.atlasTexels ? (uint16_t*)g->atlas.ptr : nullptr;
     S.pathImage = L.imageSlots ? (uint32_t*)g->pathImage.ptr : nullptr;
@@ -2325,7 +2309,6 @@ int graph_build(rive_cuda_context* ctx,
         S.qValsAlt = (uint32_t*)g->queueValsAlt.ptr;
         S.qTemp = g->queueTemp.ptr;
         S.qTempBytes = queueBytes;
-        S.qCursor = (uint32_t*)g->queueCursor.ptr;
     }
     std::vector<uint8_t> h(L.tableBytes);
     // The graph's winding grids: a cell pool sized like the context's, grown

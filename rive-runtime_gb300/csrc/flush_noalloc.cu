@@ -56,11 +56,13 @@ __global__ void tile_ranges_kernel(uint32_t pairCount,
 __global__ void raster_tile_kernel(BatchTables B,
                                    const TriRecord* tris,
                                    const uint32_t* sortedSlots,
-                                   const uint2* ranges);
+                                   const uint2* ranges,
+                                   const uint32_t* order);
 __global__ void raster_tile_feather_kernel(BatchTables B,
                                    const TriRecord* tris,
                                    const uint32_t* sortedSlots,
-                                   const uint2* ranges);
+                                   const uint2* ranges,
+                                   const uint32_t* order);
 } // namespace rivecuda
 
 using namespace rivecuda;
@@ -436,7 +438,7 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
         sortedSlots = v.Current();
     }
     (feather ? raster_tile_feather_kernel : raster_tile_kernel)<<<tiles, 256, 0, stream>>>(
-        B, tris, sortedSlots, ranges);
+        B, tris, sortedSlots, ranges, nullptr);
     CKN(cudaGetLastError());
 
     // Device status of this flush (overflow and range flags of the kernels).

@@ -3826,47 +3826,24 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
 }
 
 // The raster kernels, each without and with the feather paths (the host
-// launches the feather variant only for batches with ENABLE_FEATHER draws).
+// launches the feather variant only for batches with ENABLE_FEATHER draws). The
+// 16x16 one takes its tiles in the order of `order` (heaviest first), or as
+// they come when it is null. The hardware hands out CTAs in turn, so an ordered
+// grid is the work queue: a persistent grid with an atomic cursor over the same
+// order was slower (full-feature 2048x2048 frame 3.70 against 3.57 ms).
 #define RIVE_RASTER_KERNELS(NAME, FEATHER)                                                        \
     __global__ void __launch_bounds__(256, RIVE_RASTER_MIN_BLOCKS(FEATHER)) NAME(                           \
         BatchTables B, const TriRecord* __restrict__ tris,                                        \
-        const uint32_t* __restrict__ sortedSlots, const uint2* __restrict__ ranges)               \
+        const uint32_t* __restrict__ sortedSlots, const uint2* __restrict__ ranges,               \
+        const uint32_t* __restrict__ order)                                                       \
     {                                                                                             \
         __shared__ RasterShared<4> sh;                                                            \
-        raster_tile<4, FEATHER>(B, tris, sortedSlots, ranges, sh, blockIdx.x);                    \
+        raster_tile<4, FEATHER>(B, tris, sortedSlots, ranges, sh,                                 \
+                                order ? order[blockIdx.x] : blockIdx.x);                          \
     }
 RIVE_RASTER_KERNELS(raster_tile_kernel, false)
 RIVE_RASTER_KERNELS(raster_tile_feather_kernel, true)
 #undef RIVE_RASTER_KERNELS
-
-// The work-queue form of the 16x16 raster: a persistent grid (as many CTAs
-// as stay resident) in which each CTA takes its next tile from an atomic
-// cursor over `order`, the batch's tiles sorted by bin entries, heaviest
-// first, so the longest tiles start first and the last wave has no straggler
-// behind it. The cursor starts at zero on every launch.
-#define RIVE_RASTER_QUEUE_KERNELS(NAME, FEATHER)                                                  \
-    __global__ void __launch_bounds__(256, RIVE_RASTER_MIN_BLOCKS(FEATHER)) NAME(                           \
-        BatchTables B, const TriRecord* __restrict__ tris,                                        \
-        const uint32_t* __restrict__ sortedSlots, const uint2* __restrict__ ranges,               \
-        const uint32_t* __restrict__ order, uint32_t* __restrict__ cursor, uint32_t tiles)        \
-    {                                                                                             \
-        __shared__ RasterShared<4> sh;                                                            \
-        __shared__ uint32_t sNext;                                                                \
-        for (;;)                                                                                  \
-        {                                                                                         \
-            __syncthreads(); /* the last tile is done with the shared state */                    \
-            if (threadIdx.x == 0)                                                                 \
-                sNext = atomicAdd(cursor, 1u);                                                    \
-            __syncthreads();                                                                      \
-            const uint32_t t = sNext;                                                             \
-            if (t >= tiles)                                                                       \
-                break;                                                                            \
-            raster_tile<4, FEATHER>(B, tris, sortedSlots, ranges, sh, order[t]);                  \
-        }                                                                                         \
-    }
-RIVE_RASTER_QUEUE_KERNELS(raster_queue_kernel, false)
-RIVE_RASTER_QUEUE_KERNELS(raster_queue_feather_kernel, true)
-#undef RIVE_RASTER_QUEUE_KERNELS
 
 // The feather atlas pass (render_atlas.glsl with the floating-point target
 // and fixed-function blending; the atlas pipelines of gpu.hpp:2076-2080):
@@ -3951,7 +3928,59 @@ RIVE_ATLAS_KERNEL(raster_atlas_kernel, 4)
 RIVE_ATLAS_KERNEL(raster_atlas32_kernel, 5)
 #undef RIVE_ATLAS_KERNEL
 
-// Sort keys of the work queue: per tile, its bin entries inverted (a plain
+// The tiles of a batch of at most kOrderTiles, heaviest first to within an
+// eighth: one CTA counts them into 256 buckets (the leading four bits of a
+// tile's bin entries and their exponent, descending), per warp so that equal
+// tiles do not queue at one counter, and gives each its place. Bound by
+// latency: about 5 us for 16,384 tiles, against 45 us for a radix sort.
+__global__ void __launch_bounds__(1024, 1) tile_order_kernel(uint32_t tiles,
+                                                             const uint2* __restrict__ ranges,
+                                                             uint32_t* __restrict__ order)
+{
+    constexpr int kBuckets = 256, kWarps = 32, kPer = kBuckets * kWarps / 1024;
+    __shared__ uint32_t count[kBuckets * kWarps]; // [bucket][warp]
+    __shared__ uint32_t sums[kWarps];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    auto bucket = [&](uint32_t i) {
+        const uint2 r = ranges[i];
+        const uint32_t n = r.y > r.x ? r.y - r.x : 0u;
+        const uint32_t bits = __float_as_uint((float)n) >> 20; // exponent, 3 bits of mantissa
+        return 255u - min(n ? bits - (127u << 3) : 0u, 255u);
+    };
+    for (int i = threadIdx.x; i < kBuckets * kWarps; i += 1024)
+        count[i] = 0;
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < tiles; i += 1024)
+        atomicAdd(&count[bucket(i) * kWarps + warp], 1u);
+    __syncthreads();
+    uint32_t mine[kPer], total = 0;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j)
+    {
+        mine[j] = total;
+        total += count[threadIdx.x * kPer + j];
+    }
+    uint32_t scan = total;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, scan, o);
+        scan += lane >= o ? v : 0u;
+    }
+    if (lane == 31)
+        sums[warp] = scan;
+    __syncthreads();
+    uint32_t before = lane < warp ? sums[lane] : 0u;
+    before = __reduce_add_sync(0xffffffffu, before) + scan - total;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j)
+        count[threadIdx.x * kPer + j] = before + mine[j];
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < tiles; i += 1024)
+        order[atomicAdd(&count[bucket(i) * kWarps + warp], 1u)] = i;
+}
+
+// Sort keys of the tile order of larger batches: per tile, its bin entries inverted (a plain
 // ascending sort then puts the heaviest tile first), and its index.
 __global__ void __launch_bounds__(256) tile_order_keys_kernel(uint32_t tiles,
                                                               const uint2* __restrict__ ranges,

@@ -367,6 +367,10 @@ struct WideScatter
 // strip for every warp of 38 triangles.
 constexpr uint32_t kWideBlocks = 304;
 
+// Batches the raster grid orders its tiles for (tile_order_kernel).
+constexpr uint32_t kOrderMinTiles = 512;
+constexpr uint32_t kOrderTiles = 16384;
+
 // Index j with base[j] <= i < base[j + 1] (empty ranges skipped), n >= 1.
 __device__ __forceinline__ uint32_t find_range(const uint32_t* __restrict__ base, uint32_t n,
                                                uint32_t i)

@@ -512,8 +512,8 @@ class Context:
                    "set_winding_tiles")
 
     def set_raster_queue(self, on: bool):
-        """The raster as a persistent work queue over heaviest-first tiles
-        (16-pixel tiles), or one CTA per tile (default); same image."""
+        """Every batch's tiles heaviest first (16-pixel tiles), not only
+        those the raster orders by itself (default); same image."""
         self.check(self.lib.rive_cuda_set_raster_queue(self.h, 1 if on else 0),
                    "set_raster_queue")
 
