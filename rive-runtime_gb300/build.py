@@ -15,7 +15,8 @@ REPO = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 OUT = os.path.join(PKG, "_build")
 LIB = os.path.join(OUT, "librive_cuda.so")
-SOURCES = ["context.cu", "kernels_tess.cu", "kernels_raster.cu", "flush_noalloc.cu"]
+SOURCES = ["context.cu", "kernels_tess.cu", "kernels_raster.cu", "kernels_small.cu",
+           "flush_noalloc.cu"]
 HEADERS = ["rive_cuda_internal.cuh", "rive_fp32_math.h"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]

@@ -56,7 +56,12 @@ __global__ void center_setup_kernel(BatchTables B,
                                     TriRecord* tris,
                                     uint32_t* tileCounts,
                                     uint8_t* tileMasks);
-__global__ void scene_uniforms_kernel(FlushParams* scenes, uint32_t sceneCount, uint32_t* wide);
+__global__ void flush_start_kernel(FlushStart F);
+__global__ void small_scan_kernel(uint32_t slots, const uint32_t* counts, uint32_t* offsets,
+                                  uint32_t* hostTotal);
+__global__ void small_sort_kernel(const uint32_t* entryTotal, uint32_t capacity, bool guarded, int keyBits,
+                                  const uint16_t* keys, const uint32_t* vals, uint16_t* sortedKeys,
+                                  uint32_t* sortedVals, uint2* ranges);
 __global__ void wide_count_kernel(BatchTables B, const TriRecord* tris, uint32_t* tileCounts);
 __global__ void bin_fill_kernel(const uint32_t* pairTotal,
                                 uint32_t capacity,
@@ -330,7 +335,7 @@ struct rive_cuda_context
     // Raster configuration (rive_cuda_set_raster_config).
     int tileLog2 = kTileLog2;
     int rasterCtasPerSm = 0; // 0: as many as fit
-    bool raster32Ready = false;
+    bool raster32Ready = false, smallSortReady = false;
     size_t rasterPad[2][2] = {};      // [feather variant][8 or 16 pixel kernel]: padding
     int rasterPadFor[2] = {-1, -1};   // the CTAs-per-SM limit it was found for
     // Stage timing (rive_cuda_set_profiling).
@@ -940,7 +945,7 @@ BatchTables write_tables(rive_cuda_context* ctx,
         P.wireframe = d->wireframe;
         P.loadClear = d->color_load_action == RIVE_CUDA_LOAD_CLEAR;
         P.clearColorPremulRGBA = premul_rgba8(d->color_clear_value);
-        P.pathIDGranularity = 1; // replaced on the device by scene_uniforms_kernel
+        P.pathIDGranularity = 1; // replaced on the device by flush_start_kernel
         P.error = S.error;
         P.fb = in[i].fb;
         const uint32_t ts = 1u << L.tileLog2;
@@ -1109,20 +1114,32 @@ BatchTables write_tables(rive_cuda_context* ctx,
     return B;
 }
 
+// CTAs of flush_start_kernel: a thread per element, up to four CTAs per SM.
+uint32_t flush_start_blocks(const FlushStart& F)
+{
+    const uint32_t most = std::max({F.sceneCount, F.gradVectors, F.tiles, 1u});
+    return std::min((most + 255) / 256, 608u);
+}
+
 // Enqueues the passes up to and including the scan of tile counts (so
-// S.offsets[L.slots] holds the batch's bin-entry total on the device).
+// S.offsets[L.slots] holds the batch's bin-entry total on the device), and
+// brings the total to *hostTotal (pinned) unless that is null.
 int enqueue_front(rive_cuda_context* ctx,
                   const BatchLayout& L,
                   const BatchTables& B,
                   const Scratch& S,
-                  cudaStream_t stream)
+                  cudaStream_t stream,
+                  uint32_t* hostTotal)
 {
-    scene_uniforms_kernel<<<(L.scenes() + 127) / 128, 128, 0, stream>>>(
-        const_cast<FlushParams*>(B.scenes), L.scenes(), B.wide);
-    // Texels no span covers are never sampled; zero them so the gradient
-    // texture is deterministic.
-    CK(cudaMemsetAsync(S.grad, 0, L.gradBytes(), stream));
-    CK(cudaMemsetAsync(S.ranges, 0, (size_t)L.tiles * sizeof(uint2), stream));
+    FlushStart F = {};
+    F.scenes = const_cast<FlushParams*>(B.scenes);
+    F.sceneCount = L.scenes();
+    F.wide = B.wide;
+    F.grad = (uint4*)S.grad;
+    F.gradVectors = (uint32_t)(L.gradBytes() / 16);
+    F.ranges = S.ranges;
+    F.tiles = L.tiles;
+    flush_start_kernel<<<flush_start_blocks(F), 256, 0, stream>>>(F);
     if (L.imageSlots)
         CK(cudaMemsetAsync(S.pathImage, 0xff, (size_t)std::max(L.paths, 1u) * 4, stream));
     if (L.winding)
@@ -1179,10 +1196,21 @@ int enqueue_front(rive_cuda_context* ctx,
             wide_count_kernel<<<kWideBlocks, 256, 0, stream>>>(B, S.tris, S.counts);
         stage_end(ctx, stream);
         stage_begin(ctx, RIVE_CUDA_STAGE_BIN, stream);
-        size_t tempBytes = S.scanTempBytes;
-        CK(cudaMemsetAsync(S.offsets, 0, 4, stream));
-        CK(cub::DeviceScan::InclusiveSum(S.scanTemp, tempBytes, S.counts, S.offsets + 1, L.slots,
-                                         stream));
+        if (L.slots <= kSmallScanSlots)
+        {
+            small_scan_kernel<<<kSmallCluster, 1024, 0, stream>>>(L.slots, S.counts, S.offsets,
+                                                                  hostTotal);
+        }
+        else
+        {
+            size_t tempBytes = S.scanTempBytes;
+            CK(cudaMemsetAsync(S.offsets, 0, 4, stream));
+            CK(cub::DeviceScan::InclusiveSum(S.scanTemp, tempBytes, S.counts, S.offsets + 1,
+                                             L.slots, stream));
+            if (hostTotal)
+                CK(cudaMemcpyAsync(hostTotal, S.offsets + L.slots, 4, cudaMemcpyDeviceToHost,
+                                   stream));
+        }
         stage_end(ctx, stream);
     }
     return RIVE_CUDA_OK;
@@ -1211,6 +1239,12 @@ size_t occupancy_pad(const void* fn, int threads, int ctas)
 // configuration needs. Called before any stream capture, never inside one.
 int prepare_raster(rive_cuda_context* ctx)
 {
+    if (!ctx->smallSortReady)
+    {
+        CK(cudaFuncSetAttribute(small_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                kSmallSortSmemBytes));
+        ctx->smallSortReady = true;
+    }
     if (ctx->tileLog2 == 5 && !ctx->raster32Ready)
     {
         CK(cudaFuncSetAttribute(raster_tile32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1322,10 +1356,11 @@ int enqueue_back(rive_cuda_context* ctx,
             wide.blocks = kWideBlocks;
         }
         const uint32_t binBlocks = wide.blocks + (L.slots + 255) / 256;
+        const bool smallSort = S.keys16 && entries <= kSmallSortEntries;
         if (S.keys16)
         {
             uint16_t* keys = (uint16_t*)S.keys;
-            if (padded)
+            if (padded && !smallSort)
                 bin_fill16_kernel<<<(entries + 255) / 256, 256, 0, stream>>>(
                     S.offsets + L.slots, entries, L.tiles, keys);
             bin_scatter16_kernel<<<binBlocks, 256, 0, stream>>>(
@@ -1351,7 +1386,15 @@ int enqueue_back(rive_cuda_context* ctx,
         cub::DoubleBuffer<uint32_t> v(S.vals, S.valsAlt);
         size_t tempBytes = S.sortTempBytes;
         stage_begin(ctx, RIVE_CUDA_STAGE_SORT, stream);
-        if (S.keys16)
+        if (smallSort)
+        {
+            // Also writes the ranges, or leaves them empty on overflow.
+            small_sort_kernel<<<kSmallCluster, 1024, kSmallSortSmemBytes, stream>>>(
+                S.offsets + L.slots, entries, guarded, L.endBit(), (const uint16_t*)S.keys, S.vals,
+                (uint16_t*)S.keysAlt, S.valsAlt, S.ranges);
+            v.selector = 1;
+        }
+        else if (S.keys16)
         {
             cub::DoubleBuffer<uint16_t> k((uint16_t*)S.keys, (uint16_t*)S.keysAlt);
             CK(cub::DeviceRadixSort::SortPairs(S.sortTemp, tempBytes, k, v, (int)entries, 0,
@@ -1370,7 +1413,7 @@ int enqueue_back(rive_cuda_context* ctx,
         // A speculative pass whose total did not fit: every range emptied,
         // so the raster leaves the target as it was (or clears it) until the
         // back half runs again with exact bins.
-        if (guarded)
+        if (guarded && !smallSort)
             ranges_guard_kernel<<<(L.tiles + 255) / 256, 256, 0, stream>>>(S.offsets + L.slots,
                                                                           entries, S.ranges,
                                                                           L.tiles);
@@ -1634,13 +1677,15 @@ int run_batch_body(rive_cuda_context* ctx,
         CK(cudaEventCreateWithFlags(&ctx->tablesCopied[tslot], cudaEventDisableTiming));
     CK(cudaEventRecord(ctx->tablesCopied[tslot], stream));
 
-    rc = enqueue_front(ctx, L, B, S, stream);
-    if (rc)
-        return rc;
     // Speculative bins: a single flush on the context's stream, once a total
     // has been seen, without winding records (their cell counts are read
     // back too).
-    if (speculative && ctx->speculate && n == 1 && L.slots && !L.winding && ctx->binHighWater)
+    const bool speculates =
+        speculative && ctx->speculate && n == 1 && L.slots && !L.winding && ctx->binHighWater;
+    rc = enqueue_front(ctx, L, B, S, stream, speculates ? ctx->hSpecTotal : ctx->hPairs);
+    if (rc)
+        return rc;
+    if (speculates)
     {
         if (!ctx->pending)
         {
@@ -1656,8 +1701,6 @@ int run_batch_body(rive_cuda_context* ctx,
         if (rc)
             return rc;
         S.binError = ctx->dSpecOverflow;
-        CK(cudaMemcpyAsync(ctx->hSpecTotal, S.offsets + L.slots, 4, cudaMemcpyDeviceToHost,
-                           stream));
         CK(cudaEventRecord(p.counted, stream));
         rc = enqueue_back(ctx, L, B, S, p.capacity, true, stream, true);
         if (rc)
@@ -1682,7 +1725,6 @@ int run_batch_body(rive_cuda_context* ctx,
     uint32_t pairs = 0, windingEntries = 0;
     if (L.slots)
     {
-        CK(cudaMemcpyAsync(ctx->hPairs, S.offsets + L.slots, 4, cudaMemcpyDeviceToHost, stream));
         if (L.winding)
             CK(cudaMemcpyAsync(ctx->hGridCounters, S.gridCounters, 8, cudaMemcpyDeviceToHost,
                                stream));
@@ -2344,15 +2386,13 @@ int graph_build(rive_cuda_context* ctx,
         // (The grids' cells too, with one more run if the pool was short.)
         for (int pass = 0; pass < 2; ++pass)
         {
-            rc = enqueue_front(ctx, L, B, S, g->stream);
+            g->hError[1] = 0;
+            rc = enqueue_front(ctx, L, B, S, g->stream, g->hError);
             if (rc)
             {
                 ctx->profiling = profiling;
                 return rc;
             }
-            CK(cudaMemcpyAsync(g->hError, S.offsets + L.slots, 4, cudaMemcpyDeviceToHost,
-                               g->stream));
-            g->hError[1] = 0;
             if (L.winding)
                 CK(cudaMemcpyAsync(g->hError + 1, S.gridCounters, 4, cudaMemcpyDeviceToHost,
                                    g->stream));
@@ -2375,11 +2415,12 @@ int graph_build(rive_cuda_context* ctx,
     {
         for (DeviceBuffer* b : {&g->keys, &g->vals, &g->keysAlt, &g->valsAlt})
             CK(b->reserve((size_t)capacity * 4));
-        S.keys = (uint32_t*)g->keys.ptr;
+        S.keys16 = L.keys16();
+        S.keys = g->keys.ptr;
         S.vals = (uint32_t*)g->vals.ptr;
-        S.keysAlt = (uint32_t*)g->keysAlt.ptr;
+        S.keysAlt = g->keysAlt.ptr;
         S.valsAlt = (uint32_t*)g->valsAlt.ptr;
-        S.sortTempBytes = sort_temp_bytes(capacity, L.endBit());
+        S.sortTempBytes = sort_temp_bytes(capacity, L.endBit(), S.keys16);
         CK(g->sortTemp.reserve(S.sortTempBytes));
         S.sortTemp = g->sortTemp.ptr;
     }
@@ -2392,7 +2433,7 @@ int graph_build(rive_cuda_context* ctx,
     cudaError_t e = cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess)
     {
-        rc = enqueue_front(ctx, L, B, S, g->stream);
+        rc = enqueue_front(ctx, L, B, S, g->stream, nullptr);
         if (!rc)
             rc = enqueue_back(ctx, L, B, S, capacity, true, g->stream);
         e = cudaStreamEndCapture(g->stream, &g->graph);

@@ -11,8 +11,8 @@
 #include "rive_cuda_internal.cuh"
 
 #include <cub/device/device_radix_sort.cuh>
-#include <cub/device/device_scan.cuh>
 
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -35,9 +35,14 @@ __global__ void outer_setup_kernel(BatchTables B,
                                    TriRecord* tris,
                                    uint32_t* tileCounts,
                                    uint8_t* tileMasks);
-__global__ void scene_uniforms_kernel(FlushParams* scenes, uint32_t sceneCount, uint32_t* wide);
+__global__ void flush_start_kernel(FlushStart F);
+__global__ void small_scan_kernel(uint32_t slots, const uint32_t* counts, uint32_t* offsets,
+                                  uint32_t* hostTotal);
+__global__ void small_sort_kernel(const uint32_t* entryTotal, uint32_t capacity, bool guarded, int keyBits,
+                                  const uint16_t* keys, const uint32_t* vals, uint16_t* sortedKeys,
+                                  uint32_t* sortedVals, uint2* ranges);
 __global__ void wide_count_kernel(BatchTables B, const TriRecord* tris, uint32_t* tileCounts);
-__global__ void bin_scatter_kernel(uint32_t slotCount,
+__global__ void bin_scatter16_kernel(uint32_t slotCount,
                                    int tileLog2,
                                    const uint2* sceneTiles,
                                    const TriRecord* tris,
@@ -46,13 +51,13 @@ __global__ void bin_scatter_kernel(uint32_t slotCount,
                                    const uint32_t* offsets,
                                    uint32_t capacity,
                                    uint32_t* error,
-                                   uint32_t* keys,
+                                   uint16_t* keys,
                                    uint32_t* vals,
                                    WideScatter wide);
-__global__ void tile_ranges_kernel(uint32_t pairCount,
-                                   uint32_t tileCount,
-                                   const uint32_t* keys,
-                                   uint2* ranges);
+__global__ void tile_ranges16_kernel(uint32_t pairCount,
+                                     uint32_t tileCount,
+                                     const uint16_t* keys,
+                                     uint2* ranges);
 __global__ void raster_tile_kernel(BatchTables B,
                                    const TriRecord* tris,
                                    const uint32_t* sortedSlots,
@@ -92,7 +97,7 @@ constexpr size_t kKeysAltOff = kValsOff + align256(kPairBytes);
 constexpr size_t kValsAltOff = kKeysAltOff + align256(kPairBytes);
 constexpr size_t kRangesOff = kValsAltOff + align256(kPairBytes);
 constexpr size_t kScanTempOff = kRangesOff + align256(kMaxTiles * sizeof(uint2));
-constexpr size_t kScanTempBytes = 64u << 10;
+constexpr size_t kScanTempBytes = 64u << 10; // (kept in the layout; the scan needs none)
 constexpr size_t kSortTempOff = kScanTempOff + kScanTempBytes;
 constexpr size_t kSortTempBytes = 4u << 20;
 // Launch tables of the flush (a batch of one): FlushParams, prefix arrays and
@@ -251,6 +256,8 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
         if (!gTablesUp[dev])
         {
             CKN(ensure_feather_lut(dev));
+            CKN(cudaFuncSetAttribute(small_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     kSmallSortSmemBytes));
             gTablesUp[dev] = true;
         }
         pool = (uint8_t*)p;
@@ -290,7 +297,7 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
     P.tilesX = (d->render_target_width + kTileSize - 1) / kTileSize;
 
     // FlushUniforms (renderer/include/rive/renderer/gpu.hpp:1466-1537) stay on
-    // the device; scene_uniforms_kernel copies the fields the passes use.
+    // the device; flush_start_kernel copies the fields the passes use.
     P.uniforms = (const uint8_t*)buffers->flush_uniforms + d->flush_uniform_offset_bytes;
     P.pathIDGranularity = 1;
 
@@ -331,8 +338,6 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
     // Wide triangles: their list and strips sit in the alternate keys, which
     // only the sort uses, after them.
     uint32_t* const wideList = tiles > (uint32_t)kWideTiles ? (uint32_t*)(pool + kKeysAltOff) : nullptr;
-    scene_uniforms_kernel<<<1, 32, 0, stream>>>((FlushParams*)(dTab + kTabScenes), 1u,
-                                             wideList);
     BatchTables B = {};
     B.scenes = (const FlushParams*)(dTab + kTabScenes);
     B.gradSpanBase = (const uint32_t*)(dTab + kTabPrefix);
@@ -360,13 +365,19 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
         B.wideStrips = wideList + 1 + kWideCap;
     }
 
-    // What must start at zero on every call: the error word, the tile
-    // ranges, the gradient rows in use and the scan's leading offset.
+    // What must start at zero on every call: the error word, the tile ranges,
+    // the gradient rows in use, the wide triangles' counter.
     uint2* ranges = (uint2*)(pool + kRangesOff);
-    CKN(cudaMemsetAsync(dError, 0, 4, stream));
-    CKN(cudaMemsetAsync(ranges, 0, (size_t)tiles * sizeof(uint2), stream));
-    if (d->grad_data_height)
-        CKN(cudaMemsetAsync(P.grad, 0, (size_t)kGradTextureWidth * d->grad_data_height * 4, stream));
+    FlushStart F = {};
+    F.scenes = (FlushParams*)(dTab + kTabScenes);
+    F.sceneCount = 1;
+    F.wide = wideList;
+    F.error = dError;
+    F.grad = (uint4*)P.grad;
+    F.gradVectors = (uint32_t)(kGradTextureWidth / 4) * d->grad_data_height;
+    F.ranges = ranges;
+    F.tiles = tiles;
+    flush_start_kernel<<<(std::max(F.gradVectors, tiles) + 255) / 256, 256, 0, stream>>>(F);
 
     if (d->grad_span_count)
         color_ramp_kernel<<<d->grad_span_count, 128, 0, stream>>>(B);
@@ -387,15 +398,8 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
                                                                                masks);
         if (wideList)
             wide_count_kernel<<<kWideBlocks, 256, 0, stream>>>(B, tris, counts);
-        size_t tempBytes = 0;
-        CKN(cub::DeviceScan::InclusiveSum(nullptr, tempBytes, counts, offs + 1, slots, stream));
-        if (tempBytes > kScanTempBytes)
-            return fail(err, err_len, RIVE_CUDA_ERR_OUT_OF_MEMORY,
-                        "scan needs %zu temporary bytes, pool holds %zu", tempBytes,
-                        kScanTempBytes);
-        CKN(cudaMemsetAsync(offs, 0, 4, stream));
-        CKN(cub::DeviceScan::InclusiveSum(pool + kScanTempOff, tempBytes, counts, offs + 1, slots,
-                                          stream));
+        static_assert(kMaxSlots <= kSmallScanSlots, "the one-cluster scan holds every flush");
+        small_scan_kernel<<<kSmallCluster, 1024, 0, stream>>>(slots, counts, offs, nullptr);
         CKN(cudaMemcpyAsync(&pairs, offs + slots, 4, cudaMemcpyDeviceToHost, stream));
         CKN(cudaStreamSynchronize(stream));
         if (pairs > RIVE_CUDA_NOALLOC_MAX_BIN_ENTRIES)
@@ -404,7 +408,8 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
                         "written)",
                         pairs, RIVE_CUDA_NOALLOC_MAX_BIN_ENTRIES);
     }
-    uint32_t* keys = (uint32_t*)(pool + kKeysOff);
+    uint16_t* keys = (uint16_t*)(pool + kKeysOff); // tiles are at most kMaxTiles
+    static_assert(kMaxTiles < 0xffffu, "16-bit bin keys");
     uint32_t* vals = (uint32_t*)(pool + kValsOff);
     const uint32_t* sortedSlots = nullptr;
     if (pairs)
@@ -417,24 +422,34 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
             wide.cap = B.wideCap;
             wide.blocks = kWideBlocks;
         }
-        bin_scatter_kernel<<<wide.blocks + (slots + 255) / 256, 256, 0, stream>>>(
+        bin_scatter16_kernel<<<wide.blocks + (slots + 255) / 256, 256, 0, stream>>>(
             slots, kTileLog2, B.sceneTiles, tris, counts, masks, offs, pairs, dError, keys, vals,
             wide);
         int endBit = 1;
         while ((1u << endBit) <= tiles)
             ++endBit;
-        cub::DoubleBuffer<uint32_t> k(keys, (uint32_t*)(pool + kKeysAltOff));
+        cub::DoubleBuffer<uint16_t> k(keys, (uint16_t*)(pool + kKeysAltOff));
         cub::DoubleBuffer<uint32_t> v(vals, (uint32_t*)(pool + kValsAltOff));
-        size_t tempBytes = 0;
-        CKN(cub::DeviceRadixSort::SortPairs(nullptr, tempBytes, k, v, (int)pairs, 0, endBit, stream));
-        if (tempBytes > kSortTempBytes)
-            return fail(err, err_len, RIVE_CUDA_ERR_OUT_OF_MEMORY,
-                        "sort needs %zu temporary bytes, pool holds %zu", tempBytes,
-                        kSortTempBytes);
-        CKN(cub::DeviceRadixSort::SortPairs(pool + kSortTempOff, tempBytes, k, v, (int)pairs, 0,
-                                            endBit, stream));
-        tile_ranges_kernel<<<(pairs + 255) / 256, 256, 0, stream>>>(pairs, tiles, k.Current(),
-                                                                  ranges);
+        if (pairs <= kSmallSortEntries)
+        {
+            small_sort_kernel<<<kSmallCluster, 1024, kSmallSortSmemBytes, stream>>>(
+                offs + slots, pairs, false, endBit, keys, vals, k.Alternate(), v.Alternate(), ranges);
+            v.selector = 1;
+        }
+        else
+        {
+            size_t tempBytes = 0;
+            CKN(cub::DeviceRadixSort::SortPairs(nullptr, tempBytes, k, v, (int)pairs, 0, endBit,
+                                                stream));
+            if (tempBytes > kSortTempBytes)
+                return fail(err, err_len, RIVE_CUDA_ERR_OUT_OF_MEMORY,
+                            "sort needs %zu temporary bytes, pool holds %zu", tempBytes,
+                            kSortTempBytes);
+            CKN(cub::DeviceRadixSort::SortPairs(pool + kSortTempOff, tempBytes, k, v, (int)pairs, 0,
+                                                endBit, stream));
+            tile_ranges16_kernel<<<(pairs + 255) / 256, 256, 0, stream>>>(pairs, tiles, k.Current(),
+                                                                        ranges);
+        }
         sortedSlots = v.Current();
     }
     (feather ? raster_tile_feather_kernel : raster_tile_kernel)<<<tiles, 256, 0, stream>>>(

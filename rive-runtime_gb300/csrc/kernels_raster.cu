@@ -2103,26 +2103,6 @@ __global__ void __launch_bounds__(256) wide_count_kernel(BatchTables B,
     }
 }
 
-// FlushUniforms fields the passes use (gpu.hpp:1466-1537: pathIDGranularity
-// at byte 72, ditherScale at 88, ditherBias at 92), read on the device so no
-// pass waits for the host. One thread per flush of the batch.
-// The first of them also empties the list of wide triangles, if there is one.
-__global__ void scene_uniforms_kernel(FlushParams* __restrict__ scenes, uint32_t sceneCount,
-                                      uint32_t* __restrict__ wide)
-{
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= sceneCount)
-        return;
-    if (i == 0 && wide)
-        *wide = 0;
-    const uint8_t* u = scenes[i].uniforms;
-    const uint32_t granularity = *reinterpret_cast<const uint32_t*>(u + 72);
-    scenes[i].pathIDGranularity = granularity ? granularity : 1u;
-    scenes[i].ditherScale = *reinterpret_cast<const float*>(u + 88);
-    scenes[i].ditherBias = *reinterpret_cast<const float*>(u + 92);
-    scenes[i].mipLodBias = *reinterpret_cast<const float*>(u + 80);
-}
-
 // Fixed-capacity binning: entries [total, capacity) get the sentinel key (one
 // past the batch's last tile) so a sort over the whole capacity leaves them
 // at the end, where tile_ranges_kernel ignores them.

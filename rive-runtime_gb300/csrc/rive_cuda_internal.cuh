@@ -367,6 +367,26 @@ struct WideScatter
 // strip for every warp of 38 triangles.
 constexpr uint32_t kWideBlocks = 304;
 
+// What flush_start_kernel prepares (kernels_small.cu): the flushes' uniforms, and
+// the buffers that start at zero (gradVectors in 16-byte units; wide and error
+// may be null).
+struct FlushStart
+{
+    FlushParams* scenes;
+    uint32_t sceneCount;
+    uint32_t* wide;
+    uint32_t* error;
+    uint4* grad;
+    uint32_t gradVectors;
+    uint2* ranges;
+    uint32_t tiles;
+};
+// The scan and the sort of small frames (kernels_small.cu), one cluster each.
+constexpr uint32_t kSmallCluster = 8;
+constexpr uint32_t kSmallScanSlots = 1u << 18;
+constexpr uint32_t kSmallSortEntries = 1u << 17;
+constexpr int kSmallSortSmemBytes = (int)kSmallSortEntries / (int)kSmallCluster * 6 + 256 * 34 * 2 + 3200;
+
 // Batches the raster grid orders its tiles for (tile_order_kernel).
 constexpr uint32_t kOrderMinTiles = 512;
 constexpr uint32_t kOrderTiles = 16384;

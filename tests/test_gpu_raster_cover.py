@@ -149,6 +149,37 @@ def test_wide_triangles_around_the_capacity_of_their_list(n):
     assert (got == 1).all()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,H", [(128, 120), (640, 470)])  # one and two key bytes
+@pytest.mark.parametrize("n", [1, 1023, 8192, 8193, 131072, 131073, 262144, 262145])
+def test_bins_at_the_edges_of_the_one_cluster_passes(n, W, H):
+    """n triangles of one bin entry each, around the sizes at which the scan and
+    the sort of small frames change their share per thread or give way to the
+    library's: alone, and in a batch too large for either, the same image."""
+    import torch
+    from rive_runtime_gb300 import rive_cuda
+    rng = np.random.default_rng(n)
+    at = np.stack([rng.integers(0, W // 16, n), rng.integers(0, H // 16, n)], 1) * 16.0
+    at += rng.integers(0, 10, (n, 2))
+    tris = at[:, None] + np.array([[0, 0], [5.5, 0], [0, 5.5]])
+    ids = 1 + np.arange(n) * min(n, 60000) // n
+    f, (bufs, keep) = flush_of(tris, ids, W, H)
+    got, stats = render(f, bufs, W, H)
+    assert stats["bin_entries"] == n and stats["triangles"] == n
+    m = 300000
+    filler, (fbufs, fkeep) = flush_of(np.tile(tris[:1], (m, 1, 1)), np.full(m, 1), W, H)
+    targets = [torch.zeros((H, W, 4), dtype=torch.uint8, device="cuda") for _ in range(2)]
+    ctx = rive_cuda.Context(0)
+    ctx.flush_batch([(f, bufs, targets[0].data_ptr()), (filler, fbufs, targets[1].data_ptr())])
+    ctx.sync()
+    img = targets[0].cpu().numpy().astype(np.int64)
+    ctx.close()
+    assert np.array_equal(got, img[..., 0] | (img[..., 1] << 8) | (img[..., 2] << 16))
+    # The pixel (1, 1) of the last triangle has its colour.
+    x, y = at[-1].astype(int) + 1
+    assert got[y, x] == ids[-1]
+
+
 def test_unorm_float_is_the_correctly_rounded_quotient():
     """kUnormHi / kUnormLo of kernels_raster.cu: b / 255 for every byte by one
     rounded product and one fused step (float64 holds both exactly)."""
