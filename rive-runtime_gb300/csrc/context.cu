@@ -30,8 +30,8 @@
 namespace rivecuda
 {
 __global__ void color_ramp_kernel(BatchTables B);
-__global__ void tessellate_kernel(BatchTables B);
-__global__ void tessellate_feather_kernel(BatchTables B);
+__global__ void tessellate_kernel(BatchTables B, int lanesLog2);
+__global__ void tessellate_feather_kernel(BatchTables B, int lanesLog2);
 __global__ void patch_setup_kernel(BatchTables B,
                                    TriRecord* tris,
                                    uint32_t* tileCounts,
@@ -1163,8 +1163,10 @@ int enqueue_front(rive_cuda_context* ctx,
     if (L.tessSpans)
     {
         stage_begin(ctx, RIVE_CUDA_STAGE_TESSELLATE, stream);
-        (L.feather ? tessellate_feather_kernel : tessellate_kernel)<<<(L.tessSpans * 32u + 255u) / 256u,
-                                                                     256, 0, stream>>>(B);
+        const int lanes = tess_lanes_log2(L.tessSpans, L.feather);
+        (L.feather ? tessellate_feather_kernel
+                   : tessellate_kernel)<<<((L.tessSpans << lanes) + 255u) / 256u, 256, 0, stream>>>(
+            B, lanes);
         stage_end(ctx, stream);
     }
     if (L.slots)

@@ -21,8 +21,8 @@
 namespace rivecuda
 {
 __global__ void color_ramp_kernel(BatchTables B);
-__global__ void tessellate_kernel(BatchTables B);
-__global__ void tessellate_feather_kernel(BatchTables B);
+__global__ void tessellate_kernel(BatchTables B, int lanesLog2);
+__global__ void tessellate_feather_kernel(BatchTables B, int lanesLog2);
 __global__ void patch_setup_kernel(BatchTables B,
                                    TriRecord* tris,
                                    uint32_t* tileCounts,
@@ -382,8 +382,12 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
     if (d->grad_span_count)
         color_ramp_kernel<<<d->grad_span_count, 128, 0, stream>>>(B);
     if (d->tess_span_count)
-        (feather ? tessellate_feather_kernel : tessellate_kernel)<<<
-            (d->tess_span_count * 32u + 255u) / 256u, 256, 0, stream>>>(B);
+    {
+        const int lanes = tess_lanes_log2(d->tess_span_count, feather);
+        (feather ? tessellate_feather_kernel
+                 : tessellate_kernel)<<<((d->tess_span_count << lanes) + 255u) / 256u, 256, 0,
+                                        stream>>>(B, lanes);
+    }
 
     TriRecord* tris = (TriRecord*)(pool + kTrisOff);
     uint8_t* masks = (uint8_t*)(pool + kMasksOff);

@@ -10,10 +10,10 @@
 //    one row of the 2048-wide tessellation texture; every texel is one
 //    tessellated vertex (x, y, theta, contourIDWithFlags).
 //
-// GB300 mapping: one warp per span; the per-span set-up (tangents, polar step,
-// join step) is evaluated once per lane without divergence, then lanes stride
-// across the span's texels so each warp-wide store is 32 consecutive 16-byte
-// texels (512 B, fully coalesced). The texture is plain linear HBM memory
+// GB300 mapping: 8 or 16 lanes per span, two or four spans a warp; the per-span
+// set-up (tangents, polar step, join step) is evaluated once per lane without
+// divergence, then lanes stride across the span's vertices, so stores are runs
+// of consecutive 16-byte texels. Bound by issue slots. The texture is plain linear HBM memory
 // (row-major, 2048 texels per row), so the draw kernels read it with ordinary
 // 128-bit loads.
 #include "rive_cuda_internal.cuh"
@@ -412,12 +412,11 @@ __device__ SpanSetup span_setup(const FlushParams& P, const uint4* sp)
 
 // Per-texel half of tessellate.glsl (the fragment shader, 294-567).
 template <bool kFeather>
-__device__ uint4 tess_vertex(const SpanSetup& s, float vertexIdxF, uint32_t flagsIn)
+__device__ uint4 tess_vertex(const SpanSetup& s, float vertexIdx, uint32_t flagsIn)
 {
     float2 p0 = s.p0, p1 = s.p1, p2 = s.p2, p3 = s.p3;
     float2 tan0, tan1;
     cubic_tangents(p0, p1, p2, p3, tan0, tan1);
-    float vertexIdx = fmaxf(floorf(vertexIdxF), 0.f);
     float parametricSegmentCount = s.parametricSegmentCount;
     float radsPerPolarSegment = s.radsPerPolarSegment;
     uint32_t flags = flagsIn;
@@ -620,61 +619,93 @@ __global__ void __launch_bounds__(128) color_ramp_kernel(BatchTables B)
     }
 }
 
-// One warp per TessVertexSpan of the batch (both its forward and mirrored
-// rectangles).
+// 2^lanesLog2 lanes per TessVertexSpan of the batch (tess_lanes_log2). A span's forward rectangle
+// holds its vertices in order and its mirrored one the same vertices in reverse,
+// equal but for the mirrored flag: each is evaluated once and stored twice.
 template <bool kFeather>
-__device__ __forceinline__ void tessellate(const BatchTables& B)
+__device__ __forceinline__ void tessellate(const BatchTables& B, int lanesLog2)
 {
-    const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (gw >= B.totalTessSpans)
+    const uint32_t gs = (blockIdx.x * blockDim.x + threadIdx.x) >> lanesLog2;
+    const int lanes = 1 << lanesLog2, lane = threadIdx.x & (lanes - 1);
+    if (gs >= B.totalTessSpans)
         return;
-    const uint32_t scene = find_range(B.tessSpanBase, B.sceneCount, gw);
+    const uint32_t scene = find_range(B.tessSpanBase, B.sceneCount, gs);
     const FlushParams& P = B.scenes[scene];
-    const uint32_t warp = gw - B.tessSpanBase[scene];
-    const uint4* sp = P.tessSpans + 4 * (size_t)(P.firstTessSpan + warp);
+    const uint32_t span = gs - B.tessSpanBase[scene];
+    const uint4* sp = P.tessSpans + 4 * (size_t)(P.firstTessSpan + span);
     SpanSetup s = span_setup<kFeather>(P, sp);
     if (!s.valid)
         return;
-    uint4 q2 = sp[2], q3 = sp[3];
-    for (int second = 0; second < 2; ++second)
+    // Per rectangle: texel px = at + step * k holds vertex k (the vertex index
+    // before its clamp at 0), for k in [first, end).
+    uint4* row[2];
+    int at[2], first[2], end[2];
+    uint32_t mirrored[2];
+    const int total = (int)s.totalVertexCount;
+    const uint4 q2 = sp[2], q3 = sp[3];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
     {
-        float y = __uint_as_float(second ? q2.w : q2.z);
-        int32_t x0x1 = (int32_t)(second ? q3.y : q3.x);
-        int x0 = (int32_t)((uint32_t)x0x1 << 16) >> 16;
-        int x1 = x0x1 >> 16;
+        const float y = __uint_as_float(i ? q2.w : q2.z);
+        const int32_t x0x1 = (int32_t)(i ? q3.y : q3.x);
+        const int x0 = (int32_t)((uint32_t)x0x1 << 16) >> 16;
+        const int x1 = x0x1 >> 16;
+        first[i] = end[i] = at[i] = 0;
+        mirrored[i] = 0;
+        row[i] = nullptr;
         if (isnan(y) || x0 == x1 || y < 0.f || y >= (float)P.tessDataHeight)
             continue;
-        int rowIdx = (int)y;
-        int lo = max(min(x0, x1), 0), hi = min(max(x0, x1), kTessTextureWidth);
-        uint32_t flags = s.contourIDWithFlags;
+        row[i] = P.tess + (size_t)(int)y * kTessTextureWidth;
+        const int lo = max(min(x0, x1), 0), hi = min(max(x0, x1), kTessTextureWidth);
+        if (lo >= hi)
+            continue;
+        // Vertex index of texel px: total - |x1 - (px + 1/2)|, rounded down.
         if (x1 < x0)
-            flags |= MIRRORED_CONTOUR_CONTOUR_FLAG;
-        uint4* row = P.tess + (size_t)rowIdx * kTessTextureWidth;
-        for (int px = lo + lane; px < hi; px += 32)
         {
-            float vertexIdx = __fsub_rn(s.totalVertexCount,
-                                        fabsf(__fsub_rn((float)x1, __fadd_rn((float)px, .5f))));
-            row[px] = tess_vertex<kFeather>(s, vertexIdx, flags);
+            mirrored[i] = MIRRORED_CONTOUR_CONTOUR_FLAG;
+            at[i] = total + x1 - 1;
+            first[i] = at[i] - (hi - 1);
+            end[i] = at[i] - lo + 1;
         }
+        else
+        {
+            at[i] = x1 - total;
+            first[i] = lo - at[i];
+            end[i] = hi - at[i];
+        }
+    }
+    const bool both = first[0] < end[0] && first[1] < end[1];
+    const bool only1 = !(first[0] < end[0]);
+    const int k0 = both ? min(first[0], first[1]) : first[only1];
+    const int k1 = both ? max(end[0], end[1]) : end[only1];
+    for (int k = k0 + lane; k < k1; k += lanes)
+    {
+        const uint4 v = tess_vertex<kFeather>(s, (float)max(k, 0), s.contourIDWithFlags);
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            if (k >= first[i] && k < end[i])
+                row[i][mirrored[i] ? at[i] - k : at[i] + k] =
+                    make_uint4(v.x, v.y, v.z, v.w | mirrored[i]);
     }
 }
 
 // Resident 256-thread CTAs per SM the tessellation's registers are bounded
 // for: 4 (64 registers, a few bytes spilled) tessellates the full-feature
-// frame in 0.93 ms against 1.03 ms at the compiler's 74 registers (3 CTAs).
+// 2048x2048 frame in 0.64 ms against 0.70 and 0.69 ms with 3 and 5 (16 lanes a
+// span).
 #ifndef RIVE_TESS_MIN_BLOCKS
 #define RIVE_TESS_MIN_BLOCKS 4
 #endif
-__global__ void __launch_bounds__(256, RIVE_TESS_MIN_BLOCKS) tessellate_kernel(BatchTables B)
+__global__ void __launch_bounds__(256, RIVE_TESS_MIN_BLOCKS) tessellate_kernel(BatchTables B,
+                                                                               int lanesLog2)
 {
-    tessellate<false>(B);
+    tessellate<false>(B, lanesLog2);
 }
 
 // With feathered-fill softening and feather-join texels.
-__global__ void __launch_bounds__(256) tessellate_feather_kernel(BatchTables B)
+__global__ void __launch_bounds__(256) tessellate_feather_kernel(BatchTables B, int lanesLog2)
 {
-    tessellate<true>(B);
+    tessellate<true>(B, lanesLog2);
 }
 // The tessellation pass's device functions on n items, for the parity tests
 // (the layouts of oracle_cubic_eval and oracle_math_eval): fn 0..5 the cubic
