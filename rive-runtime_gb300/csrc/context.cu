@@ -61,7 +61,7 @@ __global__ void small_scan_kernel(uint32_t slots, const uint32_t* counts, uint32
                                   uint32_t* hostTotal);
 __global__ void small_sort_kernel(const uint32_t* entryTotal, uint32_t capacity, bool guarded, int keyBits,
                                   const uint16_t* keys, const uint32_t* vals, uint16_t* sortedKeys,
-                                  uint32_t* sortedVals, uint2* ranges);
+                                  uint32_t* sortedVals, TileHead* ranges);
 __global__ void wide_count_kernel(BatchTables B, const TriRecord* tris, uint32_t* tileCounts);
 __global__ void bin_fill_kernel(const uint32_t* pairTotal,
                                 uint32_t capacity,
@@ -82,7 +82,7 @@ __global__ void bin_scatter_kernel(uint32_t slotCount,
 __global__ void tile_ranges_kernel(uint32_t pairCount,
                                    uint32_t tileCount,
                                    const uint32_t* keys,
-                                   uint2* ranges);
+                                   TileHead* ranges);
 // The same three with 16-bit tile keys (batches of at most 65,535 tiles).
 __global__ void bin_fill16_kernel(const uint32_t* pairTotal,
                                   uint32_t capacity,
@@ -103,26 +103,26 @@ __global__ void bin_scatter16_kernel(uint32_t slotCount,
 __global__ void tile_ranges16_kernel(uint32_t pairCount,
                                      uint32_t tileCount,
                                      const uint16_t* keys,
-                                     uint2* ranges);
+                                     TileHead* ranges);
 __global__ void ranges_guard_kernel(const uint32_t* pairTotal,
                                     uint32_t capacity,
-                                    uint2* ranges,
+                                    TileHead* ranges,
                                     uint32_t tiles);
 // One mip level of an image from the level above (kernels_raster.cu).
 __global__ void mip_level_kernel(const uchar4* src, uint32_t sw, uint32_t sh, uchar4* dst,
                                  uint32_t dw, uint32_t dh);
 // The feather atlas pass at 8, 16 and 32 pixel tiles (kernels_raster.cu).
 __global__ void raster_atlas8_kernel(BatchTables B, const TriRecord* tris,
-                                     const uint32_t* sortedSlots, const uint2* ranges,
+                                     const uint32_t* sortedSlots, const TileHead* ranges,
                                      uint32_t firstTile);
 __global__ void raster_atlas_kernel(BatchTables B, const TriRecord* tris,
-                                    const uint32_t* sortedSlots, const uint2* ranges,
+                                    const uint32_t* sortedSlots, const TileHead* ranges,
                                     uint32_t firstTile);
 __global__ void raster_atlas32_kernel(BatchTables B, const TriRecord* tris,
-                                      const uint32_t* sortedSlots, const uint2* ranges,
+                                      const uint32_t* sortedSlots, const TileHead* ranges,
                                       uint32_t firstTile);
 __global__ void tile_order_keys_kernel(uint32_t tiles,
-                                       const uint2* ranges,
+                                       const TileHead* ranges,
                                        uint32_t* keys,
                                        uint32_t* vals);
 // Interior tiles as winding records (kernels_raster.cu).
@@ -147,14 +147,14 @@ __global__ void bin_scatter_winding_kernel(BatchTables B,
 // The raster kernels without and with the feather paths.
 #define RIVE_DECLARE_RASTER(NAME)                                                                  \
     __global__ void NAME(BatchTables B, const TriRecord* tris, const uint32_t* sortedSlots,        \
-                         const uint2* ranges);
+                         const TileHead* ranges);
 // (16-pixel tiles: in the order of `order`, or as they come when it is null.)
 __global__ void raster_tile_kernel(BatchTables B, const TriRecord* tris, const uint32_t* sortedSlots,
-                                   const uint2* ranges, const uint32_t* order);
+                                   const TileHead* ranges, const uint32_t* order);
 __global__ void raster_tile_feather_kernel(BatchTables B, const TriRecord* tris,
-                                           const uint32_t* sortedSlots, const uint2* ranges,
+                                           const uint32_t* sortedSlots, const TileHead* ranges,
                                            const uint32_t* order);
-__global__ void tile_order_kernel(uint32_t tiles, const uint2* ranges, uint32_t* order);
+__global__ void tile_order_kernel(uint32_t tiles, const TileHead* ranges, uint32_t* order);
 RIVE_DECLARE_RASTER(raster_tile8_kernel)
 RIVE_DECLARE_RASTER(raster_tile8_feather_kernel)
 RIVE_DECLARE_RASTER(raster_tile32_kernel)
@@ -860,7 +860,7 @@ struct Scratch
     size_t scanTempBytes = 0;
     void* sortTemp = nullptr;
     size_t sortTempBytes = 0;
-    uint2* ranges = nullptr;
+    TileHead* ranges = nullptr;
     uint32_t* error = nullptr;
     // Where the binner reports entries past the bins' capacity (error when
     // null; a scratch word for speculative passes, whose overflow is
@@ -1139,6 +1139,8 @@ int enqueue_front(rive_cuda_context* ctx,
     F.gradVectors = (uint32_t)(L.gradBytes() / 16);
     F.ranges = S.ranges;
     F.tiles = L.tiles;
+    F.tileBase = B.tileBase;
+    F.sceneTiles = B.sceneTiles;
     flush_start_kernel<<<flush_start_blocks(F), 256, 0, stream>>>(F);
     if (L.imageSlots)
         CK(cudaMemsetAsync(S.pathImage, 0xff, (size_t)std::max(L.paths, 1u) * 4, stream));
@@ -1253,6 +1255,8 @@ int prepare_raster(rive_cuda_context* ctx)
                                 kRaster32SmemBytes));
         CK(cudaFuncSetAttribute(raster_tile32_feather_kernel,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, kRaster32SmemBytes));
+        CK(cudaFuncSetAttribute(raster_atlas32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                kRaster32SmemBytes));
         ctx->raster32Ready = true;
     }
     const int slot = ctx->tileLog2 == 3 ? 0 : ctx->tileLog2 == 4 ? 1 : -1;
@@ -1291,7 +1295,7 @@ int launch_raster(rive_cuda_context* ctx,
                   const Scratch& S,
                   const TriRecord* tris,
                   const uint32_t* sortedSlots,
-                  const uint2* ranges,
+                  const TileHead* ranges,
                   uint32_t entries,
                   cudaStream_t stream)
 {
@@ -1431,7 +1435,7 @@ int enqueue_back(rive_cuda_context* ctx,
             raster_atlas8_kernel<<<atlasTiles, 64, 0, stream>>>(B, S.tris, sortedSlots, S.ranges,
                                                                 L.mainTiles);
         else if (L.tileLog2 == 5)
-            raster_atlas32_kernel<<<atlasTiles, 1024, 0, stream>>>(B, S.tris, sortedSlots,
+            raster_atlas32_kernel<<<atlasTiles, 1024, kRaster32SmemBytes, stream>>>(B, S.tris, sortedSlots,
                                                                    S.ranges, L.mainTiles);
         else
             raster_atlas_kernel<<<atlasTiles, 256, 0, stream>>>(B, S.tris, sortedSlots, S.ranges,
@@ -1592,7 +1596,7 @@ int run_batch_body(rive_cuda_context* ctx,
     CK(ctx->grad.reserve(L.gradBytes()));
     CK(ctx->hTables[tslot].reserve(L.tableBytes));
     CK(ctx->dTables.reserve(L.tableBytes));
-    CK(ctx->ranges.reserve((size_t)L.tiles * sizeof(uint2)));
+    CK(ctx->ranges.reserve((size_t)L.tiles * sizeof(TileHead)));
     CK(ctx->tris.reserve((size_t)std::max(L.slots, 1u) * sizeof(TriRecord)));
     CK(ctx->tileCounts.reserve((size_t)std::max(L.slots, 1u) * 4));
     CK(ctx->tileMasks.reserve((size_t)std::max(L.slots, 1u)));
@@ -1653,7 +1657,7 @@ int run_batch_body(rive_cuda_context* ctx,
     S.offsets = (uint32_t*)ctx->offsets.ptr;
     S.scanTemp = ctx->scanTemp.ptr;
     S.scanTempBytes = scanBytes;
-    S.ranges = (uint2*)ctx->ranges.ptr;
+    S.ranges = (TileHead*)ctx->ranges.ptr;
     S.error = ctx->dError;
     if (L.winding)
     {
@@ -2312,7 +2316,7 @@ int graph_build(rive_cuda_context* ctx,
         CK(g->atlas.reserve((size_t)L.atlasTexels * 2));
     if (L.imageSlots)
         CK(g->pathImage.reserve((size_t)std::max(L.paths, 1u) * 4));
-    CK(g->ranges.reserve((size_t)L.tiles * sizeof(uint2)));
+    CK(g->ranges.reserve((size_t)L.tiles * sizeof(TileHead)));
     CK(g->error.reserve(4));
     const bool queue = ctx->rasterQueue && L.tileLog2 == 4 && L.mainTiles > kOrderTiles;
     size_t queueBytes = 0;
@@ -2343,7 +2347,7 @@ int graph_build(rive_cuda_context* ctx,
     S.offsets = (uint32_t*)g->offsets.ptr;
     S.scanTemp = g->scanTemp.ptr;
     S.scanTempBytes = scanBytes;
-    S.ranges = (uint2*)g->ranges.ptr;
+    S.ranges = (TileHead*)g->ranges.ptr;
     S.error = (uint32_t*)g->error.ptr;
     if (queue)
     {

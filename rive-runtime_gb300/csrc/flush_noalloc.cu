@@ -40,7 +40,7 @@ __global__ void small_scan_kernel(uint32_t slots, const uint32_t* counts, uint32
                                   uint32_t* hostTotal);
 __global__ void small_sort_kernel(const uint32_t* entryTotal, uint32_t capacity, bool guarded, int keyBits,
                                   const uint16_t* keys, const uint32_t* vals, uint16_t* sortedKeys,
-                                  uint32_t* sortedVals, uint2* ranges);
+                                  uint32_t* sortedVals, TileHead* ranges);
 __global__ void wide_count_kernel(BatchTables B, const TriRecord* tris, uint32_t* tileCounts);
 __global__ void bin_scatter16_kernel(uint32_t slotCount,
                                    int tileLog2,
@@ -57,16 +57,16 @@ __global__ void bin_scatter16_kernel(uint32_t slotCount,
 __global__ void tile_ranges16_kernel(uint32_t pairCount,
                                      uint32_t tileCount,
                                      const uint16_t* keys,
-                                     uint2* ranges);
+                                     TileHead* ranges);
 __global__ void raster_tile_kernel(BatchTables B,
                                    const TriRecord* tris,
                                    const uint32_t* sortedSlots,
-                                   const uint2* ranges,
+                                   const TileHead* ranges,
                                    const uint32_t* order);
 __global__ void raster_tile_feather_kernel(BatchTables B,
                                    const TriRecord* tris,
                                    const uint32_t* sortedSlots,
-                                   const uint2* ranges,
+                                   const TileHead* ranges,
                                    const uint32_t* order);
 } // namespace rivecuda
 
@@ -96,9 +96,9 @@ constexpr size_t kValsOff = kKeysOff + align256(kPairBytes);
 constexpr size_t kKeysAltOff = kValsOff + align256(kPairBytes);
 constexpr size_t kValsAltOff = kKeysAltOff + align256(kPairBytes);
 constexpr size_t kRangesOff = kValsAltOff + align256(kPairBytes);
-constexpr size_t kScanTempOff = kRangesOff + align256(kMaxTiles * sizeof(uint2));
-constexpr size_t kScanTempBytes = 64u << 10; // (kept in the layout; the scan needs none)
-constexpr size_t kSortTempOff = kScanTempOff + kScanTempBytes;
+constexpr size_t kRangesBytes = 96u << 10;
+static_assert(kMaxTiles * sizeof(TileHead) <= kRangesBytes, "one head per tile");
+constexpr size_t kSortTempOff = kRangesOff + kRangesBytes;
 constexpr size_t kSortTempBytes = 4u << 20;
 // Launch tables of the flush (a batch of one): FlushParams, prefix arrays and
 // one PatchSegment per draw batch.
@@ -367,7 +367,7 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
 
     // What must start at zero on every call: the error word, the tile ranges,
     // the gradient rows in use, the wide triangles' counter.
-    uint2* ranges = (uint2*)(pool + kRangesOff);
+    TileHead* ranges = (TileHead*)(pool + kRangesOff);
     FlushStart F = {};
     F.scenes = (FlushParams*)(dTab + kTabScenes);
     F.sceneCount = 1;
@@ -377,6 +377,8 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
     F.gradVectors = (uint32_t)(kGradTextureWidth / 4) * d->grad_data_height;
     F.ranges = ranges;
     F.tiles = tiles;
+    F.tileBase = B.tileBase;
+    F.sceneTiles = B.sceneTiles;
     flush_start_kernel<<<(std::max(F.gradVectors, tiles) + 255) / 256, 256, 0, stream>>>(F);
 
     if (d->grad_span_count)

@@ -28,6 +28,7 @@
 
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 
@@ -2404,18 +2405,18 @@ __global__ void __launch_bounds__(256) bin_scatter_winding_kernel(BatchTables B,
 // until the back half runs again with exact bins.
 __global__ void __launch_bounds__(256) ranges_guard_kernel(const uint32_t* __restrict__ pairTotal,
                                                            uint32_t capacity,
-                                                           uint2* __restrict__ ranges,
+                                                           TileHead* __restrict__ ranges,
                                                            uint32_t tiles)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= tiles || *pairTotal <= capacity)
         return;
-    ranges[i] = make_uint2(0u, 0u);
+    ranges[i].first = ranges[i].end = 0u;
 }
 
 template <typename K>
 __device__ __forceinline__ void tile_ranges(uint32_t pairCount, uint32_t tileCount,
-                                            const K* __restrict__ keys, uint2* __restrict__ ranges)
+                                            const K* __restrict__ keys, TileHead* __restrict__ ranges)
 {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= pairCount)
@@ -2424,21 +2425,21 @@ __device__ __forceinline__ void tile_ranges(uint32_t pairCount, uint32_t tileCou
     if (k >= tileCount) // capacity padding
         return;
     if (i == 0 || keys[i - 1] != k)
-        ranges[k].x = i;
+        ranges[k].first = i;
     if (i == pairCount - 1 || keys[i + 1] != k)
-        ranges[k].y = i + 1;
+        ranges[k].end = i + 1;
 }
 __global__ void __launch_bounds__(256) tile_ranges_kernel(uint32_t pairCount,
                                                           uint32_t tileCount,
                                                           const uint32_t* __restrict__ keys,
-                                                          uint2* __restrict__ ranges)
+                                                          TileHead* __restrict__ ranges)
 {
     tile_ranges(pairCount, tileCount, keys, ranges);
 }
 __global__ void __launch_bounds__(256) tile_ranges16_kernel(uint32_t pairCount,
                                                             uint32_t tileCount,
                                                             const uint16_t* __restrict__ keys,
-                                                            uint2* __restrict__ ranges)
+                                                            TileHead* __restrict__ ranges)
 {
     tile_ranges(pairCount, tileCount, keys, ranges);
 }
@@ -3241,24 +3242,20 @@ static_assert(sizeof(TileTri) == 80, "TileTri layout");
 
 // The 512-entry feather table (the integral of the normal distribution over
 // -3..+3 standard deviations, fp16 values widened to float), written by the
-// host once per device (ensure_feather_lut, end of this file) before any flush.
-__device__ float g_featherLUT[kGaussianTableSize];
+// host once per device (ensure_feather_lut, end of this file) before any flush,
+// as pairs: entry i + 1 holds texels i and i + 1, both clamped to the table, so a
+// sample is one 8-byte load.
+__device__ float2 g_featherPairs[kGaussianTableSize + 2];
 
 // FEATHER(x) (common.glsl:53-60): the table sampled at normalised x with a
-// linear filter and clamp-to-edge addressing.
-__device__ __noinline__ float feather_lut(float x)
+// linear filter and clamp-to-edge addressing (a NaN samples the first texel).
+__device__ __forceinline__ float feather_lut(float x)
 {
     const float t = __fsub_rn(__fmul_rn(x, (float)kGaussianTableSize), .5f);
-    if (!(t == t))
-        return g_featherLUT[0];
     const float f = floorf(t);
     const float w = __fsub_rn(t, f);
-    const float fc = fminf(fmaxf(f, -1.f), (float)kGaussianTableSize);
-    const int i0 = (int)fc;
-    const int a = min(max(i0, 0), kGaussianTableSize - 1);
-    const int b = min(max(i0 + 1, 0), kGaussianTableSize - 1);
-    const float va = g_featherLUT[a], vb = g_featherLUT[b];
-    return __fadd_rn(va, __fmul_rn(__fsub_rn(vb, va), w));
+    const float2 p = g_featherPairs[(int)fminf(fmaxf(f, -1.f), (float)kGaussianTableSize) + 1];
+    return t == t ? __fadd_rn(p.x, __fmul_rn(__fsub_rn(p.y, p.x), w)) : p.x;
 }
 
 // eval_feathered_stroke (draw_path_common.glsl:242-258):
@@ -3510,25 +3507,23 @@ template <int TL, bool kFeather>
 __device__ __forceinline__ void raster_tile(const BatchTables& B,
                                             const TriRecord* __restrict__ tris,
                                             const uint32_t* __restrict__ sortedSlots,
-                                            const uint2* __restrict__ ranges,
+                                            const TileHead* __restrict__ ranges,
                                             RasterShared<TL>& sh,
                                             uint32_t gtile)
 {
     using G = RasterTile<TL>;
     constexpr uint32_t kChunk = G::kChunk;
     static_assert(sizeof(FlushParams) / 4 <= G::kThreads, "one word of FlushParams per thread");
-    const uint2 range = ranges[gtile];
+    const uint4 head = __ldg(reinterpret_cast<const uint4*>(ranges + gtile));
+    const uint2 range = make_uint2(head.x, head.y);
     // The tile's scene: its parameters are staged for the whole CTA (seen after
     // the first chunk's barrier); what comes before reads them in place.
-    const uint32_t scene = find_range(B.tileBase, B.sceneCount, gtile);
-    const FlushParams& G0 = B.scenes[scene];
+    const FlushParams& G0 = B.scenes[head.z];
     if (range.y > range.x && threadIdx.x < sizeof(FlushParams) / 4)
         reinterpret_cast<uint32_t*>(&sh.params)[threadIdx.x] =
             reinterpret_cast<const uint32_t*>(&G0)[threadIdx.x];
     const FlushParams& P = sh.params;
-    const uint32_t tilesX = G0.tilesX;
-    const uint32_t tile = gtile - B.tileBase[scene];
-    const int tx = (int)(tile % tilesX), ty = (int)(tile / tilesX);
+    const int tx = (int)(head.w & 0xffffu), ty = (int)(head.w >> 16);
     const int ox = tx * G::T, oy = ty * G::T;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int qx = (warp % G::kWarpCols) * 8, qy = (warp / G::kWarpCols) * 4;
@@ -3814,7 +3809,7 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
 #define RIVE_RASTER_KERNELS(NAME, FEATHER)                                                        \
     __global__ void __launch_bounds__(256, RIVE_RASTER_MIN_BLOCKS(FEATHER)) NAME(                           \
         BatchTables B, const TriRecord* __restrict__ tris,                                        \
-        const uint32_t* __restrict__ sortedSlots, const uint2* __restrict__ ranges,               \
+        const uint32_t* __restrict__ sortedSlots, const TileHead* __restrict__ ranges,               \
         const uint32_t* __restrict__ order)                                                       \
     {                                                                                             \
         __shared__ RasterShared<4> sh;                                                            \
@@ -3827,69 +3822,115 @@ RIVE_RASTER_KERNELS(raster_tile_feather_kernel, true)
 
 // The feather atlas pass (render_atlas.glsl with the floating-point target
 // and fixed-function blending; the atlas pipelines of gpu.hpp:2076-2080):
-// one CTA of T x T threads per atlas tile, one thread per texel, walking the
-// tile's bin entries in primitive order (fill batches, then stroke batches).
-// A fill adds its feathered coverage, subtracted when the triangle faced
-// away; a stroke keeps the maximum; every blend result rounds to fp16, as
-// the R16F target stores it. Each texel is written, covered or not (the
+// one CTA of T x T threads per atlas tile, one thread per texel. Triangles are
+// staged, listed per block and handed to the texels they cover as in
+// raster_tile; each texel then takes its own in primitive order (fill batches,
+// then stroke batches). A fill adds its feathered coverage, subtracted when the
+// triangle faced away; a stroke keeps the maximum; every blend result rounds to
+// fp16, as the R16F target stores it. Each texel is written, covered or not (the
 // atlas starts cleared). Triangles arrive clipped to their batch's scissor
 // through their pixel box, which the texel test applies exactly.
 template <int TL>
 __device__ __forceinline__ void raster_atlas_tile(const BatchTables& B,
                                                   const TriRecord* __restrict__ tris,
                                                   const uint32_t* __restrict__ sortedSlots,
-                                                  const uint2* __restrict__ ranges,
+                                                  const TileHead* __restrict__ ranges,
+                                                  RasterShared<TL>& sh,
                                                   uint32_t gtile)
 {
-    constexpr int T = 1 << TL;
-    const uint32_t scene = find_range(B.tileBase, B.sceneCount, gtile);
-    const FlushParams& P = B.scenes[scene];
-    const uint32_t tilesX = P.tilesX;
-    const uint32_t tile = gtile - B.tileBase[scene];
-    const int tx = (int)(tile % tilesX), ty = (int)(tile / tilesX);
-    const int ox = tx * T, oy = ty * T;
-    const int lxi = (int)threadIdx.x & (T - 1), lyi = (int)threadIdx.x >> TL;
+    using G = RasterTile<TL>;
+    constexpr uint32_t kChunk = G::kChunk;
+    const TileHead head = ranges[gtile];
+    const FlushParams& P = B.scenes[head.scene];
+    const int tx = (int)(head.at & 0xffffu), ty = (int)(head.at >> 16);
+    const int ox = tx * G::T, oy = ty * G::T;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int qx = (warp % G::kWarpCols) * 8, qy = (warp / G::kWarpCols) * 4;
+    const int lxi = qx + (lane & 7), lyi = qy + (lane >> 3);
     const int px = ox + lxi, py = oy + lyi;
     const float lx = (float)lxi, ly = (float)lyi;
     const float fx = (float)px + .5f, fy = (float)py + .5f;
-    const uint2 range = ranges[gtile];
     float acc = 0.f;
-    for (uint32_t k = range.x; k < range.y; ++k)
+    for (uint32_t base = head.first; base < head.end; base += kChunk)
     {
-        const uint32_t slot = __ldg(sortedSlots + k);
-        const TriRecord& R = tris[slot];
-        const uint4 meta = R.meta;
-        const int4 bb = unpack_bbox(meta);
-        if (px < bb.x || px >= bb.z || py < bb.y || py >= bb.w)
-            continue;
-        const float4 e0 = R.e0, e1 = R.e1, e2 = R.e2;
-        const float c0 = tile_edge_origin(e0, tx, ty, TL), c1 = tile_edge_origin(e1, tx, ty, TL),
-                    c2 = tile_edge_origin(e2, tx, ty, TL);
-        const float E0 = local_edge(c0, e0.z, e0.w, lx, ly);
-        const float E1 = local_edge(c1, e1.z, e1.w, lx, ly);
-        const float E2 = local_edge(c2, e2.z, e2.w, lx, ly);
-        const float emin = fminf(fminf(E0, E1), E2);
-        if (!(emin > 0.f) &&
-            !(emin == 0.f && local_inside(e0.z, e0.w, E0) && local_inside(e1.z, e1.w, E1) &&
-              local_inside(e2.z, e2.w, E2)))
-            continue;
-        const float4 cv0 = R.cov0, cv1 = R.cov1;
-        const float dx0 = (float)ox + .5f - e0.x, dy0 = (float)oy + .5f - e0.y;
-        const float cx0 = cv0.x + cv0.y * dx0 + cv0.z * dy0;
-        const float cy0 = cv0.w + cv1.x * dx0 + cv1.y * dy0;
-        const float covx = __fmaf_rn(cv0.y, lx, __fmaf_rn(cv0.z, ly, cx0));
-        const float covy = __fmaf_rn(cv1.x, lx, __fmaf_rn(cv1.y, ly, cy0));
-        float frag = feathered_fragment(B.featherPlanes, slot, fx, fy, covx, covy);
-        if (covy >= 0.f)
+        const uint32_t k = base + threadIdx.x;
+        uint32_t m = 0;
+        if (k < head.end)
         {
-            acc = h2f(f2h(fmaxf(acc, frag)));
+            const uint32_t slot = sortedSlots[k];
+            const TriRecord T = tris[slot];
+            const float4 e[3] = {T.e0, T.e1, T.e2};
+            const float c[3] = {tile_edge_origin(e[0], tx, ty, TL),
+                                tile_edge_origin(e[1], tx, ty, TL),
+                                tile_edge_origin(e[2], tx, ty, TL)};
+            const float dx0 = (float)ox + .5f - T.e0.x, dy0 = (float)oy + .5f - T.e0.y;
+            TileTri L;
+            L.v0 = make_float4(c[0], e[0].z, e[0].w, c[1]);
+            L.v1 = make_float4(e[1].z, e[1].w, c[2], e[2].z);
+            L.v2 = make_float4(e[2].w, T.cov0.w + T.cov1.x * dx0 + T.cov1.y * dy0, T.cov1.x,
+                               T.cov1.y);
+            L.v3 = make_float4(T.cov0.x + T.cov0.y * dx0 + T.cov0.z * dy0, T.cov0.y, T.cov0.z, 0.f);
+            L.v4 = make_uint4(T.meta.y, T.meta.z, T.meta.x, slot); // the pixel box, not a paint
+            sh.tris[threadIdx.x] = L;
+            m = blocks_overlapped<TL>(c, e, unpack_bbox(T.meta), ox, oy);
         }
-        else
+#pragma unroll
+        for (int b = 0; b < G::kBlocks; ++b)
         {
-            if ((meta.x >> 16) & FEATURE_ATLAS_NEGATE)
-                frag = -frag;
-            acc = h2f(f2h(acc + frag));
+            const uint32_t bits = __ballot_sync(0xffffffffu, (m >> b) & 1u);
+            if (lane == b)
+                sh.bits[b][warp] = bits;
         }
+        __syncthreads();
+        uint32_t n = 0;
+        const uint32_t words = (min(kChunk, head.end - base) + 31) / 32;
+        for (uint32_t w = 0; w < words; ++w)
+        {
+            const uint32_t bits = sh.bits[warp][w];
+            if ((bits >> lane) & 1u)
+                sh.list[warp][n + __popc(bits & ((1u << lane) - 1u))] =
+                    (typename G::Index)(w * 32 + lane);
+            n += __popc(bits);
+        }
+        __syncwarp();
+        for (uint32_t g = 0; g < n; g += 32)
+        {
+            const typename G::Index* const list = sh.list[warp] + g;
+            const uint32_t cnt = min(32u, n - g);
+            uint32_t cover = 0;
+            if (lane < cnt)
+            {
+                const TileTri& T = sh.tris[list[lane]];
+                cover = block_coverage(T.v0, T.v1, T.v2.x, (float)qx, (float)qy);
+            }
+            uint32_t hits = transpose_bits(cover, lane);
+            while (hits)
+            {
+                const TileTri& T = sh.tris[list[__ffs(hits) - 1]];
+                hits &= hits - 1;
+                const uint4 v4 = T.v4;
+                if (px < (int)(v4.x & 0xffffu) || px >= (int)(v4.x >> 16) ||
+                    py < (int)(v4.y & 0xffffu) || py >= (int)(v4.y >> 16))
+                    continue;
+                const float4 v2 = T.v2, v3 = T.v3;
+                const float covx = __fmaf_rn(v3.y, lx, __fmaf_rn(v3.z, ly, v3.x));
+                const float covy = __fmaf_rn(v2.z, lx, __fmaf_rn(v2.w, ly, v2.y));
+                float frag = feathered_fragment(B.featherPlanes, v4.w, fx, fy, covx, covy);
+                if (covy >= 0.f)
+                {
+                    acc = h2f(f2h(fmaxf(acc, frag)));
+                }
+                else
+                {
+                    if ((v4.z >> 16) & FEATURE_ATLAS_NEGATE)
+                        frag = -frag;
+                    acc = h2f(f2h(acc + frag));
+                }
+            }
+            __syncwarp();
+        }
+        if (head.end - base > kChunk)
+            __syncthreads();
     }
     if (px < (int)P.width && py < (int)P.height)
         P.atlas[(size_t)py * P.atlasW + px] = (uint16_t)f2h(acc);
@@ -3898,15 +3939,23 @@ __device__ __forceinline__ void raster_atlas_tile(const BatchTables& B,
 #define RIVE_ATLAS_KERNEL(NAME, TL)                                                                \
     __global__ void __launch_bounds__(1 << (2 * TL)) NAME(                                          \
         BatchTables B, const TriRecord* __restrict__ tris,                                        \
-        const uint32_t* __restrict__ sortedSlots, const uint2* __restrict__ ranges,               \
+        const uint32_t* __restrict__ sortedSlots, const TileHead* __restrict__ ranges,            \
         uint32_t firstTile)                                                                       \
     {                                                                                             \
-        raster_atlas_tile<TL>(B, tris, sortedSlots, ranges, firstTile + blockIdx.x);              \
+        __shared__ RasterShared<TL> sh;                                                           \
+        raster_atlas_tile<TL>(B, tris, sortedSlots, ranges, sh, firstTile + blockIdx.x);          \
     }
 RIVE_ATLAS_KERNEL(raster_atlas8_kernel, 3)
 RIVE_ATLAS_KERNEL(raster_atlas_kernel, 4)
-RIVE_ATLAS_KERNEL(raster_atlas32_kernel, 5)
 #undef RIVE_ATLAS_KERNEL
+__global__ void __launch_bounds__(1024) raster_atlas32_kernel(
+    BatchTables B, const TriRecord* __restrict__ tris, const uint32_t* __restrict__ sortedSlots,
+    const TileHead* __restrict__ ranges, uint32_t firstTile)
+{
+    extern __shared__ uint4 dyn[]; // kRaster32SmemBytes
+    raster_atlas_tile<5>(B, tris, sortedSlots, ranges, *reinterpret_cast<RasterShared<5>*>(dyn),
+                         firstTile + blockIdx.x);
+}
 
 // The tiles of a batch of at most kOrderTiles, heaviest first to within an
 // eighth: one CTA counts them into 256 buckets (the leading four bits of a
@@ -3914,7 +3963,7 @@ RIVE_ATLAS_KERNEL(raster_atlas32_kernel, 5)
 // tiles do not queue at one counter, and gives each its place. Bound by
 // latency: about 5 us for 16,384 tiles, against 45 us for a radix sort.
 __global__ void __launch_bounds__(1024, 1) tile_order_kernel(uint32_t tiles,
-                                                             const uint2* __restrict__ ranges,
+                                                             const TileHead* __restrict__ ranges,
                                                              uint32_t* __restrict__ order)
 {
     constexpr int kBuckets = 256, kWarps = 32, kPer = kBuckets * kWarps / 1024;
@@ -3922,7 +3971,7 @@ __global__ void __launch_bounds__(1024, 1) tile_order_kernel(uint32_t tiles,
     __shared__ uint32_t sums[kWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     auto bucket = [&](uint32_t i) {
-        const uint2 r = ranges[i];
+        const uint2 r = *reinterpret_cast<const uint2*>(ranges + i); // first, end
         const uint32_t n = r.y > r.x ? r.y - r.x : 0u;
         const uint32_t bits = __float_as_uint((float)n) >> 20; // exponent, 3 bits of mantissa
         return 255u - min(n ? bits - (127u << 3) : 0u, 255u);
@@ -3963,14 +4012,14 @@ __global__ void __launch_bounds__(1024, 1) tile_order_kernel(uint32_t tiles,
 // Sort keys of the tile order of larger batches: per tile, its bin entries inverted (a plain
 // ascending sort then puts the heaviest tile first), and its index.
 __global__ void __launch_bounds__(256) tile_order_keys_kernel(uint32_t tiles,
-                                                              const uint2* __restrict__ ranges,
+                                                              const TileHead* __restrict__ ranges,
                                                               uint32_t* __restrict__ keys,
                                                               uint32_t* __restrict__ vals)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= tiles)
         return;
-    const uint2 r = ranges[i];
+    const uint2 r = *reinterpret_cast<const uint2*>(ranges + i); // first, end
     keys[i] = 0xffffffffu - (r.y > r.x ? r.y - r.x : 0u);
     vals[i] = i;
 }
@@ -3978,7 +4027,7 @@ __global__ void __launch_bounds__(256) tile_order_keys_kernel(uint32_t tiles,
 #define RIVE_RASTER8_KERNELS(NAME, FEATHER)                                                       \
     __global__ void __launch_bounds__(64) NAME(BatchTables B, const TriRecord* __restrict__ tris, \
                                                const uint32_t* __restrict__ sortedSlots,         \
-                                               const uint2* __restrict__ ranges)                 \
+                                               const TileHead* __restrict__ ranges)                 \
     {                                                                                             \
         __shared__ RasterShared<3> sh;                                                            \
         raster_tile<3, FEATHER>(B, tris, sortedSlots, ranges, sh, blockIdx.x);                    \
@@ -3992,7 +4041,7 @@ RIVE_RASTER8_KERNELS(raster_tile8_feather_kernel, true)
 #define RIVE_RASTER32_KERNELS(NAME, FEATHER)                                                      \
     __global__ void __launch_bounds__(1024, 1) NAME(                                              \
         BatchTables B, const TriRecord* __restrict__ tris,                                        \
-        const uint32_t* __restrict__ sortedSlots, const uint2* __restrict__ ranges)               \
+        const uint32_t* __restrict__ sortedSlots, const TileHead* __restrict__ ranges)               \
     {                                                                                             \
         extern __shared__ uint4 dyn[];                                                            \
         RasterShared<5>& sh = *reinterpret_cast<RasterShared<5>*>(dyn);                           \
@@ -4107,7 +4156,11 @@ cudaError_t ensure_feather_lut(int device)
         return cudaSuccess;
     float table[kGaussianTableSize];
     build_feather_table(table);
-    cudaError_t e = cudaMemcpyToSymbol(g_featherLUT, table, sizeof(table));
+    float2 pairs[kGaussianTableSize + 2];
+    for (int i = -1; i <= kGaussianTableSize; ++i)
+        pairs[i + 1] = make_float2(table[std::min(std::max(i, 0), kGaussianTableSize - 1)],
+                                   table[std::min(std::max(i + 1, 0), kGaussianTableSize - 1)]);
+    cudaError_t e = cudaMemcpyToSymbol(g_featherPairs, pairs, sizeof(pairs));
     if (e == cudaSuccess)
     {
         build_inverse_feather_table(table);

@@ -15,7 +15,7 @@ namespace rivecuda
 // at byte 72, ditherScale at 88, ditherBias at 92), read on the device so no
 // pass waits for the host, one thread per flush of the batch; and what must
 // start at zero: the gradient texture (texels no span covers are never sampled;
-// zeroed so the texture is deterministic), the tile ranges, the wide triangles'
+// zeroed so the texture is deterministic), the tile heads, the wide triangles'
 // counter. One launch in the place of four.
 __global__ void __launch_bounds__(256) flush_start_kernel(FlushStart F)
 {
@@ -39,7 +39,12 @@ __global__ void __launch_bounds__(256) flush_start_kernel(FlushStart F)
     for (uint32_t i = first; i < F.gradVectors; i += stride)
         F.grad[i] = zero;
     for (uint32_t i = first; i < F.tiles; i += stride)
-        F.ranges[i] = make_uint2(0u, 0u);
+    {
+        const uint32_t scene = find_range(F.tileBase, F.sceneCount, i);
+        const uint2 st = F.sceneTiles[scene]; // (tileBase, tilesX)
+        const uint32_t y = (i - st.x) / st.y;
+        F.ranges[i] = TileHead{0u, 0u, scene, (i - st.x - y * st.y) | (y << 16)};
+    }
 }
 
 // Exclusive scan of up to kSmallScanSlots tile counts (offsets[slots] = the
@@ -173,7 +178,7 @@ __global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(1024, 1)
                       const uint32_t* __restrict__ vals,
                       uint16_t* __restrict__ sortedKeys,
                       uint32_t* __restrict__ sortedVals,
-                      uint2* __restrict__ ranges)
+                      TileHead* __restrict__ ranges)
 {
     extern __shared__ uint4 dyn[];
     SmallSortShared& sh = *reinterpret_cast<SmallSortShared*>(dyn);
@@ -290,9 +295,9 @@ __global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(1024, 1)
     {
         const uint32_t k = __ldcg(sortedKeys + i);
         if (i == 0 || __ldcg(sortedKeys + i - 1) != k)
-            ranges[k].x = i;
+            ranges[k].first = i;
         if (i == n - 1 || __ldcg(sortedKeys + i + 1) != k)
-            ranges[k].y = i + 1;
+            ranges[k].end = i + 1;
     }
 }
 } // namespace rivecuda

@@ -379,6 +379,14 @@ struct WideScatter
 // strip for every warp of 38 triangles.
 constexpr uint32_t kWideBlocks = 304;
 
+// A raster tile: its sorted bin entries [first, end), its scene, and its place
+// there (tx | ty << 16), so a raster CTA starts from one 16-byte load instead of
+// a binary search over the scenes and a division.
+struct __align__(16) TileHead
+{
+    uint32_t first, end, scene, at;
+};
+
 // What flush_start_kernel prepares (kernels_small.cu): the flushes' uniforms, and
 // the buffers that start at zero (gradVectors in 16-byte units; wide and error
 // may be null).
@@ -390,8 +398,10 @@ struct FlushStart
     uint32_t* error;
     uint4* grad;
     uint32_t gradVectors;
-    uint2* ranges;
+    TileHead* ranges;
     uint32_t tiles;
+    const uint32_t* tileBase; // BatchTables
+    const uint2* sceneTiles;
 };
 // The scan and the sort of small frames (kernels_small.cu), one cluster each.
 constexpr uint32_t kSmallCluster = 8;
