@@ -57,11 +57,6 @@ __global__ void center_setup_kernel(BatchTables B,
                                     uint32_t* tileCounts,
                                     uint8_t* tileMasks);
 __global__ void flush_start_kernel(FlushStart F);
-__global__ void small_scan_kernel(uint32_t slots, const uint32_t* counts, uint32_t* offsets,
-                                  uint32_t* hostTotal);
-__global__ void small_sort_kernel(const uint32_t* entryTotal, uint32_t capacity, bool guarded, int keyBits,
-                                  const uint16_t* keys, const uint32_t* vals, uint16_t* sortedKeys,
-                                  uint32_t* sortedVals, TileHead* ranges);
 __global__ void wide_count_kernel(BatchTables B, const TriRecord* tris, uint32_t* tileCounts);
 __global__ void bin_fill_kernel(const uint32_t* pairTotal,
                                 uint32_t capacity,
@@ -282,6 +277,11 @@ struct rive_cuda_context
 {
     int device = 0;
     cudaStream_t stream = nullptr;
+    // The context's stream runs at the device's highest priority and its rasters
+    // at the lowest: the short passes of another context's flush, whose
+    // bin-entry total its host thread waits for, go ahead of the CTAs that a
+    // raster still has to start.
+    int streamPriority = 0, rasterPriority = 0;
     cudaStream_t copyStream = nullptr; // record uploads (rive_cuda_unmap_buffer)
     cudaStream_t readStream = nullptr; // asynchronous read-backs of targets
     bool readsInFlight = false;        // read-backs queued since the last sync
@@ -335,7 +335,8 @@ struct rive_cuda_context
     // Raster configuration (rive_cuda_set_raster_config).
     int tileLog2 = kTileLog2;
     int rasterCtasPerSm = 0; // 0: as many as fit
-    bool raster32Ready = false, smallSortReady = false;
+    bool raster32Ready = false;
+    uint32_t smallCluster = 8; // small_passes_init
     size_t rasterPad[2][2] = {};      // [feather variant][8 or 16 pixel kernel]: padding
     int rasterPadFor[2] = {-1, -1};   // the CTAs-per-SM limit it was found for
     // Stage timing (rive_cuda_set_profiling).
@@ -882,6 +883,7 @@ struct Scratch
     uint32_t *qKeys = nullptr, *qVals = nullptr, *qKeysAlt = nullptr, *qValsAlt = nullptr;
     uint32_t* order = nullptr; // the grid's tile order (kOrderTiles entries)
     bool heaviestFirst = false; // whatever orders_tiles says
+    bool ownStream = false;     // on a stream of the context's or the graph's own
     void* qTemp = nullptr;
     size_t qTempBytes = 0;
 };
@@ -1202,8 +1204,7 @@ int enqueue_front(rive_cuda_context* ctx,
         stage_begin(ctx, RIVE_CUDA_STAGE_BIN, stream);
         if (L.slots <= kSmallScanSlots)
         {
-            small_scan_kernel<<<kSmallCluster, 1024, 0, stream>>>(L.slots, S.counts, S.offsets,
-                                                                  hostTotal);
+            CK(launch_small_scan(ctx->smallCluster, L.slots, S.counts, S.offsets, hostTotal, stream));
         }
         else
         {
@@ -1243,12 +1244,6 @@ size_t occupancy_pad(const void* fn, int threads, int ctas)
 // configuration needs. Called before any stream capture, never inside one.
 int prepare_raster(rive_cuda_context* ctx)
 {
-    if (!ctx->smallSortReady)
-    {
-        CK(cudaFuncSetAttribute(small_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                kSmallSortSmemBytes));
-        ctx->smallSortReady = true;
-    }
     if (ctx->tileLog2 == 5 && !ctx->raster32Ready)
     {
         CK(cudaFuncSetAttribute(raster_tile32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1272,6 +1267,27 @@ int prepare_raster(rive_cuda_context* ctx)
         ctx->rasterPadFor[slot] = ctx->rasterCtasPerSm;
     }
     return RIVE_CUDA_OK;
+}
+
+// Launches a kernel of n CTAs, at *priority unless that is null.
+template <typename... P, typename... A>
+cudaError_t launch_behind(void (*kernel)(P...), uint32_t n, int threads, size_t smem,
+                          cudaStream_t stream, const int* priority, const A&... args)
+{
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(n);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = stream;
+    cudaLaunchAttribute attr = {};
+    if (priority)
+    {
+        attr.id = cudaLaunchAttributePriority;
+        attr.val.priority = *priority;
+        c.attrs = &attr;
+        c.numAttrs = 1;
+    }
+    return cudaLaunchKernelEx(&c, kernel, P(args)...);
 }
 
 // Whether the 16-pixel grid takes its tiles heaviest first without being asked:
@@ -1299,17 +1315,24 @@ int launch_raster(rive_cuda_context* ctx,
                   uint32_t entries,
                   cudaStream_t stream)
 {
+    // Behind other streams' short passes, where it has more CTAs than start at
+    // once (760) and the passes are short: up to four million slots (16 recorded
+    // frames in turn with another context's 2.10 -> 2.03 ms, a 1080x1080 feathered
+    // frame 102 -> 86 us; above, a front half fills the GPU by itself: 1024x1024
+    // strokes, 4.4 M slots, 1.18 -> 1.20 ms).
+    const bool behind = S.ownStream && L.mainTiles > 760 && L.slots <= 1u << 22;
+    const int* priority = behind ? &ctx->rasterPriority : nullptr;
     if (L.tileLog2 == 3)
     {
         const size_t dyn = ctx->rasterCtasPerSm > 0 ? ctx->rasterPad[L.feather][0] : 0;
-        (L.feather ? raster_tile8_feather_kernel : raster_tile8_kernel)<<<L.mainTiles, 64, dyn,
-                                                                           stream>>>(
-            B, tris, sortedSlots, ranges);
+        CK(launch_behind(L.feather ? raster_tile8_feather_kernel : raster_tile8_kernel, L.mainTiles,
+                         64, dyn, stream, priority, B, tris, sortedSlots, ranges));
     }
     else if (L.tileLog2 == 5)
     {
-        (L.feather ? raster_tile32_feather_kernel : raster_tile32_kernel)<<<
-            L.mainTiles, 1024, kRaster32SmemBytes, stream>>>(B, tris, sortedSlots, ranges);
+        CK(launch_behind(L.feather ? raster_tile32_feather_kernel : raster_tile32_kernel,
+                         L.mainTiles, 1024, kRaster32SmemBytes, stream, priority, B, tris,
+                         sortedSlots, ranges));
     }
     else
     {
@@ -1329,9 +1352,8 @@ int launch_raster(rive_cuda_context* ctx,
             tile_order_kernel<<<1, 1024, 0, stream>>>(L.mainTiles, ranges, S.order);
             order = S.order;
         }
-        (L.feather ? raster_tile_feather_kernel : raster_tile_kernel)<<<L.mainTiles, 256, dyn,
-                                                                         stream>>>(
-            B, tris, sortedSlots, ranges, order);
+        CK(launch_behind(L.feather ? raster_tile_feather_kernel : raster_tile_kernel, L.mainTiles,
+                         256, dyn, stream, priority, B, tris, sortedSlots, ranges, order));
     }
     return RIVE_CUDA_OK;
 }
@@ -1362,7 +1384,8 @@ int enqueue_back(rive_cuda_context* ctx,
             wide.blocks = kWideBlocks;
         }
         const uint32_t binBlocks = wide.blocks + (L.slots + 255) / 256;
-        const bool smallSort = S.keys16 && entries <= kSmallSortEntries;
+        const bool smallSort =
+            S.keys16 && entries <= small_sort_capacity(ctx->smallCluster);
         if (S.keys16)
         {
             uint16_t* keys = (uint16_t*)S.keys;
@@ -1395,9 +1418,8 @@ int enqueue_back(rive_cuda_context* ctx,
         if (smallSort)
         {
             // Also writes the ranges, or leaves them empty on overflow.
-            small_sort_kernel<<<kSmallCluster, 1024, kSmallSortSmemBytes, stream>>>(
-                S.offsets + L.slots, entries, guarded, L.endBit(), (const uint16_t*)S.keys, S.vals,
-                (uint16_t*)S.keysAlt, S.valsAlt, S.ranges);
+            CK(launch_small_sort(ctx->smallCluster, entries, S.offsets + L.slots, guarded, L.endBit(),
+                                 (const uint16_t*)S.keys, S.vals, S.valsAlt, S.ranges, stream));
             v.selector = 1;
         }
         else if (S.keys16)
@@ -1642,6 +1664,7 @@ int run_batch_body(rive_cuda_context* ctx,
                                                  : 0;
 
     Scratch S;
+    S.ownStream = stream == ctx->stream;
     S.tables = (uint8_t*)ctx->dTables.ptr;
     S.tess = (uint4*)ctx->tess.ptr;
     S.grad = (uchar4*)ctx->grad.ptr;
@@ -1829,7 +1852,9 @@ int rive_cuda_context_create(int device, rive_cuda_context** out_ctx)
     ctx->device = device;
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess)
-        e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
+        e = cudaDeviceGetStreamPriorityRange(&ctx->rasterPriority, &ctx->streamPriority);
+    if (e == cudaSuccess)
+        e = cudaStreamCreateWithPriority(&ctx->stream, cudaStreamNonBlocking, ctx->streamPriority);
     if (e == cudaSuccess)
         e = cudaStreamCreateWithFlags(&ctx->copyStream, cudaStreamNonBlocking);
     if (e == cudaSuccess)
@@ -1850,6 +1875,8 @@ int rive_cuda_context_create(int device, rive_cuda_context** out_ctx)
         e = cudaMalloc(&ctx->dSpecOverflow, 4);
     if (e == cudaSuccess)
         e = ensure_feather_lut(device);
+    if (e == cudaSuccess)
+        e = small_passes_init(device, &ctx->smallCluster);
     if (e != cudaSuccess)
     {
         fprintf(stderr, "rive_cuda_context_create: %s\n", cudaGetErrorString(e));
@@ -2297,7 +2324,7 @@ int graph_build(rive_cuda_context* ctx,
     int rc = plan_batch(ctx, in, n, L);
     if (rc)
         return rc;
-    CK(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
+    CK(cudaStreamCreateWithPriority(&g->stream, cudaStreamNonBlocking, ctx->streamPriority));
     CK(cudaMallocHost(&g->hError, 8)); // status word; cells the grids asked for
     CK(g->tables.reserve(L.tableBytes));
     CK(g->tess.reserve(L.tessBytes()));
@@ -2332,6 +2359,7 @@ int graph_build(rive_cuda_context* ctx,
     CK(cudaMemset(g->error.ptr, 0, 4));
 
     Scratch S;
+    S.ownStream = true;
     S.tables = (uint8_t*)g->tables.ptr;
     S.tess = (uint4*)g->tess.ptr;
     S.grad = (uchar4*)g->grad.ptr;

@@ -36,11 +36,6 @@ __global__ void outer_setup_kernel(BatchTables B,
                                    uint32_t* tileCounts,
                                    uint8_t* tileMasks);
 __global__ void flush_start_kernel(FlushStart F);
-__global__ void small_scan_kernel(uint32_t slots, const uint32_t* counts, uint32_t* offsets,
-                                  uint32_t* hostTotal);
-__global__ void small_sort_kernel(const uint32_t* entryTotal, uint32_t capacity, bool guarded, int keyBits,
-                                  const uint16_t* keys, const uint32_t* vals, uint16_t* sortedKeys,
-                                  uint32_t* sortedVals, TileHead* ranges);
 __global__ void wide_count_kernel(BatchTables B, const TriRecord* tris, uint32_t* tileCounts);
 __global__ void bin_scatter16_kernel(uint32_t slotCount,
                                    int tileLog2,
@@ -256,12 +251,12 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
         if (!gTablesUp[dev])
         {
             CKN(ensure_feather_lut(dev));
-            CKN(cudaFuncSetAttribute(small_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     kSmallSortSmemBytes));
             gTablesUp[dev] = true;
         }
         pool = (uint8_t*)p;
     }
+    uint32_t cluster = 0;
+    CKN(small_passes_init(dev, &cluster));
     cudaStream_t stream = (cudaStream_t)cuda_stream;
     uint32_t* dError = (uint32_t*)(pool + kStatusOff);
 
@@ -405,7 +400,7 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
         if (wideList)
             wide_count_kernel<<<kWideBlocks, 256, 0, stream>>>(B, tris, counts);
         static_assert(kMaxSlots <= kSmallScanSlots, "the one-cluster scan holds every flush");
-        small_scan_kernel<<<kSmallCluster, 1024, 0, stream>>>(slots, counts, offs, nullptr);
+        CKN(launch_small_scan(cluster, slots, counts, offs, nullptr, stream));
         CKN(cudaMemcpyAsync(&pairs, offs + slots, 4, cudaMemcpyDeviceToHost, stream));
         CKN(cudaStreamSynchronize(stream));
         if (pairs > RIVE_CUDA_NOALLOC_MAX_BIN_ENTRIES)
@@ -436,10 +431,10 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
             ++endBit;
         cub::DoubleBuffer<uint16_t> k(keys, (uint16_t*)(pool + kKeysAltOff));
         cub::DoubleBuffer<uint32_t> v(vals, (uint32_t*)(pool + kValsAltOff));
-        if (pairs <= kSmallSortEntries)
+        if (pairs <= small_sort_capacity(cluster))
         {
-            small_sort_kernel<<<kSmallCluster, 1024, kSmallSortSmemBytes, stream>>>(
-                offs + slots, pairs, false, endBit, keys, vals, k.Alternate(), v.Alternate(), ranges);
+            CKN(launch_small_sort(cluster, pairs, offs + slots, false, endBit, keys, vals,
+                                  v.Alternate(), ranges, stream));
             v.selector = 1;
         }
         else

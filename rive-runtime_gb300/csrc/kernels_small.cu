@@ -7,6 +7,9 @@
 
 #include <cooperative_groups.h>
 
+#include <algorithm>
+#include <mutex>
+
 namespace cg = cooperative_groups;
 
 namespace rivecuda
@@ -52,7 +55,7 @@ __global__ void __launch_bounds__(256) flush_start_kernel(FlushStart F)
 // its share, the CTAs before it give it its start, and a second walk over the
 // share (from L1 or L2) writes the offsets. Bound by latency: 5 us for 115 k
 // slots, against 8 us and two launches of a decoupled look-back scan.
-__global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(1024, 1)
+__global__ void __launch_bounds__(1024, 1)
     small_scan_kernel(uint32_t slots,
                       const uint32_t* __restrict__ counts,
                       uint32_t* __restrict__ offsets,
@@ -61,10 +64,10 @@ __global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(1024, 1)
     __shared__ uint32_t sums[32];
     __shared__ uint32_t share;
     cg::cluster_group cluster = cg::this_cluster();
-    const uint32_t rank = cluster.block_rank();
+    const uint32_t rank = cluster.block_rank(), ctas = cluster.num_blocks();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t vectors = (slots + 3) / 4;
-    const uint32_t per = (vectors + kSmallCluster - 1) / kSmallCluster;
+    const uint32_t per = (vectors + ctas - 1) / ctas;
     const uint32_t lo = min(rank * per, vectors), hi = min(lo + per, vectors);
     auto load = [&](uint32_t v) {
         if (4 * v + 4 <= slots)
@@ -95,7 +98,7 @@ __global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(1024, 1)
     }
     cluster.sync();
     uint32_t before = 0, all = 0;
-    for (uint32_t r = 0; r < kSmallCluster; ++r)
+    for (uint32_t r = 0; r < ctas; ++r)
     {
         const uint32_t t = *cluster.map_shared_rank(&share, r);
         before += r < rank ? t : 0u;
@@ -146,7 +149,7 @@ __global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(1024, 1)
     cluster.sync(); // no CTA leaves while another reads its share
 }
 
-// Stable sort of up to kSmallSortEntries bin entries by 16-bit tile key, and the
+// Stable sort of up to small_sort_capacity bin entries by 16-bit tile key, and the
 // tiles' ranges, by one cluster: one counting pass per key byte. A warp ranks 32
 // entries at a time among equal digits (match), per-warp counters and the
 // CTAs' totals give every entry its place; the first pass moves entries through
@@ -154,29 +157,30 @@ __global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(1024, 1)
 // entries is read on the device. When they are more than `capacity`, the binner
 // has dropped the rest; `guarded` (a speculative flush, which then runs again)
 // leaves every range empty.
-// Bound by latency: 50 k entries in 12 us, against 45 us and seven launches and
-// fills for the library's sort and a pass for the ranges.
-constexpr int kSortWarps = 32, kSortItems = kSmallSortEntries / (kSmallCluster * 1024);
+// 512 threads and 76 KB a CTA leave room beside another stream's raster; a thread
+// holds its up to 16 entries in registers while their places are found. Bound by
+// latency and the exchange: 51 k entries of 320 tiles 14 us with 16 CTAs (18 us
+// with 8), against 45 us and seven launches and fills for the library's sort and
+// the ranges.
+constexpr int kSortThreads = 512, kSortWarps = kSortThreads / 32;
+constexpr int kSortItems = 16;
 constexpr int kSortStride = kSortWarps + 2; // counters of a digit, padded against bank conflicts
 struct SmallSortShared
 {
-    uint32_t vals[kSortItems * 1024];
-    uint16_t keys[kSortItems * 1024];
+    uint2 items[kSortItems * kSortThreads]; // (key, value)
     uint16_t count[256 * kSortStride];
     uint32_t totals[2][256]; // per pass: this CTA's entries of each digit
     uint32_t base[256];
     uint32_t sums[8];
 };
-static_assert(sizeof(SmallSortShared) <= kSmallSortSmemBytes, "kSmallSortSmemBytes");
 
-__global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(1024, 1)
+__global__ void __launch_bounds__(kSortThreads)
     small_sort_kernel(const uint32_t* __restrict__ entryTotal,
                       uint32_t capacity,
                       bool guarded,
                       int keyBits,
                       const uint16_t* __restrict__ keys,
                       const uint32_t* __restrict__ vals,
-                      uint16_t* __restrict__ sortedKeys,
                       uint32_t* __restrict__ sortedVals,
                       TileHead* __restrict__ ranges)
 {
@@ -186,35 +190,44 @@ __global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(1024, 1)
     if (n == 0 || (guarded && *entryTotal > capacity))
         return; // the whole cluster
     cg::cluster_group cluster = cg::this_cluster();
-    const uint32_t rank = cluster.block_rank();
+    const uint32_t rank = cluster.block_rank(), ctas = cluster.num_blocks();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t ltMask = (1u << lane) - 1u;
     // `per` entries a thread: CTA r holds [r chunk, (r + 1) chunk), a warp a run
     // of it, 32 entries a round. Past the last entry: key 0xffff, which sorts
     // behind every tile.
-    const uint32_t per = (n + kSmallCluster * 1024 - 1) / (kSmallCluster * 1024);
-    const uint32_t chunk = per * 1024, run = (uint32_t)warp * per * 32 + lane;
+    const uint32_t per = (n + ctas * kSortThreads - 1) / (ctas * kSortThreads);
+    const uint32_t chunk = per * kSortThreads, run = (uint32_t)warp * per * 32 + lane;
     const uint32_t perInverse = (65536 + per - 1) / per;
+    uint2 item[kSortItems];
+#pragma unroll
+    for (int r = 0; r < kSortItems; ++r)
+    {
+        const uint32_t i = rank * chunk + run + 32 * r;
+        item[r] = make_uint2(0xffffu, 0u);
+        if (r < (int)per && i < n)
+            item[r] = make_uint2(keys[i], vals[i]);
+    }
     const int passes = keyBits > 8 ? 2 : 1;
     for (int p = 0; p < passes; ++p)
     {
-        const bool last = p + 1 == passes;
-        for (int i = threadIdx.x; i < 256 * kSortStride / 2; i += 1024)
+        for (int i = threadIdx.x; i < 256 * kSortStride / 2; i += kSortThreads)
             reinterpret_cast<uint32_t*>(sh.count)[i] = 0;
+        if (p)
+        {
+#pragma unroll
+            for (int r = 0; r < kSortItems; ++r)
+                if (r < (int)per)
+                    item[r] = sh.items[run + 32 * r];
+        }
         __syncthreads();
-        auto key_of = [&](uint32_t r) -> uint32_t {
-            const uint32_t i = run + 32 * r;
-            if (p)
-                return sh.keys[i];
-            return rank * chunk + i < n ? keys[rank * chunk + i] : 0xffffu;
-        };
         uint16_t within[kSortItems]; // place among the warp's entries of the digit
 #pragma unroll
         for (int r = 0; r < kSortItems; ++r)
         {
             if (r >= (int)per)
                 break;
-            const uint32_t digit = (key_of(r) >> (8 * p)) & 0xffu;
+            const uint32_t digit = (item[r].x >> (8 * p)) & 0xffu;
             volatile uint16_t* const c = sh.count + digit * kSortStride + warp;
             const uint32_t peers = __match_any_sync(0xffffffffu, digit);
             const uint32_t old = *c;
@@ -225,23 +238,38 @@ __global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(1024, 1)
             __syncwarp();
         }
         __syncthreads();
-        if (threadIdx.x < 256)
         {
-            uint32_t sum = 0;
-            for (int w = 0; w < kSortWarps; ++w)
+            // kParts threads a digit, eight warps' counters each: their prefix
+            // within the CTA, and the CTA's total.
+            constexpr int kParts = kSortWarps / 8;
+            static_assert(kParts * 256 == kSortThreads, "a thread per digit and part");
+            const int digit = threadIdx.x / kParts, part = threadIdx.x % kParts;
+            uint16_t* const c = sh.count + digit * kSortStride + part * 8;
+            uint32_t v[8], sum = 0;
+#pragma unroll
+            for (int w = 0; w < 8; ++w)
             {
-                uint16_t* const c = sh.count + threadIdx.x * kSortStride + w;
-                const uint32_t v = *c;
-                *c = (uint16_t)sum;
-                sum += v;
+                v[w] = sum;
+                sum += c[w];
             }
-            sh.totals[p][threadIdx.x] = sum;
+            uint32_t scan = sum;
+#pragma unroll
+            for (int o = 1; o < kParts; o <<= 1)
+            {
+                const uint32_t x = __shfl_up_sync(0xffffffffu, scan, o, kParts);
+                scan += part >= o ? x : 0u;
+            }
+#pragma unroll
+            for (int w = 0; w < 8; ++w)
+                c[w] = (uint16_t)(v[w] + scan - sum);
+            if (part == kParts - 1)
+                sh.totals[p][digit] = scan;
         }
-        cluster.sync();
+        cluster.sync(); // totals are there; every CTA has its entries in registers
         uint32_t before = 0, all = 0, scan = 0;
         if (threadIdx.x < 256)
         {
-            for (uint32_t c = 0; c < kSmallCluster; ++c)
+            for (uint32_t c = 0; c < ctas; ++c)
             {
                 const uint32_t t = *cluster.map_shared_rank(&sh.totals[p][threadIdx.x], c);
                 before += c < rank ? t : 0u;
@@ -270,34 +298,121 @@ __global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(1024, 1)
         {
             if (r >= (int)per)
                 break;
-            const uint32_t i = run + 32 * r;
-            const uint32_t key = key_of(r), digit = (key >> (8 * p)) & 0xffu;
+            const uint32_t digit = (item[r].x >> (8 * p)) & 0xffu;
             const uint32_t to = sh.base[digit] + sh.count[digit * kSortStride + warp] + within[r];
-            if (last)
-            {
-                if (key != 0xffffu)
-                {
-                    sortedKeys[to] = (uint16_t)key;
-                    sortedVals[to] = p ? sh.vals[i] : vals[rank * chunk + i];
-                }
-            }
-            else
-            {
-                const uint32_t owner = ((to >> 10) * perInverse) >> 16, at = to - owner * chunk;
-                *cluster.map_shared_rank(&sh.keys[at], owner) = (uint16_t)key;
-                if (key != 0xffffu)
-                    *cluster.map_shared_rank(&sh.vals[at], owner) = vals[rank * chunk + i];
-            }
+            const uint32_t owner = ((to / kSortThreads) * perInverse) >> 16;
+            *cluster.map_shared_rank(&sh.items[to - owner * chunk], owner) = item[r];
         }
         cluster.sync(); // entries are where the next pass, or the ranges, read them
     }
-    for (uint32_t i = rank * 1024 + threadIdx.x; i < n; i += kSmallCluster * 1024)
+    for (uint32_t j = threadIdx.x; j < chunk; j += kSortThreads)
     {
-        const uint32_t k = __ldcg(sortedKeys + i);
-        if (i == 0 || __ldcg(sortedKeys + i - 1) != k)
-            ranges[k].first = i;
-        if (i == n - 1 || __ldcg(sortedKeys + i + 1) != k)
-            ranges[k].end = i + 1;
+        const uint32_t i = rank * chunk + j;
+        if (i >= n)
+            break;
+        const uint2 e = sh.items[j];
+        sortedVals[i] = e.y;
+        const uint32_t prev = j ? sh.items[j - 1].x
+                              : i ? cluster.map_shared_rank(&sh.items[chunk - 1], rank - 1)->x
+                                  : 0xffffu;
+        if (prev != e.x)
+        {
+            ranges[e.x].first = i;
+            if (prev != 0xffffu)
+                ranges[prev].end = i;
+        }
+        if (i == n - 1)
+            ranges[e.x].end = n;
     }
+    cluster.sync(); // no CTA leaves while the next one reads its last key
+}
+
+namespace
+{
+template <typename... P, typename... A>
+cudaError_t launch_cluster(void (*kernel)(P...), uint32_t ctas, int threads, size_t smem,
+                           cudaStream_t stream, const A&... args)
+{
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = ctas;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(ctas);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = stream;
+    c.attrs = &attr;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
+// CTAs of a cluster for `items` of work at `perCta` each: the smallest cluster
+// (lower latency: a 240x180 widget 54 against 56 us with 16) where it has room
+// for a few rounds, the device's largest above.
+uint32_t cluster_for(uint32_t items, uint32_t perCta, uint32_t largest)
+{
+    return items <= 8 * perCta ? std::min(8u, largest) : largest;
+}
+} // namespace
+
+cudaError_t small_passes_init(int device, uint32_t* largest)
+{
+    static std::mutex m;
+    static uint32_t found[64] = {};
+    std::lock_guard<std::mutex> lock(m);
+    if (device < 0 || device >= 64)
+        return cudaErrorInvalidDevice;
+    if (!found[device])
+    {
+        // 16 CTAs need a GPC with as many free SMs (not every partition of the
+        // device has one); 8 are portable.
+        cudaError_t e = cudaFuncSetAttribute(
+            small_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(SmallSortShared));
+        for (auto fn : {(const void*)small_sort_kernel, (const void*)small_scan_kernel})
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e != cudaSuccess)
+            return e;
+        cudaLaunchAttribute attr = {};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = 16;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cudaLaunchConfig_t c = {};
+        c.gridDim = dim3(16);
+        c.attrs = &attr;
+        c.numAttrs = 1;
+        int sorts = 0, scans = 0;
+        c.blockDim = dim3(kSortThreads);
+        c.dynamicSmemBytes = sizeof(SmallSortShared);
+        e = cudaOccupancyMaxActiveClusters(&sorts, small_sort_kernel, &c);
+        c.blockDim = dim3(1024);
+        c.dynamicSmemBytes = 0;
+        if (e == cudaSuccess)
+            e = cudaOccupancyMaxActiveClusters(&scans, small_scan_kernel, &c);
+        if (e != cudaSuccess)
+            cudaGetLastError(); // a failed query only leaves the portable size
+        found[device] = e == cudaSuccess && sorts > 0 && scans > 0 ? 16 : 8;
+    }
+    *largest = found[device];
+    return cudaSuccess;
+}
+
+uint32_t small_sort_capacity(uint32_t largest) { return largest * kSortThreads * kSortItems; }
+
+cudaError_t launch_small_scan(uint32_t largest, uint32_t slots, const uint32_t* counts,
+                              uint32_t* offsets, uint32_t* hostTotal, cudaStream_t stream)
+{
+    return launch_cluster(small_scan_kernel, cluster_for(slots, 8192, largest), 1024, 0, stream, slots,
+                          counts, offsets, hostTotal);
+}
+
+cudaError_t launch_small_sort(uint32_t largest, uint32_t entries, const uint32_t* entryTotal,
+                              bool guarded, int keyBits, const uint16_t* keys, const uint32_t* vals,
+                              uint32_t* sortedVals, TileHead* ranges, cudaStream_t stream)
+{
+    return launch_cluster(small_sort_kernel, cluster_for(entries, 2048, largest), kSortThreads,
+                          sizeof(SmallSortShared), stream, entryTotal, entries, guarded, keyBits, keys,
+                          vals, sortedVals, ranges);
 }
 } // namespace rivecuda

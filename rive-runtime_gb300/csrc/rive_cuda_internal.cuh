@@ -403,11 +403,18 @@ struct FlushStart
     const uint32_t* tileBase; // BatchTables
     const uint2* sceneTiles;
 };
-// The scan and the sort of small frames (kernels_small.cu), one cluster each.
-constexpr uint32_t kSmallCluster = 8;
+// The scan and the sort of small frames, one cluster each (kernels_small.cu).
+// small_passes_init finds the device's largest cluster for them (once per
+// device, before any stream capture); the scan takes up to kSmallScanSlots slots,
+// the sort up to small_sort_capacity entries.
 constexpr uint32_t kSmallScanSlots = 1u << 18;
-constexpr uint32_t kSmallSortEntries = 1u << 17;
-constexpr int kSmallSortSmemBytes = (int)kSmallSortEntries / (int)kSmallCluster * 6 + 256 * 34 * 2 + 3200;
+cudaError_t small_passes_init(int device, uint32_t* largest);
+uint32_t small_sort_capacity(uint32_t largest);
+cudaError_t launch_small_scan(uint32_t largest, uint32_t slots, const uint32_t* counts,
+                              uint32_t* offsets, uint32_t* hostTotal, cudaStream_t stream);
+cudaError_t launch_small_sort(uint32_t largest, uint32_t entries, const uint32_t* entryTotal,
+                              bool guarded, int keyBits, const uint16_t* keys, const uint32_t* vals,
+                              uint32_t* sortedVals, TileHead* ranges, cudaStream_t stream);
 
 // Batches the raster grid orders its tiles for (tile_order_kernel).
 constexpr uint32_t kOrderMinTiles = 512;
