@@ -884,6 +884,7 @@ struct Scratch
     uint32_t* order = nullptr; // the grid's tile order (kOrderTiles entries)
     bool heaviestFirst = false; // whatever orders_tiles says
     bool ownStream = false;     // on a stream of the context's or the graph's own
+    bool overlap = false;       // kernels start while the one before runs out (chain_launch)
     void* qTemp = nullptr;
     size_t qTempBytes = 0;
 };
@@ -1144,6 +1145,9 @@ int enqueue_front(rive_cuda_context* ctx,
     F.tileBase = B.tileBase;
     F.sceneTiles = B.sceneTiles;
     flush_start_kernel<<<flush_start_blocks(F), 256, 0, stream>>>(F);
+    // The kernels below follow one another with nothing between, but for the
+    // winding grids' passes and fills and the events of stage timing.
+    const bool overlap = S.overlap && !L.winding && !L.imageSlots && !ctx->profiling;
     if (L.imageSlots)
         CK(cudaMemsetAsync(S.pathImage, 0xff, (size_t)std::max(L.paths, 1u) * 4, stream));
     if (L.winding)
@@ -1161,35 +1165,36 @@ int enqueue_front(rive_cuda_context* ctx,
     if (L.gradSpans)
     {
         stage_begin(ctx, RIVE_CUDA_STAGE_COLOR_RAMP, stream);
-        color_ramp_kernel<<<L.gradSpans, 128, 0, stream>>>(B);
+        CK(chain_launch(color_ramp_kernel, L.gradSpans, 128, 0, stream, overlap, nullptr, B));
         stage_end(ctx, stream);
     }
     if (L.tessSpans)
     {
         stage_begin(ctx, RIVE_CUDA_STAGE_TESSELLATE, stream);
         const int lanes = tess_lanes_log2(L.tessSpans, L.feather);
-        (L.feather ? tessellate_feather_kernel
-                   : tessellate_kernel)<<<((L.tessSpans << lanes) + 255u) / 256u, 256, 0, stream>>>(
-            B, lanes);
+        CK(chain_launch(L.feather ? tessellate_feather_kernel : tessellate_kernel,
+                        ((L.tessSpans << lanes) + 255u) / 256u, 256, 0, stream, overlap, nullptr, B,
+                        lanes));
         stage_end(ctx, stream);
     }
     if (L.slots)
     {
         stage_begin(ctx, RIVE_CUDA_STAGE_PATCH_SETUP, stream);
         if (L.items[0])
-            (L.feather   ? patch_setup_feather_kernel
-             : L.winding ? patch_setup_winding_kernel
-                         : patch_setup_kernel)<<<(L.items[0] + 3) / 4, 128, 0, stream>>>(
-                B, S.tris, S.counts, S.masks);
+            CK(chain_launch(L.feather   ? patch_setup_feather_kernel
+                            : L.winding ? patch_setup_winding_kernel
+                                        : patch_setup_kernel,
+                            (L.items[0] + 3) / 4, 128, 0, stream, overlap, nullptr, B, S.tris,
+                            S.counts, S.masks));
         if (L.items[1])
-            outer_setup_kernel<<<(L.items[1] + 3) / 4, 128, 0, stream>>>(B, S.tris, S.counts,
-                                                                         S.masks);
+            CK(chain_launch(outer_setup_kernel, (L.items[1] + 3) / 4, 128, 0, stream, overlap,
+                            nullptr, B, S.tris, S.counts, S.masks));
         if (L.items[2])
-            interior_setup_kernel<<<(L.items[2] + 255) / 256, 256, 0, stream>>>(B, S.tris, S.counts,
-                                                                                S.masks);
+            CK(chain_launch(interior_setup_kernel, (L.items[2] + 255) / 256, 256, 0, stream, overlap,
+                            nullptr, B, S.tris, S.counts, S.masks));
         if (L.items[3])
-            center_setup_kernel<<<(L.items[3] + 3) / 4, 128, 0, stream>>>(B, S.tris, S.counts,
-                                                                          S.masks);
+            CK(chain_launch(center_setup_kernel, (L.items[3] + 3) / 4, 128, 0, stream, overlap,
+                            nullptr, B, S.tris, S.counts, S.masks));
         if (L.winding)
         {
             // The deferred fan triangles' winding deltas and edge tiles, then
@@ -1199,12 +1204,14 @@ int enqueue_front(rive_cuda_context* ctx,
             path_winding_kernel<<<(L.paths + 7) / 8, 256, 0, stream>>>(B, S.counts);
         }
         if (L.wide)
-            wide_count_kernel<<<kWideBlocks, 256, 0, stream>>>(B, S.tris, S.counts);
+            CK(chain_launch(wide_count_kernel, kWideBlocks, 256, 0, stream, overlap, nullptr, B,
+                            S.tris, S.counts));
         stage_end(ctx, stream);
         stage_begin(ctx, RIVE_CUDA_STAGE_BIN, stream);
         if (L.slots <= kSmallScanSlots)
         {
-            CK(launch_small_scan(ctx->smallCluster, L.slots, S.counts, S.offsets, hostTotal, stream));
+            CK(launch_small_scan(ctx->smallCluster, L.slots, S.counts, S.offsets, hostTotal, stream,
+                                 overlap));
         }
         else
         {
@@ -1269,27 +1276,6 @@ int prepare_raster(rive_cuda_context* ctx)
     return RIVE_CUDA_OK;
 }
 
-// Launches a kernel of n CTAs, at *priority unless that is null.
-template <typename... P, typename... A>
-cudaError_t launch_behind(void (*kernel)(P...), uint32_t n, int threads, size_t smem,
-                          cudaStream_t stream, const int* priority, const A&... args)
-{
-    cudaLaunchConfig_t c = {};
-    c.gridDim = dim3(n);
-    c.blockDim = dim3(threads);
-    c.dynamicSmemBytes = smem;
-    c.stream = stream;
-    cudaLaunchAttribute attr = {};
-    if (priority)
-    {
-        attr.id = cudaLaunchAttributePriority;
-        attr.val.priority = *priority;
-        c.attrs = &attr;
-        c.numAttrs = 1;
-    }
-    return cudaLaunchKernelEx(&c, kernel, P(args)...);
-}
-
 // Whether the 16-pixel grid takes its tiles heaviest first without being asked:
 // from about one wave of CTAs (760) to what one CTA can order, and where a tile
 // is long enough for the last ones to leave the GPU half empty. 3072 tiles of
@@ -1313,6 +1299,7 @@ int launch_raster(rive_cuda_context* ctx,
                   const uint32_t* sortedSlots,
                   const TileHead* ranges,
                   uint32_t entries,
+                  bool overlap,
                   cudaStream_t stream)
 {
     // Behind other streams' short passes, where it has more CTAs than start at
@@ -1325,13 +1312,13 @@ int launch_raster(rive_cuda_context* ctx,
     if (L.tileLog2 == 3)
     {
         const size_t dyn = ctx->rasterCtasPerSm > 0 ? ctx->rasterPad[L.feather][0] : 0;
-        CK(launch_behind(L.feather ? raster_tile8_feather_kernel : raster_tile8_kernel, L.mainTiles,
-                         64, dyn, stream, priority, B, tris, sortedSlots, ranges));
+        CK(chain_launch(L.feather ? raster_tile8_feather_kernel : raster_tile8_kernel, L.mainTiles,
+                         64, dyn, stream, overlap, priority, B, tris, sortedSlots, ranges));
     }
     else if (L.tileLog2 == 5)
     {
-        CK(launch_behind(L.feather ? raster_tile32_feather_kernel : raster_tile32_kernel,
-                         L.mainTiles, 1024, kRaster32SmemBytes, stream, priority, B, tris,
+        CK(chain_launch(L.feather ? raster_tile32_feather_kernel : raster_tile32_kernel,
+                         L.mainTiles, 1024, kRaster32SmemBytes, stream, overlap, priority, B, tris,
                          sortedSlots, ranges));
     }
     else
@@ -1346,14 +1333,16 @@ int launch_raster(rive_cuda_context* ctx,
             size_t tb = S.qTempBytes;
             CK(cub::DeviceRadixSort::SortPairs(S.qTemp, tb, k, v, (int)L.mainTiles, 0, 32, stream));
             order = v.Current();
+            overlap = false;
         }
         else if (S.order && (S.heaviestFirst || orders_tiles(L, entries)))
         {
-            tile_order_kernel<<<1, 1024, 0, stream>>>(L.mainTiles, ranges, S.order);
+            CK(chain_launch(tile_order_kernel, 1, 1024, 0, stream, overlap, nullptr, L.mainTiles,
+                            ranges, S.order));
             order = S.order;
         }
-        CK(launch_behind(L.feather ? raster_tile_feather_kernel : raster_tile_kernel, L.mainTiles,
-                         256, dyn, stream, priority, B, tris, sortedSlots, ranges, order));
+        CK(chain_launch(L.feather ? raster_tile_feather_kernel : raster_tile_kernel, L.mainTiles,
+                         256, dyn, stream, overlap, priority, B, tris, sortedSlots, ranges, order));
     }
     return RIVE_CUDA_OK;
 }
@@ -1372,6 +1361,11 @@ int enqueue_back(rive_cuda_context* ctx,
 {
     uint32_t* const binError = S.binError ? S.binError : S.error;
     const uint32_t* sortedSlots = nullptr;
+    // The kernels from the binner on follow one another directly where the
+    // one-cluster sort is among them.
+    const bool chained = S.overlap && !ctx->profiling && entries && L.slots && S.keys16 &&
+                         entries <= small_sort_capacity(ctx->smallCluster);
+    const bool overlap = chained;
     if (entries && L.slots)
     {
         stage_begin(ctx, RIVE_CUDA_STAGE_BIN, stream);
@@ -1419,7 +1413,8 @@ int enqueue_back(rive_cuda_context* ctx,
         {
             // Also writes the ranges, or leaves them empty on overflow.
             CK(launch_small_sort(ctx->smallCluster, entries, S.offsets + L.slots, guarded, L.endBit(),
-                                 (const uint16_t*)S.keys, S.vals, S.valsAlt, S.ranges, stream));
+                                 (const uint16_t*)S.keys, S.vals, S.valsAlt, S.ranges, stream,
+                                 overlap));
             v.selector = 1;
         }
         else if (S.keys16)
@@ -1454,18 +1449,19 @@ int enqueue_back(rive_cuda_context* ctx,
         // The feather atlases first: the main raster's blits sample them.
         const uint32_t atlasTiles = L.tiles - L.mainTiles;
         if (L.tileLog2 == 3)
-            raster_atlas8_kernel<<<atlasTiles, 64, 0, stream>>>(B, S.tris, sortedSlots, S.ranges,
-                                                                L.mainTiles);
+            CK(chain_launch(raster_atlas8_kernel, atlasTiles, 64, 0, stream, overlap, nullptr, B,
+                            S.tris, sortedSlots, S.ranges, L.mainTiles));
         else if (L.tileLog2 == 5)
-            raster_atlas32_kernel<<<atlasTiles, 1024, kRaster32SmemBytes, stream>>>(B, S.tris, sortedSlots,
-                                                                   S.ranges, L.mainTiles);
+            CK(chain_launch(raster_atlas32_kernel, atlasTiles, 1024, kRaster32SmemBytes, stream,
+                            overlap, nullptr, B, S.tris, sortedSlots, S.ranges, L.mainTiles));
         else
-            raster_atlas_kernel<<<atlasTiles, 256, 0, stream>>>(B, S.tris, sortedSlots, S.ranges,
-                                                                L.mainTiles);
+            CK(chain_launch(raster_atlas_kernel, atlasTiles, 256, 0, stream, overlap, nullptr, B,
+                            S.tris, sortedSlots, S.ranges, L.mainTiles));
     }
     if (ctx->rasterWait)
         CK(cudaStreamWaitEvent(stream, ctx->rasterWait, 0));
-    int rc = launch_raster(ctx, L, B, S, S.tris, sortedSlots, S.ranges, entries, stream);
+    int rc = launch_raster(ctx, L, B, S, S.tris, sortedSlots, S.ranges, entries,
+                           overlap && !ctx->rasterWait, stream);
     stage_end(ctx, stream);
     if (rc)
         return rc;
@@ -1665,6 +1661,7 @@ int run_batch_body(rive_cuda_context* ctx,
 
     Scratch S;
     S.ownStream = stream == ctx->stream;
+    S.overlap = L.slots <= kSmallScanSlots; // where launches count
     S.tables = (uint8_t*)ctx->dTables.ptr;
     S.tess = (uint4*)ctx->tess.ptr;
     S.grad = (uchar4*)ctx->grad.ptr;

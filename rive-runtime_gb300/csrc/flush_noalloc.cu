@@ -377,13 +377,13 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
     flush_start_kernel<<<(std::max(F.gradVectors, tiles) + 255) / 256, 256, 0, stream>>>(F);
 
     if (d->grad_span_count)
-        color_ramp_kernel<<<d->grad_span_count, 128, 0, stream>>>(B);
+        CKN(chain_launch(color_ramp_kernel, d->grad_span_count, 128, 0, stream, true, nullptr, B));
     if (d->tess_span_count)
     {
         const int lanes = tess_lanes_log2(d->tess_span_count, feather);
-        (feather ? tessellate_feather_kernel
-                 : tessellate_kernel)<<<((d->tess_span_count << lanes) + 255u) / 256u, 256, 0,
-                                        stream>>>(B, lanes);
+        CKN(chain_launch(feather ? tessellate_feather_kernel : tessellate_kernel,
+                         ((d->tess_span_count << lanes) + 255u) / 256u, 256, 0, stream, true,
+                         nullptr, B, lanes));
     }
 
     TriRecord* tris = (TriRecord*)(pool + kTrisOff);
@@ -394,13 +394,13 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
     uint32_t pairs = 0;
     if (slots)
     {
-        (feather ? patch_setup_feather_kernel : patch_setup_kernel)<<<(instAcc + 3) / 4, 128, 0,
-                                                                     stream>>>(B, tris, counts,
-                                                                               masks);
+        CKN(chain_launch(feather ? patch_setup_feather_kernel : patch_setup_kernel,
+                         (instAcc + 3) / 4, 128, 0, stream, true, nullptr, B, tris, counts, masks));
         if (wideList)
-            wide_count_kernel<<<kWideBlocks, 256, 0, stream>>>(B, tris, counts);
+            CKN(chain_launch(wide_count_kernel, kWideBlocks, 256, 0, stream, true, nullptr, B, tris,
+                             counts));
         static_assert(kMaxSlots <= kSmallScanSlots, "the one-cluster scan holds every flush");
-        CKN(launch_small_scan(cluster, slots, counts, offs, nullptr, stream));
+        CKN(launch_small_scan(cluster, slots, counts, offs, nullptr, stream, true));
         CKN(cudaMemcpyAsync(&pairs, offs + slots, 4, cudaMemcpyDeviceToHost, stream));
         CKN(cudaStreamSynchronize(stream));
         if (pairs > RIVE_CUDA_NOALLOC_MAX_BIN_ENTRIES)
@@ -434,7 +434,7 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
         if (pairs <= small_sort_capacity(cluster))
         {
             CKN(launch_small_sort(cluster, pairs, offs + slots, false, endBit, keys, vals,
-                                  v.Alternate(), ranges, stream));
+                                  v.Alternate(), ranges, stream, true));
             v.selector = 1;
         }
         else

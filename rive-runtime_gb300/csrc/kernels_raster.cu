@@ -1300,7 +1300,8 @@ __device__ __forceinline__ void patch_setup(const BatchTables& B,
     __shared__ float2 sZW[4][kFeather ? kVerts : 1];
     __shared__ bool sok[4];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t gi = blockIdx.x * 4 + w;
+    chain_next();
+    const uint32_t gi = blockIdx.x * 4 + w + chain_wait();
     if (gi >= B.totalItems[kList])
         return; // whole warp exits together
     const uint32_t seg = find_range(B.segBase[kList], B.segCount[kList], gi);
@@ -1480,7 +1481,8 @@ __device__ __forceinline__ void fan_setup(const BatchTables& B,
     __shared__ uint2 sMeta[4][kPatchVertexCount];
     constexpr uint32_t kDiscard = 1u << 31;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t gi = blockIdx.x * 4 + w;
+    chain_next();
+    const uint32_t gi = blockIdx.x * 4 + w + chain_wait();
     if (gi >= B.totalItems[0])
         return; // whole warp exits together
     const uint32_t seg = find_range(B.segBase[0], B.segCount[0], gi);
@@ -1702,10 +1704,12 @@ __global__ void __launch_bounds__(256) interior_setup_kernel(BatchTables B,
                                                              uint32_t* __restrict__ tileCounts,
                                                              uint8_t* __restrict__ tileMasks)
 {
+    chain_next();
+    const uint32_t zero = chain_wait();
     const uint32_t first = (blockIdx.x * blockDim.x) & ~31u;
     if (first >= B.totalItems[2])
         return; // whole warp exits together
-    const uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x + zero;
     const bool has = gi < B.totalItems[2];
     int4 bb = make_int4(0, 0, 0, 0);
     float4 e[3];
@@ -2077,7 +2081,8 @@ __global__ void __launch_bounds__(256) wide_count_kernel(BatchTables B,
                                                          const TriRecord* __restrict__ tris,
                                                          uint32_t* __restrict__ tileCounts)
 {
-    const uint32_t items = min(*B.wide, B.wideCap) * kWideStrips;
+    chain_next();
+    const uint32_t items = min(B.wide[chain_wait()], B.wideCap) * kWideStrips;
     const int lane = threadIdx.x & 31;
     for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < items;
          i += (gridDim.x * blockDim.x) >> 5)
@@ -2152,9 +2157,10 @@ __device__ __forceinline__ void bin_scatter_wide(int tileLog2,
                                                  uint32_t* __restrict__ error,
                                                  K* __restrict__ keys,
                                                  uint32_t* __restrict__ vals,
-                                                 const WideScatter& wide)
+                                                 const WideScatter& wide,
+                                                 uint32_t zero)
 {
-    const uint32_t items = min(*wide.list, wide.cap) * kWideStrips;
+    const uint32_t items = min(wide.list[zero], wide.cap) * kWideStrips;
     const int lane = threadIdx.x & 31;
     for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < items;
          i += (wide.blocks * blockDim.x) >> 5)
@@ -2214,12 +2220,15 @@ __device__ __forceinline__ void bin_scatter(const BatchTables* __restrict__ Bw,
                                             const WideScatter& wide)
 {
     const int lane = threadIdx.x & 31;
+    chain_next();
+    const uint32_t zero = chain_wait();
     if (blockIdx.x < wide.blocks)
     {
-        bin_scatter_wide(tileLog2, sceneTiles, tris, offsets, capacity, error, keys, vals, wide);
+        bin_scatter_wide(tileLog2, sceneTiles, tris, offsets, capacity, error, keys, vals, wide,
+                         zero);
         return;
     }
-    const uint32_t warpId = ((blockIdx.x - wide.blocks) * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t warpId = (((blockIdx.x - wide.blocks) * blockDim.x + threadIdx.x) >> 5) + zero;
     const uint32_t first = warpId * 32;
     if (first >= slotCount)
         return;
@@ -3800,6 +3809,12 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
         fb[(size_t)py * width + px] = s.color;
 }
 
+__device__ __forceinline__ uint32_t raster_index(const uint32_t* __restrict__ order)
+{
+    const uint32_t i = blockIdx.x + chain_wait();
+    return order ? order[i] : i;
+}
+
 // The raster kernels, each without and with the feather paths (the host
 // launches the feather variant only for batches with ENABLE_FEATHER draws). The
 // 16x16 one takes its tiles in the order of `order` (heaviest first), or as
@@ -3814,7 +3829,7 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
     {                                                                                             \
         __shared__ RasterShared<4> sh;                                                            \
         raster_tile<4, FEATHER>(B, tris, sortedSlots, ranges, sh,                                 \
-                                order ? order[blockIdx.x] : blockIdx.x);                          \
+                                raster_index(order));                                             \
     }
 RIVE_RASTER_KERNELS(raster_tile_kernel, false)
 RIVE_RASTER_KERNELS(raster_tile_feather_kernel, true)
@@ -3943,7 +3958,8 @@ __device__ __forceinline__ void raster_atlas_tile(const BatchTables& B,
         uint32_t firstTile)                                                                       \
     {                                                                                             \
         __shared__ RasterShared<TL> sh;                                                           \
-        raster_atlas_tile<TL>(B, tris, sortedSlots, ranges, sh, firstTile + blockIdx.x);          \
+        raster_atlas_tile<TL>(B, tris, sortedSlots, ranges, sh,                                   \
+                              firstTile + raster_index(nullptr));                                 \
     }
 RIVE_ATLAS_KERNEL(raster_atlas8_kernel, 3)
 RIVE_ATLAS_KERNEL(raster_atlas_kernel, 4)
@@ -3954,7 +3970,7 @@ __global__ void __launch_bounds__(1024) raster_atlas32_kernel(
 {
     extern __shared__ uint4 dyn[]; // kRaster32SmemBytes
     raster_atlas_tile<5>(B, tris, sortedSlots, ranges, *reinterpret_cast<RasterShared<5>*>(dyn),
-                         firstTile + blockIdx.x);
+                         firstTile + raster_index(nullptr));
 }
 
 // The tiles of a batch of at most kOrderTiles, heaviest first to within an
@@ -3970,6 +3986,7 @@ __global__ void __launch_bounds__(1024, 1) tile_order_kernel(uint32_t tiles,
     __shared__ uint32_t count[kBuckets * kWarps]; // [bucket][warp]
     __shared__ uint32_t sums[kWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    ranges += chain_wait();
     auto bucket = [&](uint32_t i) {
         const uint2 r = *reinterpret_cast<const uint2*>(ranges + i); // first, end
         const uint32_t n = r.y > r.x ? r.y - r.x : 0u;
@@ -4030,7 +4047,7 @@ __global__ void __launch_bounds__(256) tile_order_keys_kernel(uint32_t tiles,
                                                const TileHead* __restrict__ ranges)                 \
     {                                                                                             \
         __shared__ RasterShared<3> sh;                                                            \
-        raster_tile<3, FEATHER>(B, tris, sortedSlots, ranges, sh, blockIdx.x);                    \
+        raster_tile<3, FEATHER>(B, tris, sortedSlots, ranges, sh, raster_index(nullptr));         \
     }
 RIVE_RASTER8_KERNELS(raster_tile8_kernel, false)
 RIVE_RASTER8_KERNELS(raster_tile8_feather_kernel, true)
@@ -4045,7 +4062,7 @@ RIVE_RASTER8_KERNELS(raster_tile8_feather_kernel, true)
     {                                                                                             \
         extern __shared__ uint4 dyn[];                                                            \
         RasterShared<5>& sh = *reinterpret_cast<RasterShared<5>*>(dyn);                           \
-        raster_tile<5, FEATHER>(B, tris, sortedSlots, ranges, sh, blockIdx.x);                    \
+        raster_tile<5, FEATHER>(B, tris, sortedSlots, ranges, sh, raster_index(nullptr));         \
     }
 static_assert(sizeof(RasterShared<5>) <= kRaster32SmemBytes, "kRaster32SmemBytes");
 RIVE_RASTER32_KERNELS(raster_tile32_kernel, false)

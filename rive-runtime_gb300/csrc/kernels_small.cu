@@ -22,7 +22,8 @@ namespace rivecuda
 // counter. One launch in the place of four.
 __global__ void __launch_bounds__(256) flush_start_kernel(FlushStart F)
 {
-    const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x + chain_wait();
+    chain_next();
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t i = first; i < F.sceneCount; i += stride)
     {
@@ -66,6 +67,7 @@ __global__ void __launch_bounds__(1024, 1)
     cg::cluster_group cluster = cg::this_cluster();
     const uint32_t rank = cluster.block_rank(), ctas = cluster.num_blocks();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    counts += chain_wait();
     const uint32_t vectors = (slots + 3) / 4;
     const uint32_t per = (vectors + ctas - 1) / ctas;
     const uint32_t lo = min(rank * per, vectors), hi = min(lo + per, vectors);
@@ -186,6 +188,10 @@ __global__ void __launch_bounds__(kSortThreads)
 {
     extern __shared__ uint4 dyn[];
     SmallSortShared& sh = *reinterpret_cast<SmallSortShared*>(dyn);
+    const uint32_t zero = chain_wait();
+    entryTotal += zero;
+    keys += zero;
+    vals += zero;
     const uint32_t n = min(*entryTotal, capacity);
     if (n == 0 || (guarded && *entryTotal > capacity))
         return; // the whole cluster
@@ -331,19 +337,21 @@ namespace
 {
 template <typename... P, typename... A>
 cudaError_t launch_cluster(void (*kernel)(P...), uint32_t ctas, int threads, size_t smem,
-                           cudaStream_t stream, const A&... args)
+                           cudaStream_t stream, bool overlap, const A&... args)
 {
-    cudaLaunchAttribute attr = {};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = ctas;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchAttribute attr[2] = {};
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ctas;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t c = {};
     c.gridDim = dim3(ctas);
     c.blockDim = dim3(threads);
     c.dynamicSmemBytes = smem;
     c.stream = stream;
-    c.attrs = &attr;
-    c.numAttrs = 1;
+    c.attrs = attr;
+    c.numAttrs = overlap ? 2 : 1;
     return cudaLaunchKernelEx(&c, kernel, P(args)...);
 }
 
@@ -401,18 +409,20 @@ cudaError_t small_passes_init(int device, uint32_t* largest)
 uint32_t small_sort_capacity(uint32_t largest) { return largest * kSortThreads * kSortItems; }
 
 cudaError_t launch_small_scan(uint32_t largest, uint32_t slots, const uint32_t* counts,
-                              uint32_t* offsets, uint32_t* hostTotal, cudaStream_t stream)
+                              uint32_t* offsets, uint32_t* hostTotal, cudaStream_t stream,
+                              bool overlap)
 {
-    return launch_cluster(small_scan_kernel, cluster_for(slots, 8192, largest), 1024, 0, stream, slots,
-                          counts, offsets, hostTotal);
+    return launch_cluster(small_scan_kernel, cluster_for(slots, 8192, largest), 1024, 0, stream,
+                          overlap, slots, counts, offsets, hostTotal);
 }
 
 cudaError_t launch_small_sort(uint32_t largest, uint32_t entries, const uint32_t* entryTotal,
                               bool guarded, int keyBits, const uint16_t* keys, const uint32_t* vals,
-                              uint32_t* sortedVals, TileHead* ranges, cudaStream_t stream)
+                              uint32_t* sortedVals, TileHead* ranges, cudaStream_t stream,
+                              bool overlap)
 {
     return launch_cluster(small_sort_kernel, cluster_for(entries, 2048, largest), kSortThreads,
-                          sizeof(SmallSortShared), stream, entryTotal, entries, guarded, keyBits, keys,
+                          sizeof(SmallSortShared), stream, overlap, entryTotal, entries, guarded, keyBits, keys,
                           vals, sortedVals, ranges);
 }
 } // namespace rivecuda

@@ -568,7 +568,8 @@ __device__ uint4 tess_vertex(const SpanSetup& s, float vertexIdx, uint32_t flags
 // of the 512 texel columns.
 __global__ void __launch_bounds__(128) color_ramp_kernel(BatchTables B)
 {
-    const uint32_t g = blockIdx.x;
+    chain_next();
+    const uint32_t g = blockIdx.x + chain_wait();
     if (g >= B.totalGradSpans)
         return;
     const uint32_t scene = find_range(B.gradSpanBase, B.sceneCount, g);
@@ -625,7 +626,8 @@ __global__ void __launch_bounds__(128) color_ramp_kernel(BatchTables B)
 template <bool kFeather>
 __device__ __forceinline__ void tessellate(const BatchTables& B, int lanesLog2)
 {
-    const uint32_t gs = (blockIdx.x * blockDim.x + threadIdx.x) >> lanesLog2;
+    chain_next();
+    const uint32_t gs = ((blockIdx.x * blockDim.x + threadIdx.x) >> lanesLog2) + chain_wait();
     const int lanes = 1 << lanesLog2, lane = threadIdx.x & (lanes - 1);
     if (gs >= B.totalTessSpans)
         return;

@@ -411,14 +411,68 @@ constexpr uint32_t kSmallScanSlots = 1u << 18;
 cudaError_t small_passes_init(int device, uint32_t* largest);
 uint32_t small_sort_capacity(uint32_t largest);
 cudaError_t launch_small_scan(uint32_t largest, uint32_t slots, const uint32_t* counts,
-                              uint32_t* offsets, uint32_t* hostTotal, cudaStream_t stream);
+                              uint32_t* offsets, uint32_t* hostTotal, cudaStream_t stream,
+                              bool overlap);
 cudaError_t launch_small_sort(uint32_t largest, uint32_t entries, const uint32_t* entryTotal,
                               bool guarded, int keyBits, const uint16_t* keys, const uint32_t* vals,
-                              uint32_t* sortedVals, TileHead* ranges, cudaStream_t stream);
+                              uint32_t* sortedVals, TileHead* ranges, cudaStream_t stream,
+                              bool overlap);
 
 // Batches the raster grid orders its tiles for (tile_order_kernel).
 constexpr uint32_t kOrderMinTiles = 512;
 constexpr uint32_t kOrderTiles = 16384;
+
+// The start of every kernel of a flush's chain, before it reads anything another
+// one wrote: waits until the kernel before this one is complete (griddepcontrol;
+// nothing in a launch without the attribute of chain_launch). Returns 0, opaque:
+// added to the index that every load depends on, it keeps loads behind the wait
+// also where the compiler takes their memory for constant.
+__device__ __forceinline__ uint32_t chain_wait()
+{
+    uint32_t zero;
+    asm volatile("griddepcontrol.wait;\n\t"
+                 "mov.u32 %0, 0;"
+                 : "=r"(zero)::"memory");
+    return zero;
+}
+// Lets the next kernel of the chain start its CTAs once all of this one have
+// started. Not in the kernels before a raster, whose CTAs would take every SM
+// from other streams only to wait.
+__device__ __forceinline__ void chain_next()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Launches a kernel of a flush's chain. With `overlap` (the stream's last
+// operation is a kernel that starts with chain_wait) its CTAs take their places
+// while that one runs out; a small flush is eight kernels of a few microseconds,
+// and a launch after a complete kernel adds one or two to each (240x180 widget 54
+// -> 44 us, 1080x1080 recorded feathered frame 86 -> 69 us; a 1021x767
+// full-feature frame, 8.5 M slots, loses 0.3%, so the host does it for frames of
+// up to kSmallScanSlots). At *priority unless that is null.
+template <typename... P, typename... A>
+cudaError_t chain_launch(void (*kernel)(P...), uint32_t ctas, int threads, size_t smem,
+                         cudaStream_t stream, bool overlap, const int* priority, const A&... args)
+{
+    cudaLaunchAttribute attrs[2] = {};
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(ctas);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = stream;
+    c.attrs = attrs;
+    if (overlap)
+    {
+        attrs[c.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attrs[c.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (priority)
+    {
+        attrs[c.numAttrs].id = cudaLaunchAttributePriority;
+        attrs[c.numAttrs++].val.priority = *priority;
+    }
+    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
 
 // Index j with base[j] <= i < base[j + 1] (empty ranges skipped), n >= 1.
 __device__ __forceinline__ uint32_t find_range(const uint32_t* __restrict__ base, uint32_t n,
