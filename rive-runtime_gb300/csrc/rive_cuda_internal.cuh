@@ -116,6 +116,9 @@ constexpr uint32_t FEATURE_ATLAS_NEGATE = 1u << 11;
 // coordinates of the pixel (planes in the feather-plane slots), blended at
 // once, triangle by triangle.
 constexpr uint32_t FEATURE_IMAGE_MESH = 1u << 10;
+// Set by the raster as it stages a triangle: its path resolves without a clip,
+// clip rect, advanced blend mode or image, from a solid colour or a gradient.
+constexpr uint32_t FEATURE_SIMPLE = 1u << 9;
 // Two more bits of a triangle record's feature half-word, set only when the
 // batch draws interior tiles as winding records: a fan triangle whose tiles
 // are counted after its path's winding grid is complete, and the record of a
