@@ -1422,7 +1422,7 @@ int enqueue_back(rive_cuda_context* ctx,
             cub::DoubleBuffer<uint16_t> k((uint16_t*)S.keys, (uint16_t*)S.keysAlt);
             CK(cub::DeviceRadixSort::SortPairs(S.sortTemp, tempBytes, k, v, (int)entries, 0,
                                                L.endBit(), stream));
-            tile_ranges16_kernel<<<(entries + 255) / 256, 256, 0, stream>>>(entries, L.tiles,
+            tile_ranges16_kernel<<<(entries + 2047) / 2048, 256, 0, stream>>>(entries, L.tiles,
                                                                           k.Current(), S.ranges);
         }
         else
@@ -1430,7 +1430,7 @@ int enqueue_back(rive_cuda_context* ctx,
             cub::DoubleBuffer<uint32_t> k((uint32_t*)S.keys, (uint32_t*)S.keysAlt);
             CK(cub::DeviceRadixSort::SortPairs(S.sortTemp, tempBytes, k, v, (int)entries, 0,
                                                L.endBit(), stream));
-            tile_ranges_kernel<<<(entries + 255) / 256, 256, 0, stream>>>(entries, L.tiles,
+            tile_ranges_kernel<<<(entries + 1023) / 1024, 256, 0, stream>>>(entries, L.tiles,
                                                                         k.Current(), S.ranges);
         }
         // A speculative pass whose total did not fit: every range emptied,

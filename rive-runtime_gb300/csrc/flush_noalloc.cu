@@ -448,7 +448,7 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
                             kSortTempBytes);
             CKN(cub::DeviceRadixSort::SortPairs(pool + kSortTempOff, tempBytes, k, v, (int)pairs, 0,
                                                 endBit, stream));
-            tile_ranges16_kernel<<<(pairs + 255) / 256, 256, 0, stream>>>(pairs, tiles, k.Current(),
+            tile_ranges16_kernel<<<(pairs + 2047) / 2048, 256, 0, stream>>>(pairs, tiles, k.Current(),
                                                                         ranges);
         }
         sortedSlots = v.Current();

@@ -180,6 +180,36 @@ def test_bins_at_the_edges_of_the_one_cluster_passes(n, W, H):
     assert got[y, x] == ids[-1]
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,H", [(640, 470), (4112, 4112)])  # 16 and 32-bit keys
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 8, 9, 255, 1025, 140000])
+def test_tile_ranges_at_the_edges_of_a_load(n, W, H):
+    """n one-entry triangles in a batch whose keys take the vectorised range
+    pass (a filler scene brings the entries past the one-cluster sort, or the
+    canvas the tiles past 16-bit keys)."""
+    import torch
+    from rive_runtime_gb300 import rive_cuda
+    rng = np.random.default_rng(n)
+    at = np.stack([rng.integers(0, W // 16, n), rng.integers(0, H // 16, n)], 1) * 16.0
+    at[-1] = [W // 16 * 16 - 16, H // 16 * 16 - 16]  # the last full tile
+    tris = at[:, None] + np.array([[1, 1], [6.5, 1], [1, 6.5]])
+    ids = 1 + np.arange(n) * min(n, 60000) // n
+    f, (bufs, keep) = flush_of(tris, ids, W, H)
+    m = 1 if W > 1000 else 140000
+    filler, (fbufs, fkeep) = flush_of(np.tile(tris[:1], (m, 1, 1)), np.full(m, 1), W, H)
+    targets = [torch.zeros((H, W, 4), dtype=torch.uint8, device="cuda") for _ in range(2)]
+    ctx = rive_cuda.Context(0)
+    ctx.flush_batch([(filler, fbufs, targets[0].data_ptr()), (f, bufs, targets[1].data_ptr())])
+    ctx.sync()
+    img = targets[1].cpu().numpy().astype(np.int64)
+    ctx.close()
+    got = img[..., 0] | (img[..., 1] << 8) | (img[..., 2] << 16)
+    # Every tile's shape has the colour of the last triangle there.
+    want = {tuple(p): i for p, i in zip(at.astype(int), ids)}
+    assert all(got[y + 2, x + 2] == i for (x, y), i in want.items())
+    assert (got > 0).sum() == len(want) * (got[H // 16 * 16 - 16:, W // 16 * 16 - 16:] > 0).sum()
+
+
 def test_unorm_float_is_the_correctly_rounded_quotient():
     """kUnormHi / kUnormLo of kernels_raster.cu: b / 255 for every byte by one
     rounded product and one fused step (float64 holds both exactly)."""
