@@ -36,6 +36,10 @@ __global__ void patch_setup_kernel(BatchTables B,
                                    TriRecord* tris,
                                    uint32_t* tileCounts,
                                    uint8_t* tileMasks);
+__global__ void patch_setup_small_kernel(BatchTables B,
+                                         TriRecord* tris,
+                                         uint32_t* tileCounts,
+                                         uint8_t* tileMasks);
 __global__ void outer_setup_kernel(BatchTables B,
                                    TriRecord* tris,
                                    uint32_t* tileCounts,
@@ -1181,11 +1185,15 @@ int enqueue_front(rive_cuda_context* ctx,
     {
         stage_begin(ctx, RIVE_CUDA_STAGE_PATCH_SETUP, stream);
         if (L.items[0])
+        {
+            const bool three = !L.feather && !L.winding && L.items[0] > kFanWarpEach;
             CK(chain_launch(L.feather   ? patch_setup_feather_kernel
                             : L.winding ? patch_setup_winding_kernel
-                                        : patch_setup_kernel,
-                            (L.items[0] + 3) / 4, 128, 0, stream, overlap, nullptr, B, S.tris,
-                            S.counts, S.masks));
+                            : three     ? patch_setup_kernel
+                                        : patch_setup_small_kernel,
+                            three ? (L.items[0] + 11) / 12 : (L.items[0] + 3) / 4, 128, 0, stream,
+                            overlap, nullptr, B, S.tris, S.counts, S.masks));
+        }
         if (L.items[1])
             CK(chain_launch(outer_setup_kernel, (L.items[1] + 3) / 4, 128, 0, stream, overlap,
                             nullptr, B, S.tris, S.counts, S.masks));

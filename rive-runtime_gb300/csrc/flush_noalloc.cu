@@ -23,10 +23,10 @@ namespace rivecuda
 __global__ void color_ramp_kernel(BatchTables B);
 __global__ void tessellate_kernel(BatchTables B, int lanesLog2);
 __global__ void tessellate_feather_kernel(BatchTables B, int lanesLog2);
-__global__ void patch_setup_kernel(BatchTables B,
-                                   TriRecord* tris,
-                                   uint32_t* tileCounts,
-                                   uint8_t* tileMasks);
+__global__ void patch_setup_small_kernel(BatchTables B,
+                                         TriRecord* tris,
+                                         uint32_t* tileCounts,
+                                         uint8_t* tileMasks);
 __global__ void patch_setup_feather_kernel(BatchTables B,
                                            TriRecord* tris,
                                            uint32_t* tileCounts,
@@ -394,7 +394,7 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
     uint32_t pairs = 0;
     if (slots)
     {
-        CKN(chain_launch(feather ? patch_setup_feather_kernel : patch_setup_kernel,
+        CKN(chain_launch(feather ? patch_setup_feather_kernel : patch_setup_small_kernel,
                          (instAcc + 3) / 4, 128, 0, stream, true, nullptr, B, tris, counts, masks));
         if (wideList)
             CKN(chain_launch(wide_count_kernel, kWideBlocks, 256, 0, stream, true, nullptr, B, tris,

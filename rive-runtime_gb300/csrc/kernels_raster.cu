@@ -1456,107 +1456,109 @@ __device__ __forceinline__ void patch_setup(const BatchTables& B,
     }
 }
 
-// patch_setup of a midpoint fan without feathers. Its 42 vertices are 32 of the
-// AA ramps, 9 of the fan and the contour's midpoint; a warp shades the 32 in one
-// pass and makes the others from them:
-//  * fan vertex i starts from the same tessellation vertex, with the same
-//    offset, as ramp vertex 4 i (4 i + 1 when that vertex is mirrored; for
-//    i = 8, ramp vertex 30, or 28), so position and coverage are the same bits;
-//    only the discard rules differ (a stroke has no fan, a retrofitted triangle
-//    strip no ramps);
+// ---- Midpoint fans without feathers ---------------------------------------
+//
+// A patch's 42 vertices are two (outset -1 and +1: the ends of an AA ramp) at
+// each of 9 tessellation vertices, seen from one or two segments, the fan's, and
+// the contour's midpoint. As long as the patch's tessellation vertices belong to
+// one contour:
+//  * a ramp vertex depends on its tessellation vertex and outset alone, whichever
+//    segment it is seen from (mirrored vertices sit one vertex earlier);
+//  * fan vertex i is the vertex of outset -1 there, with other discard rules (a
+//    stroke has no fan, a retrofitted triangle strip no ramps);
 //  * the midpoint has no offset: a zero outset times a normal has the sign 0.
-// Shading the ten in a second pass cost as much as the 32. Vertices are snapped
-// once each, not once per triangle corner, and tile tests share their row's
-// terms: full-feature 1021x767 (356 k patches) 490 -> 372 us, 20 plain canvases
-// (653 k patches of large triangles) 1112 -> 896 us. Bound by issue slots.
-__device__ __forceinline__ void fan_setup(const BatchTables& B,
-                                          TriRecord* __restrict__ tris,
-                                          uint32_t* __restrict__ tileCounts,
-                                          uint8_t* __restrict__ tileMasks)
+// So a warp shades three patches at once, a lane per tessellation vertex
+// ("spoke") for both of its outsets, and 19 vertices a patch hold all 42. The
+// positions and coverages are the same bits as vertex by vertex; a patch that is
+// not of one contour takes that way (fan_setup_one).
+// Then the triangles of the three patches that draw (about half) are packed, so
+// that records and tile tests run on full warps. Bound by issue slots. The set-up
+// took 0.96 ms for the vertices of the full-feature 2048x2048 frame's 1.9 M patches
+// with a warp's 32 lanes on one patch's 32 ramp vertices; with three patches
+// 2016 -> 1660 us in all, 1404 with the triangles packed; 20 plain canvases
+// (653 k patches of large triangles) 897 -> 673, strokes 220 -> 164.
+constexpr int kSpokes = kPatchSegmentSpan + 1;              // 9
+constexpr int kFanVertices = 2 * kSpokes + 1;               // 19: (spoke, outset), midpoint
+constexpr int kFanPatches = 3;                              // patches a warp shades at once
+static_assert(kFanPatches * kFanVertices >= kPatchVertexCount, "fan_setup_one shares the buffers");
+
+// A warp's shaded vertices: snapped positions (1/256 px, and px), coverage, and
+// the largest coordinate and path of each (bit 31: no ramp vertex; bit 30: no
+// fan vertex).
+struct FanShared
 {
-    // Snapped positions (1/256 px, and px), coverage, and the largest
-    // coordinate and path of every vertex (bit 31: discarded).
-    __shared__ int2 sV[4][kPatchVertexCount];
-    __shared__ float2 sP[4][kPatchVertexCount], sCov[4][kPatchVertexCount];
-    __shared__ uint2 sMeta[4][kPatchVertexCount];
-    constexpr uint32_t kDiscard = 1u << 31;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    chain_next();
-    const uint32_t gi = blockIdx.x * 4 + w + chain_wait();
-    if (gi >= B.totalItems[0])
-        return; // whole warp exits together
-    const uint32_t seg = find_range(B.segBase[0], B.segCount[0], gi);
-    const PatchSegment S = B.segments[0][seg];
-    const FlushParams& P = B.scenes[S.scene];
-    const uint32_t local = gi - B.segBase[0][seg];
-    VertexOut o;
-    VertexSource src;
-    float2 zw;
-    const bool shaded = shade_patch_vertex<false>(P, patch_vertex_desc(lane), kPatchSegmentSpan,
-                                                  S.baseElement + local, o, zw, &src);
-    const bool ok = __all_sync(0xffffffffu, shaded);
-    uint32_t strokes = 0, mirrored = 0;
-    if (ok)
-    {
-        const int2 V = snap(o.pos);
-        sV[w][lane] = V;
-        sP[w][lane] = snapped_pixels(V);
-        sCov[w][lane] = o.cov;
-        sMeta[w][lane] = make_uint2(__float_as_uint(fmaxf(fabsf(o.pos.x), fabsf(o.pos.y))),
-                                    o.pathID | (o.discard ? kDiscard : 0u));
-        strokes = __ballot_sync(0xffffffffu, src.stroke);
-        mirrored = __ballot_sync(0xffffffffu, (src.flags & MIRRORED_CONTOUR_CONTOUR_FLAG) != 0);
-        __syncwarp();
-        if (lane < 9)
-        {
-            const int first = lane < 8 ? 4 * lane : 28; // starts from the same tessellation vertex
-            const int v = ((mirrored >> first) & 1u) ? (lane < 8 ? first + 1 : 28)
-                                                     : (lane < 8 ? first : 30);
-            sV[w][32 + lane] = sV[w][v];
-            sP[w][32 + lane] = sP[w][v];
-            sCov[w][32 + lane] = sCov[w][v];
-            const uint2 m = sMeta[w][v];
-            sMeta[w][32 + lane] =
-                make_uint2(m.x, (m.y & ~kDiscard) | (((strokes >> v) & 1u) ? kDiscard : 0u));
-        }
-        if (lane == 0)
-        {
-            const float2 mo = mat_mul(src.M, src.midpoint);
-            const float2 pos = make_float2(__fadd_rn(mo.x, src.translate.x),
-                                           __fadd_rn(mo.y, src.translate.y));
-            const bool negate = ((src.flags & MIRRORED_CONTOUR_CONTOUR_FLAG) != 0) !=
-                                ((src.flags & NEGATE_PATH_FILL_COVERAGE_FLAG) != 0);
-            const int2 M = snap(pos);
-            sV[w][41] = M;
-            sP[w][41] = snapped_pixels(M);
-            sCov[w][41] = make_float2(negate && !P.wireframe ? -1.f : 1.f, -1.f);
-            sMeta[w][41] = make_uint2(
-                __float_as_uint(fmaxf(fabsf(pos.x), fabsf(pos.y))),
-                o.pathID |
-                    (src.stroke || (src.flags & RETROFIT_TRI_STRIP_CONTOUR_FLAG) ? kDiscard : 0u));
-            // The path's image slot, for the raster's image paint (every patch
-            // of the path writes the same value).
-            if (S.image != kNoImage && P.pathImage && o.pathID < P.pathCount)
-                P.pathImage[o.pathID] = S.image;
-        }
-        __syncwarp();
-    }
-    const uint32_t slot = S.slotBase + local * kPatchTriangleCount + lane;
-    const bool has = lane < kPatchTriangleCount;
+    int2 v[kFanPatches * kFanVertices];
+    float2 p[kFanPatches * kFanVertices], cov[kFanPatches * kFanVertices];
+    uint2 meta[kFanPatches * kFanVertices];
+    uint32_t list[kFanPatches * kPatchTriangleCount]; // triangles that draw (fan_item)
+};
+constexpr uint32_t kNoRamp = 1u << 31, kNoFan = 1u << 30;
+
+__device__ __forceinline__ void put_vertex(FanShared& sh, int i, float2 pos, float2 cov, uint32_t meta)
+{
+    const int2 V = snap(pos);
+    sh.v[i] = V;
+    sh.p[i] = snapped_pixels(V);
+    sh.cov[i] = cov;
+    sh.meta[i] = make_uint2(__float_as_uint(fmaxf(fabsf(pos.x), fabsf(pos.y))), meta);
+}
+
+// The patch's midpoint vertex, from any of its vertices' source.
+__device__ __forceinline__ void put_midpoint(const FlushParams& P, FanShared& sh, int i,
+                                             const VertexSource& src, uint32_t pathID)
+{
+    const float2 mo = mat_mul(src.M, src.midpoint);
+    const bool negate = ((src.flags & MIRRORED_CONTOUR_CONTOUR_FLAG) != 0) !=
+                        ((src.flags & NEGATE_PATH_FILL_COVERAGE_FLAG) != 0);
+    put_vertex(sh, i,
+               make_float2(__fadd_rn(mo.x, src.translate.x), __fadd_rn(mo.y, src.translate.y)),
+               make_float2(negate && !P.wireframe ? -1.f : 1.f, -1.f),
+               pathID |
+                   (src.stroke || (src.flags & RETROFIT_TRI_STRIP_CONTOUR_FLAG) ? kNoFan : 0u));
+}
+
+// Whether triangle (a, b, c) of the shared buffers is one: none of its vertices
+// has the discard bit `hidden`, and all are in the snapping range.
+__device__ __forceinline__ bool fan_has(const FlushParams& P, const FanShared& sh, int a, int b,
+                                        int c, uint32_t hidden)
+{
+    const uint2 mA = sh.meta[a], mB = sh.meta[b], mC = sh.meta[c];
+    return !((mA.y | mB.y | mC.y) & hidden) &&
+           snapping_range(P, fmaxf(fmaxf(__uint_as_float(mA.x), __uint_as_float(mB.x)),
+                                   __uint_as_float(mC.x)));
+}
+
+// Whether it is clockwise and its box holds a pixel (setup_snapped's own tests,
+// the canvas alone for a clip).
+__device__ __forceinline__ bool fan_draws(const FlushParams& P, const FanShared& sh, int a, int b,
+                                          int c)
+{
+    const int2 V0 = sh.v[a], V1 = sh.v[b], V2 = sh.v[c];
+    const int x0 = max(-((-(min(min(V0.x, V1.x), V2.x) - 128)) >> 8), 0);
+    const int x1 = min(((max(max(V0.x, V1.x), V2.x) - 128) >> 8) + 1, (int)P.width);
+    const int y0 = max(-((-(min(min(V0.y, V1.y), V2.y) - 128)) >> 8), 0);
+    const int y1 = min(((max(max(V0.y, V1.y), V2.y) - 128) >> 8) + 1, (int)P.height);
+    return x0 < x1 && y0 < y1 &&
+           (long long)(V1.x - V0.x) * (V2.y - V0.y) > (long long)(V2.x - V0.x) * (V1.y - V0.y);
+}
+
+// Sets up the lane's triangle (a, b, c) of the shared buffers (`draws`: it has
+// one), and counts the tiles of the warp's triangles.
+__device__ __forceinline__ void fan_triangle(const BatchTables& B, const PatchSegment* Sp,
+                                             const FanShared& sh, bool has, bool draws, int a, int b,
+                                             int c, uint32_t slot, TriRecord* __restrict__ tris,
+                                             uint32_t* __restrict__ tileCounts,
+                                             uint8_t* __restrict__ tileMasks)
+{
     int4 bb = make_int4(0, 0, 0, 0);
     float4 e[3];
-    if (has && ok)
+    if (draws)
     {
-        int ia, ib, ic;
-        patch_triangle(lane, ia, ib, ic);
-        const uint2 mA = sMeta[w][ia], mB = sMeta[w][ib], mC = sMeta[w][ic];
+        const PatchSegment S = *Sp;
         TriRecord T;
-        if (!((mA.y | mB.y | mC.y) & kDiscard) &&
-            snapping_range(P, fmaxf(fmaxf(__uint_as_float(mA.x), __uint_as_float(mB.x)),
-                                    __uint_as_float(mC.x))) &&
-            setup_snapped(P, sV[w][ia], sV[w][ib], sV[w][ic], sP[w][ia], sP[w][ib], sP[w][ic],
-                          sCov[w][ia], sCov[w][ib], sCov[w][ic], mA.y, S.features, S.scene, T, bb,
-                          nullptr, float2{}, float2{}, float2{},
+        if (setup_snapped(B.scenes[S.scene], sh.v[a], sh.v[b], sh.v[c], sh.p[a], sh.p[b], sh.p[c],
+                          sh.cov[a], sh.cov[b], sh.cov[c], sh.meta[a].y & 0xffffu, S.features,
+                          S.scene, T, bb, nullptr, float2{}, float2{}, float2{},
                           make_int4((int)(S.scissorLT & 0xffffu), (int)(S.scissorLT >> 16),
                                     (int)(S.scissorRB & 0xffffu), (int)(S.scissorRB >> 16)),
                           false))
@@ -1571,21 +1573,442 @@ __device__ __forceinline__ void fan_setup(const BatchTables& B,
     count_tiles(has, B, e, bb, slot, tileCounts, tileMasks);
 }
 
+// One patch, its ramp vertices shaded one by one (32 lanes) and its fan vertices
+// copied from them: fan vertex i starts from the same tessellation vertex, with
+// the same outset, as ramp vertex 4 i (4 i + 1 when that vertex is mirrored; for
+// i = 8, ramp vertex 30, or 28).
+__device__ __forceinline__ void fan_setup_one(const BatchTables& B, uint32_t gi, FanShared& sh,
+                                           TriRecord* __restrict__ tris,
+                                           uint32_t* __restrict__ tileCounts,
+                                           uint8_t* __restrict__ tileMasks)
+{
+    const int lane = threadIdx.x & 31;
+    const uint32_t seg = find_range(B.segBase[0], B.segCount[0], gi);
+    const PatchSegment S = B.segments[0][seg];
+    const FlushParams& P = B.scenes[S.scene];
+    const uint32_t local = gi - B.segBase[0][seg];
+    VertexOut o;
+    VertexSource src;
+    float2 zw;
+    const bool shaded = shade_patch_vertex<false>(P, patch_vertex_desc(lane), kPatchSegmentSpan,
+                                                  S.baseElement + local, o, zw, &src);
+    const bool ok = __all_sync(0xffffffffu, shaded);
+    if (ok)
+    {
+        // (Here bit 31 alone is the discard bit, fan vertices being copies.)
+        put_vertex(sh, lane, o.pos, o.cov, o.pathID | (o.discard ? kNoRamp : 0u));
+        const uint32_t strokes = __ballot_sync(0xffffffffu, src.stroke);
+        const uint32_t mirrored =
+            __ballot_sync(0xffffffffu, (src.flags & MIRRORED_CONTOUR_CONTOUR_FLAG) != 0);
+        __syncwarp();
+        if (lane < 9)
+        {
+            const int first = lane < 8 ? 4 * lane : 28; // starts from the same tessellation vertex
+            const int v = ((mirrored >> first) & 1u) ? (lane < 8 ? first + 1 : 28)
+                                                     : (lane < 8 ? first : 30);
+            sh.v[32 + lane] = sh.v[v];
+            sh.p[32 + lane] = sh.p[v];
+            sh.cov[32 + lane] = sh.cov[v];
+            const uint2 m = sh.meta[v];
+            sh.meta[32 + lane] =
+                make_uint2(m.x, (m.y & ~kNoRamp) | (((strokes >> v) & 1u) ? kNoRamp : 0u));
+        }
+        if (lane == 0)
+        {
+            put_midpoint(P, sh, 41, src, o.pathID);
+            if (sh.meta[41].y & kNoFan)
+                sh.meta[41].y |= kNoRamp;
+            if (S.image != kNoImage && P.pathImage && o.pathID < P.pathCount)
+                P.pathImage[o.pathID] = S.image;
+        }
+        __syncwarp();
+    }
+    int a = 0, b = 0, c = 0;
+    const bool has = lane < kPatchTriangleCount;
+    if (has)
+        patch_triangle(lane, a, b, c);
+    fan_triangle(B, B.segments[0] + seg, sh, has,
+                 has && ok && fan_has(P, sh, a, b, c, kNoRamp), a, b, c,
+                 S.slotBase + local * kPatchTriangleCount + lane, tris, tileCounts, tileMasks);
+}
+
+__device__ __noinline__ void fan_setup_mixed(const BatchTables& B, uint32_t gi, FanShared& sh,
+                                             TriRecord* __restrict__ tris,
+                                             uint32_t* __restrict__ tileCounts,
+                                             uint8_t* __restrict__ tileMasks)
+{
+    fan_setup_one(B, gi, sh, tris, tileCounts, tileMasks);
+}
+
+// shade_patch_vertex (without feathers) of a spoke's two outsets, in the same
+// steps: pos/cov[0] of outset -1, [1] of +1. `tv` is the spoke's tessellation
+// vertex at index `idx`, `flags` its flags. Returns false on a malformed input.
+__device__ __forceinline__ bool shade_spoke(const FlushParams& P, const uint4& tv, long long idx,
+                                            uint32_t flags, float4 M, float2 translate,
+                                            float strokeRadius, float2 pos[2], float2 cov[2])
+{
+    const float theta = __uint_as_float(tv.z);
+    float sn, cs;
+    rc_sincosf(theta, &sn, &cs);
+    const float2 norm = make_float2(sn, -cs);
+    float2 offset[2];
+    if (strokeRadius != 0.f)
+    {
+        const float detM = __fsub_rn(__fmul_rn(M.x, M.w), __fmul_rn(M.z, M.y));
+        const float side = signf(detM);
+        const float aaRadius = __fmul_rn(manhattan_pixel_width(M, norm), kAARadius);
+        float globalCoverage = 1.f;
+        if (aaRadius > strokeRadius)
+        {
+            globalCoverage = __fdiv_rn(strokeRadius, aaRadius);
+            strokeRadius = aaRadius;
+        }
+        const float sr = __fadd_rn(strokeRadius, aaRadius);
+        float2 vertexOffset = make_float2(__fmul_rn(norm.x, sr), __fmul_rn(norm.y, sr));
+        const float k = __fdiv_rn(1.f, __fmul_rn(aaRadius, 2.f));
+        const uint32_t joinType = flags & JOIN_TYPE_MASK;
+        const bool join = joinType > ROUND_JOIN_CONTOUR_FLAG;
+        float2 bisector = make_float2(0.f, 0.f);
+        float clipAARadius = 0.f, bisectPixelWidth = 0.f;
+        if (join)
+        {
+            int peekDir = 2;
+            if (!(flags & JOIN_TANGENT_0_CONTOUR_FLAG))
+                peekDir = -peekDir;
+            if (flags & MIRRORED_CONTOUR_CONTOUR_FLAG)
+                peekDir = -peekDir;
+            uint4 ov;
+            if (!tess_fetch(P, idx + peekDir, ov))
+                return false;
+            float joinAngle = fabsf(__fsub_rn(__uint_as_float(ov.z), theta));
+            if (joinAngle > kPi)
+                joinAngle = __fsub_rn(k2Pi, joinAngle);
+            const bool isTan0 = (flags & JOIN_TANGENT_0_CONTOUR_FLAG) != 0;
+            const bool isLeft = (flags & LEFT_JOIN_CONTOUR_FLAG) != 0;
+            const float bisectTheta =
+                __fadd_rn(__fmul_rn(joinAngle, isTan0 == isLeft ? -.5f : .5f), theta);
+            float bs, bc;
+            rc_sincosf(bisectTheta, &bs, &bc);
+            bisector = make_float2(bs, -bc);
+            bisectPixelWidth = manhattan_pixel_width(M, bisector);
+            const float miterRatio = rc_cosf(__fmul_rn(joinAngle, .5f));
+            float clipRadius;
+            if (joinType == MITER_CLIP_JOIN_CONTOUR_FLAG ||
+                (joinType == MITER_REVERT_JOIN_CONTOUR_FLAG && miterRatio >= .25f))
+            {
+                const float inverseLimit = (flags & EMULATED_STROKE_CAP_CONTOUR_FLAG) ? 1.f : .25f;
+                clipRadius = __fmul_rn(strokeRadius,
+                                       __fdiv_rn(1.f, fmaxf(miterRatio, inverseLimit)));
+            }
+            else
+            {
+                clipRadius = __fadd_rn(__fmul_rn(strokeRadius, miterRatio),
+                                       __fmul_rn(bisectPixelWidth, .5f));
+            }
+            clipAARadius = __fadd_rn(clipRadius, __fmul_rn(bisectPixelWidth, kAARadius));
+            if (flags & JOIN_TANGENT_INNER_CONTOUR_FLAG)
+            {
+                const float strokeAARadius = __fadd_rn(strokeRadius, aaRadius);
+                const float slop = __fmul_rn(aaRadius, .125f);
+                if (strokeAARadius <= __fadd_rn(__fmul_rn(clipAARadius, miterRatio), slop))
+                {
+                    const float miterAARadius =
+                        __fmul_rn(strokeAARadius, __fdiv_rn(1.f, miterRatio));
+                    vertexOffset = make_float2(__fmul_rn(bisector.x, miterAARadius),
+                                               __fmul_rn(bisector.y, miterAARadius));
+                }
+                else
+                {
+                    const float2 bo = make_float2(__fmul_rn(bisector.x, clipAARadius),
+                                                  __fmul_rn(bisector.y, clipAARadius));
+                    const float kx = __fadd_rn(__fmul_rn(vertexOffset.x, vertexOffset.x),
+                                               __fmul_rn(vertexOffset.y, vertexOffset.y));
+                    const float ky = __fadd_rn(__fmul_rn(bo.x, bo.x), __fmul_rn(bo.y, bo.y));
+                    const float det = __fsub_rn(__fmul_rn(vertexOffset.x, bo.y),
+                                                __fmul_rn(bo.x, vertexOffset.y));
+                    const float invDet = __fdiv_rn(1.f, det);
+                    const float i00 = __fmul_rn(bo.y, invDet), i01 = __fmul_rn(-vertexOffset.y, invDet);
+                    const float i10 = __fmul_rn(-bo.x, invDet), i11 = __fmul_rn(vertexOffset.x, invDet);
+                    vertexOffset =
+                        make_float2(__fadd_rn(__fmul_rn(kx, i00), __fmul_rn(ky, i01)),
+                                    __fadd_rn(__fmul_rn(kx, i10), __fmul_rn(ky, i11)));
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+        {
+            float outset = __fmul_rn(i ? 1.f : -1.f, side);
+            if (flags & LEFT_JOIN_CONTOUR_FLAG)
+                outset = fminf(outset, 0.f);
+            if (flags & RIGHT_JOIN_CONTOUR_FLAG)
+                outset = fmaxf(outset, 0.f);
+            const float x = __fmul_rn(outset, sr);
+            float2 c = make_float2(__fadd_rn(__fmul_rn(k, __fadd_rn(x, strokeRadius)), .5f),
+                                   __fadd_rn(__fmul_rn(k, __fadd_rn(-x, strokeRadius)), .5f));
+            if (join)
+            {
+                const float ao = fabsf(outset);
+                const float2 pt =
+                    make_float2(__fmul_rn(vertexOffset.x, ao), __fmul_rn(vertexOffset.y, ao));
+                const float clipDistance =
+                    __fdiv_rn(__fsub_rn(clipAARadius, __fadd_rn(__fmul_rn(pt.x, bisector.x),
+                                                                __fmul_rn(pt.y, bisector.y))),
+                              __fmul_rn(bisectPixelWidth, kAARadius * 2.f));
+                if (flags & LEFT_JOIN_CONTOUR_FLAG)
+                    c.y = clipDistance;
+                else
+                    c.x = clipDistance;
+            }
+            c.x = __fmul_rn(c.x, globalCoverage);
+            c.y = fmaxf(__fmul_rn(c.y, globalCoverage), 1e-4f);
+            cov[i] = c;
+            offset[i] = mat_mul(M, make_float2(__fmul_rn(vertexOffset.x, outset),
+                                               __fmul_rn(vertexOffset.y, outset)));
+        }
+    }
+    else
+    {
+        // The sign of the outset normal times the inverse matrix; the other
+        // outset's is its negative.
+        const float2 on = make_float2(__fmul_rn(norm.x, -1.f), __fmul_rn(norm.y, -1.f));
+        const float det = __fsub_rn(__fmul_rn(M.x, M.w), __fmul_rn(M.z, M.y));
+        const float invDet = __fdiv_rn(1.f, det);
+        const float i00 = __fmul_rn(M.w, invDet), i01 = __fmul_rn(-M.y, invDet);
+        const float i10 = __fmul_rn(-M.z, invDet), i11 = __fmul_rn(M.x, invDet);
+        const float rx = __fadd_rn(__fmul_rn(on.x, i00), __fmul_rn(on.y, i01));
+        const float ry = __fadd_rn(__fmul_rn(on.x, i10), __fmul_rn(on.y, i11));
+        offset[0] = make_float2(signf(rx) * kAARadius, signf(ry) * kAARadius);
+        offset[1] = make_float2(-offset[0].x, -offset[0].y);
+        const bool negate = ((flags & MIRRORED_CONTOUR_CONTOUR_FLAG) != 0) !=
+                            ((flags & NEGATE_PATH_FILL_COVERAGE_FLAG) != 0);
+        cov[0] = make_float2(negate ? -1.f : 1.f, -1.f);
+        cov[1] = make_float2(negate ? -0.f : 0.f, -1.f);
+    }
+    if (P.wireframe)
+        cov[0] = cov[1] = make_float2(1.f, -1.f);
+    const float2 mo = mat_mul(M, make_float2(__uint_as_float(tv.x), __uint_as_float(tv.y)));
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+        pos[i] = make_float2(__fadd_rn(__fadd_rn(mo.x, offset[i].x), translate.x),
+                             __fadd_rn(__fadd_rn(mo.y, offset[i].y), translate.y));
+    return true;
+}
+
+__device__ __forceinline__ void fan_setup(const BatchTables& B,
+                                          TriRecord* __restrict__ tris,
+                                          uint32_t* __restrict__ tileCounts,
+                                          uint8_t* __restrict__ tileMasks)
+{
+    __shared__ FanShared shared[4];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    FanShared& sh = shared[w];
+    chain_next();
+    const uint32_t gi0 = (blockIdx.x * 4 + w) * kFanPatches + chain_wait();
+    if (gi0 >= B.totalItems[0])
+        return; // whole warp exits together
+    const int sub = min(lane / kSpokes, kFanPatches - 1), spoke = min(lane - sub * kSpokes, kSpokes - 1);
+    const uint32_t gi = min(gi0 + sub, B.totalItems[0] - 1);
+    const bool mine = lane < kFanPatches * kSpokes && gi0 + sub < B.totalItems[0];
+    const uint32_t group = ((1u << kSpokes) - 1u) << (sub * kSpokes); // the patch's lanes
+    const uint32_t seg = find_range(B.segBase[0], B.segCount[0], gi);
+    const PatchSegment* const Sp = B.segments[0] + seg;
+    const FlushParams& P = B.scenes[Sp->scene];
+    const uint32_t local = gi - B.segBase[0][seg];
+    const uint32_t instance = Sp->baseElement + local;
+    const uint32_t patchSlot = Sp->slotBase + local * kPatchTriangleCount;
+    // The spoke's tessellation vertex. `shaded`: no malformed input; `plain`: of
+    // the patch's one contour, and of one kind for both outsets.
+    bool shaded = true, plain = true;
+    uint32_t flags = 0, pathID = 0;
+    VertexSource src = {};
+    float2 pos[2], cov[2];
+    if (mine)
+    {
+        const long long first = (long long)instance * kPatchSegmentSpan;
+        long long idx = first + min(spoke, kPatchSegmentSpan - 1);
+        uint4 tv = make_uint4(0u, 0u, 0u, 0u);
+        shaded = tess_fetch(P, idx, tv);
+        flags = tv.w;
+        const uint32_t contourID = max(flags & CONTOUR_ID_MASK, 1u);
+        uint4 cd = make_uint4(0u, 0u, 0u, 0u);
+        if (shaded && contourID > P.contourCount)
+        {
+            atomicOr(P.error, ERR_BAD_CONTOUR);
+            shaded = false;
+        }
+        if (shaded)
+        {
+            cd = P.contours[P.firstContour + contourID - 1];
+            pathID = cd.z & 0xffffu;
+            if (pathID >= P.pathCount)
+            {
+                atomicOr(P.error, ERR_BAD_PATH);
+                shaded = false;
+            }
+        }
+        if (shaded)
+        {
+            const uint4* path = P.paths + 4 * (size_t)(P.firstPath + pathID);
+            const uint4 r0 = path[0], r1 = path[1];
+            const float strokeRadius = __uint_as_float(r1.z);
+            src.M = make_float4(__uint_as_float(r0.x), __uint_as_float(r0.y),
+                                __uint_as_float(r0.z), __uint_as_float(r0.w));
+            src.translate = make_float2(__uint_as_float(r1.x), __uint_as_float(r1.y));
+            src.midpoint = make_float2(__uint_as_float(cd.x), __uint_as_float(cd.y));
+            src.flags = flags;
+            src.stroke = strokeRadius != 0.f;
+            const uint32_t mirrored = flags & MIRRORED_CONTOUR_CONTOUR_FLAG;
+            const long long want = first + spoke - (mirrored ? 1 : 0);
+            uint32_t vflags = flags;
+            if (want != idx)
+            {
+                uint4 rv;
+                shaded = tess_fetch(P, want, rv);
+                if (shaded && (rv.w & (MIRRORED_CONTOUR_CONTOUR_FLAG | 0xffffu)) !=
+                                  (flags & (MIRRORED_CONTOUR_CONTOUR_FLAG | 0xffffu)))
+                {
+                    if (strokeRadius == 0.f || src.midpoint.x != 0.f) // closed
+                    {
+                        idx = cd.w;
+                        shaded = tess_fetch(P, idx, tv);
+                    }
+                    else
+                    {
+                        // An open contour keeps the vertex it started from:
+                        // another one for each outset when mirrored.
+                        plain = !mirrored;
+                    }
+                }
+                else if (shaded)
+                {
+                    idx = want;
+                    tv = rv;
+                }
+                vflags = (tv.w & ~MIRRORED_CONTOUR_CONTOUR_FLAG) | mirrored;
+            }
+            if (shaded && plain)
+            {
+                shaded = shade_spoke(P, tv, idx, vflags, src.M, src.translate, strokeRadius, pos, cov);
+                if (shaded)
+                {
+                    const int at = sub * kFanVertices + 2 * spoke;
+                    const uint32_t meta =
+                        pathID | (src.stroke ? kNoFan
+                                  : (vflags & RETROFIT_TRI_STRIP_CONTOUR_FLAG) ? kNoRamp : 0u);
+                    put_vertex(sh, at, pos[0], cov[0], meta);
+                    put_vertex(sh, at + 1, pos[1], cov[1], meta);
+                    if (spoke == 0)
+                        put_midpoint(P, sh, sub * kFanVertices + 2 * kSpokes, src, pathID);
+                }
+            }
+        }
+    }
+    // One contour: every spoke starts from the same contour and side as the
+    // patch's first.
+    constexpr uint32_t kSame = MIRRORED_CONTOUR_CONTOUR_FLAG | CONTOUR_ID_MASK;
+    const uint32_t same = __shfl_sync(0xffffffffu, flags & kSame, sub * kSpokes);
+    const uint32_t bad = __ballot_sync(0xffffffffu, mine && !shaded);
+    const uint32_t odd = __ballot_sync(0xffffffffu, mine && (!plain || (flags & kSame) != same));
+    if (mine && spoke == 0 && !((bad | odd) & group) && Sp->image != kNoImage && P.pathImage &&
+        pathID < P.pathCount)
+        P.pathImage[pathID] = Sp->image; // for the raster's image paint
+    const uint32_t mirroredPatches =
+        __ballot_sync(0xffffffffu, mine && (flags & MIRRORED_CONTOUR_CONTOUR_FLAG) != 0);
+    __syncwarp();
+    // The triangles that draw (about half of them), packed into a list so that
+    // the set-up proper runs on full warps; the others have no tiles.
+    uint32_t count = 0;
+    int a = 0, b = 0, c = 0;
+    const bool has = lane < kPatchTriangleCount;
+    if (lane >= 16 && has)
+    {
+        patch_triangle(lane, a, b, c);
+        a = a == 41 ? 2 * kSpokes : 2 * (a - 32);
+        b = b == 41 ? 2 * kSpokes : 2 * (b - 32);
+        c = c == 41 ? 2 * kSpokes : 2 * (c - 32);
+    }
+    for (int j = 0; j < kFanPatches && gi0 + j < B.totalItems[0]; ++j)
+    {
+        const uint32_t lanes = ((1u << kSpokes) - 1u) << (j * kSpokes);
+        if (odd & lanes)
+            continue;
+        const PatchSegment* const S = B.segments[0] + __shfl_sync(0xffffffffu, seg, j * kSpokes);
+        const uint32_t slot = __shfl_sync(0xffffffffu, patchSlot, j * kSpokes) + lane;
+        if (lane < 16)
+        {
+            // Segment s's ramp: its vertices 0..3 are (s, -), (s, +), (s + 1, -),
+            // (s + 1, +), or mirrored (s + 1, -), (s, -), (s + 1, +), (s, +).
+            const int s0 = lane & ~1, s1 = s0 + 2;
+            const bool m = (mirroredPatches >> (j * kSpokes)) & 1u;
+            const int v0 = m ? s1 : s0, v1 = m ? s0 : s0 + 1;
+            const int v2 = m ? s1 + 1 : s1, v3 = m ? s0 + 1 : s1 + 1;
+            a = (lane & 1) ? v2 : v0;
+            b = v1;
+            c = (lane & 1) ? v3 : v2;
+        }
+        const int base = j * kFanVertices;
+        const FlushParams& Pj = B.scenes[S->scene];
+        const bool draws = has && !(bad & lanes) &&
+                           fan_has(Pj, sh, base + a, base + b, base + c,
+                                   lane < 16 ? kNoRamp : kNoFan) &&
+                           fan_draws(Pj, sh, base + a, base + b, base + c);
+        const uint32_t drawing = __ballot_sync(0xffffffffu, draws);
+        if (draws)
+            sh.list[count + __popc(drawing & ((1u << lane) - 1u))] =
+                (uint32_t)(base + a) | ((uint32_t)(base + b) << 6) | ((uint32_t)(base + c) << 12) |
+                ((uint32_t)lane << 18) | ((uint32_t)j << 23);
+        else if (has)
+            tileCounts[slot] = 0;
+        count += __popc(drawing);
+    }
+    __syncwarp();
+    for (uint32_t i = lane; i - lane < count; i += 32)
+    {
+        const bool draws = i < count;
+        const uint32_t item = draws ? sh.list[i] : 0u;
+        const int from = (item >> 23) * kSpokes; // a lane of the patch
+        const uint32_t sj = __shfl_sync(0xffffffffu, seg, from);
+        const uint32_t slot = __shfl_sync(0xffffffffu, patchSlot, from) + ((item >> 18) & 31u);
+        fan_triangle(B, B.segments[0] + sj, sh, draws, draws, item & 63u, (item >> 6) & 63u,
+                     (item >> 12) & 63u, slot, tris, tileCounts, tileMasks);
+    }
+    for (int j = 0; odd && j < kFanPatches; ++j)
+        if (odd & (((1u << kSpokes) - 1u) << (j * kSpokes)))
+        {
+            __syncwarp();
+            fan_setup_mixed(B, gi0 + j, sh, tris, tileCounts, tileMasks);
+        }
+}
+
 // Resident 128-thread CTAs per SM the midpoint-fan set-up's registers are
-// bounded for (20 plain canvases 896, 915 and 944 us at 9, 10 and 11).
+// bounded for (20 plain canvases 691, 684, 708 and 750 us at 7, 8, 9 and 10).
 #ifndef RIVE_SETUP_MIN_BLOCKS
-#define RIVE_SETUP_MIN_BLOCKS 9
+#define RIVE_SETUP_MIN_BLOCKS 8
 #endif
-__global__ void __launch_bounds__(128, RIVE_SETUP_MIN_BLOCKS) patch_setup_kernel(BatchTables B,
-                                                          TriRecord* __restrict__ tris,
-                                                          uint32_t* __restrict__ tileCounts,
-                                                          uint8_t* __restrict__ tileMasks)
+__global__ void __launch_bounds__(128, RIVE_SETUP_MIN_BLOCKS) patch_setup_kernel(
+    BatchTables B, TriRecord* __restrict__ tris, uint32_t* __restrict__ tileCounts,
+    uint8_t* __restrict__ tileMasks)
 {
     fan_setup(B, tris, tileCounts, tileMasks);
 }
 
-// Midpoint-fan set-up for batches that draw interior tiles as winding records
-// (its own kernel, so the plain one keeps its register budget).
+// A warp per patch, for flushes of at most kFanWarpEach patches: bound by the
+// latency of one warp's chain, which three patches lengthen (1080x1920 UI
+// screen's set-up 17 us, 19 with three).
+__global__ void __launch_bounds__(128) patch_setup_small_kernel(BatchTables B,
+                                                                TriRecord* __restrict__ tris,
+                                                                uint32_t* __restrict__ tileCounts,
+                                                                uint8_t* __restrict__ tileMasks)
+{
+    __shared__ FanShared shared[4];
+    const int w = threadIdx.x >> 5;
+    chain_next();
+    const uint32_t gi = blockIdx.x * 4 + w + chain_wait();
+    if (gi < B.totalItems[0]) // whole warps
+        fan_setup_one(B, gi, shared[w], tris, tileCounts, tileMasks);
+}
+
 __global__ void __launch_bounds__(128) patch_setup_winding_kernel(BatchTables B,
                                                                   TriRecord* __restrict__ tris,
                                                                   uint32_t* __restrict__ tileCounts,

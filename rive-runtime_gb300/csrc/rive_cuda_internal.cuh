@@ -316,6 +316,10 @@ constexpr int kWideStrips = 64;
 constexpr int kWideStripTiles = 128;
 constexpr uint32_t kWideCapacity = 16384; // triangles kept; more are walked in place
 
+// Plain midpoint-fan set-up: up to kFanWarpEach patches (about a wave of warps)
+// a warp each, above that three a warp; 128-thread CTAs.
+constexpr uint32_t kFanWarpEach = 8192;
+
 // Set-up work lists: midpoint-fan patches, outer-curve patches, interior
 // triangles, center-AA midpoint-fan patches (items: instances, instances,
 // triangles, instances).

@@ -217,3 +217,39 @@ def test_unorm_float_is_the_correctly_rounded_quotient():
     b = np.arange(256, dtype=np.float64)
     got = (b * hi + f32(b * lo)).astype(np.float32)
     assert np.array_equal(got, np.arange(256, dtype=np.float32) / np.float32(255))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("name", ["plain_small_s1", "stroke_stress_s5", "strokes_s3"])
+def test_patches_three_a_warp_match_one_a_warp(name, mixed):
+    """A flush small enough for a warp per patch, and as many copies of it as
+    make a batch whose warps shade three patches at once: the same images.
+    "mixed": every third span takes another contour's number, so patches hold
+    vertices of several contours, of fills beside strokes."""
+    import torch
+    from rive_runtime_gb300 import rive_cuda
+    cap = load_golden(name)[0]
+    f = cap.flushes[0]
+    b = f.batches = np.array(f.batches)
+    b[:, 1] = np.minimum(b[:, 1], 8191)  # of plain_small_s1, the first half of its patches
+    if mixed:
+        spans = np.frombuffer(cap.buffers["tess_spans"], np.uint32).reshape(-1, 16).copy()
+        rng = np.random.default_rng(5)
+        other = rng.integers(1, f.desc["contour_count"] + 1, len(spans[::3])).astype(np.uint32)
+        spans[::3, 15] = (spans[::3, 15] & 0xffff0000) | other
+        cap.buffers["tess_spans"] = spans.tobytes()
+    bufs, keep = device_buffers(cap)
+    copies = 8192 // int(b[:, 1].sum()) + 2
+    targets = [torch.zeros((cap.height, cap.width, 4), dtype=torch.uint8, device="cuda")
+               for _ in range(copies + 1)]
+    ctx = rive_cuda.Context(0)
+    ctx.flush_device(f, bufs, targets[0].data_ptr())
+    ctx.sync()
+    ctx.flush_batch([(f, bufs, t.data_ptr()) for t in targets[1:]])
+    ctx.sync()
+    ctx.close()
+    want = targets[0].cpu().numpy()
+    assert len(np.unique(want.reshape(-1, 4), axis=0)) > 20
+    for t in targets[1:]:
+        assert np.array_equal(t.cpu().numpy(), want)
