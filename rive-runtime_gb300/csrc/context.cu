@@ -78,6 +78,19 @@ __global__ void bin_scatter_kernel(uint32_t slotCount,
                                    uint32_t* keys,
                                    uint32_t* vals,
                                    WideScatter wide);
+__global__ void bin_scatter_extended_kernel(uint32_t slotCount,
+                                            int tileLog2,
+                                            const uint2* sceneTiles,
+                                            const TriRecord* tris,
+                                            const uint32_t* tileCounts,
+                                            const uint8_t* tileMasks,
+                                            const uint32_t* offsets,
+                                            uint32_t capacity,
+                                            uint32_t* error,
+                                            uint32_t* keys,
+                                            uint32_t* vals,
+                                            WideScatter wide,
+                                            ExtendedTiles extended);
 __global__ void tile_ranges_kernel(uint32_t pairCount,
                                    uint32_t tileCount,
                                    const uint32_t* keys,
@@ -99,6 +112,19 @@ __global__ void bin_scatter16_kernel(uint32_t slotCount,
                                      uint16_t* keys,
                                      uint32_t* vals,
                                      WideScatter wide);
+__global__ void bin_scatter16_extended_kernel(uint32_t slotCount,
+                                              int tileLog2,
+                                              const uint2* sceneTiles,
+                                              const TriRecord* tris,
+                                              const uint32_t* tileCounts,
+                                              const uint8_t* tileMasks,
+                                              const uint32_t* offsets,
+                                              uint32_t capacity,
+                                              uint32_t* error,
+                                              uint16_t* keys,
+                                              uint32_t* vals,
+                                              WideScatter wide,
+                                              ExtendedTiles extended);
 __global__ void tile_ranges16_kernel(uint32_t pairCount,
                                      uint32_t tileCount,
                                      const uint16_t* keys,
@@ -153,6 +179,13 @@ __global__ void raster_tile_kernel(BatchTables B, const TriRecord* tris, const u
 __global__ void raster_tile_feather_kernel(BatchTables B, const TriRecord* tris,
                                            const uint32_t* sortedSlots, const TileHead* ranges,
                                            const uint32_t* order);
+// The two launches of a split raster (ExtendedTiles).
+__global__ void raster_extended_kernel(BatchTables B, const TriRecord* tris,
+                                       const uint32_t* sortedSlots, const TileHead* ranges,
+                                       const uint32_t* order);
+__global__ void raster_others_kernel(BatchTables B, const TriRecord* tris,
+                                     const uint32_t* sortedSlots, const TileHead* ranges,
+                                     const uint32_t* order);
 __global__ void tile_order_kernel(uint32_t tiles, const TileHead* ranges, uint32_t* order);
 RIVE_DECLARE_RASTER(raster_tile8_kernel)
 RIVE_DECLARE_RASTER(raster_tile8_feather_kernel)
@@ -688,6 +721,8 @@ struct BatchLayout
     uint32_t fanStride = kPatchTriangleCount;
     // Some scene has enough tiles for a wide triangle (BatchTables::wide).
     bool wide = false;
+    // Whether the raster splits its tiles between its two variants.
+    bool splitRaster() const { return feather && tileLog2 == 4 && mainTiles >= kSplitTiles; }
     uint32_t wideCap() const { return wide ? std::min(slots, kWideCapacity) : 0u; }
     size_t wideBytes() const { return wide ? 4 + (size_t)wideCap() * 4 * (1 + kWideStrips) : 0; }
     uint64_t tessRows = 0, gradRows = 0;
@@ -1278,6 +1313,15 @@ int prepare_raster(rive_cuda_context* ctx)
         for (int f = 0; f < 2; ++f)
             ctx->rasterPad[f][slot] =
                 occupancy_pad(fns[f][slot], slot == 0 ? 64 : 256, ctx->rasterCtasPerSm);
+        if (slot == 1) // the split's launches take the same padding
+        {
+            CK(cudaFuncSetAttribute(raster_extended_kernel,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)ctx->rasterPad[1][1]));
+            CK(cudaFuncSetAttribute(raster_others_kernel,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)ctx->rasterPad[0][1]));
+        }
         cudaGetLastError(); // a failed query only leaves the launch unpadded
         ctx->rasterPadFor[slot] = ctx->rasterCtasPerSm;
     }
@@ -1349,8 +1393,20 @@ int launch_raster(rive_cuda_context* ctx,
                             ranges, S.order));
             order = S.order;
         }
-        CK(chain_launch(L.feather ? raster_tile_feather_kernel : raster_tile_kernel, L.mainTiles,
-                         256, dyn, stream, overlap, priority, B, tris, sortedSlots, ranges, order));
+        if (L.splitRaster())
+        {
+            CK(chain_launch(raster_extended_kernel, L.mainTiles, 256, dyn, stream, overlap,
+                            priority, B, tris, sortedSlots, ranges, order));
+            const size_t dyn0 = ctx->rasterCtasPerSm > 0 ? ctx->rasterPad[0][1] : 0;
+            CK(chain_launch(raster_others_kernel, L.mainTiles, 256, dyn0, stream, true, priority, B,
+                            tris, sortedSlots, ranges, order));
+        }
+        else
+        {
+            CK(chain_launch(L.feather ? raster_tile_feather_kernel : raster_tile_kernel,
+                            L.mainTiles, 256, dyn, stream, overlap, priority, B, tris, sortedSlots,
+                            ranges, order));
+        }
     }
     return RIVE_CUDA_OK;
 }
@@ -1385,6 +1441,9 @@ int enqueue_back(rive_cuda_context* ctx,
             wide.cap = B.wideCap;
             wide.blocks = kWideBlocks;
         }
+        ExtendedTiles extended;
+        extended.heads = L.splitRaster() ? S.ranges : nullptr;
+        extended.tiles = L.mainTiles;
         const uint32_t binBlocks = wide.blocks + (L.slots + 255) / 256;
         const bool smallSort =
             S.keys16 && entries <= small_sort_capacity(ctx->smallCluster);
@@ -1394,9 +1453,14 @@ int enqueue_back(rive_cuda_context* ctx,
             if (padded && !smallSort)
                 bin_fill16_kernel<<<(entries + 255) / 256, 256, 0, stream>>>(
                     S.offsets + L.slots, entries, L.tiles, keys);
-            bin_scatter16_kernel<<<binBlocks, 256, 0, stream>>>(
-                L.slots, L.tileLog2, B.sceneTiles, S.tris, S.counts, S.masks, S.offsets, entries,
-                binError, keys, S.vals, wide);
+            if (extended.heads)
+                bin_scatter16_extended_kernel<<<binBlocks, 256, 0, stream>>>(
+                    L.slots, L.tileLog2, B.sceneTiles, S.tris, S.counts, S.masks, S.offsets,
+                    entries, binError, keys, S.vals, wide, extended);
+            else
+                bin_scatter16_kernel<<<binBlocks, 256, 0, stream>>>(
+                    L.slots, L.tileLog2, B.sceneTiles, S.tris, S.counts, S.masks, S.offsets,
+                    entries, binError, keys, S.vals, wide);
         }
         else
         {
@@ -1408,6 +1472,10 @@ int enqueue_back(rive_cuda_context* ctx,
                 bin_scatter_winding_kernel<<<(L.slots + 255) / 256, 256, 0, stream>>>(
                     B, S.tris, S.counts, S.masks, S.offsets, L.slots, entries, binError, keys,
                     S.vals);
+            else if (extended.heads)
+                bin_scatter_extended_kernel<<<binBlocks, 256, 0, stream>>>(
+                    L.slots, L.tileLog2, B.sceneTiles, S.tris, S.counts, S.masks, S.offsets, entries,
+                    binError, keys, S.vals, wide, extended);
             else
                 bin_scatter_kernel<<<binBlocks, 256, 0, stream>>>(
                     L.slots, L.tileLog2, B.sceneTiles, S.tris, S.counts, S.masks, S.offsets, entries,

@@ -951,6 +951,9 @@ __device__ __forceinline__ bool setup_snapped(const FlushParams& P,
     uint32_t key = pathID == 0 ? 0u : ((pathID + MAX_DENORM_F16) * P.pathIDGranularity) & 0xffffu;
     if (paint.x & PAINT_FLAG_EVEN_ODD_FILL)
         key ^= 0x8000u;
+    if ((features & (SF_FEATHER | FEATURE_ATLAS_BLIT | FEATURE_IMAGE_MESH)) ||
+        ((features & SF_MODULATED_IMAGE) && (paint.x & PAINT_FLAG_HAS_IMAGE)))
+        features |= FEATURE_EXTENDED;
     bb = make_int4(bx0, by0, bx1, by1);
     T.meta = make_uint4((pathID & 0xffffu) | (features << 16), (uint32_t)bx0 | ((uint32_t)bx1 << 16),
                         (uint32_t)by0 | ((uint32_t)by1 << 16), key | (scene << 16));
@@ -2568,10 +2571,17 @@ __global__ void bin_fill16_kernel(const uint32_t* __restrict__ pairTotal,
 // winding records), a deferred fan triangle's large box keeps its path's
 // edge tiles only, and an anchor winding slot writes one entry per interior
 // tile of its path with a nonzero winding.
+// With kExtended, also marks the tiles of triangles with FEATURE_EXTENDED.
+__device__ __forceinline__ void extend_tile(const ExtendedTiles& x, uint32_t tile)
+{
+    if (tile < x.tiles && !(__ldcg(&x.heads[tile].scene) & kExtendedTile))
+        atomicOr(&x.heads[tile].scene, kExtendedTile);
+}
+
 // The wide triangles' part of the binner: the first `blocks` CTAs of its grid
 // (0: no list) write their pairs, a warp per strip, each after the entries of
 // the triangle's strips before it.
-template <typename K>
+template <bool kExtended, typename K>
 __device__ __forceinline__ void bin_scatter_wide(int tileLog2,
                                                  const uint2* __restrict__ sceneTiles,
                                                  const TriRecord* __restrict__ tris,
@@ -2581,6 +2591,7 @@ __device__ __forceinline__ void bin_scatter_wide(int tileLog2,
                                                  K* __restrict__ keys,
                                                  uint32_t* __restrict__ vals,
                                                  const WideScatter& wide,
+                                                 const ExtendedTiles& extended,
                                                  uint32_t zero)
 {
     const uint32_t items = min(wide.list[zero], wide.cap) * kWideStrips;
@@ -2614,8 +2625,11 @@ __device__ __forceinline__ void bin_scatter_wide(int tileLog2,
                 const uint32_t pos = o + __popc(mask & ((1u << lane) - 1u));
                 if (pos < capacity)
                 {
-                    keys[pos] = (K)(st.x + (uint32_t)ty * st.y + (uint32_t)tx);
+                    const uint32_t tile = st.x + (uint32_t)ty * st.y + (uint32_t)tx;
+                    keys[pos] = (K)tile;
                     vals[pos] = slot;
+                    if (kExtended && (meta.x & (FEATURE_EXTENDED << 16)))
+                        extend_tile(extended, tile);
                 }
                 else
                 {
@@ -2627,7 +2641,7 @@ __device__ __forceinline__ void bin_scatter_wide(int tileLog2,
     }
 }
 
-template <bool kWinding, typename K>
+template <bool kWinding, bool kExtended, typename K>
 __device__ __forceinline__ void bin_scatter(const BatchTables* __restrict__ Bw,
                                             uint32_t slotCount,
                                             int tileLog2,
@@ -2640,15 +2654,16 @@ __device__ __forceinline__ void bin_scatter(const BatchTables* __restrict__ Bw,
                                             uint32_t* __restrict__ error,
                                             K* __restrict__ keys,
                                             uint32_t* __restrict__ vals,
-                                            const WideScatter& wide)
+                                            const WideScatter& wide,
+                                            const ExtendedTiles& extended)
 {
     const int lane = threadIdx.x & 31;
     chain_next();
     const uint32_t zero = chain_wait();
     if (blockIdx.x < wide.blocks)
     {
-        bin_scatter_wide(tileLog2, sceneTiles, tris, offsets, capacity, error, keys, vals, wide,
-                         zero);
+        bin_scatter_wide<kExtended>(tileLog2, sceneTiles, tris, offsets, capacity, error, keys,
+                                    vals, wide, extended, zero);
         return;
     }
     const uint32_t warpId = (((blockIdx.x - wide.blocks) * blockDim.x + threadIdx.x) >> 5) + zero;
@@ -2681,8 +2696,11 @@ __device__ __forceinline__ void bin_scatter(const BatchTables* __restrict__ Bw,
                 const int tx = tx0 + i % ntx, ty = ty0 + i / ntx;
                 if (o < capacity)
                 {
-                    keys[o] = (K)(st.x + (uint32_t)ty * st.y + (uint32_t)tx);
+                    const uint32_t tile = st.x + (uint32_t)ty * st.y + (uint32_t)tx;
+                    keys[o] = (K)tile;
                     vals[o] = mySlot;
+                    if (kExtended && (meta.x & (FEATURE_EXTENDED << 16)))
+                        extend_tile(extended, tile);
                 }
                 else
                 {
@@ -2762,8 +2780,11 @@ __device__ __forceinline__ void bin_scatter(const BatchTables* __restrict__ Bw,
                 const uint32_t pos = o + __popc(mask & ((1u << lane) - 1u));
                 if (pos < capacity)
                 {
-                    keys[pos] = (K)(st.x + (uint32_t)ty * st.y + (uint32_t)tx);
+                    const uint32_t tile = st.x + (uint32_t)ty * st.y + (uint32_t)tx;
+                    keys[pos] = (K)tile;
                     vals[pos] = slot;
+                    if (kExtended && (meta.x & (FEATURE_EXTENDED << 16)))
+                        extend_tile(extended, tile);
                 }
                 else
                 {
@@ -2782,38 +2803,32 @@ __device__ __forceinline__ void bin_scatter(const BatchTables* __restrict__ Bw,
 #ifndef RIVE_BIN_MIN_BLOCKS
 #define RIVE_BIN_MIN_BLOCKS 8
 #endif
-__global__ void __launch_bounds__(256, RIVE_BIN_MIN_BLOCKS) bin_scatter_kernel(uint32_t slotCount,
-                                                          int tileLog2,
-                                                          const uint2* __restrict__ sceneTiles,
-                                                          const TriRecord* __restrict__ tris,
-                                                          const uint32_t* __restrict__ tileCounts,
-                                                          const uint8_t* __restrict__ tileMasks,
-                                                          const uint32_t* __restrict__ offsets,
-                                                          uint32_t capacity,
-                                                          uint32_t* __restrict__ error,
-                                                          uint32_t* __restrict__ keys,
-                                                          uint32_t* __restrict__ vals,
-                                                          WideScatter wide)
-{
-    bin_scatter<false>(nullptr, slotCount, tileLog2, sceneTiles, tris, tileCounts, tileMasks,
-                       offsets, capacity, error, keys, vals, wide);
-}
-__global__ void __launch_bounds__(256, RIVE_BIN_MIN_BLOCKS) bin_scatter16_kernel(uint32_t slotCount,
-                                                          int tileLog2,
-                                                          const uint2* __restrict__ sceneTiles,
-                                                          const TriRecord* __restrict__ tris,
-                                                          const uint32_t* __restrict__ tileCounts,
-                                                          const uint8_t* __restrict__ tileMasks,
-                                                          const uint32_t* __restrict__ offsets,
-                                                          uint32_t capacity,
-                                                          uint32_t* __restrict__ error,
-                                                          uint16_t* __restrict__ keys,
-                                                          uint32_t* __restrict__ vals,
-                                                          WideScatter wide)
-{
-    bin_scatter<false>(nullptr, slotCount, tileLog2, sceneTiles, tris, tileCounts, tileMasks,
-                       offsets, capacity, error, keys, vals, wide);
-}
+#define RIVE_BIN_KERNELS(NAME, KEY)                                                               \
+    __global__ void __launch_bounds__(256, RIVE_BIN_MIN_BLOCKS) NAME##_kernel(                    \
+        uint32_t slotCount, int tileLog2, const uint2* __restrict__ sceneTiles,                   \
+        const TriRecord* __restrict__ tris, const uint32_t* __restrict__ tileCounts,              \
+        const uint8_t* __restrict__ tileMasks, const uint32_t* __restrict__ offsets,              \
+        uint32_t capacity, uint32_t* __restrict__ error, KEY* __restrict__ keys,                  \
+        uint32_t* __restrict__ vals, WideScatter wide)                                            \
+    {                                                                                             \
+        bin_scatter<false, false>(nullptr, slotCount, tileLog2, sceneTiles, tris, tileCounts,     \
+                                  tileMasks, offsets, capacity, error, keys, vals, wide,          \
+                                  ExtendedTiles());                                               \
+    }                                                                                             \
+    __global__ void __launch_bounds__(256, RIVE_BIN_MIN_BLOCKS) NAME##_extended_kernel(           \
+        uint32_t slotCount, int tileLog2, const uint2* __restrict__ sceneTiles,                   \
+        const TriRecord* __restrict__ tris, const uint32_t* __restrict__ tileCounts,              \
+        const uint8_t* __restrict__ tileMasks, const uint32_t* __restrict__ offsets,              \
+        uint32_t capacity, uint32_t* __restrict__ error, KEY* __restrict__ keys,                  \
+        uint32_t* __restrict__ vals, WideScatter wide, ExtendedTiles extended)                    \
+    {                                                                                             \
+        bin_scatter<false, true>(nullptr, slotCount, tileLog2, sceneTiles, tris, tileCounts,      \
+                                 tileMasks, offsets, capacity, error, keys, vals, wide,           \
+                                 extended);                                                       \
+    }
+RIVE_BIN_KERNELS(bin_scatter, uint32_t)
+RIVE_BIN_KERNELS(bin_scatter16, uint16_t)
+#undef RIVE_BIN_KERNELS
 
 // The same, for batches that draw interior tiles as winding records.
 __global__ void __launch_bounds__(256) bin_scatter_winding_kernel(BatchTables B,
@@ -2827,8 +2842,8 @@ __global__ void __launch_bounds__(256) bin_scatter_winding_kernel(BatchTables B,
                                                                   uint32_t* __restrict__ keys,
                                                                   uint32_t* __restrict__ vals)
 {
-    bin_scatter<true>(&B, slotCount, B.tileLog2, B.sceneTiles, tris, tileCounts, tileMasks,
-                      offsets, capacity, error, keys, vals, WideScatter());
+    bin_scatter<true, false>(&B, slotCount, B.tileLog2, B.sceneTiles, tris, tileCounts, tileMasks,
+                             offsets, capacity, error, keys, vals, WideScatter(), ExtendedTiles());
 }
 
 // A speculative pass whose scanned bin-entry total exceeds the capacity its
@@ -4049,7 +4064,9 @@ __device__ __forceinline__ uint32_t staged_meta(uint32_t meta, uint32_t paintX)
     return m ? m | (simple_feature(m >> 16, paintX) << 16) : 0u;
 }
 
-template <int TL, bool kFeather>
+// kSplit: one of two launches, this one for the tiles with (kFeather) or without
+// kExtendedTile.
+template <int TL, bool kFeather, bool kSplit = false>
 __device__ __forceinline__ void raster_tile(const BatchTables& B,
                                             const TriRecord* __restrict__ tris,
                                             const uint32_t* __restrict__ sortedSlots,
@@ -4064,7 +4081,9 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
     const uint2 range = make_uint2(head.x, head.y);
     // The tile's scene: its parameters are staged for the whole CTA (seen after
     // the first chunk's barrier); what comes before reads them in place.
-    const FlushParams& G0 = B.scenes[head.z];
+    if (kSplit && kFeather != ((head.z & kExtendedTile) != 0))
+        return; // the other launch's
+    const FlushParams& G0 = B.scenes[head.z & ~kExtendedTile];
     if (range.y > range.x && threadIdx.x < sizeof(FlushParams) / 4)
         reinterpret_cast<uint32_t*>(&sh.params)[threadIdx.x] =
             reinterpret_cast<const uint32_t*>(&G0)[threadIdx.x];
@@ -4353,16 +4372,24 @@ __device__ __forceinline__ uint32_t raster_index(const uint32_t* __restrict__ or
     return order ? order[i] : i;
 }
 
-// The raster kernels, each without and with the feather paths (the host
-// launches the feather variant only for batches with ENABLE_FEATHER draws). The
-// 16x16 one takes its tiles in the order of `order` (heaviest first), or as
-// they come when it is null. The hardware hands out CTAs in turn, so an ordered
-// grid is the work queue: a persistent grid with an atomic cursor over the same
-// order was slower (full-feature 2048x2048 frame 3.70 against 3.57 ms).
+// The raster kernels, each without and with the feather paths. The 16x16 ones
+// take their tiles in the order of `order` (heaviest first), or as they come when
+// it is null. The hardware hands out CTAs in turn, so an ordered grid is the work
+// queue: a persistent grid with an atomic cursor over the same order was slower
+// (full-feature 2048x2048 frame 3.70 against 3.57 ms).
+//
+// A batch without feathered draws or images takes the plain variant. Of others
+// the binner has marked the tiles that need the extended one (from kSplitTiles
+// tiles on), and each variant is launched over all tiles and leaves the other's at
+// once: the extended ones first, the plain ones as the last of those have started.
+// 64 UI screens take 1154 us of plain raster and 1484 of extended; a batch of 16
+// recorded frames, 9 of them without feathers, 1937 us of extended raster and 1854
+// split. (The extended tiles by persistent CTAs from a list: 1836, but a frame
+// with feathers on most tiles 640 -> 669.)
 #define RIVE_RASTER_KERNELS(NAME, FEATHER)                                                        \
-    __global__ void __launch_bounds__(256, RIVE_RASTER_MIN_BLOCKS(FEATHER)) NAME(                           \
+    __global__ void __launch_bounds__(256, RIVE_RASTER_MIN_BLOCKS(FEATHER)) NAME(                 \
         BatchTables B, const TriRecord* __restrict__ tris,                                        \
-        const uint32_t* __restrict__ sortedSlots, const TileHead* __restrict__ ranges,               \
+        const uint32_t* __restrict__ sortedSlots, const TileHead* __restrict__ ranges,            \
         const uint32_t* __restrict__ order)                                                       \
     {                                                                                             \
         __shared__ RasterShared<4> sh;                                                            \
@@ -4372,6 +4399,30 @@ __device__ __forceinline__ uint32_t raster_index(const uint32_t* __restrict__ or
 RIVE_RASTER_KERNELS(raster_tile_kernel, false)
 RIVE_RASTER_KERNELS(raster_tile_feather_kernel, true)
 #undef RIVE_RASTER_KERNELS
+
+__global__ void __launch_bounds__(256, RIVE_RASTER_MIN_BLOCKS(true)) raster_extended_kernel(
+    BatchTables B, const TriRecord* __restrict__ tris, const uint32_t* __restrict__ sortedSlots,
+    const TileHead* __restrict__ ranges, const uint32_t* __restrict__ order)
+{
+    __shared__ RasterShared<4> sh;
+    const uint32_t i = raster_index(order);
+    // Past the wait: everything before this launch is complete when the others'
+    // CTAs start.
+    chain_next();
+    raster_tile<4, true, true>(B, tris, sortedSlots, ranges, sh, i);
+}
+
+__global__ void __launch_bounds__(256, RIVE_RASTER_MIN_BLOCKS(false)) raster_others_kernel(
+    BatchTables B, const TriRecord* __restrict__ tris, const uint32_t* __restrict__ sortedSlots,
+    const TileHead* __restrict__ ranges, const uint32_t* __restrict__ order)
+{
+    __shared__ RasterShared<4> sh;
+    raster_tile<4, false, true>(B, tris, sortedSlots, ranges, sh,
+                                order ? order[blockIdx.x] : blockIdx.x);
+    // This grid ends after the extended tiles'.
+    if (blockIdx.x == gridDim.x - 1)
+        chain_wait();
+}
 
 // The feather atlas pass (render_atlas.glsl with the floating-point target
 // and fixed-function blending; the atlas pipelines of gpu.hpp:2076-2080):

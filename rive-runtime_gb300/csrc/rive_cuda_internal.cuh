@@ -119,6 +119,9 @@ constexpr uint32_t FEATURE_IMAGE_MESH = 1u << 10;
 // Set by the raster as it stages a triangle: its path resolves without a clip,
 // clip rect, advanced blend mode or image, from a solid colour or a gradient.
 constexpr uint32_t FEATURE_SIMPLE = 1u << 9;
+// The same bit of a triangle record: its tiles need the raster's extended variant
+// (an image mesh, an atlas blit, a feathered draw, or an image paint).
+constexpr uint32_t FEATURE_EXTENDED = 1u << 9;
 // Two more bits of a triangle record's feature half-word, set only when the
 // batch draws interior tiles as winding records: a fan triangle whose tiles
 // are counted after its path's winding grid is complete, and the record of a
@@ -382,6 +385,22 @@ struct WideScatter
     uint32_t cap = 0;
     uint32_t blocks = 0;
 };
+
+struct TileHead;
+// The binner's view of the main tiles that need the raster's extended variant
+// (heads null: the whole batch takes one variant). Binning a triangle with
+// FEATURE_EXTENDED to a tile sets kExtendedTile in the tile's head.
+struct ExtendedTiles
+{
+    TileHead* heads = nullptr;
+    uint32_t tiles = 0; // the main tiles, atlas tiles follow
+};
+constexpr uint32_t kExtendedTile = 1u << 31; // in TileHead::scene
+// Batches are split from this many main tiles on: two launches are slower where a
+// raster is short (4624 tiles of a feathered frame 38.5 -> 39.4 us; 15,645 of a
+// recorded frame 306 -> 299).
+constexpr uint32_t kSplitTiles = 8192;
+
 // CTAs (256 threads) of the two wide-triangle passes: two per SM's worth, a
 // strip for every warp of 38 triangles.
 constexpr uint32_t kWideBlocks = 304;

@@ -253,3 +253,57 @@ def test_patches_three_a_warp_match_one_a_warp(name, mixed):
     assert len(np.unique(want.reshape(-1, 4), axis=0)) > 20
     for t in targets[1:]:
         assert np.array_equal(t.cpu().numpy(), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("queue", [False, True])
+@pytest.mark.parametrize("tiles", [8191, 8192, 8193, 65600])  # one and two launches, 16 and 32-bit keys
+def test_tiles_split_between_raster_variants(tiles, queue):
+    """Feathered, atlas, image and plain frames, and a plain canvas that brings
+    the batch to `tiles` tiles: the images of single flushes."""
+    import torch
+    from conftest import render_one_by_one
+    from rive_runtime_gb300 import rive_cuda
+    names = ["feathered_s33", "feather_atlas_s35", "images_s41", "clips_s13", "feather_strokes_s31"]
+    caps = [load_golden(n)[0] for n in names]
+    pairs = [device_buffers(c) for c in caps]
+    bufs = [p[0] for p in pairs]
+    rest = tiles - sum(((c.width + 15) // 16) * ((c.height + 15) // 16) for c in caps)
+    W, H = 16 * (rest if rest < 4000 else rest // 64), 16 * (1 if rest < 4000 else 64)
+    odd = rest - (W // 16) * (H // 16)  # and what is left of it
+    sizes = [(W, H)] + ([(16 * odd, 16)] if odd else [])
+    rng = np.random.default_rng(9)
+    plain = []
+    for w, h in sizes:
+        at = np.stack([rng.integers(0, w // 16, 3000), rng.integers(0, h // 16, 3000)], 1) * 16.0
+        tris = at[:, None] + np.array([[1, 1], [14.5, 2], [3, 12.5]])
+        f, (b, keep) = flush_of(tris, np.arange(1, 3001), w, h)
+        plain.append((f, b, keep, w, h, render(f, b, w, h)[0]))
+    ctx = rive_cuda.Context(0)
+    stream = torch.cuda.current_stream().cuda_stream
+    want = render_one_by_one(ctx, caps, bufs, stream)
+    ctx.set_raster_queue(queue)
+    targets = [torch.zeros((c.height, c.width, 4), dtype=torch.uint8, device="cuda") for c in caps]
+    ptargets = [torch.zeros((h, w, 4), dtype=torch.uint8, device="cuda") for _, _, _, w, h, _ in plain]
+    assert all(len(c.flushes) == 1 for c in caps)
+    items = [(c.flushes[0], b, t.data_ptr()) for c, b, t in zip(caps, bufs, targets)]
+    items[2:2] = [(f, b, t.data_ptr()) for (f, b, _, _, _, _), t in zip(plain, ptargets)]
+    for call in ("batch", "graph"):
+        for t in targets + ptargets:
+            t.fill_(7)
+        if call == "batch":
+            ctx.flush_batch(items, stream)
+            ctx.sync(stream)
+        else:
+            g = ctx.graph(items)
+            for _ in range(2):
+                g.launch(stream)
+            g.check(stream)
+            g.close()
+        torch.cuda.synchronize()
+        for n, t, w in zip(names, targets, want):
+            assert np.array_equal(t.cpu().numpy(), w), (call, n)
+        for (_, _, _, _, _, w), t in zip(plain, ptargets):
+            img = t.cpu().numpy().astype(np.int64)
+            assert np.array_equal(img[..., 0] | (img[..., 1] << 8) | (img[..., 2] << 16), w), call
+    ctx.close()
