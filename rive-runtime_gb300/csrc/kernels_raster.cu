@@ -2671,7 +2671,16 @@ __device__ __forceinline__ void bin_scatter(const BatchTables* __restrict__ Bw,
     if (first >= slotCount)
         return;
     const uint32_t mySlot = first + lane;
-    const uint32_t myCount = mySlot < slotCount ? tileCounts[mySlot] : 0u;
+    // (Also where there is nothing to write: loads that do not wait for the count.
+    // With the mask walk's division below: scan and binner of the full-feature
+    // 2048x2048 frame 867 -> 758 us.)
+    uint32_t myCount = 0, myOffset = 0, myMask = 0;
+    if (mySlot < slotCount)
+    {
+        myCount = tileCounts[mySlot];
+        myOffset = offsets[mySlot];
+        myMask = tileMasks[mySlot];
+    }
     bool isBig = false;
     if (myCount)
     {
@@ -2687,16 +2696,19 @@ __device__ __forceinline__ void bin_scatter(const BatchTables* __restrict__ Bw,
         {
             // The set-up already tested these tiles: walk its mask.
             const uint2 st = sceneTiles[meta.w >> 16]; // (tileBase, tilesX)
-            uint32_t mask = tileMasks[mySlot];
-            uint32_t o = offsets[mySlot];
-            while (mask)
+            const uint32_t tile0 = st.x + (uint32_t)ty0 * st.y + (uint32_t)tx0;
+            // i / ntx = i * ceil(256 / ntx) / 256 for i < 8 (the quotient is never
+            // within 1/256 of a whole number; 256 / ntx + 0.99 is at least 1/100
+            // from one for ntx = 1 to 8).
+            const uint32_t inverse = (uint32_t)(__fdividef(256.f, (float)ntx) + .99f);
+            uint32_t o = myOffset;
+            while (myMask)
             {
-                const int i = __ffs(mask) - 1;
-                mask &= mask - 1;
-                const int tx = tx0 + i % ntx, ty = ty0 + i / ntx;
+                const uint32_t i = __ffs(myMask) - 1;
+                myMask &= myMask - 1;
                 if (o < capacity)
                 {
-                    const uint32_t tile = st.x + (uint32_t)ty * st.y + (uint32_t)tx;
+                    const uint32_t tile = tile0 + i + (i * inverse >> 8) * (st.y - (uint32_t)ntx);
                     keys[o] = (K)tile;
                     vals[o] = mySlot;
                     if (kExtended && (meta.x & (FEATURE_EXTENDED << 16)))
@@ -2711,7 +2723,7 @@ __device__ __forceinline__ void bin_scatter(const BatchTables* __restrict__ Bw,
         }
         else
         {
-            isBig = !(wide.blocks && tileMasks[mySlot] == kWideMask);
+            isBig = !(wide.blocks && myMask == kWideMask);
         }
     }
     uint32_t pending = __ballot_sync(0xffffffffu, isBig);
@@ -2723,7 +2735,7 @@ __device__ __forceinline__ void bin_scatter(const BatchTables* __restrict__ Bw,
         const TriRecord* T = tris + slot;
         const uint4 meta = T->meta;
         const uint2 st = sceneTiles[meta.w >> 16];
-        uint32_t o = offsets[slot];
+        uint32_t o = __shfl_sync(0xffffffffu, myOffset, t);
         if (kWinding && (meta.x & (FEATURE_WINDING_SLOT << 16)))
         {
             // The path's grid, from its winding slot's record.
