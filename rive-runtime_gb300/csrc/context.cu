@@ -30,8 +30,10 @@
 namespace rivecuda
 {
 __global__ void color_ramp_kernel(BatchTables B);
-__global__ void tessellate_kernel(BatchTables B, int lanesLog2);
-__global__ void tessellate_feather_kernel(BatchTables B, int lanesLog2);
+__global__ void tessellate_kernel(BatchTables B);
+__global__ void tessellate_feather_kernel(BatchTables B);
+__global__ void tessellate_packed_kernel(BatchTables B, int spansLog2);
+__global__ void tessellate_packed_feather_kernel(BatchTables B, int spansLog2);
 __global__ void patch_setup_kernel(BatchTables B,
                                    TriRecord* tris,
                                    uint32_t* tileCounts,
@@ -1210,10 +1212,20 @@ int enqueue_front(rive_cuda_context* ctx,
     if (L.tessSpans)
     {
         stage_begin(ctx, RIVE_CUDA_STAGE_TESSELLATE, stream);
-        const int lanes = tess_lanes_log2(L.tessSpans, L.feather);
-        CK(chain_launch(L.feather ? tessellate_feather_kernel : tessellate_kernel,
-                        ((L.tessSpans << lanes) + 255u) / 256u, 256, 0, stream, overlap, nullptr, B,
-                        lanes));
+        if (L.tessSpans >= kTessPackedSpans)
+        {
+            const int log2 =
+                tess_spans_log2(L.tessSpans, (uint64_t)L.tessRows * kTessTextureWidth);
+            CK(chain_launch(L.feather ? tessellate_packed_feather_kernel : tessellate_packed_kernel,
+                            (L.tessSpans + (4u << log2) - 1) / (4u << log2), 128, 0, stream, overlap,
+                            nullptr, B, log2));
+        }
+        else
+        {
+            CK(chain_launch(L.feather ? tessellate_feather_kernel : tessellate_kernel,
+                            (L.tessSpans * kTessLanes + 255u) / 256u, 256, 0, stream, overlap,
+                            nullptr, B));
+        }
         stage_end(ctx, stream);
     }
     if (L.slots)

@@ -21,8 +21,8 @@
 namespace rivecuda
 {
 __global__ void color_ramp_kernel(BatchTables B);
-__global__ void tessellate_kernel(BatchTables B, int lanesLog2);
-__global__ void tessellate_feather_kernel(BatchTables B, int lanesLog2);
+__global__ void tessellate_kernel(BatchTables B);
+__global__ void tessellate_feather_kernel(BatchTables B);
 __global__ void patch_setup_small_kernel(BatchTables B,
                                          TriRecord* tris,
                                          uint32_t* tileCounts,
@@ -379,12 +379,9 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
     if (d->grad_span_count)
         CKN(chain_launch(color_ramp_kernel, d->grad_span_count, 128, 0, stream, true, nullptr, B));
     if (d->tess_span_count)
-    {
-        const int lanes = tess_lanes_log2(d->tess_span_count, feather);
         CKN(chain_launch(feather ? tessellate_feather_kernel : tessellate_kernel,
-                         ((d->tess_span_count << lanes) + 255u) / 256u, 256, 0, stream, true,
-                         nullptr, B, lanes));
-    }
+                         (d->tess_span_count * kTessLanes + 255u) / 256u, 256, 0, stream, true,
+                         nullptr, B));
 
     TriRecord* tris = (TriRecord*)(pool + kTrisOff);
     uint8_t* masks = (uint8_t*)(pool + kMasksOff);

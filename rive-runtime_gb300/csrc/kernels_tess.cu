@@ -10,10 +10,10 @@
 //    one row of the 2048-wide tessellation texture; every texel is one
 //    tessellated vertex (x, y, theta, contourIDWithFlags).
 //
-// GB300 mapping: 8 or 16 lanes per span, two or four spans a warp; the per-span
-// set-up (tangents, polar step, join step) is evaluated once per lane without
-// divergence, then lanes stride across the span's vertices, so stores are runs
-// of consecutive 16-byte texels. Bound by issue slots. The texture is plain linear HBM memory
+// GB300 mapping: with many spans a warp takes 8 or 16 of them, a lane per span for
+// the set-up and then a lane per vertex, vertices that cost alike together
+// (tessellate_packed); with few, 16 lanes share a span. Stores are mostly runs of
+// consecutive 16-byte texels. Bound by issue slots. The texture is plain linear HBM memory
 // (row-major, 2048 texels per row), so the draw kernels read it with ordinary
 // 128-bit loads.
 #include "rive_cuda_internal.cuh"
@@ -79,15 +79,19 @@ __device__ __forceinline__ void cubic_tangents(float2 p0,
     t0 = f2sub(f2ne(p0, p1) ? p1 : (f2ne(p1, p2) ? p2 : p3), p0);
     t1 = f2sub(p3, f2ne(p3, p2) ? p2 : (f2ne(p2, p1) ? p1 : p0));
 }
+// The angle of a normalised vector.
+__device__ __forceinline__ float norm_angle(float2 v)
+{
+    const float theta = rc_acosf(fminf(fmaxf(v.x, -1.f), 1.f));
+    return v.y >= 0.f ? theta : -theta;
+}
 
 // common.glsl atan2(): acos of the normalized x, signed by y. The elementary
 // functions of this file come from rive_fp32_math.h, which the oracle's
 // tessellation shares, so its texels equal the oracle's bit for bit.
 __device__ __forceinline__ float rive_atan2(float2 v)
 {
-    v = f2normalize(v);
-    float theta = rc_acosf(fminf(fmaxf(v.x, -1.f), 1.f));
-    return v.y >= 0.f ? theta : -theta;
+    return norm_angle(f2normalize(v));
 }
 
 // Compensated De Casteljau (Graillat, Langlois and Louvet's compensated
@@ -302,6 +306,9 @@ struct SpanSetup
     float radsPerPolarSegment;
     float radsPerJoinSegment;
     uint32_t contourIDWithFlags; // without the mirrored flag
+    // The normalised tangents at the cubic's ends, and their angles.
+    float2 norm0, norm1;
+    float theta0, theta1;
     bool valid;
 };
 
@@ -407,7 +414,29 @@ __device__ SpanSetup span_setup(const FlushParams& P, const uint4* sp)
         s.radsPerJoinSegment = rpj;
     }
     s.contourIDWithFlags = flags;
+    s.norm0 = f2normalize(t0);
+    s.norm1 = f2normalize(t1);
+    s.theta0 = norm_angle(s.norm0);
+    s.theta1 = norm_angle(s.norm1);
     return s;
+}
+
+// Whether the tangent `tan` has turned from the unit vector `norm0` by at most
+// maxRotation (0 to pi): cos_between >= cos, as rc_cosf and correctly rounded
+// division and square root have it. Both cosines are first taken from the hardware's
+// reciprocal square root and cosine: within 2e-6 of the exact steps' values together
+// (__cosf's documented bound is 2^-21.2 there, the product of unit vectors is off by
+// a few 2^-23), so where they differ by more than 1e-5 the answer is theirs, in a
+// fifth of the instructions.
+__device__ __forceinline__ bool turned_less(float2 tan, float2 norm0, float maxRotation)
+{
+    const float len2 = __fmaf_rn(tan.x, tan.x, __fmul_rn(tan.y, tan.y));
+    const float c = __fmul_rn(__fmaf_rn(tan.x, norm0.x, __fmul_rn(tan.y, norm0.y)), rsqrtf(len2));
+    const float d = __fsub_rn(c, __cosf(maxRotation));
+    // (NaN, infinities and lengths whose square leaves the normal range: exactly.)
+    if (fabsf(d) > 1e-5f && fabsf(c) <= 1.5f && len2 > 1e-30f && len2 < 1e30f)
+        return d > 0.f;
+    return f2dot(f2normalize(tan), norm0) >= rc_cosf(maxRotation);
 }
 
 // Per-texel half of tessellate.glsl (the fragment shader, 294-567).
@@ -415,8 +444,9 @@ template <bool kFeather>
 __device__ uint4 tess_vertex(const SpanSetup& s, float vertexIdx, uint32_t flagsIn)
 {
     float2 p0 = s.p0, p1 = s.p1, p2 = s.p2, p3 = s.p3;
-    float2 tan0, tan1;
-    cubic_tangents(p0, p1, p2, p3, tan0, tan1);
+    float2 tan0norm = s.norm0;
+    float theta0 = s.theta0;
+    bool join = false;
     float parametricSegmentCount = s.parametricSegmentCount;
     float radsPerPolarSegment = s.radsPerPolarSegment;
     uint32_t flags = flagsIn;
@@ -428,9 +458,11 @@ __device__ uint4 tess_vertex(const SpanSetup& s, float vertexIdx, uint32_t flags
     }
     else
     {
+        // A join turns from the cubic's last tangent to joinTangent.
         p0 = p1 = p2 = p3;
-        tan0 = tan1;
-        tan1 = s.joinTangent;
+        tan0norm = s.norm1;
+        theta0 = s.theta1;
+        join = true;
         parametricSegmentCount = 1.f;
         mergedVertexID = __fsub_rn(mergedVertexID, mergedSegmentCount);
         mergedSegmentCount = s.joinSegmentCount;
@@ -459,7 +491,7 @@ __device__ uint4 tess_vertex(const SpanSetup& s, float vertexIdx, uint32_t flags
     {
         bool isTan0 = mergedVertexID < __fmul_rn(mergedSegmentCount, .5f);
         coord = isTan0 ? p0 : p3;
-        theta = rive_atan2(isTan0 ? tan0 : tan1);
+        theta = isTan0 ? theta0 : join ? rive_atan2(s.joinTangent) : s.theta1;
     }
     else if (flags & RETROFIT_TRI_STRIP_CONTOUR_FLAG)
     {
@@ -491,29 +523,26 @@ __device__ uint4 tess_vertex(const SpanSetup& s, float vertexIdx, uint32_t flags
             float lastParametricID = 0.f;
             float maxParametricID =
                 fminf(__fsub_rn(parametricSegmentCount, 1.f), mergedVertexID);
-            float2 tan0norm = f2normalize(tan0);
             float absRads = fabsf(radsPerPolarSegment);
             float maxRotation0 = __fmul_rn(__fadd_rn(1.f, mergedVertexID), absRads);
-#pragma unroll
-            for (int p = 9; p >= 0; --p)
+            // (Bits above maxParametricID's first would be skipped one by one.)
+#pragma unroll 1
+            for (int p = 31 - __clz(max((int)maxParametricID, 0)); p >= 0; --p)
             {
                 float testID = __fadd_rn(lastParametricID, (float)(1 << p));
                 if (testID <= maxParametricID)
                 {
                     float2 testTan = f2add(f2scale(A, testID), B_);
                     testTan = f2add(f2scale(testTan, testID), C_);
-                    float cosRotation = f2dot(f2normalize(testTan), tan0norm);
                     float maxRotation =
                         __fadd_rn(__fmul_rn(testID, -absRads), maxRotation0);
                     maxRotation = fminf(maxRotation, kPi);
-                    if (cosRotation >= rc_cosf(maxRotation))
+                    if (turned_less(testTan, tan0norm, maxRotation))
                         lastParametricID = testID;
                 }
             }
             float parametricT = __fdiv_rn(lastParametricID, parametricSegmentCount);
             float lastPolarID = __fsub_rn(mergedVertexID, lastParametricID);
-            float theta0 = rc_acosf(fminf(fmaxf(tan0norm.x, -1.f), 1.f));
-            theta0 = tan0norm.y >= 0.f ? theta0 : -theta0;
             theta = __fadd_rn(__fmul_rn(lastPolarID, radsPerPolarSegment), theta0);
             float sn, cs;
             rc_sincosf(theta, &sn, &cs);
@@ -620,30 +649,21 @@ __global__ void __launch_bounds__(128) color_ramp_kernel(BatchTables B)
     }
 }
 
-// 2^lanesLog2 lanes per TessVertexSpan of the batch (tess_lanes_log2). A span's forward rectangle
-// holds its vertices in order and its mirrored one the same vertices in reverse,
-// equal but for the mirrored flag: each is evaluated once and stored twice.
-template <bool kFeather>
-__device__ __forceinline__ void tessellate(const BatchTables& B, int lanesLog2)
+// Where a span's vertices go: texel at + step * k of its row holds vertex k (the
+// vertex index before its clamp at 0), for k in [first, end) -- per rectangle, the
+// forward one and the mirrored one, which holds the same vertices in reverse, equal
+// but for the mirrored flag: each vertex is evaluated once and stored twice.
+struct SpanRects
 {
-    chain_next();
-    const uint32_t gs = ((blockIdx.x * blockDim.x + threadIdx.x) >> lanesLog2) + chain_wait();
-    const int lanes = 1 << lanesLog2, lane = threadIdx.x & (lanes - 1);
-    if (gs >= B.totalTessSpans)
-        return;
-    const uint32_t scene = find_range(B.tessSpanBase, B.sceneCount, gs);
-    const FlushParams& P = B.scenes[scene];
-    const uint32_t span = gs - B.tessSpanBase[scene];
-    const uint4* sp = P.tessSpans + 4 * (size_t)(P.firstTessSpan + span);
-    SpanSetup s = span_setup<kFeather>(P, sp);
-    if (!s.valid)
-        return;
-    // Per rectangle: texel px = at + step * k holds vertex k (the vertex index
-    // before its clamp at 0), for k in [first, end).
-    uint4* row[2];
     int at[2], first[2], end[2];
+    int row[2]; // in rows of the texture; meaningless where the range is empty
     uint32_t mirrored[2];
-    const int total = (int)s.totalVertexCount;
+    int k0, k1; // the vertices of both
+};
+
+__device__ __forceinline__ SpanRects span_rects(const FlushParams& P, const uint4* sp, int total)
+{
+    SpanRects r;
     const uint4 q2 = sp[2], q3 = sp[3];
 #pragma unroll
     for (int i = 0; i < 2; ++i)
@@ -652,62 +672,174 @@ __device__ __forceinline__ void tessellate(const BatchTables& B, int lanesLog2)
         const int32_t x0x1 = (int32_t)(i ? q3.y : q3.x);
         const int x0 = (int32_t)((uint32_t)x0x1 << 16) >> 16;
         const int x1 = x0x1 >> 16;
-        first[i] = end[i] = at[i] = 0;
-        mirrored[i] = 0;
-        row[i] = nullptr;
+        r.first[i] = r.end[i] = r.at[i] = r.row[i] = 0;
+        r.mirrored[i] = 0;
         if (isnan(y) || x0 == x1 || y < 0.f || y >= (float)P.tessDataHeight)
             continue;
-        row[i] = P.tess + (size_t)(int)y * kTessTextureWidth;
+        r.row[i] = (int)y;
         const int lo = max(min(x0, x1), 0), hi = min(max(x0, x1), kTessTextureWidth);
         if (lo >= hi)
             continue;
         // Vertex index of texel px: total - |x1 - (px + 1/2)|, rounded down.
         if (x1 < x0)
         {
-            mirrored[i] = MIRRORED_CONTOUR_CONTOUR_FLAG;
-            at[i] = total + x1 - 1;
-            first[i] = at[i] - (hi - 1);
-            end[i] = at[i] - lo + 1;
+            r.mirrored[i] = MIRRORED_CONTOUR_CONTOUR_FLAG;
+            r.at[i] = total + x1 - 1;
+            r.first[i] = r.at[i] - (hi - 1);
+            r.end[i] = r.at[i] - lo + 1;
         }
         else
         {
-            at[i] = x1 - total;
-            first[i] = lo - at[i];
-            end[i] = hi - at[i];
+            r.at[i] = x1 - total;
+            r.first[i] = lo - r.at[i];
+            r.end[i] = hi - r.at[i];
         }
     }
-    const bool both = first[0] < end[0] && first[1] < end[1];
-    const bool only1 = !(first[0] < end[0]);
-    const int k0 = both ? min(first[0], first[1]) : first[only1];
-    const int k1 = both ? max(end[0], end[1]) : end[only1];
-    for (int k = k0 + lane; k < k1; k += lanes)
-    {
-        const uint4 v = tess_vertex<kFeather>(s, (float)max(k, 0), s.contourIDWithFlags);
+    const bool both = r.first[0] < r.end[0] && r.first[1] < r.end[1];
+    const bool only1 = !(r.first[0] < r.end[0]);
+    r.k0 = both ? min(r.first[0], r.first[1]) : only1 ? r.first[1] : r.first[0];
+    r.k1 = both ? max(r.end[0], r.end[1]) : only1 ? r.end[1] : r.end[0];
+    return r;
+}
+
+template <bool kFeather>
+__device__ __forceinline__ void put_vertex(uint4* __restrict__ tess, const SpanSetup& s,
+                                           const SpanRects& r, int k)
+{
+    const uint4 v = tess_vertex<kFeather>(s, (float)max(k, 0), s.contourIDWithFlags);
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
-            if (k >= first[i] && k < end[i])
-                row[i][mirrored[i] ? at[i] - k : at[i] + k] =
-                    make_uint4(v.x, v.y, v.z, v.w | mirrored[i]);
+    for (int i = 0; i < 2; ++i)
+        if (k >= r.first[i] && k < r.end[i])
+            tess[(size_t)r.row[i] * kTessTextureWidth +
+                 (r.mirrored[i] ? r.at[i] - k : r.at[i] + k)] =
+                make_uint4(v.x, v.y, v.z, v.w | r.mirrored[i]);
+}
+
+// 16 lanes per TessVertexSpan, which share its set-up: the shortest way for few
+// spans.
+template <bool kFeather> __device__ __forceinline__ void tessellate(const BatchTables& B)
+{
+    chain_next();
+    const uint32_t gs = ((blockIdx.x * blockDim.x + threadIdx.x) / kTessLanes) + chain_wait();
+    const int lane = threadIdx.x % kTessLanes;
+    if (gs >= B.totalTessSpans)
+        return;
+    const uint32_t scene = find_range(B.tessSpanBase, B.sceneCount, gs);
+    const FlushParams& P = B.scenes[scene];
+    const uint32_t span = gs - B.tessSpanBase[scene];
+    const uint4* sp = P.tessSpans + 4 * (size_t)(P.firstTessSpan + span);
+    const SpanSetup s = span_setup<kFeather>(P, sp);
+    if (!s.valid)
+        return;
+    const SpanRects r = span_rects(P, sp, (int)s.totalVertexCount);
+    for (int k = r.k0 + lane; k < r.k1; k += kTessLanes)
+        put_vertex<kFeather>(P.tess, s, r, k);
+}
+
+// A warp's spans, for the packed tessellation. (40 words)
+struct PackedSpan
+{
+    SpanSetup s;
+    SpanRects r;
+    uint4* tess;
+    uint32_t pad;
+};
+static_assert(sizeof(PackedSpan) == 160, "PackedSpan layout");
+
+// 8 or 16 spans a warp: a lane sets one up, then all vertices of the warp's spans
+// are dealt out to the lanes, first those between a span's ends or within a round
+// join (a search for the parametric segment, a root and an arc tangent each), then
+// the rest (a point, an angle from the set-up), so that lanes run the same code.
+// With 8 lanes per span 13 of 32 lanes were at work on 1024x1024 strokes: 129 -> 104
+// us with this, 72 with turned_less and the ends' angles from the set-up;
+// full-feature 2048x2048 frame 578 -> 482 -> 344 us, 64 UI screens 60 -> 42 -> 36.
+template <bool kFeather>
+__device__ __forceinline__ void tessellate_packed(const BatchTables& B, int spansLog2)
+{
+    __shared__ PackedSpan shared[4][kTessPacked];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    PackedSpan* const sh = shared[w];
+    chain_next();
+    const uint32_t gs0 = ((blockIdx.x * 4 + w) << spansLog2) + chain_wait();
+    if (gs0 >= B.totalTessSpans)
+        return; // whole warp exits together
+    const uint32_t gs = gs0 + lane;
+    int count[2] = {0, 0}, base = 0, low = 0, high = 0; // this lane's span
+    if (lane < 1 << spansLog2 && gs < B.totalTessSpans)
+    {
+        const uint32_t scene = find_range(B.tessSpanBase, B.sceneCount, gs);
+        const FlushParams& P = B.scenes[scene];
+        const uint32_t span = gs - B.tessSpanBase[scene];
+        const uint4* sp = P.tessSpans + 4 * (size_t)(P.firstTessSpan + span);
+        PackedSpan p;
+        p.s = span_setup<kFeather>(P, sp);
+        if (p.s.valid)
+        {
+            const int total = (int)p.s.totalVertexCount;
+            p.r = span_rects(P, sp, total);
+            p.tess = P.tess;
+            sh[lane] = p;
+            const bool bevel =
+                (p.s.contourIDWithFlags & JOIN_TYPE_MASK) > ROUND_JOIN_CONTOUR_FLAG;
+            const int inner1 = bevel ? total - (int)p.s.joinSegmentCount : total;
+            // [k0, k1) = the low part before vertex 1, the inner part, the rest.
+            base = min(max(p.r.k0, 1), p.r.k1);
+            high = max(min(p.r.k1, inner1), base);
+            count[0] = high - base;
+            low = base - p.r.k0;
+            count[1] = low + p.r.k1 - high;
+        }
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int pass = 0; pass < 2; ++pass)
+    {
+        const int mine = pass ? count[1] : count[0];
+        int start = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            const int v = __shfl_up_sync(0xffffffffu, start, o);
+            start += lane >= o ? v : 0;
+        }
+        const int all = __shfl_sync(0xffffffffu, start, 31);
+        start -= mine;
+        for (int j = lane; j - lane < all; j += 32)
+        {
+            // The last span that starts at or before j.
+            int i = 0;
+#pragma unroll
+            for (int o = 16; o >= 1; o >>= 1)
+                i += __shfl_sync(0xffffffffu, start, i + o) <= j ? o : 0;
+            const int off = j - __shfl_sync(0xffffffffu, start, i);
+            const int b = __shfl_sync(0xffffffffu, base, i), l = __shfl_sync(0xffffffffu, low, i);
+            const int h = __shfl_sync(0xffffffffu, high, i);
+            if (j < all)
+                put_vertex<kFeather>(sh[i].tess, sh[i].s, sh[i].r,
+                                     pass == 0  ? b + off
+                                     : off < l ? b - l + off
+                                               : h + off - l);
+        }
+        __syncwarp();
     }
 }
 
-// Resident 256-thread CTAs per SM the tessellation's registers are bounded
-// for: 4 (64 registers, a few bytes spilled) tessellates the full-feature
-// 2048x2048 frame in 0.64 ms against 0.70 and 0.69 ms with 3 and 5 (16 lanes a
-// span).
-#ifndef RIVE_TESS_MIN_BLOCKS
-#define RIVE_TESS_MIN_BLOCKS 4
-#endif
-__global__ void __launch_bounds__(256, RIVE_TESS_MIN_BLOCKS) tessellate_kernel(BatchTables B,
-                                                                               int lanesLog2)
-{
-    tessellate<false>(B, lanesLog2);
-}
+__global__ void __launch_bounds__(256) tessellate_kernel(BatchTables B) { tessellate<false>(B); }
 
 // With feathered-fill softening and feather-join texels.
-__global__ void __launch_bounds__(256) tessellate_feather_kernel(BatchTables B, int lanesLog2)
+__global__ void __launch_bounds__(256) tessellate_feather_kernel(BatchTables B)
 {
-    tessellate<true>(B, lanesLog2);
+    tessellate<true>(B);
+}
+
+__global__ void __launch_bounds__(128, 8) tessellate_packed_kernel(BatchTables B, int spansLog2)
+{
+    tessellate_packed<false>(B, spansLog2);
+}
+__global__ void __launch_bounds__(128, 8) tessellate_packed_feather_kernel(BatchTables B,
+                                                                          int spansLog2)
+{
+    tessellate_packed<true>(B, spansLog2);
 }
 // The tessellation pass's device functions on n items, for the parity tests
 // (the layouts of oracle_cubic_eval and oracle_math_eval): fn 0..5 the cubic

@@ -291,16 +291,20 @@ struct PatchSegment
     uint32_t mesh;
 };
 
-// Lanes that tessellate one span, as a power of two. A span of the measured
-// scenes has 6 to 40 vertices, each evaluated once for both of its rectangles,
-// and its set-up is repeated by its every lane, so few lanes waste least:
-// full-feature 2048x2048 frame 0.95 ms with a warp per span and rectangle, 0.84,
-// 0.64 and 0.58 ms with 32, 16 and 8 lanes; 64 UI screens 171, 135, 82 and 60 us.
-// Below 16,384 spans latency counts (a 240x180 widget 10 us with 16, 12 us with
-// 8), and feathered batches diverge (16 recorded frames 39 against 43 us).
-inline int tess_lanes_log2(uint32_t spans, bool feather)
+// Lanes that tessellate one span where spans are few (latency counts), and the
+// most spans a warp takes where they are many (kernels_tess.cu). A 1080x1920 UI
+// screen of 3560 spans 12 us with lanes, 15 packed; 16 recorded frames, 33 k spans,
+// 43 and 35; 64 UI screens, 133 k, 132 and 36.
+constexpr int kTessLanes = 16;
+constexpr int kTessPacked = 16;
+constexpr uint32_t kTessPackedSpans = 16384;
+// Spans a warp takes in the packed tessellation, as a power of two: 8, or 16 where
+// eight spans' vertices (half their texels) would not give every lane two and there
+// are warps enough (64 UI screens, 10 texels a span, 36 us with 16 and 43 with 8;
+// strokes, 16 texels, 79 and 72; 33 k spans of 13 texels 41 and 35).
+inline int tess_spans_log2(uint32_t spans, uint64_t texels)
 {
-    return !feather && spans >= 16384 ? 3 : 4;
+    return spans >= 1u << 16 && texels < (uint64_t)spans * 12 ? 4 : 3;
 }
 
 // Triangles with large tile boxes. One warp tests a triangle's tiles 32 at a

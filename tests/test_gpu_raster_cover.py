@@ -307,3 +307,48 @@ def test_tiles_split_between_raster_variants(tiles, queue):
             img = t.cpu().numpy().astype(np.int64)
             assert np.array_equal(img[..., 0] | (img[..., 1] << 8) | (img[..., 2] << 16), w), call
     ctx.close()
+
+
+@pytest.mark.gpu
+# Flushes of 16,384 spans on are tessellated by warps of 8 spans, of 65,536 on by
+# warps of 16 where a span has few texels.
+@pytest.mark.parametrize("name,spans", [
+    ("stroke_stress_s5", 16384), ("stroke_stress_s5", 66000), ("plain_small_s1", 16500),
+    ("full_odd_s11", 17000), ("feather_strokes_s31", 16390), ("silver_police_files_f60", 66000),
+    ("silver_rewards_f10", 66000)])
+def test_spans_by_warps_match_spans_by_lanes(name, spans):
+    """A flush's spans, and as many copies of them (each in rows of its own) as
+    take the packed tessellation: every copy has the same texels."""
+    import torch
+    from conftest import tess_written
+    from rive_runtime_gb300 import rive_cuda
+    cap = load_golden(name)[0]
+    f = cap.flushes[0]
+    d = f.desc
+    h, first, n = d["tess_data_height"], d["first_tess_span"], d["tess_span_count"]
+    written = tess_written(cap, 0)
+    ctx = rive_cuda.Context(0)
+    target = torch.zeros((cap.height, cap.width, 4), dtype=torch.uint8, device="cuda")
+
+    def texels(height):
+        bufs, keep = device_buffers(cap)
+        ctx.flush_device(f, bufs, target.data_ptr())
+        ctx.sync()
+        t = np.asarray(ctx.read_tess(height)).view(np.uint32).reshape(-1, 4)
+        return t.reshape(-1, 2048 * h, 4)[:, written], target.cpu().numpy()
+
+    want, image = texels(h)
+    one = np.frombuffer(cap.buffers["tess_spans"], np.uint32).reshape(-1, 16)[first:first + n]
+    copies = -(-spans // n)
+    all_spans = np.tile(one, (copies, 1, 1)).reshape(copies, n, 16)
+    for i in range(copies):
+        y = all_spans[i, :, 10:12].copy().view(np.float32) + np.float32(i * h)
+        all_spans[i, :, 10:12] = y.view(np.uint32)
+    cap.buffers["tess_spans"] = all_spans.tobytes()
+    d.update(first_tess_span=0, tess_span_count=copies * n, tess_data_height=copies * h)
+    got, image2 = texels(copies * h)
+    ctx.close()
+    assert len(got) == copies
+    for g in got:
+        assert np.array_equal(g, want[0])
+    assert np.array_equal(image, image2)
