@@ -599,7 +599,7 @@ int rive_cuda_get_bin_speculation(const rive_cuda_context* ctx, int* enabled);
  */
 enum
 {
-    RIVE_CUDA_STAGE_COLOR_RAMP = 0,  /* color_ramp_kernel                 */
+    RIVE_CUDA_STAGE_COLOR_RAMP = 0,  /* color_ramp_kernel (when timed)    */
     RIVE_CUDA_STAGE_TESSELLATE = 1,  /* tessellate_kernel                 */
     RIVE_CUDA_STAGE_PATCH_SETUP = 2, /* patch_setup_kernel                */
     RIVE_CUDA_STAGE_BIN = 3,         /* scan + bin_scatter_kernel         */

@@ -8,7 +8,7 @@
 // 3-deep ring (gpu::kBufferRingSize, gpu.hpp:77) of pinned, write-combined
 // host staging buffers, and unmap enqueues one host->device copy into a
 // device-resident copy of the buffer. flush() then runs, in stream order:
-//   color_ramp_kernel -> tessellate_kernel -> patch_setup_kernel (midpoint fans,
+//   color_ramp_kernel + tessellate_kernel -> patch_setup_kernel (midpoint fans,
 //   outer curves) + interior_setup_kernel ->
 //   (scan) -> bin_scatter_kernel -> (radix sort by tile) ->
 //   tile_ranges_kernel -> raster_tile_kernel.
@@ -30,8 +30,8 @@
 namespace rivecuda
 {
 __global__ void color_ramp_kernel(BatchTables B);
-__global__ void tessellate_kernel(BatchTables B);
-__global__ void tessellate_feather_kernel(BatchTables B);
+__global__ void tessellate_kernel(BatchTables B, uint32_t tessCtas);
+__global__ void tessellate_feather_kernel(BatchTables B, uint32_t tessCtas);
 __global__ void tessellate_packed_kernel(BatchTables B, int spansLog2);
 __global__ void tessellate_packed_feather_kernel(BatchTables B, int spansLog2);
 __global__ void patch_setup_kernel(BatchTables B,
@@ -723,6 +723,8 @@ struct BatchLayout
     uint32_t fanStride = kPatchTriangleCount;
     // Some scene has enough tiles for a wide triangle (BatchTables::wide).
     bool wide = false;
+    // Whether the colour ramps have a launch of their own.
+    bool rampsAlone() const { return !tessSpans || tessSpans >= kTessPackedSpans; }
     // Whether the raster splits its tiles between its two variants.
     bool splitRaster() const { return feather && tileLog2 == 4 && mainTiles >= kSplitTiles; }
     uint32_t wideCap() const { return wide ? std::min(slots, kWideCapacity) : 0u; }
@@ -1203,7 +1205,8 @@ int enqueue_front(rive_cuda_context* ctx,
             path_bounds_kernel<<<(L.tessSpans + 255) / 256, 256, 0, stream>>>(B);
         path_alloc_kernel<<<(L.paths + 255) / 256, 256, 0, stream>>>(B);
     }
-    if (L.gradSpans)
+    const bool rampsAlone = ctx->profiling || L.rampsAlone();
+    if (L.gradSpans && rampsAlone)
     {
         stage_begin(ctx, RIVE_CUDA_STAGE_COLOR_RAMP, stream);
         CK(chain_launch(color_ramp_kernel, L.gradSpans, 128, 0, stream, overlap, nullptr, B));
@@ -1222,9 +1225,10 @@ int enqueue_front(rive_cuda_context* ctx,
         }
         else
         {
+            const uint32_t ctas = (L.tessSpans * kTessLanes + 255u) / 256u;
             CK(chain_launch(L.feather ? tessellate_feather_kernel : tessellate_kernel,
-                            (L.tessSpans * kTessLanes + 255u) / 256u, 256, 0, stream, overlap,
-                            nullptr, B));
+                            ctas + (rampsAlone ? 0u : L.gradSpans), 256, 0, stream, overlap, nullptr,
+                            B, ctas));
         }
         stage_end(ctx, stream);
     }
@@ -1831,7 +1835,8 @@ int run_batch_body(rive_cuda_context* ctx,
         ctx->stats.bin_entries = 0; // known when the flush settles
         ctx->stats.winding_entries = 0;
         ctx->stats.tiles = L.tiles;
-        ctx->stats.kernel_launches = 1 + (L.gradSpans ? 1 : 0) + (L.tessSpans ? 1 : 0) + 1 + 5 +
+        ctx->stats.kernel_launches = 1 + (L.gradSpans && L.rampsAlone() ? 1 : 0) +
+                                 (L.tessSpans ? 1 : 0) + 1 + 5 +
                                      (L.wide ? 1 : 0) +
                                      1 + (L.tiles > L.mainTiles ? 1 : 0);
         return RIVE_CUDA_OK;
@@ -1868,7 +1873,8 @@ int run_batch_body(rive_cuda_context* ctx,
     ctx->stats.bin_entries = pairs;
     ctx->stats.winding_entries = windingEntries;
     ctx->stats.tiles = L.tiles;
-    ctx->stats.kernel_launches = 1 + (L.gradSpans ? 1 : 0) + (L.tessSpans ? 1 : 0) +
+    ctx->stats.kernel_launches = 1 + (L.gradSpans && L.rampsAlone() ? 1 : 0) +
+                                 (L.tessSpans ? 1 : 0) +
                                  (L.slots ? 1 + (L.wide ? 1 : 0) : 0) + (pairs ? 3 : 0) + 1 +
                                  (L.tiles > L.mainTiles ? 1 : 0) +
                                  (L.winding ? 3 + (L.tessSpans ? 1 : 0) + 1 : 0);
@@ -2567,7 +2573,8 @@ int graph_build(rive_cuda_context* ctx,
     g->stats.triangles = L.slots;
     g->stats.bin_entries = g->measured;
     g->stats.tiles = L.tiles;
-    g->stats.kernel_launches = 1 + (L.gradSpans ? 1 : 0) + (L.tessSpans ? 1 : 0) +
+    g->stats.kernel_launches = 1 + (L.gradSpans && L.rampsAlone() ? 1 : 0) +
+                                 (L.tessSpans ? 1 : 0) +
                                (L.slots ? 2 + (L.wide ? 1 : 0) : 0) + (capacity ? 4 : 0) + 1;
     return RIVE_CUDA_OK;
 }

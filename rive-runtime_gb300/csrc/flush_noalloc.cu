@@ -20,9 +20,8 @@
 
 namespace rivecuda
 {
-__global__ void color_ramp_kernel(BatchTables B);
-__global__ void tessellate_kernel(BatchTables B);
-__global__ void tessellate_feather_kernel(BatchTables B);
+__global__ void tessellate_kernel(BatchTables B, uint32_t tessCtas);
+__global__ void tessellate_feather_kernel(BatchTables B, uint32_t tessCtas);
 __global__ void patch_setup_small_kernel(BatchTables B,
                                          TriRecord* tris,
                                          uint32_t* tileCounts,
@@ -376,12 +375,12 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
     F.sceneTiles = B.sceneTiles;
     flush_start_kernel<<<(std::max(F.gradVectors, tiles) + 255) / 256, 256, 0, stream>>>(F);
 
-    if (d->grad_span_count)
-        CKN(chain_launch(color_ramp_kernel, d->grad_span_count, 128, 0, stream, true, nullptr, B));
-    if (d->tess_span_count)
+    if (d->grad_span_count || d->tess_span_count)
+    {
+        const uint32_t ctas = (d->tess_span_count * kTessLanes + 255u) / 256u;
         CKN(chain_launch(feather ? tessellate_feather_kernel : tessellate_kernel,
-                         (d->tess_span_count * kTessLanes + 255u) / 256u, 256, 0, stream, true,
-                         nullptr, B));
+                         ctas + d->grad_span_count, 256, 0, stream, true, nullptr, B, ctas));
+    }
 
     TriRecord* tris = (TriRecord*)(pool + kTrisOff);
     uint8_t* masks = (uint8_t*)(pool + kMasksOff);

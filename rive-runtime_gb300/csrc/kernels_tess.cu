@@ -1,11 +1,11 @@
 // Color-ramp and tessellation kernels (GPU passes 1 and 2 of a rasterOrdering
 // flush).
 //
-//  * color_ramp_kernel restates renderer/src/shaders/color_ramp.glsl:40-107:
+//  * color_ramp restates renderer/src/shaders/color_ramp.glsl:40-107:
 //    each GradientSpan paints a 1-texel-tall strip of the 512-wide RGBA8
 //    gradient texture: a solid left border, a linear ramp between x0 and x1,
 //    and a solid right border.
-//  * tessellate_kernel restates renderer/src/shaders/tessellate.glsl:61-567:
+//  * tessellate restates renderer/src/shaders/tessellate.glsl:61-567:
 //    each TessVertexSpan covers [x0, x1) (and optionally a mirrored range) of
 //    one row of the 2048-wide tessellation texture; every texel is one
 //    tessellated vertex (x, y, theta, contourIDWithFlags).
@@ -593,12 +593,11 @@ __device__ uint4 tess_vertex(const SpanSetup& s, float vertexIdx, uint32_t flags
 }
 } // namespace
 
-// One block of 128 threads per GradientSpan of the batch; each thread owns 4
-// of the 512 texel columns.
-__global__ void __launch_bounds__(128) color_ramp_kernel(BatchTables B)
+// GradientSpan g of the batch, by one CTA.
+__device__ __forceinline__ void color_ramp(const BatchTables& B, uint32_t g)
 {
     chain_next();
-    const uint32_t g = blockIdx.x + chain_wait();
+    g += chain_wait();
     if (g >= B.totalGradSpans)
         return;
     const uint32_t scene = find_range(B.gradSpanBase, B.sceneCount, g);
@@ -824,12 +823,29 @@ __device__ __forceinline__ void tessellate_packed(const BatchTables& B, int span
     }
 }
 
-__global__ void __launch_bounds__(256) tessellate_kernel(BatchTables B) { tessellate<false>(B); }
-
-// With feathered-fill softening and feather-join texels.
-__global__ void __launch_bounds__(256) tessellate_feather_kernel(BatchTables B)
+__global__ void __launch_bounds__(128) color_ramp_kernel(BatchTables B)
 {
-    tessellate<true>(B);
+    color_ramp(B, blockIdx.x);
+}
+
+// tessCtas CTAs of tessellation, then one for each gradient span: the two passes
+// depend on nothing of each other's, and one launch less is 2 us of a small frame
+// (240x180 widget 43 -> 41 us). Not in the packed launches, whose frames are long
+// (full-feature 1021x767 1158 -> 1167 us). The feather variants with feathered-fill
+// softening and feather-join texels.
+__global__ void __launch_bounds__(256) tessellate_kernel(BatchTables B, uint32_t tessCtas)
+{
+    if (blockIdx.x < tessCtas)
+        tessellate<false>(B);
+    else
+        color_ramp(B, blockIdx.x - tessCtas);
+}
+__global__ void __launch_bounds__(256) tessellate_feather_kernel(BatchTables B, uint32_t tessCtas)
+{
+    if (blockIdx.x < tessCtas)
+        tessellate<true>(B);
+    else
+        color_ramp(B, blockIdx.x - tessCtas);
 }
 
 __global__ void __launch_bounds__(128, 8) tessellate_packed_kernel(BatchTables B, int spansLog2)
@@ -841,6 +857,7 @@ __global__ void __launch_bounds__(128, 8) tessellate_packed_feather_kernel(Batch
 {
     tessellate_packed<true>(B, spansLog2);
 }
+
 // The tessellation pass's device functions on n items, for the parity tests
 // (the layouts of oracle_cubic_eval and oracle_math_eval): fn 0..5 the cubic
 // functions, 10..13 sin, cos, acos and the cube root.
