@@ -1144,6 +1144,7 @@ BatchTables write_tables(rive_cuda_context* ctx,
     B.fanSlotStride = L.fanStride;
     B.wide = L.wide ? S.wide : nullptr;
     B.wideCap = L.wideCap();
+    B.wideTiles = wide_tiles(L.slots);
     B.wideStrips = L.wide ? S.wide + 1 + B.wideCap : nullptr;
     B.pathBase = (const uint32_t*)(dT + L.oPathBase);
     if (L.winding)
@@ -1460,7 +1461,8 @@ int enqueue_back(rive_cuda_context* ctx,
         ExtendedTiles extended;
         extended.heads = L.splitRaster() ? S.ranges : nullptr;
         extended.tiles = L.mainTiles;
-        const uint32_t binBlocks = wide.blocks + (L.slots + 255) / 256;
+        wide.perWarp = bin_slots_per_warp(L.slots);
+        const uint32_t binBlocks = wide.blocks + (L.slots + 8 * wide.perWarp - 1) / (8 * wide.perWarp);
         const bool smallSort =
             S.keys16 && entries <= small_sort_capacity(ctx->smallCluster);
         if (S.keys16)

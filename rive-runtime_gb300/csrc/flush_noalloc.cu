@@ -356,6 +356,7 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
     {
         B.wide = wideList;
         B.wideCap = kWideCap;
+        B.wideTiles = wide_tiles((uint32_t)kMaxSlots);
         B.wideStrips = wideList + 1 + kWideCap;
     }
 
@@ -412,6 +413,7 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
     if (pairs)
     {
         WideScatter wide;
+        wide.perWarp = bin_slots_per_warp(slots);
         if (wideList)
         {
             wide.list = B.wide;
@@ -419,7 +421,8 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
             wide.cap = B.wideCap;
             wide.blocks = kWideBlocks;
         }
-        bin_scatter16_kernel<<<wide.blocks + (slots + 255) / 256, 256, 0, stream>>>(
+        bin_scatter16_kernel<<<
+            wide.blocks + (slots + 8 * wide.perWarp - 1) / (8 * wide.perWarp), 256, 0, stream>>>(
             slots, kTileLog2, B.sceneTiles, tris, counts, masks, offs, pairs, dError, keys, vals,
             wide);
         int endBit = 1;

@@ -1068,7 +1068,7 @@ __device__ __forceinline__ void count_tiles(bool has,
                 big = true;
                 // (Past the capacity the counter is only read: no contention
                 // on batches with hundreds of thousands of such triangles.)
-                if (B.wide && ntx * nty > kWideTiles &&
+                if (B.wide && ntx * nty > (int)B.wideTiles &&
                     *(volatile const uint32_t*)B.wide < B.wideCap)
                 {
                     const uint32_t i = atomicAdd(B.wide, 1u);
@@ -2667,10 +2667,10 @@ __device__ __forceinline__ void bin_scatter(const BatchTables* __restrict__ Bw,
         return;
     }
     const uint32_t warpId = (((blockIdx.x - wide.blocks) * blockDim.x + threadIdx.x) >> 5) + zero;
-    const uint32_t first = warpId * 32;
+    const uint32_t first = warpId * wide.perWarp;
     if (first >= slotCount)
         return;
-    const uint32_t mySlot = first + lane;
+    const uint32_t mySlot = lane < wide.perWarp ? first + lane : slotCount;
     // (Also where there is nothing to write: loads that do not wait for the count.
     // With the mask walk's division below: scan and binner of the full-feature
     // 2048x2048 frame 867 -> 758 us.)

@@ -319,6 +319,12 @@ inline int tess_spans_log2(uint32_t spans, uint64_t texels)
 // canvases 10.57, 10.19 and 10.17 ms with it at 256, 512 and 1024 tiles,
 // 10.15 ms without).
 constexpr int kWideTiles = 1024;
+// The line of a batch of `slots` triangles, where some scene has more than kWideTiles
+// tiles: lower for small frames, which wait for their longest warp (1080x1080
+// recorded feathered frame: scan and binner 29 -> 22 us, set-up 32 -> 29, the same
+// at 128; a 2370x1680 recorded frame's binner 32 -> 25, 35 at 128; 16 recorded
+// frames, 1.8 M slots, 71 -> 93, so not theirs).
+inline uint32_t wide_tiles(uint32_t slots) { return slots <= 1u << 18 ? 256 : kWideTiles; }
 constexpr int kWideStrips = 64;
 constexpr int kWideStripTiles = 128;
 constexpr uint32_t kWideCapacity = 16384; // triangles kept; more are walked in place
@@ -367,7 +373,7 @@ struct BatchTables
     // triangle is set aside (no scene has that many tiles, or winding records).
     uint32_t* wide;
     uint32_t* wideStrips;
-    uint32_t wideCap;
+    uint32_t wideCap, wideTiles;
     // Interior tiles as winding records (null grids: off). Midpoint-fan
     // patches then take fanSlotStride = 25 slots (24 triangles and the
     // winding slot), otherwise 24.
@@ -388,7 +394,15 @@ struct WideScatter
     const uint32_t* strips = nullptr;
     uint32_t cap = 0;
     uint32_t blocks = 0;
+    uint32_t perWarp = 32; // slots a warp takes of the others (bin_slots_per_warp)
 };
+
+// A small frame's binner waits for its longest warp, one with a backdrop's large
+// triangles one after another: 8 slots a warp, not 32 (1080x1080 recorded feathered
+// frame, 187 k slots: scan and binner 37 -> 29 us, a 240x180 widget 20.5 -> 18.5; 4
+// slots: 30 and 21). Frames of more slots have other warps to run meanwhile.
+inline uint32_t bin_slots_per_warp(uint32_t slots) { return slots <= 1u << 18 ? 8 : 32; }
+
 
 struct TileHead;
 // The binner's view of the main tiles that need the raster's extended variant
