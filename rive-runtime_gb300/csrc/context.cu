@@ -1350,7 +1350,7 @@ int prepare_raster(rive_cuda_context* ctx)
 // is long enough for the last ones to leave the GPU half empty. 3072 tiles of
 // 2366 entries: raster 737 -> 634 us; 16384 tiles of 450: 3.76 -> 3.57 ms; 1024
 // tiles of 610: no difference; UI screens (9 to 13 entries a tile) would pay the
-// order's 5 us for nothing.
+// order's 7 to 24 us for nothing.
 bool orders_tiles(const BatchLayout& L, uint32_t entries)
 {
     return L.tileLog2 == 4 && L.mainTiles >= kOrderMinTiles && L.mainTiles <= kOrderTiles &&

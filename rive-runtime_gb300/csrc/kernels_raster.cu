@@ -2877,7 +2877,8 @@ __global__ void __launch_bounds__(256) ranges_guard_kernel(const uint32_t* __res
 // 16 bytes of one load (4 or 8 keys); its neighbours' keys come from their lanes.
 // The keys are sorted, so when the one before and the one after are equal there
 // is nothing to say. (One key a thread, with its neighbours loaded: 37 us for
-// 10.9 M entries of 16,384 tiles; a quarter of that now, bound by HBM.)
+// 10.9 M entries of 16,384 tiles; now 7.3 M entries of 3,072 tiles
+// take 6 to 7 us, 2 bytes each.)
 template <typename K>
 __device__ __forceinline__ void tile_ranges(uint32_t pairCount, uint32_t tileCount,
                                             const K* __restrict__ keys, TileHead* __restrict__ ranges)
@@ -3881,8 +3882,9 @@ __device__ __noinline__ float feathered_fragment(const float4* __restrict__ plan
 }
 
 // Resident CTAs per SM the register allocation is bounded for (16x16 tiles): 5
-// (48 registers; 64 UI screens 1.94 ms against 2.15 ms with 4), with the feather
-// paths 4 (64 registers; 16 recorded frames 2.69 ms against 2.76 ms with 5).
+// (48 registers; 4 and 6 were slower everywhere, 64 UI screens by 11% with 4), with
+// the feather paths 4 (64 registers; raster of 16 recorded frames 1.84 ms, 1.94 with
+// 3 and 1.89 with 5).
 #define RIVE_RASTER_MIN_BLOCKS(FEATHER) ((FEATHER) ? 4 : 5)
 
 // Tile geometry: a CTA of T x T threads, one per pixel; warp w owns the 8x4
@@ -4578,7 +4580,8 @@ __global__ void __launch_bounds__(1024) raster_atlas32_kernel(
 // eighth: one CTA counts them into 256 buckets (the leading four bits of a
 // tile's bin entries and their exponent, descending), per warp so that equal
 // tiles do not queue at one counter, and gives each its place. Bound by
-// latency: about 5 us for 16,384 tiles, against 45 us for a radix sort.
+// latency and by equal buckets' atomics: 7 us for 3,072 tiles, 24 for 16,384, against 45
+// us for a radix sort of those.
 __global__ void __launch_bounds__(1024, 1) tile_order_kernel(uint32_t tiles,
                                                              const TileHead* __restrict__ ranges,
                                                              uint32_t* __restrict__ order)
