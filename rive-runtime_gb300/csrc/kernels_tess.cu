@@ -660,6 +660,14 @@ struct SpanRects
     int k0, k1; // the vertices of both
 };
 
+// The vertices of a span as the integer that its rectangles count with: at most
+// 6140, or 0 where the span's three counts are all zero. Those wrap to 2^32 - 1 (a
+// malformed record, drawn as the shader draws it), which no int32 holds.
+__device__ __forceinline__ int span_vertices(const SpanSetup& s)
+{
+    return s.totalVertexCount < 65536.f ? (int)s.totalVertexCount : 0;
+}
+
 __device__ __forceinline__ SpanRects span_rects(const FlushParams& P, const uint4* sp, int total)
 {
     SpanRects r;
@@ -705,10 +713,19 @@ template <bool kFeather>
 __device__ __forceinline__ void put_vertex(uint4* __restrict__ tess, const SpanSetup& s,
                                            const SpanRects& r, int k)
 {
-    const uint4 v = tess_vertex<kFeather>(s, (float)max(k, 0), s.contourIDWithFlags);
+    // (Between the two ranges: a span cut at the ends of rows.)
+    const bool in[2] = {k >= r.first[0] && k < r.end[0], k >= r.first[1] && k < r.end[1]};
+    if (!in[0] && !in[1])
+        return;
+    // Vertex k is total - |x1 - (px + 1/2)| rounded down, |x1 - (px + 1/2)| being
+    // span_vertices - k - 1/2: k itself but for the wrapped total.
+    const float index = s.totalVertexCount < 65536.f
+                            ? (float)max(k, 0)
+                            : floorf(__fsub_rn(s.totalVertexCount, __fsub_rn((float)-k, .5f)));
+    const uint4 v = tess_vertex<kFeather>(s, index, s.contourIDWithFlags);
 #pragma unroll
     for (int i = 0; i < 2; ++i)
-        if (k >= r.first[i] && k < r.end[i])
+        if (in[i])
             tess[(size_t)r.row[i] * kTessTextureWidth +
                  (r.mirrored[i] ? r.at[i] - k : r.at[i] + k)] =
                 make_uint4(v.x, v.y, v.z, v.w | r.mirrored[i]);
@@ -730,7 +747,7 @@ template <bool kFeather> __device__ __forceinline__ void tessellate(const BatchT
     const SpanSetup s = span_setup<kFeather>(P, sp);
     if (!s.valid)
         return;
-    const SpanRects r = span_rects(P, sp, (int)s.totalVertexCount);
+    const SpanRects r = span_rects(P, sp, span_vertices(s));
     for (int k = r.k0 + lane; k < r.k1; k += kTessLanes)
         put_vertex<kFeather>(P.tess, s, r, k);
 }
@@ -774,7 +791,7 @@ __device__ __forceinline__ void tessellate_packed(const BatchTables& B, int span
         p.s = span_setup<kFeather>(P, sp);
         if (p.s.valid)
         {
-            const int total = (int)p.s.totalVertexCount;
+            const int total = span_vertices(p.s);
             p.r = span_rects(P, sp, total);
             p.tess = P.tess;
             sh[lane] = p;

@@ -1,0 +1,58 @@
+"""Records and settings at the edge of what the kernels take: each against the
+oracle, or against exactly sized, unlimited renders that are themselves held to
+it by the golden tests."""
+import numpy as np
+import pytest
+
+from conftest import device_buffers, load_golden, load_package
+
+load_package()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("copies", [1, 20])  # spans by lanes, and packed in warps
+@pytest.mark.parametrize("name", ["strokes_s3", "full_odd_s11"])
+def test_spans_without_vertices_have_the_shaders_texels(name, copies):
+    """Spans whose three counts are zero: their vertex total wraps to 2^32 - 1,
+    and their texels are what the shader's arithmetic gives for it."""
+    import oracle
+    from conftest import tess_written
+    from rive_runtime_gb300 import rive_cuda
+    cap = load_golden(name)[0]
+    f = cap.flushes[0]
+    d = f.desc
+    h, first, n = d["tess_data_height"], d["first_tess_span"], d["tess_span_count"]
+    spans = np.frombuffer(cap.buffers["tess_spans"], np.uint32).reshape(-1, 16)
+    one = spans[first:first + n].copy()
+    one[np.random.default_rng(3).random(n) < .2, 14] = 0
+    # Beyond 128 texels float32 spaces the index by 256: a span across two whole
+    # rows of its own, and one that starts left of them.
+    long = np.repeat(one[:1], 2, axis=0)
+    long[:, 14] = 0
+    long[:, 10:12] = np.array([[h, h + 1], [h + 2, h + 3]], np.float32).view(np.uint32)
+    long[:, 12:14] = [[2048 << 16, 2048], [2000 << 16 | (-30 & 0xffff), -30 << 16 & 0xffffffff | 2000]]
+    one, n, h = np.concatenate([one, long]), n + 2, h + 4
+    cap.buffers["tess_spans"] = one.tobytes()
+    d.update(first_tess_span=0, tess_span_count=n, tess_data_height=h)
+    written = tess_written(cap, 0)
+    want = oracle.tessellate(cap)[written]
+    assert (one[:, 14] == 0).sum() > 8
+    many = np.tile(one, (copies, 1, 1))
+    for i in range(copies):
+        many[i, :, 10:12] = (one[:, 10:12].view(np.float32) + np.float32(i * h)).view(np.uint32)
+    cap.buffers["tess_spans"] = many.tobytes()
+    d.update(tess_span_count=copies * n, tess_data_height=copies * h)
+    assert copies == 1 or copies * n >= 16384
+    ctx = rive_cuda.Context(0)
+    import torch
+    target = torch.zeros((cap.height, cap.width, 4), dtype=torch.uint8, device="cuda")
+    bufs, keep = device_buffers(cap)
+    ctx.flush_device(f, bufs, target.data_ptr())
+    ctx.sync()
+    got = np.asarray(ctx.read_tess(copies * h)).view(np.uint32).reshape(copies, 2048 * h, 4)
+    ctx.close()
+    for g in got:
+        g = g[written]
+        assert np.array_equal(g[:, 3], want[:, 3])
+        a, b = g[:, :3].copy().view(np.float32), want[:, :3].copy().view(np.float32)
+        assert ((a.view(np.uint32) == b.view(np.uint32)) | (np.isnan(a) & np.isnan(b))).all()
