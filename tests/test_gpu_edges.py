@@ -56,3 +56,40 @@ def test_spans_without_vertices_have_the_shaders_texels(name, copies):
         assert np.array_equal(g[:, 3], want[:, 3])
         a, b = g[:, :3].copy().view(np.float32), want[:, :3].copy().view(np.float32)
         assert ((a.view(np.uint32) == b.view(np.uint32)) | (np.isnan(a) & np.isnan(b))).all()
+
+
+def parity(got, want):
+    d = np.abs(got.astype(np.int16) - want.astype(np.int16)).max(axis=2)
+    assert (d <= 2).mean() >= .999 and d.max() <= 8, (float((d <= 2).mean()), int(d.max()))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("value", [np.nan, -np.inf, -3e38])
+@pytest.mark.parametrize("where", ["v", "span", "image"])
+@pytest.mark.parametrize("name", ["strokes_s3", "feather_atlas_s35", "images_s41"])
+def test_paints_that_are_not_finite(name, where, value):
+    """Gradients whose row or span is not finite, image matrices likewise: a
+    pixel of no coverage is written, too, and its colour is not the
+    destination's (0 times NaN)."""
+    import oracle
+    from rive_runtime_gb300 import rive_cuda
+    cap = load_golden(name)[0]
+    paints = np.frombuffer(cap.buffers["paints"], np.uint32).reshape(-1, 2).copy()
+    aux = np.frombuffer(cap.buffers["paint_aux"], np.float32).reshape(-1, 32).copy()
+    n = min(len(paints), len(aux))
+    gradient = np.isin(paints[:n, 0] & 15, (2, 3))
+    image = (paints[:n, 0] & 0x800) != 0
+    hit = np.flatnonzero(image if where == "image" else gradient)[::2]
+    if not len(hit):
+        pytest.skip("no such paint in this scene")
+    if where == "v":
+        paints[hit, 1] = np.float32(value).view(np.uint32)
+    elif where == "span":
+        aux[hit, 6:8] = 0, value
+    else:
+        aux[hit, 20] = value
+    cap.buffers["paints"], cap.buffers["paint_aux"] = paints.tobytes(), aux.tobytes()
+    ctx = rive_cuda.Context(0)
+    got = ctx.render(cap)
+    ctx.close()
+    parity(got, oracle.render(cap))
