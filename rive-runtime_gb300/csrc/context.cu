@@ -1288,11 +1288,15 @@ int enqueue_front(rive_cuda_context* ctx,
     return RIVE_CUDA_OK;
 }
 
+// The most dynamic shared memory a raster kernel is padded with. Every kernel's
+// limit is set to this and never to a context's own padding: the limit belongs to
+// the kernel, and contexts differ in theirs.
+constexpr size_t kMaxPad = 160u << 10;
+
 // Dynamic shared memory (unused) that holds a raster kernel to at most
 // `ctas` resident CTAs per SM, found with the occupancy calculator.
 size_t occupancy_pad(const void* fn, int threads, int ctas)
 {
-    constexpr size_t kMaxPad = 160u << 10;
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxPad) !=
         cudaSuccess)
         return 0;
@@ -1333,11 +1337,9 @@ int prepare_raster(rive_cuda_context* ctx)
         if (slot == 1) // the split's launches take the same padding
         {
             CK(cudaFuncSetAttribute(raster_extended_kernel,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)ctx->rasterPad[1][1]));
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxPad));
             CK(cudaFuncSetAttribute(raster_others_kernel,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)ctx->rasterPad[0][1]));
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxPad));
         }
         cudaGetLastError(); // a failed query only leaves the launch unpadded
         ctx->rasterPadFor[slot] = ctx->rasterCtasPerSm;

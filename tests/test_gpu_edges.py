@@ -93,3 +93,33 @@ def test_paints_that_are_not_finite(name, where, value):
     got = ctx.render(cap)
     ctx.close()
     parity(got, oracle.render(cap))
+
+
+@pytest.mark.gpu
+def test_split_raster_under_the_limits_of_two_contexts():
+    """A frame whose tiles are split between two launches, by contexts with
+    different limits of resident CTAs in turn, single and as graphs: each keeps
+    its own."""
+    import oracle
+    import torch
+    from rive_runtime_gb300 import rive_cuda
+    cap = load_golden("silver_bankcard_f10")[0]
+    want = oracle.render(cap)
+    bufs, keep = device_buffers(cap)
+    stream = torch.cuda.Stream().cuda_stream
+    made = []
+    for ctas in (1, 4, 2, 0):
+        ctx = rive_cuda.Context(0)
+        ctx.set_raster_config(16, ctas)
+        target = torch.zeros((cap.height, cap.width, 4), dtype=torch.uint8, device="cuda")
+        made.append((ctx, target, ctx.graph([(cap.flushes[0], bufs, target.data_ptr())])))
+    for ctx, target, graph in made + made:
+        parity(ctx.render(cap), want)
+        target.zero_()
+        torch.cuda.synchronize()
+        graph.launch(stream)
+        graph.check(stream)
+        parity(target.cpu().numpy(), want)
+    for ctx, _, graph in made:
+        graph.close()
+        ctx.close()
