@@ -123,3 +123,48 @@ def test_split_raster_under_the_limits_of_two_contexts():
     for ctx, _, graph in made:
         graph.close()
         ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["strokes_s3", "clips_s13"])
+def test_noalloc_in_a_second_cuda_context(name):
+    """The no-allocation flush in a CUDA context made after the library has run
+    in the device's primary one."""
+    import ctypes
+    import oracle
+    import torch
+    from rive_runtime_gb300 import rive_cuda
+    from rive_runtime_gb300.capture import BUFFER_NAMES
+    cap = load_golden(name)[0]
+    bufs, keep = device_buffers(cap)
+    first = torch.zeros((cap.height, cap.width, 4), dtype=torch.uint8, device="cuda")
+    rive_cuda.flush_device_noalloc(cap.flushes[0], bufs, first.data_ptr(), 0)
+    torch.cuda.synchronize()
+    cu = ctypes.CDLL("libcuda.so.1")
+
+    def call(f, *args):
+        assert getattr(cu, f)(*args) == 0, f
+
+    call("cuCtxCreate_v2", ctypes.byref(ctypes.c_void_p()), 0, 0)
+    try:
+        def alloc(data):
+            p = ctypes.c_uint64()
+            call("cuMemAlloc_v2", ctypes.byref(p), ctypes.c_size_t(max(len(data), 16)))
+            call("cuMemcpyHtoD_v2", p, data, ctypes.c_size_t(len(data)))
+            return p.value
+
+        bufs2 = rive_cuda.DeviceBuffers()
+        for n in BUFFER_NAMES:
+            data = cap.buffers.get(n, b"")
+            setattr(bufs2, n, alloc(data) if data else None)
+        target = alloc(bytes(4 * cap.width * cap.height))
+        rive_cuda.flush_device_noalloc(cap.flushes[0], bufs2, target, 0)
+        got = np.zeros((cap.height, cap.width, 4), np.uint8)
+        call("cuMemcpyDtoH_v2", got.ctypes.data_as(ctypes.c_void_p), ctypes.c_uint64(target),
+             ctypes.c_size_t(got.nbytes))
+    finally:
+        old = ctypes.c_void_p()
+        call("cuCtxPopCurrent_v2", ctypes.byref(old))
+        call("cuCtxDestroy_v2", old)
+    assert np.array_equal(got, first.cpu().numpy())
+    parity(got, oracle.render(cap))
