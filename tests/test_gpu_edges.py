@@ -129,7 +129,8 @@ def test_split_raster_under_the_limits_of_two_contexts():
 @pytest.mark.parametrize("name", ["strokes_s3", "clips_s13"])
 def test_noalloc_in_a_second_cuda_context(name):
     """The no-allocation flush in a CUDA context made after the library has run
-    in the device's primary one."""
+    in the device's primary one, where the one-cluster passes' function
+    attributes were set: they hold in the other context as well."""
     import ctypes
     import oracle
     import torch
