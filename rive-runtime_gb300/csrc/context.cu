@@ -375,7 +375,7 @@ struct rive_cuda_context
     int tileLog2 = kTileLog2;
     int rasterCtasPerSm = 0; // 0: as many as fit
     bool raster32Ready = false;
-    uint32_t smallCluster = 8; // small_passes_prepare
+    uint32_t smallCluster = 8; // small_passes_init
     size_t rasterPad[2][2] = {};      // [feather variant][8 or 16 pixel kernel]: padding
     int rasterPadFor[2] = {-1, -1};   // the CTAs-per-SM limit it was found for
     // Stage timing (rive_cuda_set_profiling).
@@ -1971,7 +1971,7 @@ int rive_cuda_context_create(int device, rive_cuda_context** out_ctx)
     if (e == cudaSuccess)
         e = ensure_feather_lut(device);
     if (e == cudaSuccess)
-        e = small_passes_prepare(&ctx->smallCluster);
+        e = small_passes_init(device, &ctx->smallCluster);
     if (e != cudaSuccess)
     {
         fprintf(stderr, "rive_cuda_context_create: %s\n", cudaGetErrorString(e));

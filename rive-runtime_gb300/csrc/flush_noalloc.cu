@@ -255,7 +255,7 @@ extern "C" int rive_cuda_flush_device_noalloc(const rive_cuda_flush_desc* d,
         pool = (uint8_t*)p;
     }
     uint32_t cluster = 0;
-    CKN(small_passes_prepare(&cluster));
+    CKN(small_passes_init(dev, &cluster));
     cudaStream_t stream = (cudaStream_t)cuda_stream;
     uint32_t* dError = (uint32_t*)(pool + kStatusOff);
 

@@ -363,85 +363,46 @@ uint32_t cluster_for(uint32_t items, uint32_t perCta, uint32_t largest)
 }
 } // namespace
 
-namespace
+cudaError_t small_passes_init(int device, uint32_t* largest)
 {
-cudaError_t prepare_context(uint32_t* largest)
-{
-    // 16 CTAs need a GPC with as many free SMs (not every partition of the
-    // device has one); 8 are portable.
-    cudaError_t e = cudaFuncSetAttribute(
-        small_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(SmallSortShared));
-    for (auto fn : {(const void*)small_sort_kernel, (const void*)small_scan_kernel})
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess)
-        return e;
-    cudaLaunchAttribute attr = {};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 16;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cudaLaunchConfig_t c = {};
-    c.gridDim = dim3(16);
-    c.attrs = &attr;
-    c.numAttrs = 1;
-    int sorts = 0, scans = 0;
-    c.blockDim = dim3(kSortThreads);
-    c.dynamicSmemBytes = sizeof(SmallSortShared);
-    e = cudaOccupancyMaxActiveClusters(&sorts, small_sort_kernel, &c);
-    c.blockDim = dim3(1024);
-    c.dynamicSmemBytes = 0;
-    if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveClusters(&scans, small_scan_kernel, &c);
-    if (e != cudaSuccess)
-        cudaGetLastError(); // a failed query only leaves the portable size
-    *largest = e == cudaSuccess && sorts > 0 && scans > 0 ? 16 : 8;
-    return cudaSuccess;
-}
-
-// The number that the driver gives every CUDA context and never gives again
-// (cuCtxGetId), or 0.
-unsigned long long context_id()
-{
-    using GetId = int (*)(void*, unsigned long long*);
-    static const GetId get = [] {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult found;
-        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &fn, 12000, cudaEnableDefault, &found) !=
-                cudaSuccess ||
-            found != cudaDriverEntryPointSuccess)
-            fn = nullptr;
-        return (GetId)fn;
-    }();
-    unsigned long long id = 0;
-    return get && get(nullptr, &id) == 0 ? id : 0;
-}
-} // namespace
-
-// Function attributes belong to the CUDA context, and so do the SMs that a cluster
-// finds: what was found is kept by the context's number, for the last few contexts (a
-// call without it takes 7 us longer: 320x256 fills without allocation 115 -> 122 us).
-cudaError_t small_passes_prepare(uint32_t* largest)
-{
-    constexpr int kKept = 16;
     static std::mutex m;
-    static unsigned long long ids[kKept] = {};
-    static uint32_t found[kKept] = {}, next = 0;
-    const unsigned long long id = context_id();
+    static uint32_t found[64] = {};
     std::lock_guard<std::mutex> lock(m);
-    for (int i = 0; id && i < kKept; ++i)
-        if (ids[i] == id)
-        {
-            *largest = found[i];
-            return cudaSuccess;
-        }
-    const cudaError_t e = prepare_context(largest);
-    if (e == cudaSuccess && id)
+    if (device < 0 || device >= 64)
+        return cudaErrorInvalidDevice;
+    if (!found[device])
     {
-        ids[next] = id;
-        found[next] = *largest;
-        next = (next + 1) % kKept;
+        // 16 CTAs need a GPC with as many free SMs (not every partition of the
+        // device has one); 8 are portable.
+        cudaError_t e = cudaFuncSetAttribute(
+            small_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(SmallSortShared));
+        for (auto fn : {(const void*)small_sort_kernel, (const void*)small_scan_kernel})
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e != cudaSuccess)
+            return e;
+        cudaLaunchAttribute attr = {};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = 16;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cudaLaunchConfig_t c = {};
+        c.gridDim = dim3(16);
+        c.attrs = &attr;
+        c.numAttrs = 1;
+        int sorts = 0, scans = 0;
+        c.blockDim = dim3(kSortThreads);
+        c.dynamicSmemBytes = sizeof(SmallSortShared);
+        e = cudaOccupancyMaxActiveClusters(&sorts, small_sort_kernel, &c);
+        c.blockDim = dim3(1024);
+        c.dynamicSmemBytes = 0;
+        if (e == cudaSuccess)
+            e = cudaOccupancyMaxActiveClusters(&scans, small_scan_kernel, &c);
+        if (e != cudaSuccess)
+            cudaGetLastError(); // a failed query only leaves the portable size
+        found[device] = e == cudaSuccess && sorts > 0 && scans > 0 ? 16 : 8;
     }
-    return e;
+    *largest = found[device];
+    return cudaSuccess;
 }
 
 uint32_t small_sort_capacity(uint32_t largest) { return largest * kSortThreads * kSortItems; }

@@ -448,11 +448,11 @@ struct FlushStart
     const uint2* sceneTiles;
 };
 // The scan and the sort of small frames, one cluster each (kernels_small.cu).
-// small_passes_prepare readies them in the current CUDA context and finds the largest
-// cluster they can have there (before any stream capture); the scan takes up to
-// kSmallScanSlots slots, the sort up to small_sort_capacity entries.
+// small_passes_init finds the device's largest cluster for them (once per
+// device, before any stream capture); the scan takes up to kSmallScanSlots slots,
+// the sort up to small_sort_capacity entries.
 constexpr uint32_t kSmallScanSlots = 1u << 18;
-cudaError_t small_passes_prepare(uint32_t* largest);
+cudaError_t small_passes_init(int device, uint32_t* largest);
 uint32_t small_sort_capacity(uint32_t largest);
 cudaError_t launch_small_scan(uint32_t largest, uint32_t slots, const uint32_t* counts,
                               uint32_t* offsets, uint32_t* hostTotal, cudaStream_t stream,
