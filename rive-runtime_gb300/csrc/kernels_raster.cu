@@ -4414,11 +4414,12 @@ __device__ __forceinline__ uint32_t raster_index(const uint32_t* __restrict__ or
 // A batch without feathered draws or images takes the plain variant. Of others
 // the binner has marked the tiles that need the extended one (from kSplitTiles
 // tiles on), and each variant is launched over all tiles and leaves the other's at
-// once: the extended ones first, the plain ones as the last of those have started.
-// 64 UI screens take 1154 us of plain raster and 1484 of extended; a batch of 16
-// recorded frames, 9 of them without feathers, 1937 us of extended raster and 1854
-// split. (The extended tiles by persistent CTAs from a list: 1836, but a frame
-// with feathers on most tiles 640 -> 669.)
+// once: the extended ones first, the plain ones taking their places as those run out.
+// 64 UI screens take 1154 us of plain raster and 1484 of extended; 16 recorded frames,
+// 9 of them without feathers, 2027 us a call with one extended launch and 1993 split.
+// (Plain tiles that start before the extended ones have ended save 5 to 11 us of a
+// frame, but would read what they have not waited for; both variants in one kernel
+// take 2018, two streams 2007.)
 #define RIVE_RASTER_KERNELS(NAME, FEATHER)                                                        \
     __global__ void __launch_bounds__(256, RIVE_RASTER_MIN_BLOCKS(FEATHER)) NAME(                 \
         BatchTables B, const TriRecord* __restrict__ tris,                                        \
@@ -4439,9 +4440,7 @@ __global__ void __launch_bounds__(256, RIVE_RASTER_MIN_BLOCKS(true)) raster_exte
 {
     __shared__ RasterShared<4> sh;
     const uint32_t i = raster_index(order);
-    // Past the wait: everything before this launch is complete when the others'
-    // CTAs start.
-    chain_next();
+    chain_next(); // the others' CTAs take their places as these run out
     raster_tile<4, true, true>(B, tris, sortedSlots, ranges, sh, i);
 }
 
@@ -4450,11 +4449,7 @@ __global__ void __launch_bounds__(256, RIVE_RASTER_MIN_BLOCKS(false)) raster_oth
     const TileHead* __restrict__ ranges, const uint32_t* __restrict__ order)
 {
     __shared__ RasterShared<4> sh;
-    raster_tile<4, false, true>(B, tris, sortedSlots, ranges, sh,
-                                order ? order[blockIdx.x] : blockIdx.x);
-    // This grid ends after the extended tiles'.
-    if (blockIdx.x == gridDim.x - 1)
-        chain_wait();
+    raster_tile<4, false, true>(B, tris, sortedSlots, ranges, sh, raster_index(order));
 }
 
 // The feather atlas pass (render_atlas.glsl with the floating-point target
