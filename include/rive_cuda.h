@@ -517,7 +517,7 @@ typedef struct rive_cuda_flush_stats
     uint64_t triangles;
     uint64_t bin_entries;
     uint64_t tiles;
-    uint64_t kernel_launches;
+    uint64_t kernel_launches; /* of this library's kernels (not CUB's scan and sort) */
     uint64_t winding_entries; /* bin entries that are interior-tile windings */
 } rive_cuda_flush_stats;
 int rive_cuda_last_flush_stats(const rive_cuda_context* ctx,

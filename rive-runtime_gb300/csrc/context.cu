@@ -376,6 +376,7 @@ struct rive_cuda_context
     int rasterCtasPerSm = 0; // 0: as many as fit
     bool raster32Ready = false;
     uint32_t smallCluster = 8; // small_passes_init
+    uint32_t launches = 0;     // of the flush being enqueued
     size_t rasterPad[2][2] = {};      // [feather variant][8 or 16 pixel kernel]: padding
     int rasterPadFor[2] = {-1, -1};   // the CTAs-per-SM limit it was found for
     // Stage timing (rive_cuda_set_profiling).
@@ -1161,6 +1162,16 @@ BatchTables write_tables(rive_cuda_context* ctx,
     return B;
 }
 
+// chain_launch, counted for the flush's statistics.
+template <typename... P, typename... A>
+cudaError_t launch(rive_cuda_context* ctx, void (*kernel)(P...), uint32_t ctas, int threads,
+                   size_t smem, cudaStream_t stream, bool overlap, const int* priority,
+                   const A&... args)
+{
+    ++ctx->launches;
+    return chain_launch(kernel, ctas, threads, smem, stream, overlap, priority, args...);
+}
+
 // CTAs of flush_start_kernel: a thread per element, up to four CTAs per SM.
 uint32_t flush_start_blocks(const FlushStart& F)
 {
@@ -1188,7 +1199,7 @@ int enqueue_front(rive_cuda_context* ctx,
     F.tiles = L.tiles;
     F.tileBase = B.tileBase;
     F.sceneTiles = B.sceneTiles;
-    flush_start_kernel<<<flush_start_blocks(F), 256, 0, stream>>>(F);
+    CK(launch(ctx, flush_start_kernel, flush_start_blocks(F), 256, 0, stream, false, nullptr, F));
     // The kernels below follow one another with nothing between, but for the
     // winding grids' passes and fills and the events of stage timing.
     const bool overlap = S.overlap && !L.winding && !L.imageSlots && !ctx->profiling;
@@ -1201,16 +1212,17 @@ int enqueue_front(rive_cuda_context* ctx,
         CK(cudaMemsetAsync(S.gridWinding, 0, (size_t)S.gridCapacity * 4, stream));
         CK(cudaMemsetAsync(S.gridEdge, 0, S.gridCapacity, stream));
         CK(cudaMemsetAsync(S.gridCounters, 0, 8, stream));
-        path_init_kernel<<<(L.paths + 255) / 256, 256, 0, stream>>>(B);
+        CK(launch(ctx, path_init_kernel, (L.paths + 255) / 256, 256, 0, stream, false, nullptr, B));
         if (L.tessSpans)
-            path_bounds_kernel<<<(L.tessSpans + 255) / 256, 256, 0, stream>>>(B);
-        path_alloc_kernel<<<(L.paths + 255) / 256, 256, 0, stream>>>(B);
+            CK(launch(ctx, path_bounds_kernel, (L.tessSpans + 255) / 256, 256, 0, stream, false,
+                      nullptr, B));
+        CK(launch(ctx, path_alloc_kernel, (L.paths + 255) / 256, 256, 0, stream, false, nullptr, B));
     }
     const bool rampsAlone = ctx->profiling || L.rampsAlone();
     if (L.gradSpans && rampsAlone)
     {
         stage_begin(ctx, RIVE_CUDA_STAGE_COLOR_RAMP, stream);
-        CK(chain_launch(color_ramp_kernel, L.gradSpans, 128, 0, stream, overlap, nullptr, B));
+        CK(launch(ctx, color_ramp_kernel, L.gradSpans, 128, 0, stream, overlap, nullptr, B));
         stage_end(ctx, stream);
     }
     if (L.tessSpans)
@@ -1220,14 +1232,14 @@ int enqueue_front(rive_cuda_context* ctx,
         {
             const int log2 =
                 tess_spans_log2(L.tessSpans, (uint64_t)L.tessRows * kTessTextureWidth);
-            CK(chain_launch(L.feather ? tessellate_packed_feather_kernel : tessellate_packed_kernel,
+            CK(launch(ctx, L.feather ? tessellate_packed_feather_kernel : tessellate_packed_kernel,
                             (L.tessSpans + (4u << log2) - 1) / (4u << log2), 128, 0, stream, overlap,
                             nullptr, B, log2));
         }
         else
         {
             const uint32_t ctas = (L.tessSpans * kTessLanes + 255u) / 256u;
-            CK(chain_launch(L.feather ? tessellate_feather_kernel : tessellate_kernel,
+            CK(launch(ctx, L.feather ? tessellate_feather_kernel : tessellate_kernel,
                             ctas + (rampsAlone ? 0u : L.gradSpans), 256, 0, stream, overlap, nullptr,
                             B, ctas));
         }
@@ -1239,7 +1251,7 @@ int enqueue_front(rive_cuda_context* ctx,
         if (L.items[0])
         {
             const bool three = !L.feather && !L.winding && L.items[0] > kFanWarpEach;
-            CK(chain_launch(L.feather   ? patch_setup_feather_kernel
+            CK(launch(ctx, L.feather   ? patch_setup_feather_kernel
                             : L.winding ? patch_setup_winding_kernel
                             : three     ? patch_setup_kernel
                                         : patch_setup_small_kernel,
@@ -1247,29 +1259,31 @@ int enqueue_front(rive_cuda_context* ctx,
                             overlap, nullptr, B, S.tris, S.counts, S.masks));
         }
         if (L.items[1])
-            CK(chain_launch(outer_setup_kernel, (L.items[1] + 3) / 4, 128, 0, stream, overlap,
+            CK(launch(ctx, outer_setup_kernel, (L.items[1] + 3) / 4, 128, 0, stream, overlap,
                             nullptr, B, S.tris, S.counts, S.masks));
         if (L.items[2])
-            CK(chain_launch(interior_setup_kernel, (L.items[2] + 255) / 256, 256, 0, stream, overlap,
+            CK(launch(ctx, interior_setup_kernel, (L.items[2] + 255) / 256, 256, 0, stream, overlap,
                             nullptr, B, S.tris, S.counts, S.masks));
         if (L.items[3])
-            CK(chain_launch(center_setup_kernel, (L.items[3] + 3) / 4, 128, 0, stream, overlap,
+            CK(launch(ctx, center_setup_kernel, (L.items[3] + 3) / 4, 128, 0, stream, overlap,
                             nullptr, B, S.tris, S.counts, S.masks));
         if (L.winding)
         {
             // The deferred fan triangles' winding deltas and edge tiles, then
             // the windings of every path's grid.
-            fan_filter_kernel<<<(L.items[0] * 8u + 255u) / 256u, 256, 0, stream>>>(B, S.tris,
-                                                                                   S.counts, S.masks);
-            path_winding_kernel<<<(L.paths + 7) / 8, 256, 0, stream>>>(B, S.counts);
+            CK(launch(ctx, fan_filter_kernel, (L.items[0] * 8u + 255u) / 256u, 256, 0, stream, false,
+                      nullptr, B, S.tris, S.counts, S.masks));
+            CK(launch(ctx, path_winding_kernel, (L.paths + 7) / 8, 256, 0, stream, false, nullptr, B,
+                      S.counts));
         }
         if (L.wide)
-            CK(chain_launch(wide_count_kernel, kWideBlocks, 256, 0, stream, overlap, nullptr, B,
+            CK(launch(ctx, wide_count_kernel, kWideBlocks, 256, 0, stream, overlap, nullptr, B,
                             S.tris, S.counts));
         stage_end(ctx, stream);
         stage_begin(ctx, RIVE_CUDA_STAGE_BIN, stream);
         if (L.slots <= kSmallScanSlots)
         {
+            ++ctx->launches;
             CK(launch_small_scan(ctx->smallCluster, L.slots, S.counts, S.offsets, hostTotal, stream,
                                  overlap));
         }
@@ -1383,12 +1397,12 @@ int launch_raster(rive_cuda_context* ctx,
     if (L.tileLog2 == 3)
     {
         const size_t dyn = ctx->rasterCtasPerSm > 0 ? ctx->rasterPad[L.feather][0] : 0;
-        CK(chain_launch(L.feather ? raster_tile8_feather_kernel : raster_tile8_kernel, L.mainTiles,
+        CK(launch(ctx, L.feather ? raster_tile8_feather_kernel : raster_tile8_kernel, L.mainTiles,
                          64, dyn, stream, overlap, priority, B, tris, sortedSlots, ranges));
     }
     else if (L.tileLog2 == 5)
     {
-        CK(chain_launch(L.feather ? raster_tile32_feather_kernel : raster_tile32_kernel,
+        CK(launch(ctx, L.feather ? raster_tile32_feather_kernel : raster_tile32_kernel,
                          L.mainTiles, 1024, kRaster32SmemBytes, stream, overlap, priority, B, tris,
                          sortedSlots, ranges));
     }
@@ -1398,8 +1412,8 @@ int launch_raster(rive_cuda_context* ctx,
         const uint32_t* order = nullptr;
         if (S.qKeys)
         {
-            tile_order_keys_kernel<<<(L.mainTiles + 255) / 256, 256, 0, stream>>>(
-                L.mainTiles, ranges, S.qKeys, S.qVals);
+            CK(launch(ctx, tile_order_keys_kernel, (L.mainTiles + 255) / 256, 256, 0, stream, false,
+                      nullptr, L.mainTiles, ranges, S.qKeys, S.qVals));
             cub::DoubleBuffer<uint32_t> k(S.qKeys, S.qKeysAlt), v(S.qVals, S.qValsAlt);
             size_t tb = S.qTempBytes;
             CK(cub::DeviceRadixSort::SortPairs(S.qTemp, tb, k, v, (int)L.mainTiles, 0, 32, stream));
@@ -1408,21 +1422,21 @@ int launch_raster(rive_cuda_context* ctx,
         }
         else if (S.order && (S.heaviestFirst || orders_tiles(L, entries)))
         {
-            CK(chain_launch(tile_order_kernel, 1, 1024, 0, stream, overlap, nullptr, L.mainTiles,
+            CK(launch(ctx, tile_order_kernel, 1, 1024, 0, stream, overlap, nullptr, L.mainTiles,
                             ranges, S.order));
             order = S.order;
         }
         if (L.splitRaster())
         {
-            CK(chain_launch(raster_extended_kernel, L.mainTiles, 256, dyn, stream, overlap,
+            CK(launch(ctx, raster_extended_kernel, L.mainTiles, 256, dyn, stream, overlap,
                             priority, B, tris, sortedSlots, ranges, order));
             const size_t dyn0 = ctx->rasterCtasPerSm > 0 ? ctx->rasterPad[0][1] : 0;
-            CK(chain_launch(raster_others_kernel, L.mainTiles, 256, dyn0, stream, true, priority, B,
+            CK(launch(ctx, raster_others_kernel, L.mainTiles, 256, dyn0, stream, true, priority, B,
                             tris, sortedSlots, ranges, order));
         }
         else
         {
-            CK(chain_launch(L.feather ? raster_tile_feather_kernel : raster_tile_kernel,
+            CK(launch(ctx, L.feather ? raster_tile_feather_kernel : raster_tile_kernel,
                             L.mainTiles, 256, dyn, stream, overlap, priority, B, tris, sortedSlots,
                             ranges, order));
         }
@@ -1471,35 +1485,35 @@ int enqueue_back(rive_cuda_context* ctx,
         {
             uint16_t* keys = (uint16_t*)S.keys;
             if (padded && !smallSort)
-                bin_fill16_kernel<<<(entries + 255) / 256, 256, 0, stream>>>(
-                    S.offsets + L.slots, entries, L.tiles, keys);
+                CK(launch(ctx, bin_fill16_kernel, (entries + 255) / 256, 256, 0, stream, false,
+                          nullptr, S.offsets + L.slots, entries, L.tiles, keys));
             if (extended.heads)
-                bin_scatter16_extended_kernel<<<binBlocks, 256, 0, stream>>>(
-                    L.slots, L.tileLog2, B.sceneTiles, S.tris, S.counts, S.masks, S.offsets,
-                    entries, binError, keys, S.vals, wide, extended);
+                CK(launch(ctx, bin_scatter16_extended_kernel, binBlocks, 256, 0, stream, false,
+                          nullptr, L.slots, L.tileLog2, B.sceneTiles, S.tris, S.counts, S.masks,
+                          S.offsets, entries, binError, keys, S.vals, wide, extended));
             else
-                bin_scatter16_kernel<<<binBlocks, 256, 0, stream>>>(
-                    L.slots, L.tileLog2, B.sceneTiles, S.tris, S.counts, S.masks, S.offsets,
-                    entries, binError, keys, S.vals, wide);
+                CK(launch(ctx, bin_scatter16_kernel, binBlocks, 256, 0, stream, false, nullptr,
+                          L.slots, L.tileLog2, B.sceneTiles, S.tris, S.counts, S.masks, S.offsets,
+                          entries, binError, keys, S.vals, wide));
         }
         else
         {
             uint32_t* keys = (uint32_t*)S.keys;
             if (padded)
-                bin_fill_kernel<<<(entries + 255) / 256, 256, 0, stream>>>(
-                    S.offsets + L.slots, entries, L.tiles, keys);
+                CK(launch(ctx, bin_fill_kernel, (entries + 255) / 256, 256, 0, stream, false,
+                          nullptr, S.offsets + L.slots, entries, L.tiles, keys));
             if (L.winding)
-                bin_scatter_winding_kernel<<<(L.slots + 255) / 256, 256, 0, stream>>>(
-                    B, S.tris, S.counts, S.masks, S.offsets, L.slots, entries, binError, keys,
-                    S.vals);
+                CK(launch(ctx, bin_scatter_winding_kernel, (L.slots + 255) / 256, 256, 0, stream,
+                          false, nullptr, B, S.tris, S.counts, S.masks, S.offsets, L.slots, entries,
+                          binError, keys, S.vals));
             else if (extended.heads)
-                bin_scatter_extended_kernel<<<binBlocks, 256, 0, stream>>>(
-                    L.slots, L.tileLog2, B.sceneTiles, S.tris, S.counts, S.masks, S.offsets, entries,
-                    binError, keys, S.vals, wide, extended);
+                CK(launch(ctx, bin_scatter_extended_kernel, binBlocks, 256, 0, stream, false,
+                          nullptr, L.slots, L.tileLog2, B.sceneTiles, S.tris, S.counts, S.masks,
+                          S.offsets, entries, binError, keys, S.vals, wide, extended));
             else
-                bin_scatter_kernel<<<binBlocks, 256, 0, stream>>>(
-                    L.slots, L.tileLog2, B.sceneTiles, S.tris, S.counts, S.masks, S.offsets, entries,
-                    binError, keys, S.vals, wide);
+                CK(launch(ctx, bin_scatter_kernel, binBlocks, 256, 0, stream, false, nullptr,
+                          L.slots, L.tileLog2, B.sceneTiles, S.tris, S.counts, S.masks, S.offsets,
+                          entries, binError, keys, S.vals, wide));
         }
         stage_end(ctx, stream);
         cub::DoubleBuffer<uint32_t> v(S.vals, S.valsAlt);
@@ -1508,6 +1522,7 @@ int enqueue_back(rive_cuda_context* ctx,
         if (smallSort)
         {
             // Also writes the ranges, or leaves them empty on overflow.
+            ++ctx->launches;
             CK(launch_small_sort(ctx->smallCluster, entries, S.offsets + L.slots, guarded, L.endBit(),
                                  (const uint16_t*)S.keys, S.vals, S.valsAlt, S.ranges, stream,
                                  overlap));
@@ -1518,24 +1533,23 @@ int enqueue_back(rive_cuda_context* ctx,
             cub::DoubleBuffer<uint16_t> k((uint16_t*)S.keys, (uint16_t*)S.keysAlt);
             CK(cub::DeviceRadixSort::SortPairs(S.sortTemp, tempBytes, k, v, (int)entries, 0,
                                                L.endBit(), stream));
-            tile_ranges16_kernel<<<(entries + 2047) / 2048, 256, 0, stream>>>(entries, L.tiles,
-                                                                          k.Current(), S.ranges);
+            CK(launch(ctx, tile_ranges16_kernel, (entries + 2047) / 2048, 256, 0, stream, false,
+                      nullptr, entries, L.tiles, k.Current(), S.ranges));
         }
         else
         {
             cub::DoubleBuffer<uint32_t> k((uint32_t*)S.keys, (uint32_t*)S.keysAlt);
             CK(cub::DeviceRadixSort::SortPairs(S.sortTemp, tempBytes, k, v, (int)entries, 0,
                                                L.endBit(), stream));
-            tile_ranges_kernel<<<(entries + 1023) / 1024, 256, 0, stream>>>(entries, L.tiles,
-                                                                        k.Current(), S.ranges);
+            CK(launch(ctx, tile_ranges_kernel, (entries + 1023) / 1024, 256, 0, stream, false, nullptr,
+                      entries, L.tiles, k.Current(), S.ranges));
         }
         // A speculative pass whose total did not fit: every range emptied,
         // so the raster leaves the target as it was (or clears it) until the
         // back half runs again with exact bins.
         if (guarded && !smallSort)
-            ranges_guard_kernel<<<(L.tiles + 255) / 256, 256, 0, stream>>>(S.offsets + L.slots,
-                                                                          entries, S.ranges,
-                                                                          L.tiles);
+            CK(launch(ctx, ranges_guard_kernel, (L.tiles + 255) / 256, 256, 0, stream, false, nullptr,
+                      S.offsets + L.slots, entries, S.ranges, L.tiles));
         stage_end(ctx, stream);
         sortedSlots = v.Current();
     }
@@ -1545,13 +1559,13 @@ int enqueue_back(rive_cuda_context* ctx,
         // The feather atlases first: the main raster's blits sample them.
         const uint32_t atlasTiles = L.tiles - L.mainTiles;
         if (L.tileLog2 == 3)
-            CK(chain_launch(raster_atlas8_kernel, atlasTiles, 64, 0, stream, overlap, nullptr, B,
+            CK(launch(ctx, raster_atlas8_kernel, atlasTiles, 64, 0, stream, overlap, nullptr, B,
                             S.tris, sortedSlots, S.ranges, L.mainTiles));
         else if (L.tileLog2 == 5)
-            CK(chain_launch(raster_atlas32_kernel, atlasTiles, 1024, kRaster32SmemBytes, stream,
+            CK(launch(ctx, raster_atlas32_kernel, atlasTiles, 1024, kRaster32SmemBytes, stream,
                             overlap, nullptr, B, S.tris, sortedSlots, S.ranges, L.mainTiles));
         else
-            CK(chain_launch(raster_atlas_kernel, atlasTiles, 256, 0, stream, overlap, nullptr, B,
+            CK(launch(ctx, raster_atlas_kernel, atlasTiles, 256, 0, stream, overlap, nullptr, B,
                             S.tris, sortedSlots, S.ranges, L.mainTiles));
     }
     if (ctx->rasterWait)
@@ -1666,7 +1680,11 @@ int settle_pending(rive_cuda_context* ctx)
         S.binError = nullptr;
         int rc = reserve_bins(ctx, p->L, total, S);
         if (!rc)
+        {
+            ctx->launches = (uint32_t)ctx->stats.kernel_launches;
             rc = enqueue_back(ctx, p->L, p->B, S, total, false, p->stream);
+            ctx->stats.kernel_launches = ctx->launches;
+        }
         if (!rc && ctx->lastDone)
         {
             CK(cudaEventRecord(ctx->lastDone, p->stream));
@@ -1804,6 +1822,7 @@ int run_batch_body(rive_cuda_context* ctx,
     // back too).
     const bool speculates =
         speculative && ctx->speculate && n == 1 && L.slots && !L.winding && ctx->binHighWater;
+    ctx->launches = 0;
     rc = enqueue_front(ctx, L, B, S, stream, speculates ? ctx->hSpecTotal : ctx->hPairs);
     if (rc)
         return rc;
@@ -1839,10 +1858,7 @@ int run_batch_body(rive_cuda_context* ctx,
         ctx->stats.bin_entries = 0; // known when the flush settles
         ctx->stats.winding_entries = 0;
         ctx->stats.tiles = L.tiles;
-        ctx->stats.kernel_launches = 1 + (L.gradSpans && L.rampsAlone() ? 1 : 0) +
-                                 (L.tessSpans ? 1 : 0) + 1 + 5 +
-                                     (L.wide ? 1 : 0) +
-                                     1 + (L.tiles > L.mainTiles ? 1 : 0);
+        ctx->stats.kernel_launches = ctx->launches;
         return RIVE_CUDA_OK;
     }
     uint32_t pairs = 0, windingEntries = 0;
@@ -1877,11 +1893,7 @@ int run_batch_body(rive_cuda_context* ctx,
     ctx->stats.bin_entries = pairs;
     ctx->stats.winding_entries = windingEntries;
     ctx->stats.tiles = L.tiles;
-    ctx->stats.kernel_launches = 1 + (L.gradSpans && L.rampsAlone() ? 1 : 0) +
-                                 (L.tessSpans ? 1 : 0) +
-                                 (L.slots ? 1 + (L.wide ? 1 : 0) : 0) + (pairs ? 3 : 0) + 1 +
-                                 (L.tiles > L.mainTiles ? 1 : 0) +
-                                 (L.winding ? 3 + (L.tessSpans ? 1 : 0) + 1 : 0);
+    ctx->stats.kernel_launches = ctx->launches;
     return RIVE_CUDA_OK;
 }
 
@@ -2559,6 +2571,7 @@ int graph_build(rive_cuda_context* ctx,
         ctx->profiling = profiling;
         return rc;
     }
+    ctx->launches = 0; // the captured ones, not the sizing run's
     cudaError_t e = cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess)
     {
@@ -2577,9 +2590,7 @@ int graph_build(rive_cuda_context* ctx,
     g->stats.triangles = L.slots;
     g->stats.bin_entries = g->measured;
     g->stats.tiles = L.tiles;
-    g->stats.kernel_launches = 1 + (L.gradSpans && L.rampsAlone() ? 1 : 0) +
-                                 (L.tessSpans ? 1 : 0) +
-                               (L.slots ? 2 + (L.wide ? 1 : 0) : 0) + (capacity ? 4 : 0) + 1;
+    g->stats.kernel_launches = ctx->launches;
     return RIVE_CUDA_OK;
 }
 } // namespace

@@ -169,3 +169,42 @@ def test_noalloc_in_a_second_cuda_context(name):
         call("cuCtxDestroy_v2", old)
     assert np.array_equal(got, first.cpu().numpy())
     parity(got, oracle.render(cap))
+
+
+@pytest.mark.gpu
+def test_kernel_launches_are_counted():
+    """flush_stats.kernel_launches: the library's own kernels of the last flush,
+    where a setting or a size adds one."""
+    import torch
+    from rive_runtime_gb300 import rive_cuda
+    ctx = rive_cuda.Context(0)
+    ctx.set_bin_speculation(False)
+
+    def launches(cap):
+        ctx.render(cap)
+        return ctx.stats()["kernel_launches"]
+
+    small = load_golden("strokes_s3")[0]  # with gradients, 256 tiles
+    # Preparation, tessellation with ramps, set-up, scan, binner, sort, raster.
+    assert launches(small) == 7
+    bufs, keep = device_buffers(small)
+    target = torch.zeros((small.height, small.width, 4), dtype=torch.uint8, device="cuda")
+    graph = ctx.graph([(small.flushes[0], bufs, target.data_ptr())])
+    assert graph.stats()["kernel_launches"] == 7
+    graph.close()
+    ctx.set_raster_queue(True)
+    assert launches(small) == 8  # and the tiles' order
+    ctx.set_raster_queue(False)
+    ctx.set_profiling(True)
+    assert launches(small) == 8  # and the ramps by themselves
+    ctx.set_profiling(False)
+    ctx.set_bin_speculation(True)
+    assert launches(small) == 7
+    ctx.set_bin_speculation(False)
+    # 15,645 tiles: set-up passes of fans, center-AA fans, triangles; the wide
+    # triangles' count; the atlas; two rasters.
+    large = load_golden("silver_bankcard_f10")[0]
+    split = launches(large)
+    ctx.set_raster_config(32)
+    assert launches(large) == split - 1
+    ctx.close()
