@@ -219,7 +219,16 @@ typedef struct rive_cuda_flush_desc
 
 typedef struct rive_cuda_context rive_cuda_context;
 
-/* Creates a context bound to CUDA device `device`. */
+/*
+ * Creates a context bound to CUDA device `device`.
+ *
+ * The context's own stream has the device's highest stream priority: its
+ * kernels start before those that the caller has waiting on streams of lower
+ * priority, kernels that run already go on. On it, rasters of more than 760
+ * tiles and of at most 2^22 triangle slots (24 a patch) have the lowest one, so
+ * that they give way to the short passes of other contexts. A flush on a
+ * caller's stream runs at that stream's priority.
+ */
 int rive_cuda_context_create(int device, rive_cuda_context** out_ctx);
 void rive_cuda_context_destroy(rive_cuda_context* ctx);
 
@@ -409,6 +418,8 @@ int rive_cuda_flush_batch(rive_cuda_context* ctx,
  * rive_cuda_graph_check (waits for the stream) returns as
  * RIVE_CUDA_ERR_DEVICE_STATUS. Launches on one graph must not overlap in
  * time (they share its intermediates); NULL stream: the graph's own stream.
+ * That stream has the device's highest priority; on another one the graph
+ * runs at its priority.
  */
 typedef struct rive_cuda_graph rive_cuda_graph;
 int rive_cuda_graph_create(rive_cuda_context* ctx,
@@ -599,8 +610,11 @@ int rive_cuda_get_bin_speculation(const rive_cuda_context* ctx, int* enabled);
  */
 enum
 {
-    RIVE_CUDA_STAGE_COLOR_RAMP = 0,  /* color_ramp_kernel (when timed)    */
-    RIVE_CUDA_STAGE_TESSELLATE = 1,  /* tessellate_kernel                 */
+    RIVE_CUDA_STAGE_COLOR_RAMP = 0,  /* color_ramp_kernel; while stages are
+                                        not timed, flushes of 1 to 16,383
+                                        tessellation spans make the ramps in
+                                        tessellate_kernel's launch       */
+    RIVE_CUDA_STAGE_TESSELLATE = 1,  /* tessellate(_packed)_kernel        */
     RIVE_CUDA_STAGE_PATCH_SETUP = 2, /* patch_setup_kernel                */
     RIVE_CUDA_STAGE_BIN = 3,         /* scan + bin_scatter_kernel         */
     RIVE_CUDA_STAGE_SORT = 4,        /* radix sort + tile_ranges_kernel   */
