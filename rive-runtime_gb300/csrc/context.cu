@@ -319,7 +319,7 @@ struct rive_cuda_context
     // The context's stream runs at the device's highest priority and its rasters
     // at the lowest: the short passes of another context's flush, whose
     // bin-entry total its host thread waits for, go ahead of the CTAs that a
-    // raster still has to start.
+    // raster still has to start. (Stated at rive_cuda_context_create.)
     int streamPriority = 0, rasterPriority = 0;
     cudaStream_t copyStream = nullptr; // record uploads (rive_cuda_unmap_buffer)
     cudaStream_t readStream = nullptr; // asynchronous read-backs of targets

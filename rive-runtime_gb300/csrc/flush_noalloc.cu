@@ -2,8 +2,9 @@
 // small frame whose every intermediate (tessellation and gradient textures,
 // triangle records, tile bins, scan/sort temporaries, status words) lives in
 // one fixed, file-scope device pool. The call allocates nothing: no
-// cudaMalloc/cudaFree, no allocating library routine. It launches the same
-// kernels, in the same order, as rive_cuda_flush_device.
+// cudaMalloc/cudaFree, no allocating library routine. Its kernels are those of a
+// rive_cuda_flush_device of a small frame, in the same order; its tiles are
+// rendered as they come.
 //
 // The pool is one per device and per process, so calls that overlap in time
 // (two host threads, or two streams of one device) race on it.

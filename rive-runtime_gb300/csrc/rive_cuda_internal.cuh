@@ -367,10 +367,10 @@ struct BatchTables
     float4* featherPlanes;
     // Image meshes of the batch (PatchSegment::mesh indexes it).
     const MeshDesc* meshes;
-    // Triangles whose tile box holds more than kWideTiles tiles: wide[0] of
+    // Triangles whose tile box holds more than wideTiles tiles: wide[0] of
     // them (at most wideCap are kept), slots from wide[1] on, and per kept
-    // triangle the entries of each of its kWideStrips strips. Null: no such
-    // triangle is set aside (no scene has that many tiles, or winding records).
+    // triangle the entries of each of its kWideStrips strips. Null: none is set
+    // aside (no scene has more than kWideTiles tiles, or winding records).
     uint32_t* wide;
     uint32_t* wideStrips;
     uint32_t wideCap, wideTiles;
