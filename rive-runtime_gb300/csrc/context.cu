@@ -1362,11 +1362,15 @@ int prepare_raster(rive_cuda_context* ctx)
 }
 
 // Whether the 16-pixel grid takes its tiles heaviest first without being asked:
-// from about one wave of CTAs (760) to what one CTA can order, and where a tile
-// is long enough for the last ones to leave the GPU half empty. 3072 tiles of
-// 2366 entries: raster 737 -> 634 us; 16384 tiles of 450: 3.76 -> 3.57 ms; 1024
-// tiles of 610: no difference; UI screens (9 to 13 entries a tile) would pay the
-// order's 7 to 24 us for nothing.
+// from about one wave of CTAs (760) on, up to what one CTA orders quickly, and where a
+// tile is long enough for the last ones to leave the GPU half empty. Raster with the
+// order and without, full-feature frames: 256 tiles of 2,007 entries 135 us and 135,
+// 625 of 2,193 209 and 214, 1,024 of 2,197 259 and 310, 4,096 of 2,527 878 and 966,
+// 4,096 of 280 120 and 159, 16,384 of 527 (four flushes) 3,700 and 3,856; plain fills:
+// 1,936 tiles of 95 entries 60 and 67, 3,969 of 532 552 and 600. UI screens pay the
+// order's 7 to 24 us for nothing: 8,160 tiles of 11 entries 76 and 64, 9,275 of 82,
+// just above the line, 134 and 123. Above kOrderTiles the order's radix sort takes what
+// the order gives: 24,450 tiles of a full-feature frame 6.07 ms with it, 6.01 without.
 bool orders_tiles(const BatchLayout& L, uint32_t entries)
 {
     return L.tileLog2 == 4 && L.mainTiles >= kOrderMinTiles && L.mainTiles <= kOrderTiles &&
@@ -1388,10 +1392,11 @@ int launch_raster(rive_cuda_context* ctx,
                   cudaStream_t stream)
 {
     // Behind other streams' short passes, where it has more CTAs than start at
-    // once (760) and the passes are short: up to four million slots (16 recorded
-    // frames in turn with another context's 2.10 -> 2.03 ms, a 1080x1080 feathered
-    // frame 102 -> 86 us; above, a front half fills the GPU by itself: 1024x1024
-    // strokes, 4.4 M slots, 1.18 -> 1.20 ms).
+    // once (760) and the passes are short: up to four million slots (in
+    // turn with two other contexts' calls, with it and without: 16 recorded frames 2.00
+    // and 2.17 ms, a 1080x1080 feathered frame 68 and 89 us, a 1080x1920 UI screen 81 and
+    // 91, 64 UI screens, 4.1 M slots, 1.37 and 1.40 ms; above, a front half fills the
+    // GPU by itself: 1024x1024 strokes, 4.4 M slots, 1.00 and 0.99 ms).
     const bool behind = S.ownStream && L.mainTiles > 760 && L.slots <= 1u << 22;
     const int* priority = behind ? &ctx->rasterPriority : nullptr;
     if (L.tileLog2 == 3)

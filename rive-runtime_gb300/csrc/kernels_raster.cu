@@ -1475,11 +1475,10 @@ __device__ __forceinline__ void patch_setup(const BatchTables& B,
 // positions and coverages are the same bits as vertex by vertex; a patch that is
 // not of one contour takes that way (fan_setup_one).
 // Then the triangles of the three patches that draw (about half) are packed, so
-// that records and tile tests run on full warps. Bound by issue slots. The set-up
-// took 0.96 ms for the vertices of the full-feature 2048x2048 frame's 1.9 M patches
-// with a warp's 32 lanes on one patch's 32 ramp vertices; with three patches
-// 2016 -> 1660 us in all, 1404 with the triangles packed; 20 plain canvases
-// (653 k patches of large triangles) 897 -> 673, strokes 220 -> 164.
+// that records and tile tests run on full warps. Bound by issue slots. Set-up with a
+// warp per patch (patch_setup_small_kernel) and with this: full-feature 2048x2048
+// frame (1.9 M patches) 2,054 and 1,417 us, 20 plain canvases (655 k patches of large
+// triangles) 889 and 673, 1024x1024 strokes 220 and 165, 64 UI screens 184 and 124.
 constexpr int kSpokes = kPatchSegmentSpan + 1;              // 9
 constexpr int kFanVertices = 2 * kSpokes + 1;               // 19: (spoke, outset), midpoint
 constexpr int kFanPatches = 3;                              // patches a warp shades at once
@@ -1985,7 +1984,8 @@ __device__ __forceinline__ void fan_setup(const BatchTables& B,
 }
 
 // Resident 128-thread CTAs per SM the midpoint-fan set-up's registers are
-// bounded for (20 plain canvases 691, 684, 708 and 750 us at 7, 8, 9 and 10).
+// bounded for: at 7, 8, 9 and 10 20 plain canvases' set-up takes 687, 674, 704 and 747
+// us, the full-feature 2048x2048 frame's 1.48, 1.42, 1.52 and 1.61 ms.
 #ifndef RIVE_SETUP_MIN_BLOCKS
 #define RIVE_SETUP_MIN_BLOCKS 8
 #endif
@@ -1998,7 +1998,8 @@ __global__ void __launch_bounds__(128, RIVE_SETUP_MIN_BLOCKS) patch_setup_kernel
 
 // A warp per patch, for flushes of at most kFanWarpEach patches: bound by the
 // latency of one warp's chain, which three patches lengthen (1080x1920 UI
-// screen's set-up 17 us, 19 with three).
+// screen, 6,232 patches: set-up 18 us, 22 with three; four 800x600 screens, 12,318: 24
+// and 22).
 __global__ void __launch_bounds__(128) patch_setup_small_kernel(BatchTables B,
                                                                 TriRecord* __restrict__ tris,
                                                                 uint32_t* __restrict__ tileCounts,
@@ -2671,9 +2672,7 @@ __device__ __forceinline__ void bin_scatter(const BatchTables* __restrict__ Bw,
     if (first >= slotCount)
         return;
     const uint32_t mySlot = lane < wide.perWarp ? first + lane : slotCount;
-    // (Also where there is nothing to write: loads that do not wait for the count.
-    // With the mask walk's division below: scan and binner of the full-feature
-    // 2048x2048 frame 867 -> 758 us.)
+    // (Also where there is nothing to write: loads that do not wait for the count.)
     uint32_t myCount = 0, myOffset = 0, myMask = 0;
     if (mySlot < slotCount)
     {
@@ -2809,9 +2808,9 @@ __device__ __forceinline__ void bin_scatter(const BatchTables* __restrict__ Bw,
 }
 
 // Resident 256-thread CTAs per SM the binner's registers are bounded for. It
-// waits for its scattered loads, so more warps win over a few spilled
-// registers: scan and binner of the full-feature 2048x2048 frame 1.06, 0.96 and
-// 0.85 ms at 5, 6 and 8 CTAs.
+// waits for its scattered loads, so more warps win over the 32 registers' spills (124 to
+// 148 bytes a thread): scan and binner of the full-feature 2048x2048 frame 866, 823 and
+// 776 us at 5, 6 and 8 CTAs, of 1024x1024 strokes 117, 113 and 112.
 #ifndef RIVE_BIN_MIN_BLOCKS
 #define RIVE_BIN_MIN_BLOCKS 8
 #endif
@@ -2876,9 +2875,8 @@ __global__ void __launch_bounds__(256) ranges_guard_kernel(const uint32_t* __res
 // Where each tile's entries start and end in the sorted keys. A thread takes the
 // 16 bytes of one load (4 or 8 keys); its neighbours' keys come from their lanes.
 // The keys are sorted, so when the one before and the one after are equal there
-// is nothing to say. (One key a thread, with its neighbours loaded: 37 us for
-// 10.9 M entries of 16,384 tiles; now 7.3 M entries of 3,072 tiles
-// take 6 to 7 us, 2 bytes each.)
+// is nothing to say. Bound by the keys' bytes: 8.6 M entries of 16,384 tiles, 2 bytes
+// each, take 9 us.
 template <typename K>
 __device__ __forceinline__ void tile_ranges(uint32_t pairCount, uint32_t tileCount,
                                             const K* __restrict__ keys, TileHead* __restrict__ ranges)
@@ -3528,8 +3526,8 @@ __device__ __noinline__ void image_modulate(const FlushParams& P, uint32_t pathI
 // paint's colour is 0 unless that colour is not finite. A solid colour is bytes; a
 // gradient's texel is finite unless its row, or the place of a one-texel ramp, is not or
 // overflows as it becomes texels. An image's is sampled and decides for itself. (Tested
-// here and not as a triangle is set up, which costs more: 20 plain canvases 8.13 -> 8.15
-// ms against 8.24, strokes 984 -> 987 us against 1013.)
+// here and not as a triangle is set up: 20 plain canvases 8.15 ms against 8.24, strokes
+// 987 us against 1,013.)
 __device__ __forceinline__ bool paint_vanishes(const FlushParams& P, uint32_t paintX,
                                                uint32_t paintY, uint32_t pathID, uint32_t features)
 {
@@ -3901,9 +3899,10 @@ __device__ __noinline__ float feathered_fragment(const float4* __restrict__ plan
 }
 
 // Resident CTAs per SM the register allocation is bounded for (16x16 tiles): 5
-// (48 registers; 4 and 6 were slower everywhere, 64 UI screens by 11% with 4), with
-// the feather paths 4 (64 registers; raster of 16 recorded frames 1.84 ms, 1.94 with
-// 3 and 1.89 with 5).
+// (48 registers, 108 bytes spilled), with the feather paths 4 (64 registers, 140 bytes).
+// Raster at 4, 5 and 6: 64 UI screens 1,150, 1,147 and 1,288 us, 20 plain canvases 6.27,
+// 6.63 and 7.53 ms, the full-feature 2048x2048 frame 3.61, 3.70 and 4.18 ms. With feathers
+// at 3, 4 and 5: a 1080x1080 recorded frame 43, 40 and 42 us.
 #define RIVE_RASTER_MIN_BLOCKS(FEATHER) ((FEATHER) ? 4 : 5)
 
 // Tile geometry: a CTA of T x T threads, one per pixel; warp w owns the 8x4
@@ -4269,8 +4268,7 @@ __device__ __forceinline__ void raster_tile(const BatchTables& B,
                 // in primitive order, so when the stream moves to another path
                 // every pixel still holding the previous path's coverage has
                 // seen all of it: resolve them together. (Inlined here and at
-                // the tile's end: out of line it cost 8% of the 20 plain
-                // canvases' frame time, and one shared site 1%.)
+                // the tile's end: out of line it keeps the planes in memory.)
                 if (moves & rest & (0u - rest))
                 {
                     if (pendMeta)
@@ -4408,15 +4406,14 @@ __device__ __forceinline__ uint32_t raster_index(const uint32_t* __restrict__ or
 // The raster kernels, each without and with the feather paths. The 16x16 ones
 // take their tiles in the order of `order` (heaviest first), or as they come when
 // it is null. The hardware hands out CTAs in turn, so an ordered grid is the work
-// queue: a persistent grid with an atomic cursor over the same order was slower
-// (full-feature 2048x2048 frame 3.70 against 3.57 ms).
+// queue.
 //
 // A batch without feathered draws or images takes the plain variant. Of others
 // the binner has marked the tiles that need the extended one (from kSplitTiles
 // tiles on), and each variant is launched over all tiles and leaves the other's at
 // once: the extended ones first, the plain ones taking their places as those run out.
-// 64 UI screens take 1154 us of plain raster and 1484 of extended; 16 recorded frames,
-// 9 of them without feathers, 2027 us a call with one extended launch and 1993 split.
+// 16 recorded frames, 9 of them without feathers, take 2,026 us a call with one extended
+// launch and 1,995 split.
 // (Plain tiles that start before the extended ones have ended save 5 to 11 us of a
 // frame, but would read what they have not waited for; both variants in one kernel
 // take 2018, two streams 2007.)
@@ -4594,8 +4591,8 @@ __global__ void __launch_bounds__(1024) raster_atlas32_kernel(
 // eighth: one CTA counts them into 256 buckets (the leading four bits of a
 // tile's bin entries and their exponent, descending), per warp so that equal
 // tiles do not queue at one counter, and gives each its place. Bound by
-// latency and by equal buckets' atomics: 7 us for 3,072 tiles, 24 for 16,384, against 45
-// us for a radix sort of those.
+// latency and by equal buckets' atomics: 7 us for 3,072 tiles, 12 for 8,160, 22 for
+// 16,384.
 __global__ void __launch_bounds__(1024, 1) tile_order_kernel(uint32_t tiles,
                                                              const TileHead* __restrict__ ranges,
                                                              uint32_t* __restrict__ order)

@@ -766,9 +766,8 @@ static_assert(sizeof(PackedSpan) == 160, "PackedSpan layout");
 // are dealt out to the lanes, first those between a span's ends or within a round
 // join (a search for the parametric segment, a root and an arc tangent each), then
 // the rest (a point, an angle from the set-up), so that lanes run the same code.
-// With 8 lanes per span 13 of 32 lanes were at work on 1024x1024 strokes: 129 -> 104
-// us with this, 72 with turned_less and the ends' angles from the set-up;
-// full-feature 2048x2048 frame 578 -> 482 -> 344 us, 64 UI screens 60 -> 42 -> 36.
+// With 16 lanes a span and with this: 1024x1024 strokes 144 and 72 us, full-feature
+// 1021x767 133 and 65, 64 UI screens 138 and 35.
 template <bool kFeather>
 __device__ __forceinline__ void tessellate_packed(const BatchTables& B, int spansLog2)
 {
@@ -847,8 +846,8 @@ __global__ void __launch_bounds__(128) color_ramp_kernel(BatchTables B)
 
 // tessCtas CTAs of tessellation, then one for each gradient span: the two passes
 // depend on nothing of each other's, and one launch less is 2 us of a small frame
-// (240x180 widget 43 -> 41 us). Not in the packed launches, whose frames are long
-// (full-feature 1021x767 1158 -> 1167 us). The feather variants with feathered-fill
+// (240x180 widget 44 us with two, 41 with one; 1080x1920 UI screen 82 and 81). Not in
+// the packed launches, whose frames are long. The feather variants with feathered-fill
 // softening and feather-join texels.
 __global__ void __launch_bounds__(256) tessellate_kernel(BatchTables B, uint32_t tessCtas)
 {

@@ -293,15 +293,17 @@ struct PatchSegment
 
 // Lanes that tessellate one span where spans are few (latency counts), and the
 // most spans a warp takes where they are many (kernels_tess.cu). A 1080x1920 UI
-// screen of 3560 spans 12 us with lanes, 15 packed; 16 recorded frames, 33 k spans,
-// 43 and 35; 64 UI screens, 133 k, 132 and 36.
+// screen of 4.6 k spans 11 us with lanes, 14 packed; 4, 8 and 16 800x600 screens, 10, 16
+// and 36 k spans, 18, 22 and 41 with lanes, 15, 15 and 19 packed, whose colour ramps
+// then need a launch (4 screens' whole call 112 us with lanes, 114 packed; 8: 157 and
+// 147); 16 recorded frames, 33 k, 43 and 35; 64 UI screens, 139 k, 138 and 35.
 constexpr int kTessLanes = 16;
 constexpr int kTessPacked = 16;
 constexpr uint32_t kTessPackedSpans = 16384;
 // Spans a warp takes in the packed tessellation, as a power of two: 8, or 16 where
 // eight spans' vertices (half their texels) would not give every lane two and there
 // are warps enough (64 UI screens, 10 texels a span, 36 us with 16 and 43 with 8;
-// strokes, 16 texels, 79 and 72; 33 k spans of 13 texels 41 and 35).
+// strokes, 16 texels, 77 and 73; 16 recorded frames, 33 k spans of 13 texels, 41 and 35).
 inline int tess_spans_log2(uint32_t spans, uint64_t texels)
 {
     return spans >= 1u << 16 && texels < (uint64_t)spans * 12 ? 4 : 3;
@@ -309,21 +311,21 @@ inline int tess_spans_log2(uint32_t spans, uint64_t texels)
 
 // Triangles with large tile boxes. One warp tests a triangle's tiles 32 at a
 // time; a canvas-wide triangle of a backdrop has 8,000 to 65,000 of them, and a
-// patch of such triangles kept its warp busy for hundreds of microseconds while
-// the rest of the GPU was idle (a 1739x2831 recorded frame: set-up 589 us,
-// binner 550 us). Boxes above kWideTiles tiles are therefore set aside and cut
-// into up to kWideStrips strips of at least kWideStripTiles tiles, a warp each.
-// 1080x1920 UI screen with uploads and read-back: 556 -> 368 us; 16 recorded
-// frames alone: 3.71 -> 2.74 ms. The line lies where the two extra passes
-// stop costing batches whose many such triangles fill the GPU anyway (20 plain
-// canvases 10.57, 10.19 and 10.17 ms with it at 256, 512 and 1024 tiles,
-// 10.15 ms without).
+// patch of such triangles keeps its warp busy for hundreds of microseconds while
+// the rest of the GPU is idle. Large boxes are therefore set aside and cut into up
+// to kWideStrips strips of at least kWideStripTiles tiles, a warp each. With and
+// without: set-up and binner of a 1080x1920 UI screen 18 + 24 us, 49 + 146; of 16
+// recorded frames 175 + 71, 419 + 846 (the call alone 2.37 and 3.39 ms). The line of
+// large batches lies where the two extra passes stop costing those whose many such
+// triangles fill the GPU anyway: 20 plain canvases 8.56, 8.17 and 8.15 ms with it
+// at 256, 512 and 1024 tiles, 8.15 ms without.
 constexpr int kWideTiles = 1024;
 // The line of a batch of `slots` triangles, where some scene has more than kWideTiles
 // tiles: lower for small frames, which wait for their longest warp (1080x1080
-// recorded feathered frame: scan and binner 29 -> 22 us, set-up 32 -> 29, the same
-// at 128; a 2370x1680 recorded frame's binner 32 -> 25, 35 at 128; 16 recorded
-// frames, 1.8 M slots, 71 -> 93, so not theirs).
+// recorded feathered frame, 109 k slots: scan and binner 21, 21, 21 and 29 us at 128,
+// 256, 512 and 1024 tiles, the call alone 133, 133, 134 and 145; a 1080x1920 UI screen
+// the same at all four; 16 recorded frames, 1.8 M slots, 161, 94, 71 and 68, so not
+// theirs).
 inline uint32_t wide_tiles(uint32_t slots) { return slots <= 1u << 18 ? 256 : kWideTiles; }
 constexpr int kWideStrips = 64;
 constexpr int kWideStripTiles = 128;
@@ -398,11 +400,12 @@ struct WideScatter
 };
 
 // A small frame's binner waits for its longest warp, one with a backdrop's large
-// triangles one after another: 8 slots a warp, not 32 (1080x1080 recorded feathered
-// frame, 187 k slots: scan and binner 37 -> 29 us, a 240x180 widget 20.5 -> 18.5; 4
-// slots: 30 and 21). Frames of more slots have other warps to run meanwhile.
+// triangles one after another: 8 slots a warp, not 32. Scan and binner at 4, 8, 16
+// and 32: 1080x1080 recorded feathered frame, 109 k slots, 21, 21, 23 and 25 us; 240x180
+// widget 18, 19, 21 and 21; 1080x1920 UI screen, 150 k, 26, 24, 27 and 28. Frames of
+// more slots have other warps to run meanwhile: 16 recorded frames, 1.8 M, 113, 83, 72
+// and 70; full-feature 1021x767, 8.4 M, 392, 242, 173 and 141.
 inline uint32_t bin_slots_per_warp(uint32_t slots) { return slots <= 1u << 18 ? 8 : 32; }
-
 
 struct TileHead;
 // The binner's view of the main tiles that need the raster's extended variant
@@ -415,8 +418,9 @@ struct ExtendedTiles
 };
 constexpr uint32_t kExtendedTile = 1u << 31; // in TileHead::scene
 // Batches are split from this many main tiles on: two launches are slower where a
-// raster is short (4624 tiles of a feathered frame 38.5 -> 39.4 us). Of 15,645 tiles,
-// feathers on some: 313 -> 303 us; of 19,293, feathers on most: 646 -> 653.
+// raster is short (4,624 tiles of a feathered frame 40 us, 44 split) or most of its tiles
+// are extended (19,293 tiles: 647 and 656 us). 15,645 tiles, feathers on some: 312 and
+// 301; 16 recorded frames, the whole call 2,026 and 1,995.
 constexpr uint32_t kSplitTiles = 8192;
 
 // CTAs (256 threads) of the two wide-triangle passes: two per SM's worth, a
@@ -490,10 +494,12 @@ __device__ __forceinline__ void chain_next()
 // Launches a kernel of a flush's chain. With `overlap` (the stream's last
 // operation is a kernel that starts with chain_wait) its CTAs take their places
 // while that one runs out; a small flush is eight kernels of a few microseconds,
-// and a launch after a complete kernel adds one or two to each (240x180 widget 54
-// -> 44 us, 1080x1080 recorded feathered frame 86 -> 69 us; a 1021x767
-// full-feature frame, 8.5 M slots, loses 0.3%, so the host does it for frames of
-// up to kSmallScanSlots). At *priority unless that is null.
+// and a launch after a complete kernel adds one or two to each. With and without,
+// other contexts' calls in the gaps: 240x180 widget 41 and 48 us, 1080x1080 recorded
+// feathered frame 68 and 82; alone 73 and 90, 133 and 153, 1080x1920 UI screen 158 and
+// 173 (81 and 77 among others). The host does it for frames of up to kSmallScanSlots:
+// above, 64 UI screens, 4.1 M slots, lose 1% by it, a full-feature 1021x767 frame, 8.4
+// M, gains 1%. At *priority unless that is null.
 template <typename... P, typename... A>
 cudaError_t chain_launch(void (*kernel)(P...), uint32_t ctas, int threads, size_t smem,
                          cudaStream_t stream, bool overlap, const int* priority, const A&... args)
