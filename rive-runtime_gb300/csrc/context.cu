@@ -323,6 +323,7 @@ struct rive_cuda_context
     int streamPriority = 0, rasterPriority = 0;
     cudaStream_t copyStream = nullptr; // record uploads (rive_cuda_unmap_buffer)
     cudaStream_t readStream = nullptr; // asynchronous read-backs of targets
+    cudaStream_t clearStream = nullptr; // new memory's clears (clear_new)
     bool readsInFlight = false;        // read-backs queued since the last sync
     // Set by rive_cuda_flush for one flush: the raster waits for it (a
     // read-back of the target still in flight), the front half does not.
@@ -1951,6 +1952,18 @@ int run_flush(rive_cuda_context* ctx,
 }
 } // namespace
 
+namespace
+{
+// Zeroes memory just allocated, before it returns. Not on the legacy default stream
+// (cudaMemset), which the context's streams and a caller's non-blocking ones do not wait
+// for: behind other work there, the clear would come after their first use of the memory.
+cudaError_t clear_new(rive_cuda_context* ctx, void* p, size_t bytes)
+{
+    const cudaError_t e = cudaMemsetAsync(p, 0, bytes, ctx->clearStream);
+    return e == cudaSuccess ? cudaStreamSynchronize(ctx->clearStream) : e;
+}
+} // namespace
+
 extern "C" {
 
 int rive_cuda_context_create(int device, rive_cuda_context** out_ctx)
@@ -1972,9 +1985,12 @@ int rive_cuda_context_create(int device, rive_cuda_context** out_ctx)
     if (e == cudaSuccess)
         e = cudaStreamCreateWithFlags(&ctx->readStream, cudaStreamNonBlocking);
     if (e == cudaSuccess)
+        e = cudaStreamCreateWithPriority(&ctx->clearStream, cudaStreamNonBlocking,
+                                         ctx->streamPriority);
+    if (e == cudaSuccess)
         e = cudaMalloc(&ctx->dError, 4);
     if (e == cudaSuccess)
-        e = cudaMemset(ctx->dError, 0, 4);
+        e = clear_new(ctx, ctx->dError, 4);
     if (e == cudaSuccess)
         e = cudaMallocHost(&ctx->hError, 4);
     if (e == cudaSuccess)
@@ -2070,6 +2086,8 @@ void rive_cuda_context_destroy(rive_cuda_context* ctx)
         }
     for (cudaEvent_t e : ctx->eventPool)
         cudaEventDestroy(e);
+    if (ctx->clearStream)
+        cudaStreamDestroy(ctx->clearStream);
     if (ctx->stream)
         cudaStreamDestroy(ctx->stream);
     if (ctx->copyStream)
@@ -2237,7 +2255,7 @@ int rive_cuda_render_target_create(rive_cuda_context* ctx,
         delete t;
         return cuda_fail(ctx, e, "render target alloc");
     }
-    e = cudaMemset(t->pixels, 0, (size_t)width * height * 4);
+    e = clear_new(ctx, t->pixels, (size_t)width * height * 4);
     if (e != cudaSuccess)
     {
         cudaFree(t->pixels);
@@ -2468,7 +2486,7 @@ int graph_build(rive_cuda_context* ctx,
     }
     const size_t scanBytes = scan_temp_bytes(L.slots);
     CK(g->scanTemp.reserve(scanBytes));
-    CK(cudaMemset(g->error.ptr, 0, 4));
+    CK(clear_new(ctx, g->error.ptr, 4));
 
     Scratch S;
     S.ownStream = true;
@@ -2863,7 +2881,7 @@ int rive_cuda_render_buffer_create(rive_cuda_context* ctx,
     // stay inside the allocation.
     cudaError_t e = cudaMalloc(&b->mem, (bytes + 15) & ~(size_t)15);
     if (e == cudaSuccess)
-        e = cudaMemset(b->mem, 0, (bytes + 15) & ~(size_t)15);
+        e = clear_new(ctx, b->mem, (bytes + 15) & ~(size_t)15);
     if (e != cudaSuccess)
     {
         cudaFree(b->mem);

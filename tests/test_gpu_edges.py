@@ -258,3 +258,30 @@ def test_contexts_on_threads_against_the_oracle():
         assert len(got) == 15
         parity(got[0], oracle.render(cap))
         assert all(np.array_equal(g, got[0]) for g in got)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["clips_s13", "image_meshes_s43"])
+def test_new_memory_is_clear_before_it_is_used(name):
+    """Targets and render buffers made and used while the legacy default stream is
+    busy: their clears neither wait for it nor come after the flush."""
+    import torch
+    from rive_runtime_gb300 import rive_cuda
+    cap, warm = load_golden(name)[0], load_golden(name)[0]
+    ctx = rive_cuda.Context(0)
+    want = ctx.render(warm)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(200_000_000)  # on the legacy stream, about 0.1 s
+    target = ctx.render_target(cap.width, cap.height)
+    images = []
+    for _ in range(2):
+        ctx.upload_frame(cap)
+        for f in cap.flushes:
+            ctx.flush(f, target)
+        ctx.sync()
+        images.append(ctx.read_target(target, cap.width, cap.height))
+        torch.cuda.synchronize()
+        images.append(ctx.read_target(target, cap.width, cap.height))
+    ctx.close()
+    for image in images:
+        assert np.array_equal(image, want)
