@@ -2537,9 +2537,17 @@ int graph_build(rive_cuda_context* ctx,
         S.gridCapacity = gridCap;
         return e;
     };
+    // On the graph's stream and waited for: from pageable memory a plain copy may
+    // return before the tables have arrived, and that stream, or the one of the first
+    // launch, does not wait for the default one.
+    auto upload_tables = [&]() -> cudaError_t {
+        const cudaError_t e = cudaMemcpyAsync(S.tables, h.data(), L.tableBytes,
+                                              cudaMemcpyHostToDevice, g->stream);
+        return e == cudaSuccess ? cudaStreamSynchronize(g->stream) : e;
+    };
     CK(placeGrids());
     BatchTables B = write_tables(ctx, in, L, S, h.data());
-    CK(cudaMemcpy(S.tables, h.data(), L.tableBytes, cudaMemcpyHostToDevice));
+    CK(upload_tables());
 
     const bool profiling = ctx->profiling;
     ctx->profiling = false; // stage events are not recorded inside a graph
@@ -2568,7 +2576,7 @@ int graph_build(rive_cuda_context* ctx,
             gridCap = asked + asked / 8;
             CK(placeGrids());
             B = write_tables(ctx, in, L, S, h.data());
-            CK(cudaMemcpy(S.tables, h.data(), L.tableBytes, cudaMemcpyHostToDevice));
+            CK(upload_tables());
         }
         capacity = g->measured + g->measured / 8 + 4096;
     }

@@ -4798,6 +4798,10 @@ cudaError_t ensure_feather_lut(int device)
         build_inverse_feather_table(table);
         e = upload_inverse_feather_lut(table);
     }
+    // (A copy from pageable memory may return before it has arrived, and the flushes'
+    // streams do not wait for the default one.)
+    if (e == cudaSuccess)
+        e = cudaStreamSynchronize(cudaStreamLegacy);
     if (e == cudaSuccess && device >= 0 && device < 64)
         done[device] = true;
     return e;
