@@ -308,7 +308,7 @@ void rive_cuda_render_buffer_destroy(rive_cuda_context* ctx, rive_cuda_render_bu
 
 /*
  * Render targets (gpu::RenderTarget, render_target.hpp): an RGBA8 image in
- * device memory, rows of width*4 bytes, row 0 at the top.
+ * device memory, rows of width*4 bytes, row 0 at the top; zeroed when created.
  */
 typedef struct rive_cuda_render_target rive_cuda_render_target;
 int rive_cuda_render_target_create(rive_cuda_context* ctx,
